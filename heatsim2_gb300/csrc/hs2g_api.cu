@@ -41,7 +41,9 @@ struct hs2g_handle {
   double* M = nullptr;
   uint8_t* compute = nullptr;
   uint8_t* vclass = nullptr;
-  double* coef_block = nullptr;
+  double* coef_x = nullptr;  // a0, b0
+  double* coef_yz[2] = {nullptr, nullptr};  // a1, b1 and a2, b2 in voxel order, unless their lines have classes
+  hs2g::LineTables tables[2];               // the y and z lines' classes
   int64_t xb_len = 0;
   Coeffs c{};
   // per-step scratch (device)
@@ -64,10 +66,8 @@ struct hs2g_handle {
   int64_t* shape_tiles = nullptr;
   unsigned long long* err_dev = nullptr;
   int* status_dev = nullptr;
-  bool bulk_y = false, bulk_z = false, z_discard = true;
   bool graph_pdl = true;  // the captured step graphs launch their sweeps with programmatic dependent launch
   bool per_row = false;  // compiled from per-row conductances (hs2g_create_rows): no shared face arrays
-  hs2g::TensorMapCache* tmaps = nullptr;
   int64_t bytes = 0;
   // host-buffer steps overlap their copies with the sweeps: a copy stream, one stream per upload slab for
   // its x sweep, and per-chunk events
@@ -227,35 +227,27 @@ int alloc_common(hs2g_handle* h, bool faces = true) {
   if ((rc = dalloc(h, &h->vclass, n, "source classes"))) return rc;
   if ((rc = dalloc(h, &h->W0, np, "stage buffer 0"))) return rc;
   if ((rc = dalloc(h, &h->W1, np, "stage buffer 1"))) return rc;
-  if ((rc = dalloc(h, &h->coef_block, np * hs2g::kNumCoeffArrays, "step coefficients"))) return rc;
+  if ((rc = dalloc(h, &h->coef_x, 2 * n, "step coefficients"))) return rc;
+  for (double*& c : h->coef_yz)
+    if ((rc = dalloc(h, &c, 2 * np, "step coefficients"))) return rc;
   h->c.nchunks = (h->d.nx + 31) / 32;
   h->xb_len = h->d.nz * h->d.ny * h->c.nchunks * hs2g::kXBlockCoeffs * 32;
   if ((rc = dalloc(h, &h->c.xb, h->xb_len, "x stencil coefficients"))) return rc;
   HS2G_CUDA(cudaMemsetAsync(h->c.xb, 0, sizeof(double) * h->xb_len, h->stream), "clear x coefficients");
   if ((rc = dalloc(h, &h->err_dev, 1, "error word"))) return rc;
   if ((rc = dalloc(h, &h->status_dev, 1, "status word"))) return rc;
-  double** slots[hs2g::kNumCoeffArrays] = {&h->c.a0, &h->c.b0, &h->c.a1, &h->c.b1, &h->c.a2, &h->c.b2};
-  for (int s = 0; s < hs2g::kNumCoeffArrays; ++s) *slots[s] = h->coef_block + (int64_t)s * np;
+  h->c.a0 = h->coef_x;
+  h->c.b0 = h->coef_x + n;
+  h->c.a1 = h->coef_yz[0];
+  h->c.b1 = h->coef_yz[0] + np;
+  h->c.a2 = h->coef_yz[1];
+  h->c.b2 = h->coef_yz[1] + np;
   HS2G_CUDA(cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned long long), h->stream), "clear error word");
   HS2G_CUDA(cudaMemsetAsync(h->status_dev, 0, sizeof(int), h->stream), "clear status word");
-  // tensor-tile line sweeps need 16-byte aligned coefficient arrays (an even voxel count) and even row pitches
-  HS2G_CUDA(hs2g::lines_bulk_prepare(), "configure line-sweep kernels");
-  // Kernel variants (defaults are the fastest measured on GB300; the others stay selectable for comparison
-  // and testing): HS2G_LINE_SWEEP=plain the plain-load y sweep, HS2G_Z_SWEEP=tma the TMA tensor-tile z sweep,
-  // HS2G_Z_DISCARD=0 the plain z sweep leaving its forward values to L2's own eviction, HS2G_PDL=0 the step
-  // graphs' sweeps launched without programmatic dependent launch (0.5702 against 0.5689 ms per step at
-  // 65x512x512).
-  const char* ymode = getenv("HS2G_LINE_SWEEP");
-  const char* zmode = getenv("HS2G_Z_SWEEP");
-  const char* zdiscard = getenv("HS2G_Z_DISCARD");
+  HS2G_CUDA(hs2g::sweeps_prepare(), "configure sweep kernels");
+  // HS2G_PDL=0: the step graphs' sweeps launched without programmatic dependent launch
   const char* pdl = getenv("HS2G_PDL");
-  h->z_discard = !(zdiscard && strcmp(zdiscard, "0") == 0);
   h->graph_pdl = !(pdl && strcmp(pdl, "0") == 0);
-  h->bulk_y = !(ymode && strcmp(ymode, "plain") == 0) && hs2g::lines_bulk_supported(h->d, 1, h->c.px);
-  h->bulk_z = (zmode && strcmp(zmode, "tma") == 0) && h->c.px == h->d.nx && (n % 2 == 0) &&
-              hs2g::lines_bulk_supported(h->d, 2, h->d.nx);
-
-  h->tmaps = hs2g::tensor_map_cache_create();
   return HS2G_OK;
 }
 
@@ -267,11 +259,6 @@ hs2g::StepArgs make_args(const hs2g_handle* h, const double* T_in, const double*
   a.W1 = h->W1;
   a.vclass = h->vclass;
   a.status = h->status_dev;
-  const bool aligned = ((reinterpret_cast<uintptr_t>(T_in) | reinterpret_cast<uintptr_t>(T_out)) & 15u) == 0;
-  a.bulk_y = h->bulk_y;
-  a.bulk_z = h->bulk_z && aligned;
-  a.z_discard = h->z_discard;
-  a.tmaps = h->tmaps;
   return a;
 }
 
@@ -300,6 +287,29 @@ int new_handle(int device, const Dims& d, hs2g_handle** out) {
   return HS2G_OK;
 }
 
+// Replace the y and z coefficients by tables per line class where the lines have few classes.
+int classify(hs2g_handle* h) {
+  const Dims& d = h->d;
+  Coeffs& c = h->c;
+  const int64_t np = d.nz * d.ny * c.px;
+  for (int ax = 0; ax < 2; ++ax) {
+    double *&a = ax ? c.a2 : c.a1, *&b = ax ? c.b2 : c.b1;
+    const int64_t lines = (ax ? d.ny : d.nz) * d.nx, n = ax ? d.nz : d.ny;
+    hs2g::LineTables& t = h->tables[ax];
+    cudaError_t e = ax ? hs2g::classify_lines(a, b, d.ny, d.nx, c.px, n, d.ny * c.px, &t, h->stream)
+                       : hs2g::classify_lines(a, b, d.nz, d.nx, d.ny * c.px, n, c.px, &t, h->stream);
+    if (e == cudaErrorMemoryAllocation) continue;  // no room for the tables: the arrays stay
+    if (e != cudaSuccess) return cuda_fail(e, "line classes");
+    if (!t.cls) continue;
+    (ax ? c.cls2 : c.cls1) = t.cls;
+    a = t.a;
+    b = t.b;
+    h->bytes += (int64_t)(sizeof(double) * 2 * t.nclass * n + sizeof(int32_t) * lines);
+    dfree(h, h->coef_yz[ax], 2 * np);
+  }
+  return HS2G_OK;
+}
+
 int factor(hs2g_handle* h) {
   const int64_t n = h->d.nvox();
   double *s2 = nullptr, *sigma = nullptr;
@@ -315,7 +325,7 @@ int factor(hs2g_handle* h) {
   dfree(h, sigma, n);
   if (e != cudaSuccess) return cuda_fail(e, "factor kernels");
   if (e2 != cudaSuccess) return cuda_fail(e2, "factor kernels");
-  return HS2G_OK;
+  return classify(h);
 }
 
 int ensure_staging(hs2g_handle* h) {
@@ -377,7 +387,7 @@ int step_host_pipelined(hs2g_handle* h, hs2g::StepArgs& a, const hs2g::QTable& q
   if (e != cudaSuccess) return cuda_fail(e, "y sweep");
   for (int c = 0; c < nout; ++c) {
     const int64_t j0 = d.ny * c / nout, j1 = d.ny * (c + 1) / nout;
-    e = hs2g::launch_z_range(a, h->c, j0 * d.nx, j1 * d.nx, s);
+    e = hs2g::launch_z_rows(a, h->c, j0, j1, s);
     if (e != cudaSuccess) return cuda_fail(e, "z sweep");
     HS2G_CUDA(cudaEventRecord(h->ev_out[c], s), "download T");
     HS2G_CUDA(cudaStreamWaitEvent(cs, h->ev_out[c], 0), "download T");
@@ -458,8 +468,6 @@ void hs2g_destroy(hs2g_handle* h) {
   if (h->own_stream) cudaStreamSynchronize(h->own_stream);
   const int64_t n = h->d.nvox();
   dfree(h, h->status_dev, 1);
-  hs2g::tensor_map_cache_destroy(h->tmaps);
-  h->tmaps = nullptr;
   dfree(h, h->Gz, 0);
   dfree(h, h->Gy, 0);
   dfree(h, h->Gx, 0);
@@ -467,7 +475,13 @@ void hs2g_destroy(hs2g_handle* h) {
   dfree(h, h->compute, n);
   dfree(h, h->vclass, n);
   const int64_t np = h->d.nz * h->d.ny * h->c.px;
-  dfree(h, h->coef_block, np * hs2g::kNumCoeffArrays);
+  dfree(h, h->coef_x, 2 * n);
+  for (double*& c : h->coef_yz) dfree(h, c, 2 * np);
+  for (hs2g::LineTables& t : h->tables) {
+    if (t.a) cudaFree(t.a);
+    if (t.b) cudaFree(t.b);
+    if (t.cls) cudaFree(t.cls);
+  }
   dfree(h, h->c.xb, h->xb_len);
   dfree(h, h->W0, np);
   dfree(h, h->W1, np);
@@ -690,6 +704,7 @@ int hs2g_create_rows(const hs2g_rows_problem* p, int device, hs2g_handle** out) 
   rows = nullptr;
   if (e != cudaSuccess) return bail(cuda_fail(e, "factor kernels"));
   if (e2 != cudaSuccess) return bail(cuda_fail(e2, "factor kernels"));
+  if ((rc = classify(h))) return bail(rc);
   *out = h;
   return HS2G_OK;
 }
@@ -804,7 +819,7 @@ int hs2g_step(hs2g_handle* h, const double* T_in, double* T_out, const double* q
   }
   a.T_in = Tin_d;
   a.T_out = Tout_d;
-  if (!dev && !a.bulk_z && n >= kPipelineMinVoxels && d.nz >= 8 && d.ny >= 8) {
+  if (!dev && n >= kPipelineMinVoxels && d.nz >= 8 && d.ny >= 8) {
     int rc = ensure_copy_pipeline(h);
     if (rc) return rc;
     return step_host_pipelined(h, a, q, T_in, T_out);

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "hs2g_internal.cuh"
+#include "hs2g_pair.cuh"
 
 namespace hs2g {
 namespace {
@@ -27,6 +28,12 @@ struct Inst {
   int64_t off;      // voxel offset in the concatenated fields
   int64_t xb_off;   // element offset of the instance's stencil blocks
   int64_t nchunks;  // 32-column chunks per x-line
+  int64_t woff;     // offset of the instance in W0 and W1, whose rows have pitch px (nx rounded up to 16 bytes)
+  int64_t px;
+  // y and z coefficients (axis 0: y, 1: z): rows of pitch px like W0, or with cls tables per line class
+  const void* a[2];
+  const void* b[2];
+  const int32_t* cls[2];
 };
 
 struct XWork {
@@ -37,7 +44,7 @@ struct XWork {
 struct LWork {
   int32_t inst;
   int32_t pad;
-  int64_t g0;  // first line of the block (y: k*nx + i, z: j*nx + i)
+  int64_t g0;  // first group of neighbouring lines (y: rows of lines k, z: rows of lines j)
 };
 
 template <typename R>
@@ -49,10 +56,6 @@ struct BatchView {
   const R* xb;
   const R* a0;
   const R* b0;
-  const R* a1;
-  const R* b1;
-  const R* a2;
-  const R* b2;
   const uint8_t* vclass;
   const R* qtabs;          // [nsched][ninst][nclass]
   const uint8_t* active;   // [nsched][ninst] any source active
@@ -109,7 +112,8 @@ __device__ void batch_x_block(const BatchView<R>& v, const Inst& I, int64_t L0_,
   const IX nx = (IX)d.nx, L0 = (IX)L0_;
   const IX nlines = (IX)(d.nz * d.ny);
   const int nchunks = (int)I.nchunks;
-  R* W0 = v.W0 + I.off;
+  R* W0 = v.W0 + I.woff;
+  const IX px = (IX)I.px;
   const R* a0 = v.a0 + I.off;
   const R* b0 = v.b0 + I.off;
   R carry = 0;
@@ -150,7 +154,7 @@ __device__ void batch_x_block(const BatchView<R>& v, const Inst& I, int64_t L0_,
     for (int ll = 0; ll < 8; ++ll) {
       const int l = warp * 8 + ll;
       const IX L = L0 + l;
-      if (L < nlines && i < nx) W0[L * nx + i] = sr[l][lane];
+      if (L < nlines && i < nx) W0[L * px + i] = sr[l][lane];
     }
     __syncthreads();
   }
@@ -163,7 +167,7 @@ __device__ void batch_x_block(const BatchView<R>& v, const Inst& I, int64_t L0_,
       const IX L = L0 + l;
       R z = 0, b = 0;
       if (L < nlines && i < nx) {
-        z = W0[L * nx + i];
+        z = W0[L * px + i];
         b = b0[L * nx + i];
       }
       sr[l][lane] = z;
@@ -192,7 +196,7 @@ __device__ void batch_x_block(const BatchView<R>& v, const Inst& I, int64_t L0_,
     for (int ll = 0; ll < 8; ++ll) {
       const int l = warp * 8 + ll;
       const IX L = L0 + l;
-      if (L < nlines && i < nx) W0[L * nx + i] = sr[l][lane];
+      if (L < nlines && i < nx) W0[L * px + i] = sr[l][lane];
     }
     __syncthreads();
   }
@@ -225,66 +229,45 @@ __global__ void __launch_bounds__(128, 7) batch_x_kernel(BatchView<R> v) {
   }
 }
 
-// y lines (thread per line): W1 = s2*dT1 from W0 = sigma*dT0
-template <typename R>
-__global__ void batch_y_kernel(BatchView<R> v) {
-  for (int64_t w = blockIdx.x; w < v.ny_work; w += gridDim.x) {
-    const LWork item = v.yw[w];
-    const Inst I = v.inst[item.inst];
-    const Dims& d = I.d;
-    const int64_t g = item.g0 + threadIdx.x;
-    if (g >= d.nz * d.nx) continue;
-    const int64_t k = g / d.nx, i = g - k * d.nx;
-    const R* W0 = v.W0 + I.off;
-    const R* a1 = v.a1 + I.off;
-    const R* b1 = v.b1 + I.off;
-    R* W1 = v.W1 + I.off;
-    int64_t p = k * d.nxy() + i;
-    R z = 0;
-#pragma unroll 4
-    for (int64_t j = 0; j < d.ny; ++j, p += d.nx) {
-      z = fma(-a1[p], z, W0[p]);
-      W1[p] = z;
-    }
-    R x = 0;
-#pragma unroll 4
-    for (int64_t j = d.ny - 1; j >= 0; --j) {
-      p -= d.nx;
-      x = fma(-b1[p], x, W1[p]);
-      W1[p] = x;
-    }
-  }
-}
-
-// z lines (thread per line): T += dT2 from W1 = s2*dT1, W0 as scratch
-template <typename R>
-__global__ void batch_z_kernel(BatchView<R> v) {
-  for (int64_t w = blockIdx.x; w < v.nz_work; w += gridDim.x) {
-    const LWork item = v.zw[w];
-    const Inst I = v.inst[item.inst];
-    const Dims& d = I.d;
-    const int64_t nxy = d.nxy();
-    const int64_t g = item.g0 + threadIdx.x;
-    if (g >= nxy) continue;
-    const R* W1 = v.W1 + I.off;
-    const R* a2 = v.a2 + I.off;
-    const R* b2 = v.b2 + I.off;
-    R* Z = v.W0 + I.off;
-    R* T = v.T + I.off;
-    int64_t p = g;
-    R z = 0;
-#pragma unroll 4
-    for (int64_t k = 0; k < d.nz; ++k, p += nxy) {
-      z = fma(-a2[p], z, W1[p]);
-      Z[p] = z;
-    }
-    R x = 0;
-#pragma unroll 4
-    for (int64_t k = d.nz - 1; k >= 0; --k) {
-      p -= nxy;
-      x = fma(-b2[p], x, Z[p]);
-      T[p] = T[p] + x;
-    }
+// y lines (W1 = s2*dT1 from W0 = sigma*dT0) and z lines (ADD_T: T += dT2 from W1 = s2*dT1, W0 as scratch): a CTA takes
+// one work item, kPairMaxWarps groups of 16 (FP64, both ends) or 32 (FP32) neighbouring lines of one instance, a
+// group per warp.  DENSE: some instance keeps its coefficients in voxel order.
+template <typename R, bool ADD_T, bool KEEP, bool DENSE>
+__global__ void __launch_bounds__(32 * kPairMaxWarps) batch_pair_kernel(BatchView<R> v, int64_t smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char batch_sm[];
+  constexpr bool TWO = sizeof(R) == 8;
+  constexpr int G = pair_lines<TWO>(), VEC = 16 / sizeof(R);
+  const LWork item = (ADD_T ? v.zw : v.yw)[blockIdx.x];
+  const Inst& I = v.inst[item.inst];
+  const int64_t nx = I.d.nx, ny = I.d.ny, gpr = (nx + G - 1) / G;
+  const int64_t grp = item.g0 + (threadIdx.x >> 5);
+  const int64_t row = grp / gpr, i0 = (grp % gpr) * G;
+  if (row >= (ADD_T ? ny : I.d.nz)) return;
+  const int64_t w = ADD_T ? row * I.px + i0 : row * ny * I.px + i0, wst = ADD_T ? ny * I.px : I.px;
+  const int32_t* cls = I.cls[ADD_T];
+  PairLines<R> p;
+  p.W = (ADD_T ? v.W1 : v.W0) + I.woff + w;
+  p.wst = p.cst = p.zst = wst;
+  p.a = (const R*)I.a[ADD_T] + (cls ? 0 : w);
+  p.b = (const R*)I.b[ADD_T] + (cls ? 0 : w);
+  p.cls = cls ? cls + row * nx + i0 : nullptr;
+  p.T = ADD_T ? v.T + I.off + row * nx + i0 : nullptr;
+  p.out = ADD_T ? v.T + I.off + row * nx + i0 : v.W1 + I.woff + w;
+  p.st = ADD_T ? nx * ny : wst;
+  p.Z = (ADD_T ? v.W0 : v.W1) + I.woff + w;
+  const int n = (int)(ADD_T ? I.d.nz : ny), width = (int)min((int64_t)G, nx - i0);
+  R* sm = reinterpret_cast<R*>(batch_sm + (threadIdx.x >> 5) * smem_per_warp);
+  const bool t16 = !ADD_T || (nx % VEC == 0 && I.off % VEC == 0);
+  if (!DENSE || cls) {
+    if (t16)
+      pair_solve<R, TWO, ADD_T, KEEP, true, VEC, VEC>(p, n, width, sm);
+    else
+      pair_solve<R, TWO, ADD_T, KEEP, true, VEC, 1>(p, n, width, sm);
+  } else {
+    if (t16)
+      pair_solve<R, TWO, ADD_T, KEEP, false, VEC, VEC>(p, n, width, sm);
+    else
+      pair_solve<R, TWO, ADD_T, KEEP, false, VEC, 1>(p, n, width, sm);
   }
 }
 
@@ -305,8 +288,7 @@ __global__ void widen_kernel(const R* __restrict__ src, double* __restrict__ dst
 
 struct Tuning {
   int x_grid;
-  int y_block, y_grid;
-  int z_block, z_grid;
+  bool y_keep, z_keep;  // the forward values of the y / z lines stay in shared memory
 };
 
 }  // namespace
@@ -326,7 +308,9 @@ struct Batch {
   void* T = nullptr;  // R*
   void* W0 = nullptr;
   void* W1 = nullptr;
-  void* coef = nullptr;  // 6 arrays of nvox R
+  void* coef = nullptr;  // a0 and b0, nvox R each
+  std::vector<void*> line_mem;  // the instances' y and z coefficients
+  int64_t nw = 0;               // elements of W0 and W1
   void* xb = nullptr;
   uint8_t* vclass = nullptr;
   void* qtabs = nullptr;
@@ -337,7 +321,9 @@ struct Batch {
   LWork* yw = nullptr;
   LWork* zw = nullptr;
   int64_t nxw = 0, nyw = 0, nzw = 0;
-  Tuning tune{0, 128, 0, 128, 0};
+  Tuning tune{0, true, true};
+  int64_t max_ny = 0, max_nz = 0;  // longest y and z line
+  bool dense[2] = {false, false};  // some instance keeps its y / z coefficients in voxel order
   bool ix32 = false;  // every instance's voxels and stencil blocks below 2^31 elements: 32-bit x-sweep indices
   cudaGraphExec_t graph = nullptr;
   int64_t bytes = 0;
@@ -356,10 +342,6 @@ BatchView<R> view(const Batch& b) {
   R* c = (R*)b.coef;
   v.a0 = c;
   v.b0 = c + b.nvox;
-  v.a1 = c + 2 * b.nvox;
-  v.b1 = c + 3 * b.nvox;
-  v.a2 = c + 4 * b.nvox;
-  v.b2 = c + 5 * b.nvox;
   v.xb = (const R*)b.xb;
   v.vclass = b.vclass;
   v.qtabs = (const R*)b.qtabs;
@@ -378,6 +360,45 @@ BatchView<R> view(const Batch& b) {
 }
 
 template <typename R>
+using BatchPairKernel = void (*)(BatchView<R>, int64_t);
+template <typename R, bool ADD_T>
+BatchPairKernel<R> batch_pair_for(bool keep, bool dense) {
+  return keep ? (dense ? batch_pair_kernel<R, ADD_T, true, true> : batch_pair_kernel<R, ADD_T, true, false>)
+              : (dense ? batch_pair_kernel<R, ADD_T, false, true> : batch_pair_kernel<R, ADD_T, false, false>);
+}
+// launch shape of an axis (force_keep: -1 by rule); CTAs have kPairMaxWarps warps
+template <typename R, bool ADD_T>
+PairShape batch_shape(const Batch& b, int force_keep) {
+  constexpr bool TWO = sizeof(R) == 8;
+  const int64_t len = ADD_T ? b.max_nz : b.max_ny, groups = (ADD_T ? b.nzw : b.nyw) * kPairMaxWarps;
+  PairShape sh = b.dense[ADD_T] ? pair_shape<R, TWO, ADD_T, false>(len, groups, force_keep)
+                                : pair_shape<R, TWO, ADD_T, true>(len, groups, force_keep);
+  size_t each = b.dense[ADD_T] ? pair_smem<R, TWO, ADD_T, true, false>(len) : pair_smem<R, TWO, ADD_T, true, true>(len);
+  if (each * kPairMaxWarps > 226 * 1024) sh.keep = false;
+  if (!sh.keep) each = b.dense[ADD_T] ? pair_smem<R, TWO, ADD_T, false, false>(len) : pair_smem<R, TWO, ADD_T, false, true>(len);
+  sh.warps = kPairMaxWarps;
+  sh.smem = each * kPairMaxWarps;
+  return sh;
+}
+template <typename R, bool ADD_T>
+cudaError_t launch_batch_pair(const Batch& b, const BatchView<R>& v, bool keep, cudaStream_t s) {
+  const PairShape sh = batch_shape<R, ADD_T>(b, keep ? 1 : 0);
+  const int64_t work = ADD_T ? b.nzw : b.nyw;
+  batch_pair_for<R, ADD_T>(sh.keep, b.dense[ADD_T])<<<(unsigned)work, 32 * kPairMaxWarps, sh.smem, s>>>(
+      v, (int64_t)(sh.smem / kPairMaxWarps));
+  return cudaGetLastError();
+}
+template <typename R>
+cudaError_t batch_prepare() {
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 8 && e == cudaSuccess; ++k) {
+    const void* f = k & 4 ? (const void*)batch_pair_for<R, true>(k & 1, k & 2) : (const void*)batch_pair_for<R, false>(k & 1, k & 2);
+    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  }
+  return e;
+}
+
+template <typename R>
 cudaError_t launch_axis(const Batch& b, int axis, const Tuning& t, cudaStream_t s) {
   BatchView<R> v = view<R>(b);
   if (axis == 0) {
@@ -386,9 +407,9 @@ cudaError_t launch_axis(const Batch& b, int axis, const Tuning& t, cudaStream_t 
     else
       batch_x_kernel<R><<<(unsigned)std::max(1, t.x_grid), 128, 0, s>>>(v);
   } else if (axis == 1) {
-    batch_y_kernel<R><<<(unsigned)std::max(1, t.y_grid), t.y_block, 0, s>>>(v);
+    return launch_batch_pair<R, false>(b, v, t.y_keep, s);
   } else if (axis == 2) {
-    batch_z_kernel<R><<<(unsigned)std::max(1, t.z_grid), t.z_block, 0, s>>>(v);
+    return launch_batch_pair<R, true>(b, v, t.z_keep, s);
   } else {
     batch_advance_kernel<<<1, 32, 0, s>>>(b.step);
   }
@@ -407,12 +428,13 @@ cudaError_t launch_step_batch(const Batch& b, cudaStream_t s) {
 
 }  // namespace
 
-// Work lists: blocks of 32 x-lines / block_y y-lines / block_z z-lines per instance, longest lines first.
-void batch_build_work(Batch& b, int block_y, int block_z, std::vector<XWork>& xw, std::vector<LWork>& yw,
-                      std::vector<LWork>& zw) {
+// Work lists: blocks of 32 x-lines, and of the line solves' y and z lines, per instance, longest lines first.
+void batch_build_work(Batch& b, std::vector<XWork>& xw, std::vector<LWork>& yw, std::vector<LWork>& zw) {
   xw.clear();
   yw.clear();
   zw.clear();
+  const int per = b.precision == 64 ? pair_lines<true>() : pair_lines<false>();
+  auto groups = [&](const Dims& d) { return (d.nx + per - 1) / per; };  // of neighbouring lines in a row of lines
   std::vector<int> order(b.ninst);
   for (int i = 0; i < b.ninst; ++i) order[i] = i;
   auto by = [&](auto len) {
@@ -426,18 +448,18 @@ void batch_build_work(Batch& b, int block_y, int block_z, std::vector<XWork>& xw
   }
   for (int ib : by([](const Dims& d) { return d.ny; })) {
     const Dims& d = b.inst[ib].d;
-    for (int64_t g0 = 0; g0 < d.nz * d.nx; g0 += block_y) yw.push_back(LWork{ib, 0, g0});
+    for (int64_t g0 = 0; g0 < d.nz * groups(d); g0 += kPairMaxWarps) yw.push_back(LWork{ib, 0, g0});
   }
   for (int ib : by([](const Dims& d) { return d.nz; })) {
     const Dims& d = b.inst[ib].d;
-    for (int64_t g0 = 0; g0 < d.nxy(); g0 += block_z) zw.push_back(LWork{ib, 0, g0});
+    for (int64_t g0 = 0; g0 < d.ny * groups(d); g0 += kPairMaxWarps) zw.push_back(LWork{ib, 0, g0});
   }
 }
 
-cudaError_t batch_upload_work(Batch& b, int block_y, int block_z) {
+cudaError_t batch_upload_work(Batch& b) {
   std::vector<XWork> xw;
   std::vector<LWork> yw, zw;
-  batch_build_work(b, block_y, block_z, xw, yw, zw);
+  batch_build_work(b, xw, yw, zw);
   if (b.xw) cudaFree(b.xw);
   if (b.yw) cudaFree(b.yw);
   if (b.zw) cudaFree(b.zw);
@@ -507,33 +529,23 @@ cudaError_t batch_autotune(Batch& b, std::string& report) {
       if (ms < bt) bt = ms, best.x_grid = t.x_grid;
     }
   }
-  // y and z: block size (work list granularity) and persistent grid
+  // y and z: forward values in shared memory or through global memory
   for (int axis = 1; axis <= 2; ++axis) {
     float bt = 1e30f;
-    int bb = 128, bg = 0;
-    for (int blk : {64, 128, 256}) {
-      if ((e = batch_upload_work(b, axis == 1 ? blk : best.y_block, axis == 2 ? blk : best.z_block)) != cudaSuccess)
-        return e;
-      for (int per : {8, 16, 32}) {
-        Tuning t = best;
-        const int64_t nwork = axis == 1 ? b.nyw : b.nzw;
-        const int grid = (int)std::min<int64_t>(nwork, (int64_t)sms * per * 256 / blk);
-        if (axis == 1) t.y_block = blk, t.y_grid = grid;
-        else t.z_block = blk, t.z_grid = grid;
-        float ms;
-        if ((e = batch_time_axis(b, axis, t, 2, &ms)) != cudaSuccess) return e;
-        snprintf(line, sizeof line, "%s block %d grid %d: %.3f ms\n", axis == 1 ? "y" : "z", blk, grid, ms);
-        report += line;
-        if (ms < bt) bt = ms, bb = blk, bg = grid;
-      }
+    for (int keep = 1; keep >= 0; --keep) {
+      Tuning t = best;
+      (axis == 1 ? t.y_keep : t.z_keep) = keep != 0;
+      float ms;
+      if ((e = batch_time_axis(b, axis, t, 2, &ms)) != cudaSuccess) return e;
+      snprintf(line, sizeof line, "%s forward values in %s memory: %.3f ms\n", axis == 1 ? "y" : "z",
+               keep ? "shared" : "global", ms);
+      report += line;
+      if (ms < bt) bt = ms, (axis == 1 ? best.y_keep : best.z_keep) = keep != 0;
     }
-    if (axis == 1) best.y_block = bb, best.y_grid = bg;
-    else best.z_block = bb, best.z_grid = bg;
-    if ((e = batch_upload_work(b, best.y_block, best.z_block)) != cudaSuccess) return e;
   }
   b.tune = best;
-  snprintf(line, sizeof line, "chosen: x grid %d, y block %d grid %d, z block %d grid %d\n", best.x_grid,
-           best.y_block, best.y_grid, best.z_block, best.z_grid);
+  snprintf(line, sizeof line, "chosen: x grid %d, y values in %s memory, z values in %s memory\n", best.x_grid,
+           best.y_keep ? "shared" : "global", best.z_keep ? "shared" : "global");
   report += line;
   return e;
 }
@@ -587,6 +599,7 @@ void batch_free(Batch& b) {
   for (void* p : {(void*)b.inst_dev, b.T, b.W0, b.W1, b.coef, b.xb, (void*)b.vclass, b.qtabs, (void*)b.active,
                   (void*)b.step, (void*)b.xw, (void*)b.yw, (void*)b.zw})
     if (p) cudaFree(p);
+  for (void* p : b.line_mem) cudaFree(p);
   if (b.stream) cudaStreamDestroy(b.stream);
 }
 
@@ -594,12 +607,12 @@ int64_t xb_elems(const hs2g::Dims& d) { return d.nz * d.ny * ((d.nx + 31) / 32) 
 
 // Compile instance `ib` of problem p into the batch (FP64 workspace ws, then into the batch's storage type).
 int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, unsigned long long* err) {
-  const hs2g::Inst& I = b.inst[ib];
+  hs2g::Inst& I = b.inst[ib];
   const hs2g::Dims& d = I.d;
-  const int64_t n = d.nvox();
+  const int64_t n = d.nvox(), np = d.nz * d.ny * I.px;
   const int64_t nfz = (d.nz + 1) * d.nxy(), nfy = d.nz * (d.ny + 1) * d.nx, nfx = d.nz * d.ny * (d.nx + 1);
   cudaStream_t s = b.stream;
-  // workspace layout (doubles): faces z, y, x | M s2 sigma | 6 coefficient arrays | x blocks | bytes:
+  // workspace layout (doubles): faces z, y, x | M s2 sigma | a0 b0 | a1 b1 a2 b2 | x blocks | bytes:
   // compute mask, material, boundary classes | material table | boundary forms
   double* fz = ws;
   double* fy = fz + nfz;
@@ -607,8 +620,9 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   double* M = fx + nfx;
   double* s2 = M + n;
   double* sg = s2 + n;
-  double* c6 = sg + n;
-  double* xbw = c6 + 6 * n;
+  double* c2 = sg + n;
+  double* c4 = c2 + 2 * n;
+  double* xbw = c4 + 4 * np;
   uint8_t* u8 = reinterpret_cast<uint8_t*>(xbw + xb_elems(d));
   uint8_t* comp = u8;
   uint8_t* mat = comp + n;
@@ -648,26 +662,63 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   }
   hs2g::Coeffs c{};
   c.nchunks = I.nchunks;
-  c.px = d.nx;  // the batched sweeps use plain loads on unpadded rows
+  c.px = I.px;
   const bool f64 = b.precision == 64;
-  double* cbase = f64 ? (double*)b.coef : c6;
-  const int64_t cstride = f64 ? b.nvox : n;
-  const int64_t coff = f64 ? I.off : 0;
-  c.a0 = cbase + coff;
-  c.b0 = cbase + cstride + coff;
-  c.a1 = cbase + 2 * cstride + coff;
-  c.b1 = cbase + 3 * cstride + coff;
-  c.a2 = cbase + 4 * cstride + coff;
-  c.b2 = cbase + 5 * cstride + coff;
+  c.a0 = f64 ? (double*)b.coef + I.off : c2;
+  c.b0 = f64 ? (double*)b.coef + b.nvox + I.off : c2 + n;
+  c.a1 = c4;
+  c.b1 = c4 + np;
+  c.a2 = c4 + 2 * np;
+  c.b2 = c4 + 3 * np;
   c.xb = f64 ? (double*)b.xb + I.xb_off : xbw;
   if (!f64 && (e = cudaMemsetAsync(xbw, 0, sizeof(double) * xb_elems(d), s)) != cudaSuccess)
     return bcuda(e, "batch compile");
-  if ((e = hs2g::launch_factor(d, fz, fy, fx, M, comp, s2, sg, c, s)) != cudaSuccess)
+  if ((e = hs2g::launch_factor(d, fz, fy, fx, M, comp, s2, sg, c, s, f64)) != cudaSuccess)
     return bcuda(e, "batch factor");
   if (!f64) {
-    for (int a = 0; a < 6 && e == cudaSuccess; ++a)
-      e = hs2g::batch_convert(c6 + a * n, (float*)b.coef + a * b.nvox + I.off, n, 32, s);
+    for (int a = 0; a < 2 && e == cudaSuccess; ++a)
+      e = hs2g::batch_convert(c2 + a * n, (float*)b.coef + a * b.nvox + I.off, n, 32, s);
     if (e == cudaSuccess) e = hs2g::batch_convert(xbw, (float*)b.xb + I.xb_off, xb_elems(d), 32, s);
+  }
+  // the y and z coefficients: tables per line class, or the arrays where the lines have too many classes
+  for (int ax = 0; ax < 2 && e == cudaSuccess; ++ax) {
+    const double *a = ax ? c.a2 : c.a1, *bb = ax ? c.b2 : c.b1;
+    hs2g::LineTables t;
+    e = ax ? hs2g::classify_lines(a, bb, d.ny, d.nx, I.px, d.nz, d.ny * I.px, &t, s)
+           : hs2g::classify_lines(a, bb, d.nz, d.nx, d.ny * I.px, d.ny, I.px, &t, s);
+    if (e != cudaSuccess) break;
+    const int64_t count = t.cls ? t.nclass * (ax ? d.nz : d.ny) : np;
+    if (t.cls) {
+      b.line_mem.push_back(t.cls);
+      b.bytes += (int64_t)sizeof(int32_t) * (ax ? d.ny : d.nz) * d.nx;
+      a = t.a;
+      bb = t.b;
+    } else {
+      b.dense[ax] = true;
+    }
+    I.cls[ax] = t.cls;
+    const void** dst[2] = {&I.a[ax], &I.b[ax]};
+    const double* src[2] = {a, bb};
+    for (int q = 0; q < 2; ++q) {
+      if (t.cls && f64) {  // the tables as they are
+        b.line_mem.push_back((void*)src[q]);
+        *dst[q] = src[q];
+      } else {
+        void* m = nullptr;
+        if (e == cudaSuccess) e = cudaMalloc(&m, b.elem() * count);
+        if (e == cudaSuccess) {
+          b.line_mem.push_back(m);
+          *dst[q] = m;
+          e = hs2g::batch_convert(src[q], m, count, b.precision, s);
+        }
+      }
+      b.bytes += (int64_t)b.elem() * count;
+    }
+    if (t.cls && !f64) {
+      cudaStreamSynchronize(s);
+      cudaFree(t.a);
+      cudaFree(t.b);
+    }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e == cudaSuccess ? HS2G_OK : bcuda(e, "batch factor");
@@ -732,6 +783,10 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     I.off = off;
     I.xb_off = xoff;
     I.nchunks = (I.d.nx + 31) / 32;
+    I.woff = b.nw;
+    const int64_t quad = 16 / (int64_t)b.elem();
+    I.px = (I.d.nx + quad - 1) / quad * quad;
+    b.nw += I.d.nz * I.d.ny * I.px;
     b.inst.push_back(I);
     const hs2g::Dims& d = I.d;
     const int64_t nn = d.nvox();
@@ -739,7 +794,7 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     xoff += xb_elems(d);
     b.offsets.push_back(off);
     const int64_t faces = (d.nz + 1) * d.nxy() + d.nz * (d.ny + 1) * d.nx + d.nz * d.ny * (d.nx + 1);
-    const int64_t need = faces + 9 * nn + xb_elems(d) + (faces + 3 * nn) / 8 + 2048 +
+    const int64_t need = faces + 5 * nn + 4 * d.nz * d.ny * I.px + xb_elems(d) + (faces + 3 * nn) / 8 + 2048 +
                          (int64_t)(sizeof(hs2g_material) * HS2G_MAX_CLASSES + sizeof(hs2g_face_form) * 3 *
                                    HS2G_MAX_CLASSES) / 8 + 256;
     ws = std::max(ws, need);
@@ -748,14 +803,14 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   b.xb_len = xoff;
   b.ix32 = true;
   for (const hs2g::Inst& I : b.inst)
-    b.ix32 = b.ix32 && I.d.nvox() < ((int64_t)1 << 31) && xb_elems(I.d) < ((int64_t)1 << 31);
+    b.ix32 = b.ix32 && I.d.nz * I.d.ny * I.px < ((int64_t)1 << 31) && xb_elems(I.d) < ((int64_t)1 << 31);
   const size_t el = b.elem();
   double* wsp = nullptr;
   unsigned long long* err = nullptr;
   if ((e = balloc(b, &b.inst_dev, n)) != cudaSuccess || (e = balloc(b, (char**)&b.T, b.nvox * el)) != cudaSuccess ||
-      (e = balloc(b, (char**)&b.W0, b.nvox * el)) != cudaSuccess ||
-      (e = balloc(b, (char**)&b.W1, b.nvox * el)) != cudaSuccess ||
-      (e = balloc(b, (char**)&b.coef, 6 * b.nvox * el)) != cudaSuccess ||
+      (e = balloc(b, (char**)&b.W0, b.nw * el)) != cudaSuccess ||
+      (e = balloc(b, (char**)&b.W1, b.nw * el)) != cudaSuccess ||
+      (e = balloc(b, (char**)&b.coef, 2 * b.nvox * el)) != cudaSuccess ||
       (e = balloc(b, (char**)&b.xb, b.xb_len * el)) != cudaSuccess ||
       (e = balloc(b, &b.vclass, b.nvox)) != cudaSuccess || (e = balloc(b, &b.step, 1)) != cudaSuccess ||
       (e = cudaMalloc(&wsp, sizeof(double) * ws)) != cudaSuccess ||
@@ -767,12 +822,11 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   }
   cudaMemsetAsync(b.xb, 0, b.xb_len * el, b.stream);
   cudaMemsetAsync(b.T, 0, b.nvox * el, b.stream);
-  cudaMemsetAsync(b.W0, 0, b.nvox * el, b.stream);
-  cudaMemsetAsync(b.W1, 0, b.nvox * el, b.stream);
-  cudaMemsetAsync(b.coef, 0, 6 * b.nvox * el, b.stream);
+  cudaMemsetAsync(b.W0, 0, b.nw * el, b.stream);
+  cudaMemsetAsync(b.W1, 0, b.nw * el, b.stream);
+  cudaMemsetAsync(b.coef, 0, 2 * b.nvox * el, b.stream);
   cudaMemsetAsync(b.vclass, 0, b.nvox, b.stream);
   cudaMemsetAsync(b.step, 0, sizeof(int), b.stream);
-  cudaMemcpyAsync(b.inst_dev, b.inst.data(), sizeof(hs2g::Inst) * n, cudaMemcpyHostToDevice, b.stream);
   int rc = HS2G_OK;
   for (int i = 0; i < n && rc == HS2G_OK; ++i) {
     cudaMemsetAsync(err, 0, sizeof(unsigned long long), b.stream);
@@ -781,12 +835,26 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   cudaFree(wsp);
   cudaFree(err);
   if (rc != HS2G_OK) return bail(rc);
-  if ((e = hs2g::batch_upload_work(b, 128, 128)) != cudaSuccess) return bail(bcuda(e, "work lists"));
+  e = cudaMemcpyAsync(b.inst_dev, b.inst.data(), sizeof(hs2g::Inst) * n, cudaMemcpyHostToDevice, b.stream);
+  if (e != cudaSuccess) return bail(bcuda(e, "instances"));
+  if ((e = hs2g::batch_upload_work(b)) != cudaSuccess) return bail(bcuda(e, "work lists"));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   b.tune.x_grid = (int)std::min<int64_t>(b.nxw, (int64_t)sms * 7);  // the x kernel's 7 resident CTAs per SM
-  b.tune.y_grid = (int)std::min<int64_t>(b.nyw, (int64_t)sms * 16);
-  b.tune.z_grid = (int)std::min<int64_t>(b.nzw, (int64_t)sms * 16);
+  for (const hs2g::Inst& I : b.inst) {
+    b.max_ny = std::max(b.max_ny, I.d.ny);
+    b.max_nz = std::max(b.max_nz, I.d.nz);
+  }
+  if (precision == 64) {
+    e = hs2g::batch_prepare<double>();
+    b.tune.y_keep = hs2g::batch_shape<double, false>(b, -1).keep;
+    b.tune.z_keep = hs2g::batch_shape<double, true>(b, -1).keep;
+  } else {
+    e = hs2g::batch_prepare<float>();
+    b.tune.y_keep = hs2g::batch_shape<float, false>(b, -1).keep;
+    b.tune.z_keep = hs2g::batch_shape<float, true>(b, -1).keep;
+  }
+  if (e != cudaSuccess) return bail(bcuda(e, "configure sweep kernels"));
   if ((e = cudaStreamSynchronize(b.stream)) != cudaSuccess) return bail(bcuda(e, "batch create"));
   *out = hb;
   return HS2G_OK;

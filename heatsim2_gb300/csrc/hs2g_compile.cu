@@ -187,50 +187,104 @@ struct RowFaces {
   __device__ double xhi(const Dims&, int64_t p, int64_t, int64_t, int64_t) const { return xh[p]; }
 };
 
-// z lines (one thread per (j,i)): stage-2 coefficients and s2.
+// z lines (one thread per (j,i)): stage-2 coefficients and s2.  The y and z lines are eliminated from both ends
+// towards the middle row m = n/2 (hs2g_pair.cuh): below it a = lo/piv, b = hi/piv, above it the same with lo and
+// hi exchanged, and the middle row keeps both couplings, a = lo/piv and b = hi/piv.  The two ends advance in one
+// loop, so their divisions overlap.  One way (the FP32 batch, two_ended false): m is the last row, which has no
+// upper neighbour.
 template <class F>
 __global__ void factor_z_kernel(Dims d, F g, const double* __restrict__ M, const uint8_t* __restrict__ compute,
-                                double* __restrict__ s2, double* __restrict__ a2, double* __restrict__ b2) {
+                                double* __restrict__ s2, double* __restrict__ a2, double* __restrict__ b2,
+                                int64_t px, bool two_ended) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= d.nxy()) return;
   const int64_t j = t / d.nx, i = t - j * d.nx;
-  double u_prev = 0.0;
-  for (int64_t k = 0; k < d.nz; ++k) {
+  const int64_t m = two_ended ? d.nz / 2 : d.nz - 1;
+  auto at2 = [&](int64_t k) { return (k * d.ny + j) * px + i; };  // a2 / b2 row pitch
+  auto row = [&](int64_t k) {
     const int64_t p = k * d.nxy() + t;
     const bool comp = compute[p] != 0;
-    const RowIn r = stage_row(comp, M[p], comp ? g.zlo(d, p, k, j, i) : 0.0, comp ? g.zhi(d, p, k, j, i) : 0.0);
-    const double piv = r.d - u_prev * r.lo;
-    const double u = r.hi / piv;
-    a2[p] = r.lo / piv;
-    b2[p] = u;
+    return stage_row(comp, M[p], comp ? g.zlo(d, p, k, j, i) : 0.0, comp ? g.zhi(d, p, k, j, i) : 0.0);
+  };
+  double u = 0.0, v = 0.0;  // upper factor of the last eliminated row at each end
+  auto up = [&](int64_t k) {
+    const int64_t p = k * d.nxy() + t;
+    const RowIn r = row(k);
+    const double piv = r.d - u * r.lo;
+    u = r.hi / piv;
+    a2[at2(k)] = r.lo / piv;
+    b2[at2(k)] = u;
     s2[p] = M[p] / piv;
-    u_prev = u;
+  };
+  auto down = [&](int64_t k) {
+    const int64_t p = k * d.nxy() + t;
+    const RowIn r = row(k);
+    const double piv = r.d - v * r.hi;
+    v = r.lo / piv;
+    a2[at2(k)] = r.hi / piv;
+    b2[at2(k)] = v;
+    s2[p] = M[p] / piv;
+  };
+  for (int64_t e = 0; e < m; ++e) {
+    up(e);
+    if (d.nz - 1 - e > m) down(d.nz - 1 - e);
   }
+  const int64_t p = m * d.nxy() + t;
+  const RowIn r = row(m);
+  const double piv = r.d - u * r.lo - v * r.hi;
+  a2[at2(m)] = r.lo / piv;
+  b2[at2(m)] = r.hi / piv;
+  s2[p] = M[p] / piv;
 }
 
 // y lines (one thread per (k,i)): stage-1 coefficients and sigma.
 template <class F>
 __global__ void factor_y_kernel(Dims d, F g, const double* __restrict__ M, const uint8_t* __restrict__ compute,
                                 const double* __restrict__ s2, double* __restrict__ sigma, double* __restrict__ a1,
-                                double* __restrict__ b1, int64_t px) {
+                                double* __restrict__ b1, int64_t px, bool two_ended) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= d.nz * d.nx) return;
   const int64_t k = t / d.nx, i = t - k * d.nx;
-  double u_prev = 0.0, s2_prev = 1.0;
-  for (int64_t j = 0; j < d.ny; ++j) {
-    const int64_t p = (k * d.ny + j) * d.nx + i;
-    const int64_t pp = (k * d.ny + j) * px + i;  // a1 / b1 row pitch
+  const int64_t m = two_ended ? d.ny / 2 : d.ny - 1;
+  auto at = [&](int64_t j) { return (k * d.ny + j) * d.nx + i; };
+  auto row = [&](int64_t j) {
+    const int64_t p = at(j);
     const bool comp = compute[p] != 0;
-    const RowIn r = stage_row(comp, M[p], comp ? g.ylo(d, p, k, j, i) : 0.0, comp ? g.yhi(d, p, k, j, i) : 0.0);
-    const double piv = r.d - u_prev * r.lo;
-    const double u = r.hi / piv;
-    const double s2p = s2[p];
-    sigma[p] = s2p * M[p] / piv;
-    a1[pp] = (j > 0) ? s2p * r.lo / (piv * s2_prev) : 0.0;
-    b1[pp] = (j + 1 < d.ny) ? s2p * u / s2[p + d.nx] : 0.0;
-    u_prev = u;
-    s2_prev = s2p;
+    return stage_row(comp, M[p], comp ? g.ylo(d, p, k, j, i) : 0.0, comp ? g.yhi(d, p, k, j, i) : 0.0);
+  };
+  // W1 carries the scale s2, so a row's couplings are scaled by its own s2 and the neighbour's is divided out; f:
+  // the coupling, q: the pivot where it is still to be divided by it
+  auto lower = [&](int64_t j, double f, double q) { return j > 0 ? s2[at(j)] * f / (q * s2[at(j - 1)]) : 0.0; };
+  auto upper = [&](int64_t j, double f, double q) { return j + 1 < d.ny ? s2[at(j)] * f / (q * s2[at(j + 1)]) : 0.0; };
+  double u = 0.0, v = 0.0;
+  auto up = [&](int64_t j) {
+    const int64_t pp = (k * d.ny + j) * px + i;  // a1 / b1 row pitch
+    const RowIn r = row(j);
+    const double piv = r.d - u * r.lo;
+    u = r.hi / piv;
+    sigma[at(j)] = s2[at(j)] * M[at(j)] / piv;
+    a1[pp] = lower(j, r.lo, piv);
+    b1[pp] = upper(j, u, 1.0);
+  };
+  auto down = [&](int64_t j) {
+    const int64_t pp = (k * d.ny + j) * px + i;
+    const RowIn r = row(j);
+    const double piv = r.d - v * r.hi;
+    v = r.lo / piv;
+    sigma[at(j)] = s2[at(j)] * M[at(j)] / piv;
+    a1[pp] = upper(j, r.hi, piv);
+    b1[pp] = lower(j, v, 1.0);
+  };
+  for (int64_t e = 0; e < m; ++e) {
+    up(e);
+    if (d.ny - 1 - e > m) down(d.ny - 1 - e);
   }
+  const int64_t pp = (k * d.ny + m) * px + i;
+  const RowIn r = row(m);
+  const double piv = r.d - u * r.lo - v * r.hi;
+  sigma[at(m)] = s2[at(m)] * M[at(m)] / piv;
+  a1[pp] = lower(m, r.lo, piv);
+  b1[pp] = upper(m, r.hi, piv);
 }
 
 // x lines (one thread per (k,j)): stage-0 stencil, forward and back coefficients.
@@ -325,24 +379,25 @@ cudaError_t launch_validate_dense(const Dims& d, const double* Gz, const double*
 
 template <class F>
 cudaError_t launch_factor_with(const Dims& d, F g, const double* M, const uint8_t* compute, double* s2,
-                               double* sigma, const Coeffs& c, cudaStream_t s) {
+                               double* sigma, const Coeffs& c, cudaStream_t s, bool two_ended) {
   const int th = 128;
-  factor_z_kernel<F><<<grid_for(d.nxy(), th), th, 0, s>>>(d, g, M, compute, s2, c.a2, c.b2);
+  factor_z_kernel<F><<<grid_for(d.nxy(), th), th, 0, s>>>(d, g, M, compute, s2, c.a2, c.b2, c.px, two_ended);
   factor_y_kernel<F><<<grid_for(d.nz * d.nx, th), th, 0, s>>>(d, g, M, compute, s2, sigma, c.a1, c.b1,
-                                                                c.px ? c.px : d.nx);
+                                                                c.px, two_ended);
   factor_x_kernel<F><<<grid_for(d.nz * d.ny, th), th, 0, s>>>(d, g, M, compute, sigma, c);
   return cudaGetLastError();
 }
 
 cudaError_t launch_factor(const Dims& d, const double* Gz, const double* Gy, const double* Gx, const double* M,
-                          const uint8_t* compute, double* s2, double* sigma, const Coeffs& c, cudaStream_t s) {
-  return launch_factor_with(d, SharedFaces{Gz, Gy, Gx}, M, compute, s2, sigma, c, s);
+                          const uint8_t* compute, double* s2, double* sigma, const Coeffs& c, cudaStream_t s,
+                          bool two_ended) {
+  return launch_factor_with(d, SharedFaces{Gz, Gy, Gx}, M, compute, s2, sigma, c, s, two_ended);
 }
 
 cudaError_t launch_factor_rows(const Dims& d, const double* const rows[6], const double* M, const uint8_t* compute,
                                double* s2, double* sigma, const Coeffs& c, cudaStream_t s) {
   const RowFaces g{rows[0], rows[1], rows[2], rows[3], rows[4], rows[5]};
-  return launch_factor_with(d, g, M, compute, s2, sigma, c, s);
+  return launch_factor_with(d, g, M, compute, s2, sigma, c, s, true);
 }
 
 cudaError_t launch_validate_rows(const Dims& d, const double* const rows[6], double* M, uint8_t* compute,

@@ -17,8 +17,8 @@ struct Dims {
 // Per-voxel coefficients of the scaled delta-form Douglas step.
 //   stage 0 (x lines):  z_i = wc*T + wxl*T[i-1] + wxh*T[i+1] + wyl*T[j-1] + wyh*T[j+1] + wzl*T[k-1]
 //                             + wzh*T[k+1] + wq*Q - a0*z_{i-1};   W0_i = z_i - b0*W0_{i+1}
-//   stage 1 (y lines):  z_j = W0_j - a1*z_{j-1};                   W1_j = z_j - b1*W1_{j+1}
-//   stage 2 (z lines):  z_k = W1_k - a2*z_{k-1};                   dT_k = z_k - b2*dT_{k+1};  T' = T + dT
+//   stage 1 (y lines):  the same recurrences with a1, b1 from W0 to W1, from both ends towards the middle row
+//   stage 2 (z lines):  the same with a2, b2 from W1 to dT;  T' = T + dT            (hs2g_pair.cuh)
 // The eight stage-0 stencil coefficients are chunk-blocked: for x-line L = k*ny + j and 32-column chunk ch,
 // block (L*nchunks + ch) holds [wc, wxl, wxh, wyl, wyh, wzl, wzh, wq] x 32 columns (2 KB, zero-padded past
 // nx), so a warp's stencil reads one contiguous stream instead of eight.  The other coefficients are
@@ -28,17 +28,32 @@ enum XCoeff { kWc = 0, kWxl, kWxh, kWyl, kWyh, kWzl, kWzh, kWq };
 struct Coeffs {
   double* xb;   // stage-0 stencil blocks, nz*ny*nchunks*8*32 doubles
   int64_t nchunks;
-  // Row pitch of the arrays the y sweep moves with TMA tiles (W0, W1, a1, b1): nx, or nx rounded up so that
-  // the rows start on 16-byte boundaries (an odd nx gets one pad column).  All other arrays have pitch nx.
+  // Row pitch of the arrays the y and z sweeps copy 16 bytes at a time (W0, W1, a1, b1, a2, b2): nx, or nx rounded
+  // up so that the rows start on 16-byte boundaries (an odd nx gets one pad column).  All other arrays have pitch nx.
   int64_t px;
   double* a0;
   double* b0;
+  // y and z lines: arrays in voxel order (row pitch px), or with cls1 / cls2 tables of a line's rows per class
+  // (classify_lines), the class of y line (k, i) at cls1[k*nx + i] and of z line (j, i) at cls2[j*nx + i]
   double* a1;
   double* b1;
   double* a2;
   double* b2;
+  int32_t* cls1;
+  int32_t* cls2;
 };
-constexpr int kNumCoeffArrays = 6;  // voxel-order arrays besides xb
+
+// The distinct lines of an axis: a[c*n + r], b[c*n + r] per class and row, cls[line]; cls is null when there are too
+// many.  Device memory owned by the caller.
+struct LineTables {
+  double* a = nullptr;
+  double* b = nullptr;
+  int32_t* cls = nullptr;
+  int64_t nclass = 0;
+};
+// lines (o, i), i fastest, with row r at o*ost + r*rst + i of a and b (hs2g_classes.cu); waits for the stream
+cudaError_t classify_lines(const double* a, const double* b, int64_t outer, int64_t nx, int64_t ost, int64_t n,
+                           int64_t rst, LineTables* out, cudaStream_t s);
 
 struct QTable {
   double q[HS2G_MAX_CLASSES];
@@ -126,7 +141,8 @@ cudaError_t launch_capacity_from_classes(const Dims& d, const uint8_t* material,
 cudaError_t launch_validate_dense(const Dims& d, const double* Gz, const double* Gy, const double* Gx,
                                   double* M, uint8_t* compute, unsigned long long* err, cudaStream_t s);
 cudaError_t launch_factor(const Dims& d, const double* Gz, const double* Gy, const double* Gx, const double* M,
-                          const uint8_t* compute, double* s2, double* sigma, const Coeffs& c, cudaStream_t s);
+                          const uint8_t* compute, double* s2, double* sigma, const Coeffs& c, cudaStream_t s,
+                          bool two_ended = true);
 // per-row problems: rows = {z lo, z hi, y lo, y hi, x lo, x hi}, each (nz, ny, nx)
 cudaError_t launch_validate_rows(const Dims& d, const double* const rows[6], double* M, uint8_t* compute,
                                  unsigned long long* err, cudaStream_t s);
@@ -155,23 +171,12 @@ struct StepArgs {
   const double* qshape;  // per-voxel multiplier of the class sources (null: 1 everywhere)
   bool has_qtab;
   int* status;           // device word: 0, or HS2G_ERR_TIMEOUT when a bounded wait in a kernel ran out
-  bool bulk_y, bulk_z;   // use the TMA tensor-tile line sweeps (hs2g_lines.cu) for y / z
-  bool z_discard;        // the plain z sweep drops its forward values from L2 after reading them
-  struct TensorMapCache* tmaps;
   bool pdl;              // launch the y and z sweeps with programmatic dependent launch (captured step graphs)
   bool pdl_x;            // the same for the x sweep (not for the first kernel of a graph)
 };
 
-// TMA tensor-tile line sweeps (hs2g_lines.cu); axis 1 = y, 2 = z.
-struct TensorMapCache;
-TensorMapCache* tensor_map_cache_create();
-void tensor_map_cache_destroy(TensorMapCache* c);
-bool lines_bulk_supported(const Dims& d, int axis, int64_t px);
-cudaError_t lines_bulk_prepare();
-// axis 1 (y): A, alpha, scratch, beta and out have row pitch px; axis 2 (z): every array has pitch nx (px = nx)
-cudaError_t launch_lines_bulk(const Dims& d, int axis, const double* A, const double* alpha, double* scratch,
-                              const double* beta, const double* T_in, double* out, int* status,
-                              TensorMapCache* cache, cudaStream_t s, int64_t px, bool pdl = false);
+// raise the dynamic shared-memory limits of the sweep kernels on the current device (when a handle is created)
+cudaError_t sweeps_prepare();
 cudaError_t launch_step(const StepArgs& a, const Coeffs& c, const QTable& q, cudaStream_t s);
 // the same three kernels with an event recorded before each and after the last (ev[0..3])
 cudaError_t launch_step_events(const StepArgs& a, const Coeffs& c, const QTable& q, cudaStream_t s,
@@ -196,11 +201,11 @@ cudaError_t launch_surface_estimate(int64_t nxy, const double* T, double dz, dou
 // one bounded mbarrier wait on a barrier that receives its arrival (arrive != 0) or none (hs2g_lines.cu)
 cudaError_t wait_selftest(uint64_t limit_ns, int arrive, int* status_dev, cudaStream_t s);
 // the step in pieces, for overlapping host copies with it: the x sweep over x-lines [line_begin, line_end)
-// (line = k*ny + j) with 32, 16 or 8 x-lines per CTA, the whole y sweep, the plain z sweep over columns
-// [col_begin, col_end) (col = j*nx + i)
+// (line = k*ny + j) with 32, 16 or 8 x-lines per CTA, the whole y sweep, the z sweep over the rows of columns
+// [j_begin, j_end)
 cudaError_t launch_x_range(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t line_begin,
                            int64_t line_end, int lines_per_cta, cudaStream_t s);
 cudaError_t launch_y(const StepArgs& a, const Coeffs& c, cudaStream_t s);
-cudaError_t launch_z_range(const StepArgs& a, const Coeffs& c, int64_t col_begin, int64_t col_end, cudaStream_t s);
+cudaError_t launch_z_rows(const StepArgs& a, const Coeffs& c, int64_t j_begin, int64_t j_end, cudaStream_t s);
 
 }  // namespace hs2g

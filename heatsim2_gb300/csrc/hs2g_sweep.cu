@@ -13,15 +13,15 @@
 //            along x (coalesced loads of T and of the line's coefficient block), staged through shared memory,
 //            and one warp runs the 32 line recurrences down the transposed chunk (lane = line).  The forward
 //            values are kept in the output array W0 and re-read by the back substitution in the same CTA.
-//   y sweep: TMA tensor tiles (hs2g_lines.cu), or one thread per y-line with plain loads.
-//   z sweep: one thread per z-line (j,i); neighbouring lanes have neighbouring i, so each k step is one
-//            coalesced 256-byte access per array per warp (a TMA variant exists, HS2G_Z_SWEEP=tma).
+//   y, z sweeps: one warp per 16 neighbouring lines, both ends of each line at once, rows copied ahead into shared
+//            memory and coefficients from tables per line class (hs2g_pair.cuh, hs2g_classes.cu).
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
 
 #include "hs2g_internal.cuh"
+#include "hs2g_pair.cuh"
 
 namespace hs2g {
 namespace {
@@ -37,7 +37,6 @@ constexpr int kXWarps = kXThreads / 32;
 // whole-grid kernels set the budget directly (__maxnreg__); the host-buffer step's line-range kernels keep a
 // bound of 6 blocks (kXMinBlocks).  Check -Xptxas -v after a change.
 constexpr int kXMinBlocks = 6;
-constexpr int kLineThreads = 128;
 
 // Stage-0 right-hand side of voxel (L, i) of x-line L = k*ny + j, pre-scaled by the line's pivot:
 // wc*T + wxl*T[i-1] + wxh*T[i+1] + wyl*T[j-1] + wyh*T[j+1] + wzl*T[k-1] + wzh*T[k+1] (+ wq*Q).
@@ -350,101 +349,44 @@ void launch_x_row(const StepArgs& a, const Coeffs& c, const DevSchedule* ds, cud
     launch_kernel(sweep_x_row_kernel<2>, dim3(gx), dim3(kXThreads), 0, s, a.pdl_x, d, a.T_in, c, a.vclass, ds, a.W0);
 }
 
-// y lines: W1 = s2 * dT1 from W0 = sigma * dT0
-__global__ void __launch_bounds__(kLineThreads) sweep_y_kernel(Dims d, const double* __restrict__ W0,
-                                                                const double* __restrict__ a1,
-                                                                const double* __restrict__ b1,
-                                                                double* __restrict__ W1, int64_t px) {
+// The y sweep (ADD_T false: W1 = s2 * dT1 from W0 = sigma * dT0; rows of lines k) and the z sweep (ADD_T: T_out =
+// T_in + dT2 from W1 = s2 * dT1; rows of lines j; W0 the scratch of the forward values, T_in may be T_out) over the
+// rows of lines [begin, end).  One warp per group of 16 neighbouring lines.
+struct PairArgs {
+  Dims d;
+  int64_t px;
+  const double* W;
+  const double* a;
+  const double* b;
+  const int32_t* cls;
+  const double* T;
+  double* out;
+  double* Z;
+  int64_t begin, end;
+};
+template <bool ADD_T, bool KEEP, bool TABLE, int TVEC>
+__global__ void __launch_bounds__(32 * kPairMaxWarps) pair_sweep_kernel(PairArgs g, int64_t smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char pair_sm[];
+  const int64_t nx = g.d.nx, gpr = (nx + 15) / 16;  // groups per row of lines
+  const int64_t grp = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t row = g.begin + grp / gpr, i0 = (grp % gpr) * 16;
+  if (row >= g.end) return;
+  PairLines<double> p;
+  const int64_t w = ADD_T ? row * g.px + i0 : row * g.d.ny * g.px + i0;  // first line's first row in the padded arrays
+  const int64_t wst = ADD_T ? g.d.ny * g.px : g.px;
+  p.W = g.W + w;
+  p.wst = p.cst = p.zst = wst;
+  p.a = TABLE ? g.a : g.a + w;
+  p.b = TABLE ? g.b : g.b + w;
+  p.cls = TABLE ? g.cls + row * nx + i0 : nullptr;
+  p.T = ADD_T ? g.T + row * nx + i0 : nullptr;
+  p.out = g.out + (ADD_T ? row * nx + i0 : w);
+  p.st = ADD_T ? g.d.nxy() : wst;
+  p.Z = g.Z + w;
   wait_prior_grid();
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= d.nz * d.nx) return;
-  const int64_t k = t / d.nx, i = t - k * d.nx;
-  int64_t p = k * d.ny * px + i;  // the y-sweep arrays have row pitch px
-  double z = 0.0;
-#pragma unroll 4
-  for (int64_t j = 0; j < d.ny; ++j, p += px) {
-    z = fma(-a1[p], z, W0[p]);
-    W1[p] = z;
-  }
-  double x = 0.0;
-#pragma unroll 4
-  for (int64_t j = d.ny - 1; j >= 0; --j) {
-    p -= px;
-    x = fma(-b1[p], x, W1[p]);
-    W1[p] = x;
-  }
-}
-
-// z lines: dT2 from W1 = s2 * dT1; T_out = T_in + dT2.  Z is scratch (the x sweep's buffer, free by now).
-// T_in may equal T_out: each voxel's T_in is read by the same thread just before its T_out is written.
-// DISCARD: the forward values are read once by the back substitution and never again, so once a warp has read
-// a group of 4 rows k .. k+3 (k a multiple of 4) it drops their Z lines from L2 (lanes 0 and 16 each own one
-// 128-byte line of a row), which saves the write-back of every line still cached; only warps whose 32 columns
-// are whole lines of every plane do this (nxy a multiple of 16, warp-aligned columns inside the launch's range),
-// and the rows above the top group (nz mod 4 of them) are left as they are.
-// 16 CTAs per SM (32 registers): the 2048 CTAs of a 512x512-column grid are resident at once.
-template <bool DISCARD>
-__global__ void __launch_bounds__(kLineThreads, 16) sweep_z_kernel(Dims d, const double* __restrict__ W1,
-                                                                const double* __restrict__ a2,
-                                                                const double* __restrict__ b2, const double* T_in,
-                                                                double* __restrict__ Z, double* T_out,
-                                                                int64_t col_begin, int64_t col_end, int64_t px) {
-  // this launch covers the z-lines (columns j*nx + i) [col_begin, col_end); W1 has row pitch px
-  const int64_t t = col_begin + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t nxy = d.nxy();
-  const int64_t t0 = t - (threadIdx.x & 31);  // the warp's first column
-  const bool drop = DISCARD && nxy % 16 == 0 && t0 % 32 == 0 && t0 + 32 <= col_end;  // warp-uniform
-  wait_prior_grid();
-  if (t >= col_end) return;
-  int64_t p = t;
-  const int64_t jw = t / d.nx;
-  int64_t pw = jw * px + (t - jw * d.nx);
-  const int64_t nxyw = d.ny * px;
-  const uint64_t keep = l2_evict_last();  // the forward values come back to this thread after its last row
-  double z = 0.0;
-#pragma unroll 4
-  for (int64_t k = 0; k < d.nz; ++k, p += nxy, pw += nxyw) {
-    z = fma(-a2[p], z, W1[pw]);
-    st_hint(Z + p, z, keep);
-  }
-  double x = 0.0;
-  if (!DISCARD) {
-#pragma unroll 4
-    for (int64_t k = d.nz - 1; k >= 0; --k) {
-      p -= nxy;
-      x = fma(-b2[p], x, Z[p]);
-      T_out[p] = T_in[p] + x;
-    }
-    return;
-  }
-  int64_t k = d.nz - 1;
-#pragma unroll 1
-  for (; (k & 3) != 3; --k) {  // rows above the last whole group of 4
-    p -= nxy;
-    x = fma(-b2[p], x, Z[p]);
-    T_out[p] = T_in[p] + x;
-  }
-#pragma unroll 1
-  for (; k >= 3; k -= 4) {  // rows k-3 .. k, then their Z lines dropped
-    p -= 4 * nxy;
-    double z3 = Z[p + 3 * nxy], z2 = Z[p + 2 * nxy], z1 = Z[p + nxy], z0 = Z[p];
-    x = fma(-b2[p + 3 * nxy], x, z3);
-    T_out[p + 3 * nxy] = T_in[p + 3 * nxy] + x;
-    x = fma(-b2[p + 2 * nxy], x, z2);
-    T_out[p + 2 * nxy] = T_in[p + 2 * nxy] + x;
-    x = fma(-b2[p + nxy], x, z1);
-    T_out[p + nxy] = T_in[p + nxy] + x;
-    x = fma(-b2[p], x, z0);
-    T_out[p] = T_in[p] + x;
-    if (!drop) continue;
-    __syncwarp();  // every lane of the warp has read its four rows of Z
-    if ((threadIdx.x & 15) == 0) {
-      l2_discard_line(Z + p);
-      l2_discard_line(Z + p + nxy);
-      l2_discard_line(Z + p + 2 * nxy);
-      l2_discard_line(Z + p + 3 * nxy);
-    }
-  }
+  pair_solve<double, true, ADD_T, KEEP, TABLE, 2, TVEC>(
+      p, (int)(ADD_T ? g.d.nz : g.d.ny), (int)min((int64_t)16, nx - i0),
+      reinterpret_cast<double*>(pair_sm + (threadIdx.x >> 5) * smem_per_warp));
 }
 
 __global__ void copy_layer_kernel(Dims d, const double* __restrict__ T, int layer, double* __restrict__ dst) {
@@ -550,26 +492,47 @@ cudaError_t fp64_fma_rate(double* fma_per_s) {
 }
 
 namespace {
+using PairKernel = void (*)(PairArgs, int64_t);
+template <bool ADD_T>
+PairKernel pair_kernel(bool keep, bool table, bool t16) {
+  // T moves 16 bytes at a time when its rows start on 16-byte boundaries (an even nx)
+  if (table)
+    return keep ? (ADD_T && !t16 ? pair_sweep_kernel<ADD_T, true, true, 1> : pair_sweep_kernel<ADD_T, true, true, 2>)
+                : (ADD_T && !t16 ? pair_sweep_kernel<ADD_T, false, true, 1> : pair_sweep_kernel<ADD_T, false, true, 2>);
+  return keep ? (ADD_T && !t16 ? pair_sweep_kernel<ADD_T, true, false, 1> : pair_sweep_kernel<ADD_T, true, false, 2>)
+              : (ADD_T && !t16 ? pair_sweep_kernel<ADD_T, false, false, 1> : pair_sweep_kernel<ADD_T, false, false, 2>);
+}
+template <bool ADD_T>
+cudaError_t launch_pair(const PairArgs& g, cudaStream_t s, bool pdl) {
+  if (g.end <= g.begin) return cudaSuccess;
+  const int64_t n = ADD_T ? g.d.nz : g.d.ny, groups = (g.end - g.begin) * ((g.d.nx + 15) / 16);
+  const bool table = g.cls != nullptr;
+  const bool t16 = g.d.nx % 2 == 0 && ((reinterpret_cast<uintptr_t>(g.T) & 15) == 0);
+  const PairShape sh = table ? pair_shape<double, true, ADD_T, true>(n, groups) : pair_shape<double, true, ADD_T, false>(n, groups);
+  return launch_kernel(pair_kernel<ADD_T>(sh.keep, table, t16), dim3((unsigned)((groups + sh.warps - 1) / sh.warps)),
+                       dim3(32 * sh.warps), sh.smem, s, pdl, g, (int64_t)(sh.smem / sh.warps));
+}
 // the y and z sweeps of a step, with events before each and after the last when ev is given
 cudaError_t launch_yz(const StepArgs& a, const Coeffs& c, cudaStream_t s, cudaEvent_t* ev) {
-  const Dims& d = a.d;
-  cudaError_t e = cudaSuccess;
-  if (a.bulk_y)
-    e = launch_lines_bulk(d, 1, a.W0, c.a1, a.W1, c.b1, nullptr, a.W1, a.status, a.tmaps, s, c.px, a.pdl);
-  else
-    e = launch_kernel(sweep_y_kernel, dim3(blocks(d.nz * d.nx, kLineThreads)), dim3(kLineThreads), 0, s, a.pdl, d,
-                      a.W0, c.a1, c.b1, a.W1, c.px);
+  cudaError_t e = launch_y(a, c, s);
   if (e != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[2], s);
-  if (a.bulk_z)
-    e = launch_lines_bulk(d, 2, a.W1, c.a2, a.W0, c.b2, a.T_in, a.T_out, a.status, a.tmaps, s, d.nx, a.pdl);
-  else
-    e = launch_z_range(a, c, 0, d.nxy(), s);
+  e = launch_z_rows(a, c, 0, a.d.ny, s);
   if (e != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[3], s);
   return cudaGetLastError();
 }
 }  // namespace
+
+cudaError_t sweeps_prepare() {
+  cudaError_t e = cudaSuccess;
+  for (int v = 0; v < 16 && e == cudaSuccess; ++v) {
+    const bool keep = v & 1, table = v & 2, t16 = v & 4;
+    const void* k = v & 8 ? (const void*)pair_kernel<true>(keep, table, t16) : (const void*)pair_kernel<false>(keep, table, t16);
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  }
+  return e;
+}
 
 cudaError_t launch_step_events(const StepArgs& a, const Coeffs& c, const QTable& q, cudaStream_t s,
                                cudaEvent_t ev[4]) {
@@ -626,22 +589,12 @@ cudaError_t launch_x_range(const StepArgs& a, const Coeffs& c, const QTable& q, 
 }
 
 cudaError_t launch_y(const StepArgs& a, const Coeffs& c, cudaStream_t s) {
-  const Dims& d = a.d;
-  if (a.bulk_y)
-    return launch_lines_bulk(d, 1, a.W0, c.a1, a.W1, c.b1, nullptr, a.W1, a.status, a.tmaps, s, c.px);
-  sweep_y_kernel<<<blocks(d.nz * d.nx, kLineThreads), kLineThreads, 0, s>>>(d, a.W0, c.a1, c.b1, a.W1, c.px);
-  return cudaGetLastError();
+  return launch_pair<false>(PairArgs{a.d, c.px, a.W0, c.a1, c.b1, c.cls1, nullptr, a.W1, a.W1, 0, a.d.nz}, s, a.pdl);
 }
 
-cudaError_t launch_z_range(const StepArgs& a, const Coeffs& c, int64_t col_begin, int64_t col_end, cudaStream_t s) {
-  const Dims& d = a.d;
-  if (col_end <= col_begin) return cudaSuccess;
-  const unsigned grid = blocks(col_end - col_begin, kLineThreads);
-  if (a.z_discard)
-    return launch_kernel(sweep_z_kernel<true>, dim3(grid), dim3(kLineThreads), 0, s, a.pdl, d, a.W1, c.a2, c.b2,
-                         a.T_in, a.W0, a.T_out, col_begin, col_end, c.px);
-  return launch_kernel(sweep_z_kernel<false>, dim3(grid), dim3(kLineThreads), 0, s, a.pdl, d, a.W1, c.a2, c.b2, a.T_in,
-                       a.W0, a.T_out, col_begin, col_end, c.px);
+cudaError_t launch_z_rows(const StepArgs& a, const Coeffs& c, int64_t j_begin, int64_t j_end, cudaStream_t s) {
+  return launch_pair<true>(PairArgs{a.d, c.px, a.W1, c.a2, c.b2, c.cls2, a.T_in, a.T_out, a.W0, j_begin, j_end}, s,
+                           a.pdl);
 }
 
 cudaError_t launch_copy_layer(const Dims& d, const double* T, int layer, double* dst, cudaStream_t s) {

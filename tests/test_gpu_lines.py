@@ -1,0 +1,59 @@
+"""The sweeps' line solves at the sizes where they can go wrong: line lengths around the blocks of eight rows of a half
+line (1 to 3 rows, 15 to 18, 33), row widths around the warps' 16 lines with odd ones among them, coefficients from
+tables per line class (a layered problem) and in voxel order (faces drawn at random, so that no two lines are alike),
+forward values kept in shared memory and, for long lines, sent through global memory; double and float.  Against the
+oracle, 2 steps: FP64 within the parity bar of 1e-12 of max|T|, FP32 within the 1e-7 of its stated error."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+import oracle
+from oracle_shim import HS
+import heatsim2_gb300 as hs
+from heatsim2_gb300 import workloads as W
+from heatsim2_gb300.batch import Batch
+
+pytestmark = pytest.mark.gpu
+
+SMALL = [(1, 2, 16), (2, 1, 15), (3, 3, 17), (15, 18, 33), (16, 17, 1), (17, 16, 31), (33, 15, 16), (18, 33, 47)]
+LONG = [(2, 700, 80), (700, 2, 40), (8, 300, 1700), (300, 8, 1700)]
+
+
+def _spec(shape, random_faces):
+    nz, ny, nx = shape
+    spec = W.line_grid(shape, dt=0.01)
+    spec["boundaries"] = [["conducting"], ["insulating"]] + [["thininsulatinglayer", 50.0 + 37.0 * c] for c in range(40)]
+    spec["volumetric"] = [["none"], ["stepped", 0.0, 1.0, 2e8]]
+    a = spec["arrays"]
+    a["volumetric"][:] = 0
+    a["volumetric"][0] = 1
+    if random_faces:
+        rng = np.random.default_rng(sum(shape))
+        for key, cut in (("boundary_z", np.s_[1:-1]), ("boundary_y", np.s_[:, 1:-1]), ("boundary_x", np.s_[:, :, 1:-1])):
+            a[key][cut] = rng.choice([0] + list(range(2, 42)), size=a[key][cut].shape)
+    return spec
+
+
+def _field(shape):
+    return 293.0 + np.random.default_rng(4).random(shape)
+
+
+@pytest.mark.parametrize("random_faces", [False, True])
+@pytest.mark.parametrize("shape", SMALL + LONG)
+def test_line_solves_vs_oracle(cuda_ok, shape, random_faces):
+    spec = _spec(shape, random_faces)
+    vol = W.volumetric_tuple(hs, spec)
+    P, S = hs.setup(*W.setup_args(hs, spec))
+    Po, _ = oracle.setup(*W.setup_args(HS, spec))
+    T = ref = _field(shape)
+    for t in (0.0, 0.01):
+        T = hs.run_adi_steps(P, S, t, spec["dt"], T, spec["arrays"]["volumetric"], vol)
+        ref = oracle.run_adi_steps(Po, None, t, spec["dt"], ref, spec["arrays"]["volumetric"], vol)
+    assert rel_err(T, ref) <= 1e-12
+    for precision, tol in ((64, 0.0), (32, 1e-7)):      # the batched form: the same bits in double
+        b = Batch([W.setup_args(hs, spec)], precision=precision)
+        b.set_temperature([_field(shape)])
+        b.set_sources([0.0, 0.01], spec["dt"])
+        b.run(2)
+        got = b.get_temperature()[0]
+        assert rel_err(got, T) <= tol, precision
