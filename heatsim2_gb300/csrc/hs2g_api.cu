@@ -22,11 +22,6 @@ using hs2g::Dims;
 // its columns.  The host link (~0.2 TB/s each way on GB300) is then busy while the sweeps run.
 constexpr int kCopyChunks = 4;
 constexpr double kSlabEnd[kCopyChunks] = {0.55, 0.80, 0.93, 1.0};  // upload slab c ends at this fraction of nz
-// x-lines per CTA of each slab's x sweep: a small launch lasts as long as one CTA's chunk loop, so the later,
-// smaller slabs take smaller CTAs and finish sooner after their upload (64x512x512 composite panel: 1.77 ms
-// per host-buffer step against 1.85 ms with 32 lines throughout; 16 for every slab 1.80, 8 for the last two
-// 1.83)
-constexpr int kSlabLines[kCopyChunks] = {32, 32, 16, 8};
 constexpr int64_t kPipelineMinVoxels = int64_t(1) << 20;
 
 struct hs2g_handle {
@@ -41,10 +36,8 @@ struct hs2g_handle {
   double* M = nullptr;
   uint8_t* compute = nullptr;
   uint8_t* vclass = nullptr;
-  double* coef_x = nullptr;  // a0, b0
-  double* coef_yz[2] = {nullptr, nullptr};  // a1, b1 and a2, b2 in voxel order, unless their lines have classes
-  hs2g::LineTables tables[2];               // the y and z lines' classes
-  int64_t xb_len = 0;
+  double* coef[3] = {nullptr, nullptr, nullptr};  // the x, y, z line coefficients in voxel order, unless tabulated
+  hs2g::Compressed kept;                    // the stencil blocks and the lines' tables
   Coeffs c{};
   // per-step scratch (device)
   double* W0 = nullptr;
@@ -227,24 +220,19 @@ int alloc_common(hs2g_handle* h, bool faces = true) {
   if ((rc = dalloc(h, &h->vclass, n, "source classes"))) return rc;
   if ((rc = dalloc(h, &h->W0, np, "stage buffer 0"))) return rc;
   if ((rc = dalloc(h, &h->W1, np, "stage buffer 1"))) return rc;
-  if ((rc = dalloc(h, &h->coef_x, 2 * n, "step coefficients"))) return rc;
-  for (double*& c : h->coef_yz)
+  for (double*& c : h->coef)
     if ((rc = dalloc(h, &c, 2 * np, "step coefficients"))) return rc;
   h->c.nchunks = (h->d.nx + 31) / 32;
-  h->xb_len = h->d.nz * h->d.ny * h->c.nchunks * hs2g::kXBlockCoeffs * 32;
-  if ((rc = dalloc(h, &h->c.xb, h->xb_len, "x stencil coefficients"))) return rc;
-  HS2G_CUDA(cudaMemsetAsync(h->c.xb, 0, sizeof(double) * h->xb_len, h->stream), "clear x coefficients");
   if ((rc = dalloc(h, &h->err_dev, 1, "error word"))) return rc;
   if ((rc = dalloc(h, &h->status_dev, 1, "status word"))) return rc;
-  h->c.a0 = h->coef_x;
-  h->c.b0 = h->coef_x + n;
-  h->c.a1 = h->coef_yz[0];
-  h->c.b1 = h->coef_yz[0] + np;
-  h->c.a2 = h->coef_yz[1];
-  h->c.b2 = h->coef_yz[1] + np;
+  h->c.a0 = h->coef[0];
+  h->c.b0 = h->coef[0] + np;
+  h->c.a1 = h->coef[1];
+  h->c.b1 = h->coef[1] + np;
+  h->c.a2 = h->coef[2];
+  h->c.b2 = h->coef[2] + np;
   HS2G_CUDA(cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned long long), h->stream), "clear error word");
   HS2G_CUDA(cudaMemsetAsync(h->status_dev, 0, sizeof(int), h->stream), "clear status word");
-  HS2G_CUDA(hs2g::sweeps_prepare(), "configure sweep kernels");
   // HS2G_PDL=0: the step graphs' sweeps launched without programmatic dependent launch
   const char* pdl = getenv("HS2G_PDL");
   h->graph_pdl = !(pdl && strcmp(pdl, "0") == 0);
@@ -287,45 +275,41 @@ int new_handle(int device, const Dims& d, hs2g_handle** out) {
   return HS2G_OK;
 }
 
-// Replace the y and z coefficients by tables per line class where the lines have few classes.
-int classify(hs2g_handle* h) {
+// Factorise the problem, keep what the steps read of it and give the rest of the coefficient arrays back.
+int factor(hs2g_handle* h, const hs2g::Faces& faces) {
   const Dims& d = h->d;
   Coeffs& c = h->c;
-  const int64_t np = d.nz * d.ny * c.px;
-  for (int ax = 0; ax < 2; ++ax) {
-    double *&a = ax ? c.a2 : c.a1, *&b = ax ? c.b2 : c.b1;
-    const int64_t lines = (ax ? d.ny : d.nz) * d.nx, n = ax ? d.nz : d.ny;
-    hs2g::LineTables& t = h->tables[ax];
-    cudaError_t e = ax ? hs2g::classify_lines(a, b, d.ny, d.nx, c.px, n, d.ny * c.px, &t, h->stream)
-                       : hs2g::classify_lines(a, b, d.nz, d.nx, d.ny * c.px, n, c.px, &t, h->stream);
-    if (e == cudaErrorMemoryAllocation) continue;  // no room for the tables: the arrays stay
-    if (e != cudaSuccess) return cuda_fail(e, "line classes");
-    if (!t.cls) continue;
-    (ax ? c.cls2 : c.cls1) = t.cls;
-    a = t.a;
-    b = t.b;
-    h->bytes += (int64_t)(sizeof(double) * 2 * t.nclass * n + sizeof(int32_t) * lines);
-    dfree(h, h->coef_yz[ax], 2 * np);
-  }
-  return HS2G_OK;
-}
-
-int factor(hs2g_handle* h) {
-  const int64_t n = h->d.nvox();
-  double *s2 = nullptr, *sigma = nullptr;
+  const int64_t n = d.nvox(), np = d.nz * d.ny * c.px;
+  double* sc = nullptr;  // s2, sigma and the scratch of the search for equal lines and blocks
+  const int64_t len = 2 * n + (int64_t)(hs2g::compress_scratch(d) + 7) / 8;
   int rc;
-  if ((rc = dalloc(h, &s2, n, "factor scratch"))) return rc;
-  if ((rc = dalloc(h, &sigma, n, "factor scratch"))) {
-    dfree(h, s2, n);
-    return rc;
-  }
-  cudaError_t e = hs2g::launch_factor(h->d, h->Gz, h->Gy, h->Gx, h->M, h->compute, s2, sigma, h->c, h->stream);
+  if ((rc = dalloc(h, &sc, len, "factor scratch"))) return rc;
+  cudaError_t e = hs2g::launch_factor(d, faces, h->M, h->compute, sc, sc + n, c, h->stream, true);
+  if (e == cudaSuccess) e = hs2g::compress_coeffs(d, faces, h->compute, sc, c, 64, (unsigned char*)(sc + 2 * n), &h->kept, h->stream);
   cudaError_t e2 = cudaStreamSynchronize(h->stream);
-  dfree(h, s2, n);
-  dfree(h, sigma, n);
+  dfree(h, sc, len);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return fail(HS2G_ERR_NOMEM, "no device memory for the stencil coefficients");
+  }
   if (e != cudaSuccess) return cuda_fail(e, "factor kernels");
   if (e2 != cudaSuccess) return cuda_fail(e2, "factor kernels");
-  return classify(h);
+  c.xb = (double*)h->kept.blocks.pool;
+  c.bidx = h->kept.blocks.bidx;
+  h->bytes += (int64_t)h->kept.blocks.bytes;
+  double** coeffs[3][2] = {{&c.a0, &c.b0}, {&c.a1, &c.b1}, {&c.a2, &c.b2}};
+  int32_t** cls[3] = {&c.cls0, &c.cls1, &c.cls2};
+  for (int ax = 0; ax < 3; ++ax) {
+    const hs2g::LineTables& t = h->kept.lines[ax];
+    if (!t.cls) continue;
+    *coeffs[ax][0] = t.a;
+    *coeffs[ax][1] = t.b;
+    *cls[ax] = t.cls;
+    h->bytes += (int64_t)t.bytes;
+    dfree(h, h->coef[ax], 2 * np);
+  }
+  HS2G_CUDA(hs2g::sweeps_prepare(d, c), "configure sweep kernels");
+  return HS2G_OK;
 }
 
 int ensure_staging(hs2g_handle* h) {
@@ -376,7 +360,7 @@ int step_host_pipelined(hs2g_handle* h, hs2g::StepArgs& a, const hs2g::QTable& q
     HS2G_CUDA(cudaStreamWaitEvent(xs, h->ev_begin, 0), "upload T");
     HS2G_CUDA(cudaStreamWaitEvent(xs, h->ev_in[c], 0), "upload T");
     const int64_t upto = (k1 == d.nz ? d.nz : k1 - 1) * d.ny;
-    cudaError_t e = hs2g::launch_x_range(a, h->c, q, done, upto, kSlabLines[c], xs);
+    cudaError_t e = hs2g::launch_x_range(a, h->c, q, done, upto, xs);
     if (e != cudaSuccess) return cuda_fail(e, "x sweep");
     HS2G_CUDA(cudaEventRecord(h->ev_x[c], xs), "x sweep");
     HS2G_CUDA(cudaStreamWaitEvent(s, h->ev_x[c], 0), "x sweep");
@@ -399,6 +383,18 @@ int step_host_pipelined(hs2g_handle* h, hs2g::StepArgs& a, const hs2g::QTable& q
   HS2G_CUDA(cudaStreamSynchronize(cs), "step");
   HS2G_CUDA(cudaStreamSynchronize(s), "step");
   return check_status(h);
+}
+
+// Whether host memory at p is page-locked.  Overlapped copies pay only then: the runtime stages pageable memory through
+// its own buffers while the caller waits, piece by piece (49x220x200 numpy steps: 1.05 ms with one copy each way, 1.8 ms
+// in four slabs and blocks; page-locked at 65x512x512: 1.80 ms and 1.57 ms).
+bool page_locked(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
 }
 
 // The shape field applies to a step whose table gives a shaped class a non-zero value.
@@ -475,14 +471,8 @@ void hs2g_destroy(hs2g_handle* h) {
   dfree(h, h->compute, n);
   dfree(h, h->vclass, n);
   const int64_t np = h->d.nz * h->d.ny * h->c.px;
-  dfree(h, h->coef_x, 2 * n);
-  for (double*& c : h->coef_yz) dfree(h, c, 2 * np);
-  for (hs2g::LineTables& t : h->tables) {
-    if (t.a) cudaFree(t.a);
-    if (t.b) cudaFree(t.b);
-    if (t.cls) cudaFree(t.cls);
-  }
-  dfree(h, h->c.xb, h->xb_len);
+  for (double*& c : h->coef) dfree(h, c, 2 * np);
+  h->kept.release();
   dfree(h, h->W0, np);
   dfree(h, h->W1, np);
   dfree(h, h->Tin_dev, n);
@@ -534,28 +524,24 @@ int hs2g_create_classes(const hs2g_class_problem* p, int device, hs2g_handle** o
   if (rc) return rc;
   const Dims& d = h->d;
   const int64_t n = d.nvox();
-  uint8_t *mat = nullptr, *bz = nullptr, *by = nullptr, *bx = nullptr;
-  hs2g_material* mats = nullptr;
-  hs2g_face_form* forms = nullptr;
-  auto cleanup_tmp = [&]() {
-    dfree(h, mat, n);
-    dfree(h, bz, 0);
-    dfree(h, by, 0);
-    dfree(h, bx, 0);
-    dfree(h, mats, p->nmat);
-    dfree(h, forms, p->nbnd * 3);
-  };
   const int64_t nfz = (d.nz + 1) * d.nxy(), nfy = d.nz * (d.ny + 1) * d.nx, nfx = d.nz * d.ny * (d.nx + 1);
-  if ((rc = alloc_common(h)) || (rc = dalloc(h, &mat, n, "material classes")) ||
-      (rc = dalloc(h, &bz, nfz, "z boundary classes")) || (rc = dalloc(h, &by, nfy, "y boundary classes")) ||
-      (rc = dalloc(h, &bx, nfx, "x boundary classes")) || (rc = dalloc(h, &mats, p->nmat, "material table")) ||
-      (rc = dalloc(h, &forms, p->nbnd * 3, "boundary forms"))) {
+  // one allocation for what only the compilation reads: the class maps, the material table, the boundary forms and the
+  // faces' values per class and material pair
+  const size_t sizes[7] = {(size_t)n, (size_t)nfz, (size_t)nfy, (size_t)nfx, sizeof(hs2g_material) * p->nmat,
+                           sizeof(hs2g_face_form) * p->nbnd * 3, hs2g::face_table_bytes(p->nmat, p->nbnd)};
+  int64_t at[8] = {};
+  for (int k = 0; k < 7; ++k) at[k + 1] = at[k] + (int64_t)((sizes[k] + 255) & ~size_t(255));
+  uint8_t* tmp = nullptr;
+  if ((rc = alloc_common(h)) || (rc = dalloc(h, &tmp, at[7], "class maps"))) {
     std::string msg = g_last_error;
-    cleanup_tmp();
     hs2g_destroy(h);
     g_last_error = msg;
     return rc;
   }
+  uint8_t *mat = tmp, *bz = tmp + at[1], *by = tmp + at[2], *bx = tmp + at[3];
+  hs2g_material* mats = reinterpret_cast<hs2g_material*>(tmp + at[4]);
+  hs2g_face_form* forms = reinterpret_cast<hs2g_face_form*>(tmp + at[5]);
+  void* table = tmp + at[6];
   cudaStream_t s = h->stream;
   cudaError_t e = cudaSuccess;
   auto up = [&](void* dst, const void* src, size_t bytes) {
@@ -571,19 +557,19 @@ int hs2g_create_classes(const hs2g_class_problem* p, int device, hs2g_handle** o
     up(h->vclass, p->volumetric, (size_t)n);
   else if (e == cudaSuccess)
     e = cudaMemsetAsync(h->vclass, 0, (size_t)n, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 0, mat, bz, mats, p->nmat, forms, p->nbnd, h->Gz, h->err_dev, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 1, mat, by, mats, p->nmat, forms, p->nbnd, h->Gy, h->err_dev, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 2, mat, bx, mats, p->nmat, forms, p->nbnd, h->Gx, h->err_dev, s);
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, 0, mat, bz, mats, p->nmat, forms, p->nbnd, h->Gz, h->err_dev, table, s);
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, 1, mat, by, mats, p->nmat, forms, p->nbnd, h->Gy, h->err_dev, table, s);
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, 2, mat, bx, mats, p->nmat, forms, p->nbnd, h->Gx, h->err_dev, table, s);
   if (e == cudaSuccess)
     e = hs2g::launch_capacity_from_classes(d, mat, mats, p->nmat, h->M, h->compute, h->err_dev, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cleanup_tmp();
+  dfree(h, tmp, at[7]);
   if (e != cudaSuccess) {
     rc = cuda_fail(e, "compile kernels");
   } else {
     rc = check_kernel_error(h);
   }
-  if (!rc) rc = factor(h);
+  if (!rc) rc = factor(h, hs2g::Faces{h->Gz, h->Gy, h->Gx, {}});
   if (rc) {
     std::string msg = g_last_error;
     hs2g_destroy(h);
@@ -631,7 +617,7 @@ int hs2g_create_dense(const hs2g_dense_problem* p, int device, hs2g_handle** out
   if (e == cudaSuccess) e = hs2g::launch_validate_dense(d, h->Gz, h->Gy, h->Gx, h->M, h->compute, h->err_dev, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   rc = (e != cudaSuccess) ? cuda_fail(e, "dense compile") : check_kernel_error(h);
-  if (!rc) rc = factor(h);
+  if (!rc) rc = factor(h, hs2g::Faces{h->Gz, h->Gy, h->Gx, {}});
   if (rc) {
     std::string msg = g_last_error;
     hs2g_destroy(h);
@@ -690,21 +676,10 @@ int hs2g_create_rows(const hs2g_rows_problem* p, int device, hs2g_handle** out) 
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   rc = (e != cudaSuccess) ? cuda_fail(e, "per-row compile") : check_kernel_error(h);
   if (rc) return bail(rc);
-  double *s2 = nullptr, *sigma = nullptr;
-  if ((rc = dalloc(h, &s2, n, "factor scratch"))) return bail(rc);
-  if ((rc = dalloc(h, &sigma, n, "factor scratch"))) {
-    dfree(h, s2, n);
-    return bail(rc);
-  }
-  e = hs2g::launch_factor_rows(d, dev_rows, h->M, h->compute, s2, sigma, h->c, s);
-  cudaError_t e2 = cudaStreamSynchronize(s);
-  dfree(h, s2, n);
-  dfree(h, sigma, n);
+  hs2g::Faces faces;
+  for (int r = 0; r < 6; ++r) faces.rows[r] = dev_rows[r];
+  if ((rc = factor(h, faces))) return bail(rc);
   dfree(h, rows, 6 * n);
-  rows = nullptr;
-  if (e != cudaSuccess) return bail(cuda_fail(e, "factor kernels"));
-  if (e2 != cudaSuccess) return bail(cuda_fail(e2, "factor kernels"));
-  if ((rc = classify(h))) return bail(rc);
   *out = h;
   return HS2G_OK;
 }
@@ -819,7 +794,7 @@ int hs2g_step(hs2g_handle* h, const double* T_in, double* T_out, const double* q
   }
   a.T_in = Tin_d;
   a.T_out = Tout_d;
-  if (!dev && n >= kPipelineMinVoxels && d.nz >= 8 && d.ny >= 8) {
+  if (!dev && n >= kPipelineMinVoxels && d.nz >= 8 && d.ny >= 8 && page_locked(T_in) && page_locked(T_out)) {
     int rc = ensure_copy_pipeline(h);
     if (rc) return rc;
     return step_host_pipelined(h, a, q, T_in, T_out);

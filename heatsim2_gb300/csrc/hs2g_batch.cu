@@ -15,10 +15,12 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hs2g_internal.cuh"
 #include "hs2g_pair.cuh"
+#include "hs2g_x.cuh"
 
 namespace hs2g {
 namespace {
@@ -26,14 +28,15 @@ namespace {
 struct Inst {
   Dims d;
   int64_t off;      // voxel offset in the concatenated fields
-  int64_t xb_off;   // element offset of the instance's stencil blocks
   int64_t nchunks;  // 32-column chunks per x-line
   int64_t woff;     // offset of the instance in W0 and W1, whose rows have pitch px (nx rounded up to 16 bytes)
   int64_t px;
-  // y and z coefficients (axis 0: y, 1: z): rows of pitch px like W0, or with cls tables per line class
-  const void* a[2];
-  const void* b[2];
-  const int32_t* cls[2];
+  const void* pool;      // stencil blocks, and their index per (line, chunk) or null
+  const int32_t* bidx;
+  // x, y and z line coefficients: in voxel order (row pitch px), or with cls tables per line class
+  const void* a[3];
+  const void* b[3];
+  const int32_t* cls[3];
 };
 
 struct XWork {
@@ -53,9 +56,6 @@ struct BatchView {
   R* T;
   R* W0;
   R* W1;
-  const R* xb;
-  const R* a0;
-  const R* b0;
   const uint8_t* vclass;
   const R* qtabs;          // [nsched][ninst][nclass]
   const uint8_t* active;   // [nsched][ninst] any source active
@@ -69,164 +69,49 @@ struct BatchView {
   int64_t nz_work;
 };
 
-constexpr int kMaxBatchClasses = HS2G_MAX_CLASSES;
 
-// IX: index type of the voxel, line and stencil-block arithmetic within an instance (int32_t when every
-// instance and its stencil blocks have fewer than 2^31 elements)
-template <typename R, bool HAS_Q, typename IX = int64_t>
-__device__ __forceinline__ R batch_stencil(const Inst& I, const R* __restrict__ T, const R* __restrict__ xb,
-                                           const uint8_t* __restrict__ vclass, const R* sq, IX L, int ch,
-                                           int lane) {
-  const Dims& d = I.d;
-  const IX nx = (IX)d.nx, ny = (IX)d.ny, nz = (IX)d.nz;
-  const IX i = (IX)ch * 32 + lane;
-  const IX k = L / ny, j = L - k * ny;
-  const IX p = L * nx + i;
-  const IX nxy = nx * ny;
-  const R* __restrict__ w = xb + I.xb_off + ((L * (IX)I.nchunks + ch) * kXBlockCoeffs) * 32 + lane;
-  const R* Ti = T + I.off;
-  const R t = Ti[p];
-  const R txl = i > 0 ? Ti[p - 1] : t;
-  const R txh = i + 1 < nx ? Ti[p + 1] : t;
-  const R tyl = j > 0 ? Ti[p - nx] : t;
-  const R tyh = j + 1 < ny ? Ti[p + nx] : t;
-  const R tzl = k > 0 ? Ti[p - nxy] : t;
-  const R tzh = k + 1 < nz ? Ti[p + nxy] : t;
-  R r = w[kWc * 32] * t;
-  r = fma(w[kWxl * 32], txl, r);
-  r = fma(w[kWxh * 32], txh, r);
-  r = fma(w[kWyl * 32], tyl, r);
-  r = fma(w[kWyh * 32], tyh, r);
-  r = fma(w[kWzl * 32], tzl, r);
-  r = fma(w[kWzh * 32], tzh, r);
-  if (HAS_Q) r = fma(w[kWq * 32], sq[vclass[I.off + p]], r);
-  return r;
+template <typename R>
+__device__ __forceinline__ XProblem<R> x_problem(const BatchView<R>& v, const Inst& I) {
+  return {I.d.nz, I.d.ny, I.d.nx, v.T + I.off, (const R*)I.pool, I.bidx, I.nchunks, (const R*)I.a[0], (const R*)I.b[0],
+          I.cls[0], v.vclass + I.off, nullptr, nullptr, v.W0 + I.woff, I.px};
 }
-
-// One block of 32 x-lines of one instance (CTA of 128 threads), same structure as sweep_x_kernel.
-template <typename R, bool HAS_Q, typename IX = int64_t>
-__device__ void batch_x_block(const BatchView<R>& v, const Inst& I, int64_t L0_, const R* sq, R (*sr)[33],
-                              R (*sa)[33]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const Dims& d = I.d;
-  const IX nx = (IX)d.nx, L0 = (IX)L0_;
-  const IX nlines = (IX)(d.nz * d.ny);
-  const int nchunks = (int)I.nchunks;
-  R* W0 = v.W0 + I.woff;
-  const IX px = (IX)I.px;
-  const R* a0 = v.a0 + I.off;
-  const R* b0 = v.b0 + I.off;
-  R carry = 0;
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const IX i = (IX)ch * 32 + lane;
-#pragma unroll
-    for (int ll = 0; ll < 8; ++ll) {
-      const int l = warp * 8 + ll;
-      const IX L = L0 + l;
-      R r = 0, a = 0;
-      if (L < nlines && i < nx) {
-        r = batch_stencil<R, HAS_Q, IX>(I, v.T, v.xb, v.vclass, sq, L, ch, lane);
-        a = a0[L * nx + i];
-      }
-      sr[l][lane] = r;
-      sa[l][lane] = a;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const int cw = (int)min((int64_t)32, d.nx - (int64_t)ch * 32);
-      R z = carry;
-      if (cw == 32) {  // full chunks unrolled: the shared loads of later rows issue ahead of the chain
-#pragma unroll 4
-        for (int cc = 0; cc < 32; ++cc) {
-          z = fma(-sa[lane][cc], z, sr[lane][cc]);
-          sr[lane][cc] = z;
-        }
-      } else {
-        for (int cc = 0; cc < cw; ++cc) {
-          z = fma(-sa[lane][cc], z, sr[lane][cc]);
-          sr[lane][cc] = z;
-        }
-      }
-      carry = z;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int ll = 0; ll < 8; ++ll) {
-      const int l = warp * 8 + ll;
-      const IX L = L0 + l;
-      if (L < nlines && i < nx) W0[L * px + i] = sr[l][lane];
-    }
-    __syncthreads();
-  }
-  carry = 0;
-  for (int ch = nchunks - 1; ch >= 0; --ch) {
-    const IX i = (IX)ch * 32 + lane;
-#pragma unroll
-    for (int ll = 0; ll < 8; ++ll) {
-      const int l = warp * 8 + ll;
-      const IX L = L0 + l;
-      R z = 0, b = 0;
-      if (L < nlines && i < nx) {
-        z = W0[L * px + i];
-        b = b0[L * nx + i];
-      }
-      sr[l][lane] = z;
-      sa[l][lane] = b;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const int cw = (int)min((int64_t)32, d.nx - (int64_t)ch * 32);
-      R x = carry;
-      if (cw == 32) {
-#pragma unroll 4
-        for (int cc = 31; cc >= 0; --cc) {
-          x = fma(-sa[lane][cc], x, sr[lane][cc]);
-          sr[lane][cc] = x;
-        }
-      } else {
-        for (int cc = cw - 1; cc >= 0; --cc) {
-          x = fma(-sa[lane][cc], x, sr[lane][cc]);
-          sr[lane][cc] = x;
-        }
-      }
-      carry = x;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int ll = 0; ll < 8; ++ll) {
-      const int l = warp * 8 + ll;
-      const IX L = L0 + l;
-      if (L < nlines && i < nx) W0[L * px + i] = sr[l][lane];
-    }
-    __syncthreads();
-  }
-}
-
-// 72 registers (7 CTAs of 128 threads per SM): more loads in flight per thread than at 64 registers, which
-// left the kernel load-latency bound (2.25e10 against 2.47e10 voxel-steps/s on the 256-instance batch).
-// IX = int32_t (every batch whose instances have fewer than 2^31 voxels and stencil-block elements): 32-bit
-// line, voxel and block arithmetic within an instance, 9.55 against 10.65 ms per FP64 step of that batch (the
-// same for the y and z sweeps changed nothing there).
-template <typename R, typename IX = int64_t>
-__global__ void __launch_bounds__(128, 7) batch_x_kernel(BatchView<R> v) {
-  __shared__ R sr[32][33];
-  __shared__ R sa[32][33];
-  __shared__ R sq[kMaxBatchClasses];
+// x sweep: a work item is kXItemLines consecutive x-lines of one instance.  The stencil takes a CTA per item and
+// gridDim.y-th chunk of columns (IX = int32_t when every instance has fewer than 2^31 voxels); the line solves a warp
+// per 16 (FP64) or 32 (FP32) lines of an item.  DENSE: some instance keeps its coefficients in voxel order.
+constexpr int kXItemLines = 64;
+template <typename R, typename IX>
+__global__ void __launch_bounds__(32 * kXStencilWarps, kXStencilCtas) batch_stencil_kernel(BatchView<R> v) {
+  __shared__ XLine<IX> lines[kXStencilLines];
+  __shared__ R sq[HS2G_MAX_CLASSES];
+  constexpr int SUB = kXItemLines / kXStencilLines;
+  const XWork item = v.xw[blockIdx.x / SUB];
+  const Inst& I = v.inst[item.inst];
+  const int64_t L0 = item.L0 + (int)(blockIdx.x % SUB) * kXStencilLines, end = I.d.nz * I.d.ny;
+  if (L0 >= end || blockIdx.y >= I.nchunks) return;
+  const XProblem<R> P = x_problem(v, I);
   const int step = *v.step;
-  const bool sched = step < v.nsched;
-  for (int64_t w = blockIdx.x; w < v.nx_work; w += gridDim.x) {
-    const XWork item = v.xw[w];
-    const Inst I = v.inst[item.inst];
-    const bool has_q = sched && v.active[(int64_t)step * v.ninst + item.inst];
-    if (has_q) {
-      const R* q = v.qtabs + ((int64_t)step * v.ninst + item.inst) * v.nclass;
-      for (int c = threadIdx.x; c < kMaxBatchClasses; c += blockDim.x) sq[c] = c < v.nclass ? q[c] : R(0);
-      __syncthreads();
-      batch_x_block<R, true, IX>(v, I, item.L0, sq, sr, sa);
-    } else {
-      batch_x_block<R, false, IX>(v, I, item.L0, sq, sr, sa);
-    }
+  if (step < v.nsched && v.active[(int64_t)step * v.ninst + item.inst]) {
+    const R* q = v.qtabs + ((int64_t)step * v.ninst + item.inst) * v.nclass;
+    for (int c = threadIdx.x; c < HS2G_MAX_CLASSES; c += 32 * kXStencilWarps) sq[c] = c < v.nclass ? q[c] : R(0);
+    x_stencil_lines<R, true, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
+  } else {
+    x_stencil_lines<R, false, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
   }
+}
+template <typename R, bool KEEP, bool DENSE>
+__global__ void __launch_bounds__(32 * kPairMaxWarps) batch_x_solve_kernel(BatchView<R> v, int64_t smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char batch_x_sm[];
+  constexpr bool TWO = sizeof(R) == 8;
+  const XWork item = v.xw[blockIdx.x];
+  const Inst& I = v.inst[item.inst];
+  const int64_t L0 = item.L0 + (threadIdx.x >> 5) * x_lines<TWO>(), end = I.d.nz * I.d.ny;
+  if (L0 >= end) return;
+  const int count = (int)min((int64_t)x_lines<TWO>(), end - L0);
+  R* sm = reinterpret_cast<R*>(batch_x_sm + (threadIdx.x >> 5) * smem_per_warp);
+  if (!DENSE || I.cls[0])
+    x_solve_lines<R, TWO, true, KEEP>(x_problem(v, I), L0, count, sm);
+  else
+    x_solve_lines<R, TWO, false, KEEP>(x_problem(v, I), L0, count, sm);
 }
 
 // y lines (W1 = s2*dT1 from W0 = sigma*dT0) and z lines (ADD_T: T += dT2 from W1 = s2*dT1, W0 as scratch): a CTA takes
@@ -244,12 +129,13 @@ __global__ void __launch_bounds__(32 * kPairMaxWarps) batch_pair_kernel(BatchVie
   const int64_t row = grp / gpr, i0 = (grp % gpr) * G;
   if (row >= (ADD_T ? ny : I.d.nz)) return;
   const int64_t w = ADD_T ? row * I.px + i0 : row * ny * I.px + i0, wst = ADD_T ? ny * I.px : I.px;
-  const int32_t* cls = I.cls[ADD_T];
+  constexpr int AX = ADD_T ? 2 : 1;
+  const int32_t* cls = I.cls[AX];
   PairLines<R> p;
   p.W = (ADD_T ? v.W1 : v.W0) + I.woff + w;
   p.wst = p.cst = p.zst = wst;
-  p.a = (const R*)I.a[ADD_T] + (cls ? 0 : w);
-  p.b = (const R*)I.b[ADD_T] + (cls ? 0 : w);
+  p.a = (const R*)I.a[AX] + (cls ? 0 : w);
+  p.b = (const R*)I.b[AX] + (cls ? 0 : w);
   p.cls = cls ? cls + row * nx + i0 : nullptr;
   p.T = ADD_T ? v.T + I.off + row * nx + i0 : nullptr;
   p.out = ADD_T ? v.T + I.off + row * nx + i0 : v.W1 + I.woff + w;
@@ -287,8 +173,8 @@ __global__ void widen_kernel(const R* __restrict__ src, double* __restrict__ dst
 }
 
 struct Tuning {
-  int x_grid;
-  bool y_keep, z_keep;  // the forward values of the y / z lines stay in shared memory
+  int x_split;                  // the stencil's CTAs per item: each takes every x_split-th chunk of columns
+  bool x_keep, y_keep, z_keep;  // the forward values of the x / y / z lines stay in shared memory
 };
 
 }  // namespace
@@ -303,15 +189,13 @@ struct Batch {
   cudaStream_t stream = nullptr;
   std::vector<Inst> inst;
   std::vector<int64_t> offsets;  // [ninst+1] voxel offsets
-  int64_t nvox = 0, xb_len = 0;
+  int64_t nvox = 0;
   Inst* inst_dev = nullptr;
   void* T = nullptr;  // R*
   void* W0 = nullptr;
   void* W1 = nullptr;
-  void* coef = nullptr;  // a0 and b0, nvox R each
-  std::vector<void*> line_mem;  // the instances' y and z coefficients
+  std::vector<void*> coef_mem;  // the instances' coefficients
   int64_t nw = 0;               // elements of W0 and W1
-  void* xb = nullptr;
   uint8_t* vclass = nullptr;
   void* qtabs = nullptr;
   uint8_t* active = nullptr;
@@ -321,9 +205,9 @@ struct Batch {
   LWork* yw = nullptr;
   LWork* zw = nullptr;
   int64_t nxw = 0, nyw = 0, nzw = 0;
-  Tuning tune{0, true, true};
-  int64_t max_ny = 0, max_nz = 0;  // longest y and z line
-  bool dense[2] = {false, false};  // some instance keeps its y / z coefficients in voxel order
+  Tuning tune{1, true, true, true};
+  int64_t max_nx = 0, max_ny = 0, max_nz = 0;  // longest x, y and z line
+  bool dense[3] = {false, false, false};  // some instance keeps its x / y / z coefficients in voxel order
   bool ix32 = false;  // every instance's voxels and stencil blocks below 2^31 elements: 32-bit x-sweep indices
   cudaGraphExec_t graph = nullptr;
   int64_t bytes = 0;
@@ -339,10 +223,6 @@ BatchView<R> view(const Batch& b) {
   v.T = (R*)b.T;
   v.W0 = (R*)b.W0;
   v.W1 = (R*)b.W1;
-  R* c = (R*)b.coef;
-  v.a0 = c;
-  v.b0 = c + b.nvox;
-  v.xb = (const R*)b.xb;
   v.vclass = b.vclass;
   v.qtabs = (const R*)b.qtabs;
   v.active = b.active;
@@ -371,11 +251,11 @@ template <typename R, bool ADD_T>
 PairShape batch_shape(const Batch& b, int force_keep) {
   constexpr bool TWO = sizeof(R) == 8;
   const int64_t len = ADD_T ? b.max_nz : b.max_ny, groups = (ADD_T ? b.nzw : b.nyw) * kPairMaxWarps;
-  PairShape sh = b.dense[ADD_T] ? pair_shape<R, TWO, ADD_T, false>(len, groups, force_keep)
+  PairShape sh = b.dense[ADD_T ? 2 : 1] ? pair_shape<R, TWO, ADD_T, false>(len, groups, force_keep)
                                 : pair_shape<R, TWO, ADD_T, true>(len, groups, force_keep);
-  size_t each = b.dense[ADD_T] ? pair_smem<R, TWO, ADD_T, true, false>(len) : pair_smem<R, TWO, ADD_T, true, true>(len);
+  size_t each = b.dense[ADD_T ? 2 : 1] ? pair_smem<R, TWO, ADD_T, true, false>(len) : pair_smem<R, TWO, ADD_T, true, true>(len);
   if (each * kPairMaxWarps > 226 * 1024) sh.keep = false;
-  if (!sh.keep) each = b.dense[ADD_T] ? pair_smem<R, TWO, ADD_T, false, false>(len) : pair_smem<R, TWO, ADD_T, false, true>(len);
+  if (!sh.keep) each = b.dense[ADD_T ? 2 : 1] ? pair_smem<R, TWO, ADD_T, false, false>(len) : pair_smem<R, TWO, ADD_T, false, true>(len);
   sh.warps = kPairMaxWarps;
   sh.smem = each * kPairMaxWarps;
   return sh;
@@ -384,13 +264,36 @@ template <typename R, bool ADD_T>
 cudaError_t launch_batch_pair(const Batch& b, const BatchView<R>& v, bool keep, cudaStream_t s) {
   const PairShape sh = batch_shape<R, ADD_T>(b, keep ? 1 : 0);
   const int64_t work = ADD_T ? b.nzw : b.nyw;
-  batch_pair_for<R, ADD_T>(sh.keep, b.dense[ADD_T])<<<(unsigned)work, 32 * kPairMaxWarps, sh.smem, s>>>(
+  batch_pair_for<R, ADD_T>(sh.keep, b.dense[ADD_T ? 2 : 1])<<<(unsigned)work, 32 * kPairMaxWarps, sh.smem, s>>>(
       v, (int64_t)(sh.smem / kPairMaxWarps));
   return cudaGetLastError();
 }
 template <typename R>
+BatchPairKernel<R> batch_x_solve_for(bool keep, bool dense) {
+  return keep ? (dense ? batch_x_solve_kernel<R, true, true> : batch_x_solve_kernel<R, true, false>)
+              : (dense ? batch_x_solve_kernel<R, false, true> : batch_x_solve_kernel<R, false, false>);
+}
+// the same for the x line solves, whose CTAs have a warp per x_lines of an item
+template <typename R>
+PairShape batch_x_shape(const Batch& b, int force_keep) {
+  constexpr bool TWO = sizeof(R) == 8;
+  const int warps = kXItemLines / x_lines<TWO>();
+  const int64_t groups = b.nxw * warps;
+  PairShape sh = b.dense[0] ? x_solve_shape<R, TWO, false>(b.max_nx, groups, force_keep)
+                            : x_solve_shape<R, TWO, true>(b.max_nx, groups, force_keep);
+  size_t each = b.dense[0] ? x_solve_smem<R, TWO, false, true>(b.max_nx) : x_solve_smem<R, TWO, true, true>(b.max_nx);
+  if (each * warps > 226 * 1024) sh.keep = false;
+  if (!sh.keep) each = b.dense[0] ? x_solve_smem<R, TWO, false, false>(b.max_nx) : x_solve_smem<R, TWO, true, false>(b.max_nx);
+  sh.warps = warps;
+  sh.smem = each * warps;
+  return sh;
+}
+template <typename R>
 cudaError_t batch_prepare() {
   cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 4 && e == cudaSuccess; ++k)
+    e = cudaFuncSetAttribute((const void*)batch_x_solve_for<R>(k & 1, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             226 * 1024);
   for (int k = 0; k < 8 && e == cudaSuccess; ++k) {
     const void* f = k & 4 ? (const void*)batch_pair_for<R, true>(k & 1, k & 2) : (const void*)batch_pair_for<R, false>(k & 1, k & 2);
     e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
@@ -402,10 +305,14 @@ template <typename R>
 cudaError_t launch_axis(const Batch& b, int axis, const Tuning& t, cudaStream_t s) {
   BatchView<R> v = view<R>(b);
   if (axis == 0) {
+    const dim3 grid((unsigned)(b.nxw * (kXItemLines / kXStencilLines)), (unsigned)t.x_split);
     if (b.ix32)
-      batch_x_kernel<R, int32_t><<<(unsigned)std::max(1, t.x_grid), 128, 0, s>>>(v);
+      batch_stencil_kernel<R, int32_t><<<grid, 32 * kXStencilWarps, 0, s>>>(v);
     else
-      batch_x_kernel<R><<<(unsigned)std::max(1, t.x_grid), 128, 0, s>>>(v);
+      batch_stencil_kernel<R, int64_t><<<grid, 32 * kXStencilWarps, 0, s>>>(v);
+    const PairShape sh = batch_x_shape<R>(b, t.x_keep ? 1 : 0);
+    batch_x_solve_for<R>(sh.keep, b.dense[0])<<<(unsigned)b.nxw, 32 * sh.warps, sh.smem, s>>>(
+        v, (int64_t)(sh.smem / sh.warps));
   } else if (axis == 1) {
     return launch_batch_pair<R, false>(b, v, t.y_keep, s);
   } else if (axis == 2) {
@@ -428,7 +335,7 @@ cudaError_t launch_step_batch(const Batch& b, cudaStream_t s) {
 
 }  // namespace
 
-// Work lists: blocks of 32 x-lines, and of the line solves' y and z lines, per instance, longest lines first.
+// Work lists: blocks of consecutive x-lines, and of groups of y and z lines, per instance, longest lines first.
 void batch_build_work(Batch& b, std::vector<XWork>& xw, std::vector<LWork>& yw, std::vector<LWork>& zw) {
   xw.clear();
   yw.clear();
@@ -444,7 +351,7 @@ void batch_build_work(Batch& b, std::vector<XWork>& xw, std::vector<LWork>& yw, 
   };
   for (int ib : by([](const Dims& d) { return d.nx; })) {
     const Dims& d = b.inst[ib].d;
-    for (int64_t L0 = 0; L0 < d.nz * d.ny; L0 += 32) xw.push_back(XWork{ib, 0, L0});
+    for (int64_t L0 = 0; L0 < d.nz * d.ny; L0 += kXItemLines) xw.push_back(XWork{ib, 0, L0});
   }
   for (int ib : by([](const Dims& d) { return d.ny; })) {
     const Dims& d = b.inst[ib].d;
@@ -515,19 +422,21 @@ cudaError_t batch_autotune(Batch& b, std::string& report) {
   Tuning best = b.tune;
   char line[256];
   cudaError_t e = cudaSuccess;
-  // x: persistent grid size (CTAs of 128 threads)
+  // x: the stencil's CTAs per item, and the line solves' forward values in shared or global memory
   {
     float bt = 1e30f;
-    // per = 0: one CTA per work item, the hardware's block scheduler doing the balancing
-    for (int per : {4, 5, 6, 7, 8, 10, 0}) {
-      Tuning t = best;
-      t.x_grid = (int)std::min<int64_t>(std::min<int64_t>(b.nxw, 1 << 30), per ? (int64_t)sms * per : b.nxw);
-      float ms;
-      if ((e = batch_time_axis(b, 0, t, 2, &ms)) != cudaSuccess) return e;
-      snprintf(line, sizeof line, "x grid %d: %.3f ms\n", t.x_grid, ms);
-      report += line;
-      if (ms < bt) bt = ms, best.x_grid = t.x_grid;
-    }
+    for (int keep = 1; keep >= 0; --keep)
+      for (int split : {1, 2, 4}) {
+        Tuning t = best;
+        t.x_split = split;
+        t.x_keep = keep != 0;
+        float ms;
+        if ((e = batch_time_axis(b, 0, t, 2, &ms)) != cudaSuccess) return e;
+        snprintf(line, sizeof line, "x split %d, forward values in %s memory: %.3f ms\n", split,
+                 keep ? "shared" : "global", ms);
+        report += line;
+        if (ms < bt) bt = ms, best.x_split = split, best.x_keep = keep != 0;
+      }
   }
   // y and z: forward values in shared memory or through global memory
   for (int axis = 1; axis <= 2; ++axis) {
@@ -544,8 +453,8 @@ cudaError_t batch_autotune(Batch& b, std::string& report) {
     }
   }
   b.tune = best;
-  snprintf(line, sizeof line, "chosen: x grid %d, y values in %s memory, z values in %s memory\n", best.x_grid,
-           best.y_keep ? "shared" : "global", best.z_keep ? "shared" : "global");
+  snprintf(line, sizeof line, "chosen: x split %d, x values in %s memory, y in %s, z in %s\n", best.x_split,
+           best.x_keep ? "shared" : "global", best.y_keep ? "shared" : "global", best.z_keep ? "shared" : "global");
   report += line;
   return e;
 }
@@ -596,14 +505,12 @@ cudaError_t balloc(Batch& b, T** p, int64_t count) {
 void batch_free(Batch& b) {
   if (b.graph) cudaGraphExecDestroy(b.graph);
   b.graph = nullptr;
-  for (void* p : {(void*)b.inst_dev, b.T, b.W0, b.W1, b.coef, b.xb, (void*)b.vclass, b.qtabs, (void*)b.active,
+  for (void* p : {(void*)b.inst_dev, b.T, b.W0, b.W1, (void*)b.vclass, b.qtabs, (void*)b.active,
                   (void*)b.step, (void*)b.xw, (void*)b.yw, (void*)b.zw})
     if (p) cudaFree(p);
-  for (void* p : b.line_mem) cudaFree(p);
+  for (void* p : b.coef_mem) cudaFree(p);
   if (b.stream) cudaStreamDestroy(b.stream);
 }
-
-int64_t xb_elems(const hs2g::Dims& d) { return d.nz * d.ny * ((d.nx + 31) / 32) * hs2g::kXBlockCoeffs * 32; }
 
 // Compile instance `ib` of problem p into the batch (FP64 workspace ws, then into the batch's storage type).
 int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, unsigned long long* err) {
@@ -612,7 +519,7 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   const int64_t n = d.nvox(), np = d.nz * d.ny * I.px;
   const int64_t nfz = (d.nz + 1) * d.nxy(), nfy = d.nz * (d.ny + 1) * d.nx, nfx = d.nz * d.ny * (d.nx + 1);
   cudaStream_t s = b.stream;
-  // workspace layout (doubles): faces z, y, x | M s2 sigma | a0 b0 | a1 b1 a2 b2 | x blocks | bytes:
+  // workspace layout (doubles): faces z, y, x | M s2 sigma | a0 b0 | a1 b1 a2 b2 | bytes:
   // compute mask, material, boundary classes | material table | boundary forms
   double* fz = ws;
   double* fy = fz + nfz;
@@ -621,9 +528,8 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   double* s2 = M + n;
   double* sg = s2 + n;
   double* c2 = sg + n;
-  double* c4 = c2 + 2 * n;
-  double* xbw = c4 + 4 * np;
-  uint8_t* u8 = reinterpret_cast<uint8_t*>(xbw + xb_elems(d));
+  double* c4 = c2 + 2 * np;
+  uint8_t* u8 = reinterpret_cast<uint8_t*>(c4 + 4 * np);
   uint8_t* comp = u8;
   uint8_t* mat = comp + n;
   uint8_t* bz = mat + n;
@@ -632,6 +538,10 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   hs2g_material* mats = reinterpret_cast<hs2g_material*>((reinterpret_cast<uintptr_t>(bx + nfx) + 255) & ~uintptr_t(255));
   hs2g_face_form* forms = reinterpret_cast<hs2g_face_form*>(
       (reinterpret_cast<uintptr_t>(mats + HS2G_MAX_CLASSES) + 255) & ~uintptr_t(255));
+  // then the faces' values per class and material pair, and the scratch of the search for equal lines and blocks
+  unsigned char* table = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(forms + 3 * HS2G_MAX_CLASSES) + 255) & ~uintptr_t(255));
+  unsigned char* scratch = table + ((hs2g::face_table_bytes(p.nmat, p.nbnd) + 255) & ~size_t(255));
   cudaError_t e = cudaSuccess;
   auto up = [&](void* dst, const void* src, size_t bytes) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
@@ -644,9 +554,9 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   up(forms, p.forms, sizeof(hs2g_face_form) * p.nbnd * 3);
   if (p.volumetric) up(b.vclass + I.off, p.volumetric, (size_t)n);
   else if (e == cudaSuccess) e = cudaMemsetAsync(b.vclass + I.off, 0, (size_t)n, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 0, mat, bz, mats, p.nmat, forms, p.nbnd, fz, err, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 1, mat, by, mats, p.nmat, forms, p.nbnd, fy, err, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 2, mat, bx, mats, p.nmat, forms, p.nbnd, fx, err, s);
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, 0, mat, bz, mats, p.nmat, forms, p.nbnd, fz, err, table, s);
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, 1, mat, by, mats, p.nmat, forms, p.nbnd, fy, err, table, s);
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, 2, mat, bx, mats, p.nmat, forms, p.nbnd, fx, err, table, s);
   if (e == cudaSuccess) e = hs2g::launch_capacity_from_classes(d, mat, mats, p.nmat, M, comp, err, s);
   if (e != cudaSuccess) return bcuda(e, "batch compile");
   unsigned long long v = 0;
@@ -664,60 +574,47 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   c.nchunks = I.nchunks;
   c.px = I.px;
   const bool f64 = b.precision == 64;
-  c.a0 = f64 ? (double*)b.coef + I.off : c2;
-  c.b0 = f64 ? (double*)b.coef + b.nvox + I.off : c2 + n;
+  c.a0 = c2;
+  c.b0 = c2 + np;
   c.a1 = c4;
   c.b1 = c4 + np;
   c.a2 = c4 + 2 * np;
   c.b2 = c4 + 3 * np;
-  c.xb = f64 ? (double*)b.xb + I.xb_off : xbw;
-  if (!f64 && (e = cudaMemsetAsync(xbw, 0, sizeof(double) * xb_elems(d), s)) != cudaSuccess)
-    return bcuda(e, "batch compile");
-  if ((e = hs2g::launch_factor(d, fz, fy, fx, M, comp, s2, sg, c, s, f64)) != cudaSuccess)
+  const hs2g::Faces faces{fz, fy, fx, {}};
+  if ((e = hs2g::launch_factor(d, faces, M, comp, s2, sg, c, s, f64)) != cudaSuccess) return bcuda(e, "batch factor");
+  hs2g::Compressed kept;
+  if ((e = hs2g::compress_coeffs(d, faces, comp, s2, c, b.precision, scratch, &kept, s)) != cudaSuccess)
     return bcuda(e, "batch factor");
-  if (!f64) {
-    for (int a = 0; a < 2 && e == cudaSuccess; ++a)
-      e = hs2g::batch_convert(c2 + a * n, (float*)b.coef + a * b.nvox + I.off, n, 32, s);
-    if (e == cudaSuccess) e = hs2g::batch_convert(xbw, (float*)b.xb + I.xb_off, xb_elems(d), 32, s);
-  }
-  // the y and z coefficients: tables per line class, or the arrays where the lines have too many classes
-  for (int ax = 0; ax < 2 && e == cudaSuccess; ++ax) {
-    const double *a = ax ? c.a2 : c.a1, *bb = ax ? c.b2 : c.b1;
-    hs2g::LineTables t;
-    e = ax ? hs2g::classify_lines(a, bb, d.ny, d.nx, I.px, d.nz, d.ny * I.px, &t, s)
-           : hs2g::classify_lines(a, bb, d.nz, d.nx, d.ny * I.px, d.ny, I.px, &t, s);
-    if (e != cudaSuccess) break;
-    const int64_t count = t.cls ? t.nclass * (ax ? d.nz : d.ny) : np;
+  b.coef_mem.push_back(kept.blocks.pool);
+  I.pool = kept.blocks.pool;
+  I.bidx = kept.blocks.bidx;
+  b.bytes += (int64_t)kept.blocks.bytes;
+  const double* coeffs[3][2] = {{c.a0, c.b0}, {c.a1, c.b1}, {c.a2, c.b2}};
+  for (int ax = 0; ax < 3; ++ax) {
+    hs2g::LineTables& t = kept.lines[ax];
     if (t.cls) {
-      b.line_mem.push_back(t.cls);
-      b.bytes += (int64_t)sizeof(int32_t) * (ax ? d.ny : d.nz) * d.nx;
-      a = t.a;
-      bb = t.b;
+      b.coef_mem.push_back(t.a);
+      b.bytes += (int64_t)t.bytes;
     } else {
       b.dense[ax] = true;
     }
     I.cls[ax] = t.cls;
     const void** dst[2] = {&I.a[ax], &I.b[ax]};
-    const double* src[2] = {a, bb};
-    for (int q = 0; q < 2; ++q) {
-      if (t.cls && f64) {  // the tables as they are
-        b.line_mem.push_back((void*)src[q]);
-        *dst[q] = src[q];
-      } else {
-        void* m = nullptr;
-        if (e == cudaSuccess) e = cudaMalloc(&m, b.elem() * count);
-        if (e == cudaSuccess) {
-          b.line_mem.push_back(m);
-          *dst[q] = m;
-          e = hs2g::batch_convert(src[q], m, count, b.precision, s);
-        }
-      }
-      b.bytes += (int64_t)b.elem() * count;
+    if (t.cls && f64) {  // the tables as they are
+      I.a[ax] = t.a;
+      I.b[ax] = t.b;
+      continue;
     }
-    if (t.cls && !f64) {
-      cudaStreamSynchronize(s);
-      cudaFree(t.a);
-      cudaFree(t.b);
+    // float tables beside the classes, or the arrays where the lines have too many classes
+    const int64_t count = t.cls ? t.nclass * (ax == 0 ? d.nx : ax == 1 ? d.ny : d.nz) : np;
+    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+      void* m = nullptr;
+      e = cudaMalloc(&m, b.elem() * count);
+      if (e != cudaSuccess) break;
+      b.coef_mem.push_back(m);
+      b.bytes += (int64_t)b.elem() * count;
+      *dst[q] = m;
+      e = hs2g::batch_convert(t.cls ? (q ? t.b : t.a) : coeffs[ax][q], m, count, b.precision, s);
     }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -775,13 +672,12 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     delete hb;
     return bcuda(e, "cudaStreamCreate");
   }
-  int64_t off = 0, xoff = 0, ws = 0;
+  int64_t off = 0, ws = 0;
   b.offsets.push_back(0);
   for (int i = 0; i < n; ++i) {
     hs2g::Inst I{};
     I.d = hs2g::Dims{problems[i].nz, problems[i].ny, problems[i].nx};
     I.off = off;
-    I.xb_off = xoff;
     I.nchunks = (I.d.nx + 31) / 32;
     I.woff = b.nw;
     const int64_t quad = 16 / (int64_t)b.elem();
@@ -791,27 +687,24 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     const hs2g::Dims& d = I.d;
     const int64_t nn = d.nvox();
     off += nn + (nn & 1);  // keep every instance 16-byte aligned
-    xoff += xb_elems(d);
     b.offsets.push_back(off);
     const int64_t faces = (d.nz + 1) * d.nxy() + d.nz * (d.ny + 1) * d.nx + d.nz * d.ny * (d.nx + 1);
-    const int64_t need = faces + 5 * nn + 4 * d.nz * d.ny * I.px + xb_elems(d) + (faces + 3 * nn) / 8 + 2048 +
+    const int64_t need = faces + 3 * nn + 6 * d.nz * d.ny * I.px + (faces + 3 * nn) / 8 + 2048 +
                          (int64_t)(sizeof(hs2g_material) * HS2G_MAX_CLASSES + sizeof(hs2g_face_form) * 3 *
-                                   HS2G_MAX_CLASSES) / 8 + 256;
+                                   HS2G_MAX_CLASSES) / 8 + 512 +
+                         (int64_t)(hs2g::face_table_bytes(problems[i].nmat, problems[i].nbnd) + hs2g::compress_scratch(d)) / 8;
     ws = std::max(ws, need);
   }
   b.nvox = off;
-  b.xb_len = xoff;
   b.ix32 = true;
   for (const hs2g::Inst& I : b.inst)
-    b.ix32 = b.ix32 && I.d.nz * I.d.ny * I.px < ((int64_t)1 << 31) && xb_elems(I.d) < ((int64_t)1 << 31);
+    b.ix32 = b.ix32 && I.d.nz * I.d.ny * I.px < ((int64_t)1 << 31);
   const size_t el = b.elem();
   double* wsp = nullptr;
   unsigned long long* err = nullptr;
   if ((e = balloc(b, &b.inst_dev, n)) != cudaSuccess || (e = balloc(b, (char**)&b.T, b.nvox * el)) != cudaSuccess ||
       (e = balloc(b, (char**)&b.W0, b.nw * el)) != cudaSuccess ||
       (e = balloc(b, (char**)&b.W1, b.nw * el)) != cudaSuccess ||
-      (e = balloc(b, (char**)&b.coef, 2 * b.nvox * el)) != cudaSuccess ||
-      (e = balloc(b, (char**)&b.xb, b.xb_len * el)) != cudaSuccess ||
       (e = balloc(b, &b.vclass, b.nvox)) != cudaSuccess || (e = balloc(b, &b.step, 1)) != cudaSuccess ||
       (e = cudaMalloc(&wsp, sizeof(double) * ws)) != cudaSuccess ||
       (e = cudaMalloc(&err, sizeof(unsigned long long))) != cudaSuccess) {
@@ -820,11 +713,9 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     hs2g::set_last_error(HS2G_ERR_NOMEM, "hs2g_batch_create: device allocation failed");
     return bail(HS2G_ERR_NOMEM);
   }
-  cudaMemsetAsync(b.xb, 0, b.xb_len * el, b.stream);
   cudaMemsetAsync(b.T, 0, b.nvox * el, b.stream);
   cudaMemsetAsync(b.W0, 0, b.nw * el, b.stream);
   cudaMemsetAsync(b.W1, 0, b.nw * el, b.stream);
-  cudaMemsetAsync(b.coef, 0, 2 * b.nvox * el, b.stream);
   cudaMemsetAsync(b.vclass, 0, b.nvox, b.stream);
   cudaMemsetAsync(b.step, 0, sizeof(int), b.stream);
   int rc = HS2G_OK;
@@ -840,17 +731,19 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   if ((e = hs2g::batch_upload_work(b)) != cudaSuccess) return bail(bcuda(e, "work lists"));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  b.tune.x_grid = (int)std::min<int64_t>(b.nxw, (int64_t)sms * 7);  // the x kernel's 7 resident CTAs per SM
   for (const hs2g::Inst& I : b.inst) {
+    b.max_nx = std::max(b.max_nx, I.d.nx);
     b.max_ny = std::max(b.max_ny, I.d.ny);
     b.max_nz = std::max(b.max_nz, I.d.nz);
   }
   if (precision == 64) {
     e = hs2g::batch_prepare<double>();
+    b.tune.x_keep = hs2g::batch_x_shape<double>(b, -1).keep;
     b.tune.y_keep = hs2g::batch_shape<double, false>(b, -1).keep;
     b.tune.z_keep = hs2g::batch_shape<double, true>(b, -1).keep;
   } else {
     e = hs2g::batch_prepare<float>();
+    b.tune.x_keep = hs2g::batch_x_shape<float>(b, -1).keep;
     b.tune.y_keep = hs2g::batch_shape<float, false>(b, -1).keep;
     b.tune.z_keep = hs2g::batch_shape<float, true>(b, -1).keep;
   }

@@ -1,4 +1,4 @@
-// Line classes: the y and z lines of a problem have few distinct sequences of coefficients (a layered specimen with
+// Line classes: the lines of a problem have few distinct sequences of coefficients (a layered specimen with
 // some flaws has one per layer and flaw pattern), so the step keeps one table per distinct line and a class per line
 // instead of two values per voxel.  At 65x512x512 that takes 16 of the y sweep's 32 bytes per voxel and 16 of the z
 // sweep's 40 out of its HBM traffic.  Lines are compared bit for bit: the step's arithmetic does not change.
@@ -10,14 +10,6 @@ namespace hs2g {
 namespace {
 
 constexpr int kTh = 256;
-
-struct LineGrid {
-  const double* a;
-  const double* b;
-  int64_t outer, nx, ost, n, rst;  // line (o, i): rows r at o*ost + r*rst + i
-  __device__ int64_t lines() const { return outer * nx; }
-  __device__ int64_t base(int64_t l) const { return (l / nx) * ost + l % nx; }
-};
 
 __device__ __forceinline__ unsigned long long mix(unsigned long long h, double v) {
   h = (h ^ (unsigned long long)__double_as_longlong(v)) * 0x9E3779B97F4A7C15ull;
@@ -62,72 +54,57 @@ __global__ void assign_lines_kernel(LineGrid g, const int* slot, const int* id, 
           __double_as_longlong(g.b[p]) == __double_as_longlong(g.b[q]);
   if (!eq) *same = 0;
 }
-__global__ void gather_lines_kernel(LineGrid g, const int* rep, int64_t nclass, double* ta, double* tb) {
+__global__ void gather_lines_kernel(LineGrid g, const int* rep, int64_t nclass, int64_t mid, double* ta, double* tb) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= nclass * g.n) return;
-  const int64_t p = g.base(rep[t / g.n]) + (t % g.n) * g.rst;
+  int64_t r = t % g.n;
+  if (mid >= 0 && r > mid) r = mid + g.n - r;
+  const int64_t p = g.base(rep[t / g.n]) + r * g.rst;
   ta[t] = g.a[p];
   tb[t] = g.b[p];
 }
 
 }  // namespace
 
-cudaError_t classify_lines(const double* a, const double* b, int64_t outer, int64_t nx, int64_t ost, int64_t n,
-                           int64_t rst, LineTables* out, cudaStream_t s) {
-  *out = LineTables{};
-  const int64_t lines = outer * nx;
-  // Worth it when the tables are an eighth of the arrays: the classes of a warp's 16 lines then cost it no more
-  // than reading the arrays would.
-  const int64_t max_class = std::max<int64_t>(1, lines / 8);
-  if (lines >= ((int64_t)1 << 30)) return cudaSuccess;
-  int64_t cap = 64;
-  while (cap < 2 * lines) cap *= 2;
-  const LineGrid g{a, b, outer, nx, ost, n, rst};
-  unsigned long long* keys = nullptr;
-  int *ints = nullptr, host[2] = {0, 1};
-  int32_t* cls = nullptr;
-  // ints: owner[cap], id[cap], slot[lines], rep[max_class], {count, same}
-  cudaError_t e = cudaMalloc(&keys, sizeof(*keys) * cap);
-  if (e == cudaSuccess) e = cudaMalloc(&ints, sizeof(int) * (2 * cap + lines + max_class + 2));
-  if (e == cudaSuccess) e = cudaMalloc(&cls, sizeof(int32_t) * lines);
-  int *owner = ints, *id = ints + cap, *slot = id + cap, *rep = slot + lines, *count = rep + max_class;
+size_t LineJob::scratch_bytes(int64_t lines) {
+  const ClassTable t(lines);
+  return t.bytes() + sizeof(int) * (size_t)max_class(lines) + 256;
+}
+
+cudaError_t LineJob::begin(unsigned char* scratch, cudaStream_t s) {
+  const int64_t lines = grid.lines();
+  table = ClassTable(lines);
+  rep = reinterpret_cast<int*>(table.place(scratch));
+  cudaError_t e = table.clear(s);
+  if (e != cudaSuccess) return e;
   const unsigned blocks = (unsigned)((lines + kTh - 1) / kTh);
-  if (e == cudaSuccess) e = cudaMemsetAsync(keys, 0, sizeof(*keys) * cap, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(owner, 0x7f, sizeof(int) * cap, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(count, host, sizeof host, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) {
-    hash_lines_kernel<<<blocks, kTh, 0, s>>>(g, keys, owner, cap - 1, slot);
-    number_lines_kernel<<<blocks, kTh, 0, s>>>(lines, owner, slot, id, rep, count, (int)max_class);
-    e = cudaGetLastError();
+  hash_lines_kernel<<<blocks, kTh, 0, s>>>(grid, table.keys, table.owner, table.cap - 1, table.slot);
+  number_lines_kernel<<<blocks, kTh, 0, s>>>(lines, table.owner, table.slot, table.id, rep, table.count,
+                                             (int)max_class(lines));
+  return cudaGetLastError();
+}
+
+cudaError_t LineJob::finish(int64_t nclass, LineTables* out, cudaStream_t s) {
+  *out = LineTables{};
+  const int64_t lines = grid.lines(), n = grid.n;
+  if (nclass > max_class(lines)) return cudaSuccess;
+  unsigned char* m = nullptr;
+  const size_t half = sizeof(double) * (size_t)(nclass * n);
+  cudaError_t e = cudaMalloc(&m, 2 * half + sizeof(int32_t) * lines);
+  if (e == cudaErrorMemoryAllocation) {  // no room for the tables: the arrays stay
+    cudaGetLastError();
+    return cudaSuccess;
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(host, count, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  const int64_t nclass = host[0];
-  if (e == cudaSuccess && nclass <= max_class) {
-    e = cudaMalloc(&out->a, sizeof(double) * nclass * n);
-    if (e == cudaSuccess) e = cudaMalloc(&out->b, sizeof(double) * nclass * n);
-    if (e == cudaSuccess) {
-      assign_lines_kernel<<<blocks, kTh, 0, s>>>(g, slot, id, rep, cls, count + 1);
-      gather_lines_kernel<<<(unsigned)((nclass * n + kTh - 1) / kTh), kTh, 0, s>>>(g, rep, nclass, out->a, out->b);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(host + 1, count + 1, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && host[1]) {
-      out->cls = cls;
-      out->nclass = nclass;
-      cls = nullptr;
-    } else {
-      cudaFree(out->a);
-      cudaFree(out->b);
-      out->a = out->b = nullptr;
-    }
-  }
-  cudaFree(keys);
-  cudaFree(ints);
-  cudaFree(cls);
-  if (e != cudaSuccess) cudaGetLastError();
-  return e;
+  if (e != cudaSuccess) return e;
+  out->a = reinterpret_cast<double*>(m);
+  out->b = reinterpret_cast<double*>(m + half);
+  out->cls = reinterpret_cast<int32_t*>(m + 2 * half);
+  out->nclass = nclass;
+  out->bytes = 2 * half + sizeof(int32_t) * lines;
+  assign_lines_kernel<<<(unsigned)((lines + kTh - 1) / kTh), kTh, 0, s>>>(grid, table.slot, table.id, rep, out->cls,
+                                                                         table.count + 1);
+  gather_lines_kernel<<<(unsigned)((nclass * n + kTh - 1) / kTh), kTh, 0, s>>>(grid, rep, nclass, mid, out->a, out->b);
+  return cudaGetLastError();
 }
 
 }  // namespace hs2g

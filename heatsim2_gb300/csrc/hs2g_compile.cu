@@ -5,7 +5,10 @@
 // Replaces the reference's Python voxel loop and symbolic assembly (crank_nicolson.pyx:272-491,
 // alternatingdirection_c.c:102-199) and its LU factorisation at finalize (tridiag.pyx:9-43,
 // alternatingdirection_c_pyx.pyx:279).  All FP64.  One thread per face (compiler) or per grid line (LU).
+#include <algorithm>
+
 #include "hs2g_internal.cuh"
+#include "hs2g_x.cuh"
 
 namespace hs2g {
 namespace {
@@ -24,65 +27,78 @@ __device__ __forceinline__ double eval_form(const double* f, const double* klo, 
   return acc;
 }
 
+// The conductance and error code (0: none) that class b gives a face between materials of the tables mlo and mhi (the
+// voxel below and above it; nmat: outside the grid) on `axis`; exterior: it has a side outside the grid.
+struct FaceValue {
+  double g;
+  int code;
+};
+__device__ FaceValue face_value(const hs2g_material* __restrict__ mats, int nmat, const hs2g_face_form& form, int mlo,
+                                int mhi) {
+  const bool lo_c = mlo < nmat && mats[mlo].kind == HS2G_TEMPERATURE_COMPUTE;
+  const bool hi_c = mhi < nmat && mats[mhi].kind == HS2G_TEMPERATURE_COMPUTE;
+  if (!lo_c && !hi_c) return {0.0, 0};
+  const double* klo = lo_c ? mats[mlo].k : mats[mhi].k;
+  const double* khi = hi_c ? mats[mhi].k : mats[mlo].k;
+  const double g = eval_form(form.normal, klo, khi);
+  if (!(g == g) || isinf(g)) return {0.0, HS2G_ERR_KTYPE};
+  const double tol = 1e-12 * fabs(g);
+  int code = 0;
+  for (int z = 0; z < form.nzero; ++z) {
+    const double v = eval_form(form.zero[z], klo, khi);
+    if (!(fabs(v) <= tol) && code == 0) code = form.zero_code[z];
+  }
+  if (code == 0 && (mlo >= nmat || mhi >= nmat) && g != 0.0) code = HS2G_ERR_EXTERIOR;
+  return {g, code};
+}
+// The values of every (class, low material, high material), nmat standing for outside the grid: one thread each.
+__global__ void face_values_kernel(int axis, const hs2g_material* __restrict__ mats, int nmat,
+                                   const hs2g_face_form* __restrict__ forms, int nbnd, FaceValue* __restrict__ table) {
+  const int m1 = nmat + 1, n = nbnd * m1 * m1;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+    table[t] = face_value(mats, nmat, forms[t / (m1 * m1) * 3 + axis], t / m1 % m1, t % m1);
+}
+
 // One thread per face of `axis`.  The two voxels that meet at a face are lo (index - 1 along the axis) and hi.
 // A face only matters to the compute voxels beside it; the reference evaluates its flux from a compute
 // voxel's equation with the neighbour's k replaced by the voxel's own when the neighbour is fixed or outside
 // the grid (crank_nicolson.pyx:298-338), so both compute sides see the same k pair and one value per face
-// serves both.
+// serves both.  table: face_values_kernel's, or null when there are too many classes and materials for one (each face's
+// forms evaluated in its own thread take 20 times as long: 6.5 ms against 0.3 ms per axis at 65x512x512).
 __global__ void faces_kernel(Dims d, int axis, const uint8_t* __restrict__ material,
                              const uint8_t* __restrict__ bclass, const hs2g_material* __restrict__ mats, int nmat,
-                             const hs2g_face_form* __restrict__ forms, int nbnd, double* __restrict__ G,
-                             unsigned long long* err) {
+                             const hs2g_face_form* __restrict__ forms, int nbnd, const FaceValue* __restrict__ table,
+                             double* __restrict__ G, unsigned long long* err) {
   const int64_t fz = d.nz + (axis == 0), fy = d.ny + (axis == 1), fx = d.nx + (axis == 2);
   const int64_t nfaces = fz * fy * fx;
+  const int64_t n_axis = axis == 0 ? d.nz : (axis == 1 ? d.ny : d.nx);
+  const int64_t back = axis == 0 ? d.nxy() : (axis == 1 ? d.nx : 1);  // from a face's hi voxel to its lo voxel
   for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < nfaces;
        f += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = f % fx;
-    const int64_t j = (f / fx) % fy;
-    const int64_t k = f / (fx * fy);
+    const int64_t row = f / fx, i = f - row * fx, k = row / fy, j = row - k * fy;
     const int64_t c = axis == 0 ? k : (axis == 1 ? j : i);
-    const int64_t n_axis = axis == 0 ? d.nz : (axis == 1 ? d.ny : d.nx);
-    const bool lo_in = c > 0, hi_in = c < n_axis;
-    // the hi voxel has the face's coordinates, the lo voxel is one step back along the axis
-    const int64_t phi = hi_in ? (k * d.ny + j) * d.nx + i : -1;
-    const int64_t plo =
-        lo_in ? ((k - (axis == 0)) * d.ny + (j - (axis == 1))) * d.nx + (i - (axis == 2)) : -1;
-    int mlo = -1, mhi = -1;
-    if (lo_in) mlo = material[plo];
-    if (hi_in) mhi = material[phi];
-    if ((lo_in && mlo >= nmat) || (hi_in && mhi >= nmat)) {
+    const int64_t p = (k * d.ny + j) * d.nx + i;  // the hi voxel's place
+    int mlo = nmat, mhi = nmat;
+    if (c > 0) mlo = material[p - back];
+    if (c < n_axis) mhi = material[p];
+    if ((c > 0 && mlo >= nmat) || (c < n_axis && mhi >= nmat)) {
       record_error(err, HS2G_ERR_ARG, axis, f);
-      G[f] = 0.0;
-      continue;
-    }
-    const bool lo_c = lo_in && mats[mlo].kind == HS2G_TEMPERATURE_COMPUTE;
-    const bool hi_c = hi_in && mats[mhi].kind == HS2G_TEMPERATURE_COMPUTE;
-    if (!lo_c && !hi_c) {
       G[f] = 0.0;
       continue;
     }
     const int b = bclass[f];
     if (b >= nbnd) {
-      record_error(err, HS2G_ERR_ARG, axis, f);
+      // no class of the table: an error unless the face lies between voxels that are not computed
+      if ((mlo < nmat && mats[mlo].kind == HS2G_TEMPERATURE_COMPUTE) ||
+          (mhi < nmat && mats[mhi].kind == HS2G_TEMPERATURE_COMPUTE))
+        record_error(err, HS2G_ERR_ARG, axis, f);
       G[f] = 0.0;
       continue;
     }
-    const double* klo = lo_c ? mats[mlo].k : mats[mhi].k;
-    const double* khi = hi_c ? mats[mhi].k : mats[mlo].k;
-    const hs2g_face_form& form = forms[b * 3 + axis];
-    const double g = eval_form(form.normal, klo, khi);
-    if (!(g == g) || isinf(g)) {
-      record_error(err, HS2G_ERR_KTYPE, axis, f);
-      G[f] = 0.0;
-      continue;
-    }
-    const double tol = 1e-12 * fabs(g);
-    for (int z = 0; z < form.nzero; ++z) {
-      const double v = eval_form(form.zero[z], klo, khi);
-      if (!(fabs(v) <= tol)) record_error(err, form.zero_code[z], axis, f);
-    }
-    if ((!lo_in || !hi_in) && g != 0.0) record_error(err, HS2G_ERR_EXTERIOR, axis, f);
-    G[f] = g;
+    const FaceValue v = table ? table[(b * (nmat + 1) + mlo) * (nmat + 1) + mhi]
+                              : face_value(mats, nmat, forms[b * 3 + axis], mlo, mhi);
+    if (v.code) record_error(err, v.code, axis, f);
+    G[f] = v.g;
   }
 }
 
@@ -212,8 +228,8 @@ __global__ void factor_z_kernel(Dims d, F g, const double* __restrict__ M, const
     const RowIn r = row(k);
     const double piv = r.d - u * r.lo;
     u = r.hi / piv;
-    a2[at2(k)] = r.lo / piv;
-    b2[at2(k)] = u;
+    a2[at2(k)] = -(r.lo / piv);
+    b2[at2(k)] = -(u);
     s2[p] = M[p] / piv;
   };
   auto down = [&](int64_t k) {
@@ -221,8 +237,8 @@ __global__ void factor_z_kernel(Dims d, F g, const double* __restrict__ M, const
     const RowIn r = row(k);
     const double piv = r.d - v * r.hi;
     v = r.lo / piv;
-    a2[at2(k)] = r.hi / piv;
-    b2[at2(k)] = v;
+    a2[at2(k)] = -(r.hi / piv);
+    b2[at2(k)] = -(v);
     s2[p] = M[p] / piv;
   };
   for (int64_t e = 0; e < m; ++e) {
@@ -232,8 +248,8 @@ __global__ void factor_z_kernel(Dims d, F g, const double* __restrict__ M, const
   const int64_t p = m * d.nxy() + t;
   const RowIn r = row(m);
   const double piv = r.d - u * r.lo - v * r.hi;
-  a2[at2(m)] = r.lo / piv;
-  b2[at2(m)] = r.hi / piv;
+  a2[at2(m)] = -(r.lo / piv);
+  b2[at2(m)] = -(r.hi / piv);
   s2[p] = M[p] / piv;
 }
 
@@ -263,8 +279,8 @@ __global__ void factor_y_kernel(Dims d, F g, const double* __restrict__ M, const
     const double piv = r.d - u * r.lo;
     u = r.hi / piv;
     sigma[at(j)] = s2[at(j)] * M[at(j)] / piv;
-    a1[pp] = lower(j, r.lo, piv);
-    b1[pp] = upper(j, u, 1.0);
+    a1[pp] = -(lower(j, r.lo, piv));
+    b1[pp] = -(upper(j, u, 1.0));
   };
   auto down = [&](int64_t j) {
     const int64_t pp = (k * d.ny + j) * px + i;
@@ -272,8 +288,8 @@ __global__ void factor_y_kernel(Dims d, F g, const double* __restrict__ M, const
     const double piv = r.d - v * r.hi;
     v = r.lo / piv;
     sigma[at(j)] = s2[at(j)] * M[at(j)] / piv;
-    a1[pp] = upper(j, r.hi, piv);
-    b1[pp] = lower(j, v, 1.0);
+    a1[pp] = -(upper(j, r.hi, piv));
+    b1[pp] = -(lower(j, v, 1.0));
   };
   for (int64_t e = 0; e < m; ++e) {
     up(e);
@@ -283,46 +299,261 @@ __global__ void factor_y_kernel(Dims d, F g, const double* __restrict__ M, const
   const RowIn r = row(m);
   const double piv = r.d - u * r.lo - v * r.hi;
   sigma[at(m)] = s2[at(m)] * M[at(m)] / piv;
-  a1[pp] = lower(m, r.lo, piv);
-  b1[pp] = upper(m, r.hi, piv);
+  a1[pp] = -(lower(m, r.lo, piv));
+  b1[pp] = -(upper(m, r.hi, piv));
 }
 
-// x lines (one thread per (k,j)): stage-0 stencil, forward and back coefficients.
+// x lines (one thread per (k,j)): the coefficients a0, b0 and the row scale f0 = sigma/piv of the stage-0 right-hand
+// side; two-ended about column x_mid, or one way (m the last column).
 template <class F>
 __global__ void factor_x_kernel(Dims d, F g, const double* __restrict__ M, const uint8_t* __restrict__ compute,
-                                const double* __restrict__ sigma, Coeffs c) {
+                                const double* __restrict__ sigma, double* __restrict__ f0, double* __restrict__ a0,
+                                double* __restrict__ b0, int64_t px, bool two_ended) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= d.nz * d.ny) return;
   const int64_t k = t / d.ny, j = t - k * d.ny;
-  double u_prev = 0.0, sg_prev = 1.0;
-  for (int64_t i = 0; i < d.nx; ++i) {
+  const int64_t m = two_ended ? x_mid(d.nx) : d.nx - 1;
+  const double* sg = sigma + t * d.nx;
+  auto row = [&](int64_t i) {
     const int64_t p = t * d.nx + i;
     const bool comp = compute[p] != 0;
-    const double gxl = comp ? g.xlo(d, p, k, j, i) : 0.0, gxh = comp ? g.xhi(d, p, k, j, i) : 0.0;
-    const double gyl = comp ? g.ylo(d, p, k, j, i) : 0.0, gyh = comp ? g.yhi(d, p, k, j, i) : 0.0;
-    const double gzl = comp ? g.zlo(d, p, k, j, i) : 0.0, gzh = comp ? g.zhi(d, p, k, j, i) : 0.0;
-    const RowIn r = stage_row(comp, M[p], gxl, gxh);
-    const double piv = r.d - u_prev * r.lo;
-    const double u = r.hi / piv;
-    const double sg = sigma[p];
-    const double f0 = sg / piv;
-    const double center = -(((gxl + gxh) + (gyl + gyh)) + (gzl + gzh));
-    double* blk = c.xb + ((t * c.nchunks + i / 32) * kXBlockCoeffs) * 32 + (i % 32);
-    blk[kWc * 32] = f0 * center;
-    blk[kWxl * 32] = f0 * gxl;
-    blk[kWxh * 32] = f0 * gxh;
-    blk[kWyl * 32] = f0 * gyl;
-    blk[kWyh * 32] = f0 * gyh;
-    blk[kWzl * 32] = f0 * gzl;
-    blk[kWzh * 32] = f0 * gzh;
-    blk[kWq * 32] = comp ? f0 : 0.0;
-    const double a0 = (i > 0) ? sg * r.lo / (piv * sg_prev) : 0.0;
-    const double b0 = (i + 1 < d.nx) ? sg * u / sigma[p + 1] : 0.0;
-    c.a0[p] = a0;
-    c.b0[p] = b0;
-    u_prev = u;
-    sg_prev = sg;
+    return stage_row(comp, M[p], comp ? g.xlo(d, p, k, j, i) : 0.0, comp ? g.xhi(d, p, k, j, i) : 0.0);
+  };
+  // W0 carries the scale sigma (see factor_y_kernel)
+  auto lower = [&](int64_t i, double f, double q) { return i > 0 ? sg[i] * f / (q * sg[i - 1]) : 0.0; };
+  auto upper = [&](int64_t i, double f, double q) { return i + 1 < d.nx ? sg[i] * f / (q * sg[i + 1]) : 0.0; };
+  double u = 0.0, v = 0.0;
+  auto up = [&](int64_t i) {
+    const RowIn r = row(i);
+    const double piv = r.d - u * r.lo;
+    u = r.hi / piv;
+    f0[t * d.nx + i] = sg[i] / piv;
+    a0[t * px + i] = -(lower(i, r.lo, piv));
+    b0[t * px + i] = -(upper(i, u, 1.0));
+  };
+  auto down = [&](int64_t i) {
+    const RowIn r = row(i);
+    const double piv = r.d - v * r.hi;
+    v = r.lo / piv;
+    f0[t * d.nx + i] = sg[i] / piv;
+    a0[t * px + i] = -(upper(i, r.hi, piv));
+    b0[t * px + i] = -(lower(i, v, 1.0));
+  };
+  for (int64_t e = 0; e < max(m, d.nx - 1 - m); ++e) {
+    if (e < m) up(e);
+    if (d.nx - 1 - e > m) down(d.nx - 1 - e);
   }
+  const RowIn r = row(m);
+  const double piv = r.d - u * r.lo - v * r.hi;
+  f0[t * d.nx + m] = sg[m] / piv;
+  a0[t * px + m] = -(lower(m, r.lo, piv));
+  b0[t * px + m] = -(upper(m, r.hi, piv));
+}
+
+// The eight stage-0 coefficients of column i of x-line t (zeros past the line's end).
+template <class F>
+__device__ __forceinline__ void block_values(const Dims& d, const F& g, const uint8_t* __restrict__ compute,
+                                             const double* __restrict__ f0, int64_t t, int64_t i, double (&v)[8]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = 0.0;
+  const int64_t k = t / d.ny, j = t - k * d.ny, p = t * d.nx + i;
+  if (i >= d.nx || !compute[p]) return;
+  const double gxl = g.xlo(d, p, k, j, i), gxh = g.xhi(d, p, k, j, i);
+  const double gyl = g.ylo(d, p, k, j, i), gyh = g.yhi(d, p, k, j, i);
+  const double gzl = g.zlo(d, p, k, j, i), gzh = g.zhi(d, p, k, j, i);
+  const double f = f0[p];
+  v[0] = f * -(((gxl + gxh) + (gyl + gyh)) + (gzl + gzh));
+  v[1] = f * gxl;
+  v[2] = f * gxh;
+  v[3] = f * gyl;
+  v[4] = f * gyh;
+  v[5] = f * gzl;
+  v[6] = f * gzh;
+  v[7] = f;
+}
+// which of the voxel's faces are on the grid's exterior (bit f, in the weights' order); 0 past the line's end
+__device__ __forceinline__ int exterior_faces(const Dims& d, int64_t t, int64_t i) {
+  if (i >= d.nx) return 0;
+  const int64_t k = t / d.ny, j = t - k * d.ny;
+  return (i == 0) | (i + 1 == d.nx) << 1 | (j == 0) << 2 | (j + 1 == d.ny) << 3 | (k == 0) << 4 | (k + 1 == d.nz) << 5;
+}
+// writes a block (one warp); true when two products do for each of its voxels (kXTwoWeights)
+template <typename R>
+__device__ __forceinline__ bool store_block(R* blk, int lane, const double (&v)[8], int exterior) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) blk[c * 32 + lane] = (R)v[c];
+  bool two = false;
+  if constexpr (sizeof(R) == 8) {
+    double w[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) w[f] = exterior >> f & 1 ? (exterior >> (f ^ 1) & 1 ? 0.0 : v[1 + (f ^ 1)]) : v[1 + f];
+    if ((exterior & 3) == 3) w[0] = w[1] = w[3];  // one column: the x weights may be the y weights too, and y's x's
+    if ((exterior & 12) == 12) w[2] = w[3] = w[1];
+    two = __all_sync(0xffffffffu, w[0] == w[1] && w[0] == w[2] && w[0] == w[3] && w[4] == w[5]);
+    uint2 wi[6];
+    const int e4 = x_int_weights(w, wi);
+    uint2* iw = reinterpret_cast<uint2*>(blk + 8 * 32) + lane;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) iw[f * 32] = wi[f];
+    reinterpret_cast<int*>(blk + 14 * 32)[lane] = e4;
+  }
+  return two;
+}
+
+// Distinct blocks (one warp per block): hashed into an open-addressing table, numbered, written once each, and every
+// block compared with the one it is replaced by (bit for bit; a clash of hashes clears *same).
+template <class F>
+__global__ void hash_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
+                                   int64_t nchunks, unsigned long long* keys, int* owner, int64_t mask, int* slot) {
+  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (b >= d.nz * d.ny * nchunks) return;
+  double v[8];
+  block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + lane, v);
+  unsigned long long h = (unsigned long long)lane * 0xD6E8FEB86659FD93ull + 1 +
+                         ((unsigned long long)exterior_faces(d, b / nchunks, (b % nchunks) * 32 + lane) << 40);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    h = (h ^ (unsigned long long)__double_as_longlong(v[c])) * 0x9E3779B97F4A7C15ull;
+    h ^= h >> 29;
+  }
+  for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+  if (lane) return;
+  h = (h ^ (h >> 32)) * 0x9E3779B97F4A7C15ull;
+  if (h == 0) h = 1;
+  int64_t e = (int64_t)(h >> 17) & mask;
+  for (;; e = (e + 1) & mask) {  // the table has twice as many entries as there are blocks
+    const unsigned long long k = atomicCAS(keys + e, 0ull, h);
+    if (k == 0ull || k == h) break;
+  }
+  slot[b] = (int)e;
+  atomicMin(owner + e, (int)b);
+}
+__global__ void number_blocks_kernel(int64_t blocks, const int* owner, const int* slot, int* id, int* count) {
+  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (b < blocks && owner[slot[b]] == (int)b) id[slot[b]] = atomicAdd(count, 1);
+}
+// writes the owners' blocks (slot null: every block at its own place)
+template <typename R, class F>
+__global__ void write_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
+                                    int64_t nchunks, const int* owner, const int* slot, int* id, R* pool) {
+  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (b >= d.nz * d.ny * nchunks) return;
+  if (slot && owner[slot[b]] != (int)b) return;
+  double v[8];
+  block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31), v);
+  const int64_t at = slot ? (int64_t)id[slot[b]] : b;
+  const bool two = store_block(pool + at * x_block_elems<R>(), threadIdx.x & 31, v,
+                               exterior_faces(d, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31)));
+  __syncwarp();
+  if (two && slot && (threadIdx.x & 31) == 0) id[slot[b]] = (int)at | kXTwoWeights;
+}
+template <class F>
+__global__ void index_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
+                                    int64_t nchunks, const int* owner, const int* slot, const int* id, int32_t* bidx,
+                                    int* same) {
+  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (b >= d.nz * d.ny * nchunks) return;
+  const int64_t o = owner[slot[b]];
+  double v[8], w[8];
+  block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + lane, v);
+  block_values(d, g, compute, f0, o / nchunks, (o % nchunks) * 32 + lane, w);
+  bool eq = exterior_faces(d, b / nchunks, (b % nchunks) * 32 + lane) == exterior_faces(d, o / nchunks, (o % nchunks) * 32 + lane);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) eq &= __double_as_longlong(v[c]) == __double_as_longlong(w[c]);
+  if (!eq) *same = 0;
+  if (lane == 0) bidx[b] = id[slot[b]];
+}
+
+inline int64_t block_count(const Dims& d) { return d.nz * d.ny * ((d.nx + 31) / 32); }
+// things are numbered in 32 bits, and the index keeps a bit for kXTwoWeights
+inline bool blocks_countable(const Dims& d) { return block_count(d) < ((int64_t)1 << 29); }
+
+template <typename R, class F>
+cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const double* f0, const Coeffs& c, bool two_ended,
+                          unsigned char* scratch, Compressed* out, cudaStream_t s) {
+  const int64_t nch = (d.nx + 31) / 32, blocks = block_count(d);
+  const unsigned wgrid = (unsigned)((blocks + 7) / 8), tgrid = (unsigned)((blocks + 255) / 256);
+  const size_t bytes = sizeof(R) * x_block_elems<R>();
+  LineJob job[3];
+  job[0].grid = {c.a0, c.b0, d.nz * d.ny, 1, c.px, d.nx, 1};
+  job[0].mid = two_ended ? x_mid(d.nx) : -1;
+  job[1].grid = {c.a1, c.b1, d.nz, d.nx, d.ny * c.px, d.ny, c.px};
+  job[2].grid = {c.a2, c.b2, d.ny, d.nx, c.px, d.nz, d.ny * c.px};
+  // all four searches are queued, then their counts read at once, and the checks' outcomes likewise
+  unsigned char* at = scratch;
+  bool on[4] = {};
+  int host[4][2] = {};
+  cudaError_t e = cudaSuccess;
+  for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
+    const int64_t lines = job[a].grid.lines();
+    if (lines >= ((int64_t)1 << 29)) continue;
+    on[a] = true;
+    e = job[a].begin(at, s);
+    at += (LineJob::scratch_bytes(lines) + 255) & ~size_t(255);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(host[a], job[a].table.count, sizeof(int), cudaMemcpyDeviceToHost, s);
+  }
+  ClassTable t(blocks_countable(d) ? blocks : 0);
+  if (e == cudaSuccess && blocks_countable(d)) {
+    on[3] = true;
+    t.place(at);
+    e = t.clear(s);
+    if (e == cudaSuccess) {
+      hash_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.keys, t.owner, t.cap - 1, t.slot);
+      number_blocks_kernel<<<tgrid, 256, 0, s>>>(blocks, t.owner, t.slot, t.id, t.count);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host[3], t.count, sizeof(int), cudaMemcpyDeviceToHost, s);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  for (int a = 0; a < 3 && e == cudaSuccess; ++a)
+    if (on[a]) {
+      e = job[a].finish(host[a][0], &out->lines[a], s);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(host[a] + 1, job[a].table.count + 1, sizeof(int), cudaMemcpyDeviceToHost, s);
+    }
+  // An index is worth it when at most a quarter of the blocks are distinct: the sweep then reads them from L2, and the
+  // index costs it a dependent load
+  XBlocks& x = out->blocks;
+  const size_t index = sizeof(int32_t) * (size_t)blocks;
+  bool shared = on[3] && host[3][0] <= std::max<int64_t>(1, blocks / 4);
+  if (e == cudaSuccess && shared) {
+    x.count = host[3][0];
+    x.bytes = bytes * x.count + index;
+    e = cudaMalloc(&x.pool, x.bytes);
+    if (e == cudaSuccess) {
+      x.bidx = reinterpret_cast<int32_t*>((unsigned char*)x.pool + bytes * x.count);
+      write_blocks_kernel<R><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, (R*)x.pool);
+      index_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, x.bidx, t.count + 1);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host[3] + 1, t.count + 1, sizeof(int), cudaMemcpyDeviceToHost, s);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  for (int a = 0; a < 3 && e == cudaSuccess; ++a)
+    if (out->lines[a].cls && !host[a][1]) {
+      cudaFree(out->lines[a].a);
+      out->lines[a] = LineTables{};
+    }
+  if (e == cudaSuccess && shared && !host[3][1]) {
+    cudaFree(x.pool);
+    x = XBlocks{};
+    shared = false;
+  }
+  if (e == cudaSuccess && !shared) {  // every block for itself
+    x.count = blocks;
+    x.bytes = bytes * blocks;
+    e = cudaMalloc(&x.pool, x.bytes);
+    if (e == cudaSuccess) {
+      write_blocks_kernel<R><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, nullptr, nullptr, nullptr, (R*)x.pool);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
+  if (e != cudaSuccess) out->release();
+  return e;
 }
 
 // per-row problem: capacities positive and finite, coefficients finite, exterior sides zero on computed
@@ -355,12 +586,21 @@ inline unsigned grid_for(int64_t n, int threads) {
 
 }  // namespace
 
+size_t face_table_bytes(int nmat, int nbnd) {
+  const int64_t entries = (int64_t)nbnd * (nmat + 1) * (nmat + 1);
+  return entries <= 65536 ? sizeof(FaceValue) * (size_t)entries : 0;
+}
+
 cudaError_t launch_faces(const Dims& d, int axis, const uint8_t* material, const uint8_t* bclass,
                          const hs2g_material* mats, int nmat, const hs2g_face_form* forms, int nbnd, double* G,
-                         unsigned long long* err, cudaStream_t s) {
+                         unsigned long long* err, void* table, cudaStream_t s) {
   const int64_t nfaces = (d.nz + (axis == 0)) * (d.ny + (axis == 1)) * (d.nx + (axis == 2));
+  FaceValue* values = face_table_bytes(nmat, nbnd) ? static_cast<FaceValue*>(table) : nullptr;
+  if (values)
+    face_values_kernel<<<grid_for((int64_t)nbnd * (nmat + 1) * (nmat + 1), 64), 64, 0, s>>>(axis, mats, nmat, forms, nbnd,
+                                                                                         values);
   faces_kernel<<<grid_for(nfaces, kThreads), kThreads, 0, s>>>(d, axis, material, bclass, mats, nmat, forms, nbnd,
-                                                               G, err);
+                                                               values, G, err);
   return cudaGetLastError();
 }
 
@@ -384,20 +624,40 @@ cudaError_t launch_factor_with(const Dims& d, F g, const double* M, const uint8_
   factor_z_kernel<F><<<grid_for(d.nxy(), th), th, 0, s>>>(d, g, M, compute, s2, c.a2, c.b2, c.px, two_ended);
   factor_y_kernel<F><<<grid_for(d.nz * d.nx, th), th, 0, s>>>(d, g, M, compute, s2, sigma, c.a1, c.b1,
                                                                 c.px, two_ended);
-  factor_x_kernel<F><<<grid_for(d.nz * d.ny, th), th, 0, s>>>(d, g, M, compute, sigma, c);
+  factor_x_kernel<F><<<grid_for(d.nz * d.ny, th), th, 0, s>>>(d, g, M, compute, sigma, s2, c.a0, c.b0, c.px, two_ended);
   return cudaGetLastError();
 }
 
-cudaError_t launch_factor(const Dims& d, const double* Gz, const double* Gy, const double* Gx, const double* M,
-                          const uint8_t* compute, double* s2, double* sigma, const Coeffs& c, cudaStream_t s,
-                          bool two_ended) {
-  return launch_factor_with(d, SharedFaces{Gz, Gy, Gx}, M, compute, s2, sigma, c, s, two_ended);
+cudaError_t launch_factor(const Dims& d, const Faces& f, const double* M, const uint8_t* compute, double* s2,
+                          double* sigma, const Coeffs& c, cudaStream_t s, bool two_ended) {
+  if (f.rows[0])
+    return launch_factor_with(d, RowFaces{f.rows[0], f.rows[1], f.rows[2], f.rows[3], f.rows[4], f.rows[5]}, M, compute,
+                              s2, sigma, c, s, two_ended);
+  return launch_factor_with(d, SharedFaces{f.Gz, f.Gy, f.Gx}, M, compute, s2, sigma, c, s, two_ended);
 }
 
-cudaError_t launch_factor_rows(const Dims& d, const double* const rows[6], const double* M, const uint8_t* compute,
-                               double* s2, double* sigma, const Coeffs& c, cudaStream_t s) {
-  const RowFaces g{rows[0], rows[1], rows[2], rows[3], rows[4], rows[5]};
-  return launch_factor_with(d, g, M, compute, s2, sigma, c, s, true);
+void Compressed::release() {
+  cudaFree(blocks.pool);
+  for (LineTables& t : lines) cudaFree(t.a);
+  *this = Compressed{};
+}
+
+size_t compress_scratch(const Dims& d) {
+  size_t n = 256 + (blocks_countable(d) ? ClassTable(block_count(d)).bytes() : 0);
+  for (int64_t lines : {d.nz * d.ny, d.nz * d.nx, d.nxy()})
+    if (lines < ((int64_t)1 << 29)) n += (LineJob::scratch_bytes(lines) + 255) & ~size_t(255);
+  return n;
+}
+
+cudaError_t compress_coeffs(const Dims& d, const Faces& f, const uint8_t* compute, const double* f0, const Coeffs& c,
+                            int precision, unsigned char* scratch, Compressed* out, cudaStream_t s) {
+  *out = Compressed{};
+  if (f.rows[0])
+    return compress_with<double>(d, RowFaces{f.rows[0], f.rows[1], f.rows[2], f.rows[3], f.rows[4], f.rows[5]}, compute,
+                                 f0, c, true, scratch, out, s);
+  const SharedFaces g{f.Gz, f.Gy, f.Gx};
+  return precision == 64 ? compress_with<double>(d, g, compute, f0, c, true, scratch, out, s)
+                         : compress_with<float>(d, g, compute, f0, c, false, scratch, out, s);
 }
 
 cudaError_t launch_validate_rows(const Dims& d, const double* const rows[6], double* M, uint8_t* compute,

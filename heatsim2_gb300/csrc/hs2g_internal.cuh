@@ -14,46 +14,108 @@ struct Dims {
   __host__ __device__ int64_t nxy() const { return ny * nx; }
 };
 
+constexpr int kXBlockDoubles = (8 + 6) * 32 + 16;  // an FP64 stencil block (hs2g_x.cuh)
+
+// middle column of the two-ended x elimination
+__host__ __device__ inline int64_t x_mid(int64_t nx) { return (nx - 1) / 2; }
+
 // Per-voxel coefficients of the scaled delta-form Douglas step.
-//   stage 0 (x lines):  z_i = wc*T + wxl*T[i-1] + wxh*T[i+1] + wyl*T[j-1] + wyh*T[j+1] + wzl*T[k-1]
-//                             + wzh*T[k+1] + wq*Q - a0*z_{i-1};   W0_i = z_i - b0*W0_{i+1}
-//   stage 1 (y lines):  the same recurrences with a1, b1 from W0 to W1, from both ends towards the middle row
-//   stage 2 (z lines):  the same with a2, b2 from W1 to dT;  T' = T + dT            (hs2g_pair.cuh)
-// The eight stage-0 stencil coefficients are chunk-blocked: for x-line L = k*ny + j and 32-column chunk ch,
-// block (L*nchunks + ch) holds [wc, wxl, wxh, wyl, wyh, wzl, wzh, wq] x 32 columns (2 KB, zero-padded past
-// nx), so a warp's stencil reads one contiguous stream instead of eight.  The other coefficients are
-// (nz, ny, nx) arrays in voxel order, a1 and b1 (and the stage buffers W0, W1) with row pitch px.
-constexpr int kXBlockCoeffs = 8;
-enum XCoeff { kWc = 0, kWxl, kWxh, kWyl, kWyh, kWzl, kWzh, kWq };
+//   stage 0 (x lines):  right-hand side wc*T + wxl*T[i-1] + wxh*T[i+1] + wyl*T[j-1] + wyh*T[j+1] + wzl*T[k-1]
+//                       + wzh*T[k+1] + wq*Q, the line recurrences with a0, b0 to W0          (hs2g_x.cuh)
+//   stage 1 (y lines):  the recurrences with a1, b1 from W0 to W1                            (hs2g_pair.cuh)
+//   stage 2 (z lines):  the same with a2, b2 from W1 to dT;  T' = T + dT
+// In FP64 every line is eliminated from both ends towards a middle row; the FP32 batch goes one way.  The line
+// coefficients are stored negated, as the recurrences' multiply-adds take them.
+// The stage-0 stencil coefficients come in blocks of 32 columns of an x-line (x-line L = k*ny + j, chunk ch), so that
+// a warp reads one contiguous stream; equal blocks are kept once (bidx[L*nchunks + ch], null when there are too many
+// distinct ones).  Lines whose coefficients are equal bit for bit share a table (cls0 per x-line, cls1 per y line
+// (k, i) at k*nx + i, cls2 per z line (j, i) at j*nx + i); a null class array: values in voxel order with row pitch px.
 struct Coeffs {
-  double* xb;   // stage-0 stencil blocks, nz*ny*nchunks*8*32 doubles
+  double* xb;
+  int32_t* bidx;
   int64_t nchunks;
-  // Row pitch of the arrays the y and z sweeps copy 16 bytes at a time (W0, W1, a1, b1, a2, b2): nx, or nx rounded
+  // Row pitch of the arrays the line solves copy 16 bytes at a time (W0, W1 and the line coefficients): nx, or nx rounded
   // up so that the rows start on 16-byte boundaries (an odd nx gets one pad column).  All other arrays have pitch nx.
   int64_t px;
   double* a0;
   double* b0;
-  // y and z lines: arrays in voxel order (row pitch px), or with cls1 / cls2 tables of a line's rows per class
-  // (classify_lines), the class of y line (k, i) at cls1[k*nx + i] and of z line (j, i) at cls2[j*nx + i]
   double* a1;
   double* b1;
   double* a2;
   double* b2;
+  int32_t* cls0;
   int32_t* cls1;
   int32_t* cls2;
 };
 
 // The distinct lines of an axis: a[c*n + r], b[c*n + r] per class and row, cls[line]; cls is null when there are too
-// many.  Device memory owned by the caller.
+// many.  One device allocation, at a, owned by the caller.
 struct LineTables {
   double* a = nullptr;
   double* b = nullptr;
   int32_t* cls = nullptr;
   int64_t nclass = 0;
+  size_t bytes = 0;
 };
-// lines (o, i), i fastest, with row r at o*ost + r*rst + i of a and b (hs2g_classes.cu); waits for the stream
-cudaError_t classify_lines(const double* a, const double* b, int64_t outer, int64_t nx, int64_t ost, int64_t n,
-                           int64_t rst, LineTables* out, cudaStream_t s);
+// Stencil blocks of a problem: the distinct ones with an index per (line, chunk), or all of them (bidx null).  Device
+// memory owned by the caller.
+struct XBlocks {
+  void* pool = nullptr;
+  int32_t* bidx = nullptr;
+  int64_t count = 0;
+  size_t bytes = 0;
+};
+
+// An open-addressing table over n things, by 64-bit hash: keys, the smallest thing of each key, the number it gets,
+// each thing's slot, and {count of numbers, 1 while no two different things were found under one key}.
+struct ClassTable {
+  int64_t n = 0, cap = 64;
+  unsigned long long* keys = nullptr;
+  int *owner = nullptr, *id = nullptr, *slot = nullptr, *count = nullptr;
+  explicit ClassTable(int64_t things = 0) : n(things) {
+    while (cap < 2 * n) cap *= 2;
+  }
+  size_t bytes() const { return sizeof(*keys) * (size_t)cap + sizeof(int) * (size_t)(2 * cap + n + 2); }
+  unsigned char* place(unsigned char* at) {  // returns what follows it
+    keys = reinterpret_cast<unsigned long long*>(at);
+    owner = reinterpret_cast<int*>(keys + cap);
+    id = owner + cap;
+    slot = id + cap;
+    count = slot + n;
+    return reinterpret_cast<unsigned char*>(count + 2);
+  }
+  cudaError_t clear(cudaStream_t s) {
+    static const int start[2] = {0, 1};
+    cudaError_t e = cudaMemsetAsync(keys, 0, sizeof(*keys) * cap, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(owner, 0x7f, sizeof(int) * cap, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(count, start, sizeof start, cudaMemcpyHostToDevice, s);
+    return e;
+  }
+};
+
+// lines (o, i), i fastest, with row r at o*ost + r*rst + i of a and b
+struct LineGrid {
+  const double* a;
+  const double* b;
+  int64_t outer, nx, ost, n, rst;
+  __host__ __device__ int64_t lines() const { return outer * nx; }
+  __device__ int64_t base(int64_t l) const { return (l / nx) * ost + l % nx; }
+};
+// Finding the line classes of an axis (hs2g_classes.cu): begin queues the hashing and numbering, the caller reads
+// table.count[0] (and waits), finish queues the tables and the check that clears table.count[1] on a clash of hashes.
+// mid >= 0: the rows above mid are tabulated last first (row r at position mid + n - r).
+struct LineJob {
+  LineGrid grid{};
+  int64_t mid = -1;
+  ClassTable table;
+  int* rep = nullptr;
+  // Worth it when the tables are an eighth of the arrays: the classes of a warp's 16 lines then cost it no more than
+  // reading the arrays would
+  static int64_t max_class(int64_t lines) { return lines / 8 > 1 ? lines / 8 : 1; }
+  static size_t scratch_bytes(int64_t lines);
+  cudaError_t begin(unsigned char* scratch, cudaStream_t s);
+  cudaError_t finish(int64_t nclass, LineTables* out, cudaStream_t s);
+};
 
 struct QTable {
   double q[HS2G_MAX_CLASSES];
@@ -134,20 +196,36 @@ __device__ __forceinline__ void record_error(unsigned long long* err, int code, 
 // setup kernels (hs2g_compile.cu)
 cudaError_t launch_faces(const Dims& d, int axis, const uint8_t* material, const uint8_t* bclass,
                          const hs2g_material* mats, int nmat, const hs2g_face_form* forms, int nbnd, double* G,
-                         unsigned long long* err, cudaStream_t s);
+                         unsigned long long* err, void* table, cudaStream_t s);
+size_t face_table_bytes(int nmat, int nbnd);  // of launch_faces's table; 0: it takes none
 cudaError_t launch_capacity_from_classes(const Dims& d, const uint8_t* material, const hs2g_material* mats,
                                          int nmat, double* M, uint8_t* compute, unsigned long long* err,
                                          cudaStream_t s);
 cudaError_t launch_validate_dense(const Dims& d, const double* Gz, const double* Gy, const double* Gx,
                                   double* M, uint8_t* compute, unsigned long long* err, cudaStream_t s);
-cudaError_t launch_factor(const Dims& d, const double* Gz, const double* Gy, const double* Gx, const double* M,
-                          const uint8_t* compute, double* s2, double* sigma, const Coeffs& c, cudaStream_t s,
-                          bool two_ended = true);
-// per-row problems: rows = {z lo, z hi, y lo, y hi, x lo, x hi}, each (nz, ny, nx)
+// The face conductances a problem is factorised from: one array per axis indexed by face, or (rows[0] set) per-row
+// conductances {z lo, z hi, y lo, y hi, x lo, x hi}, each (nz, ny, nx).
+struct Faces {
+  const double *Gz = nullptr, *Gy = nullptr, *Gx = nullptr;
+  const double* rows[6] = {};
+};
+// The line factors into c (row pitch c.px), in FP64 from both ends; s2 and sigma are scratch, s2 holds the stage-0 row
+// scale f0 afterwards.
+cudaError_t launch_factor(const Dims& d, const Faces& f, const double* M, const uint8_t* compute, double* s2,
+                          double* sigma, const Coeffs& c, cudaStream_t s, bool two_ended);
+// What the step keeps of the factors (hs2g_compile.cu): the stencil blocks, and the x, y and z line tables where the
+// lines have few classes (lines[a].cls null: c's arrays stay).  scratch: compress_scratch(d) bytes.  Waits for the
+// stream.
+struct Compressed {
+  XBlocks blocks;
+  LineTables lines[3];
+  void release();
+};
+size_t compress_scratch(const Dims& d);
+cudaError_t compress_coeffs(const Dims& d, const Faces& f, const uint8_t* compute, const double* f0, const Coeffs& c,
+                            int precision, unsigned char* scratch, Compressed* out, cudaStream_t s);
 cudaError_t launch_validate_rows(const Dims& d, const double* const rows[6], double* M, uint8_t* compute,
                                  unsigned long long* err, cudaStream_t s);
-cudaError_t launch_factor_rows(const Dims& d, const double* const rows[6], const double* M, const uint8_t* compute,
-                               double* s2, double* sigma, const Coeffs& c, cudaStream_t s);
 
 // per-voxel source shapes (hs2g_sources.cu)
 cudaError_t launch_fill(double* p, int64_t n, double v, cudaStream_t s);
@@ -175,8 +253,9 @@ struct StepArgs {
   bool pdl_x;            // the same for the x sweep (not for the first kernel of a graph)
 };
 
-// raise the dynamic shared-memory limits of the sweep kernels on the current device (when a handle is created)
-cudaError_t sweeps_prepare();
+// raise the dynamic shared-memory limits of the sweep kernels that a problem launches, on the current device (when a
+// handle is created)
+cudaError_t sweeps_prepare(const Dims& d, const Coeffs& c);
 cudaError_t launch_step(const StepArgs& a, const Coeffs& c, const QTable& q, cudaStream_t s);
 // the same three kernels with an event recorded before each and after the last (ev[0..3])
 cudaError_t launch_step_events(const StepArgs& a, const Coeffs& c, const QTable& q, cudaStream_t s,
@@ -201,10 +280,10 @@ cudaError_t launch_surface_estimate(int64_t nxy, const double* T, double dz, dou
 // one bounded mbarrier wait on a barrier that receives its arrival (arrive != 0) or none (hs2g_lines.cu)
 cudaError_t wait_selftest(uint64_t limit_ns, int arrive, int* status_dev, cudaStream_t s);
 // the step in pieces, for overlapping host copies with it: the x sweep over x-lines [line_begin, line_end)
-// (line = k*ny + j) with 32, 16 or 8 x-lines per CTA, the whole y sweep, the z sweep over the rows of columns
+// (line = k*ny + j), the whole y sweep, the z sweep over the rows of columns
 // [j_begin, j_end)
 cudaError_t launch_x_range(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t line_begin,
-                           int64_t line_end, int lines_per_cta, cudaStream_t s);
+                           int64_t line_end, cudaStream_t s);
 cudaError_t launch_y(const StepArgs& a, const Coeffs& c, cudaStream_t s);
 cudaError_t launch_z_rows(const StepArgs& a, const Coeffs& c, int64_t j_begin, int64_t j_end, cudaStream_t s);
 

@@ -6,9 +6,9 @@
 //     z_r = W_r - a_r z_{r-1} (r < m),   z_r = W_r - a_r z_{r+1} (r > m),
 //     x_m = W_m - a_m z_{m-1} - b_m z_{m+1},
 //     x_r = z_r - b_r x_{r+1} (r < m),   x_r = z_r - b_r x_{r-1} (r > m),
-// one FMA per row and pass as in a one-way elimination, but two independent chains of half the length.  A
-// dependent FP64 FMA takes 64 cycles here and a warp issues one FP64 instruction per 64 cycles whatever its active
-// lanes, so a warp takes 16 lines: lanes 0-15 their lower ends, lanes 16-31 their upper ends.
+// (the coefficients are stored negated) one FMA per row and pass as in a one-way elimination, but two independent
+// chains of half the length.  A dependent FP64 FMA takes 64 cycles here and a warp issues one FP64 instruction per 64
+// cycles whatever its active lanes, so a warp takes 16 lines: lanes 0-15 their lower ends, lanes 16-31 their upper ends.
 // FP32: 32 lines per warp, eliminated one way (m = n); a float chain is not what bounds the sweep.
 //
 // A warp's lines are neighbours along x in one row of lines, so a row of any array is one contiguous piece.
@@ -237,14 +237,14 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
     if (q < nfull) {
 #pragma unroll
       for (int k = 0; k < RB; ++k) {
-        z = fma(-a[k], z, w[k]);
+        z = fma(a[k], z, w[k]);
         put(k);
       }
     } else {
 #pragma unroll
       for (int k = 0; k < RB; ++k)
         if (k < left) {
-          z = fma(-a[k], z, w[k]);
+          z = fma(a[k], z, w[k]);
           put(k);
         }
     }
@@ -252,12 +252,12 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
   R x = 0;
   if (TWO) {
     const R other = __shfl_xor_sync(0xffffffffu, z, 16);
-    x = fma(-bm, upper ? z : other, fma(-am, upper ? other : z, wm));  // the same value in both halves
+    x = fma(bm, upper ? z : other, fma(am, upper ? other : z, wm));  // the same value in both halves
     if (!upper && live) p.out[m * p.st + mine] = ADD_T ? tm + x : x;
   }
   if (!KEEP) {
     cp_async_wait_pending<0>();
-    __threadfence_block();  // the forward values before the copies that read them back
+    __threadfence();  // the forward values before the copies that read them back from L2
     __syncwarp();
 #pragma unroll 1
     for (int i = nb; i < nb + LA; ++i) issue(i, true);
@@ -287,14 +287,14 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
     if (q < nfull) {
 #pragma unroll
       for (int k = RB - 1; k >= 0; --k) {
-        x = fma(-b[k], x, zz[k]);
+        x = fma(b[k], x, zz[k]);
         put(k);
       }
     } else {
 #pragma unroll
       for (int k = RB - 1; k >= 0; --k)
         if (k < left) {
-          x = fma(-b[k], x, zz[k]);
+          x = fma(b[k], x, zz[k]);
           put(k);
         }
     }

@@ -3,350 +3,115 @@
 // source-field assembly and three permute / CSR mat-vec / tridiagonal-solve stages
 // (alternatingdirection_c_pyx.pyx:294-416, tridiag.pyx:46-69).
 //
-// FP64 is the binding resource on GB300 (about 0.6e12 DFMA/s against ~6.5 TB/s of HBM), so the step is
-// arranged for the fewest FP64 operations: 7 stencil FMAs (+1 when a source is active) and 2 recurrence
+// FP64 is the binding resource on GB300 (about 0.6e12 DFMA/s against ~6.5 TB/s of HBM and 32-bit integer units 64
+// times as wide), so the step is arranged for the fewest FP64 operations: the stencil in integers and 2 recurrence
 // FMAs per voxel in the x sweep, 2 FMAs per voxel in the y sweep, 2 FMAs and 1 add per voxel in the z sweep.
-//
-// Memory layout: every field is (nz, ny, nx) with x fastest; the stage-0 stencil coefficients are
-// chunk-blocked (hs2g_internal.cuh).
-//   x sweep: a CTA owns 32 consecutive x-lines.  The stencil is evaluated in 32-column chunks with lanes
-//            along x (coalesced loads of T and of the line's coefficient block), staged through shared memory,
-//            and one warp runs the 32 line recurrences down the transposed chunk (lane = line).  The forward
-//            values are kept in the output array W0 and re-read by the back substitution in the same CTA.
+//   x sweep: hs2g_x.cuh
 //   y, z sweeps: one warp per 16 neighbouring lines, both ends of each line at once, rows copied ahead into shared
 //            memory and coefficients from tables per line class (hs2g_pair.cuh, hs2g_classes.cu).
+#include <algorithm>
 #include <cmath>
-#include <cstdlib>
-#include <cstring>
 #include <type_traits>
 
 #include "hs2g_internal.cuh"
 #include "hs2g_pair.cuh"
+#include "hs2g_x.cuh"
 
 namespace hs2g {
 namespace {
 
-constexpr int kXLines = 32;   // x-lines per CTA
-constexpr int kXChunk = 32;   // columns per staged chunk
-constexpr int kXThreads = 128;
-constexpr int kXWarps = kXThreads / 32;
-// Register budget of the x sweep: at 72 registers 7 CTAs of 128 threads fit on an SM, so the 1040 CTAs of a
-// 65 x 512-line grid run in one wave on 152 SMs with the most loads in flight per thread (332 us at
-// 65x512x512; 80 registers: 6 CTAs per SM and a second wave, 530 us; the compiler's own choice of 48
-// registers: 415 us; a bound of 7 blocks also gives 72 registers but schedules worse: 347-363 us).  The
-// whole-grid kernels set the budget directly (__maxnreg__); the host-buffer step's line-range kernels keep a
-// bound of 6 blocks (kXMinBlocks).  Check -Xptxas -v after a change.
-constexpr int kXMinBlocks = 6;
+// Where a launch's class source values come from: nowhere, the kernel's parameter table, or row ds->step of the
+// handle's device schedule (an inactive row or one past the schedule's end gives zeros).
+enum XSource { kNoSource, kTable, kRow };
+template <int SRC>
+using XTable = typename std::conditional<SRC == kTable, QTable, int>::type;
 
-// Stage-0 right-hand side of voxel (L, i) of x-line L = k*ny + j, pre-scaled by the line's pivot:
-// wc*T + wxl*T[i-1] + wxh*T[i+1] + wyl*T[j-1] + wyh*T[j+1] + wzl*T[k-1] + wzh*T[k+1] (+ wq*Q).
-// Out-of-grid neighbours carry a zero coefficient (exterior faces are insulating): T[p] is read instead.
-// Column i = ch*32 + lane of the chunk; the coefficients come from the line's chunk block.
-// A sweep's forward values are written and read back by the same thread block within microseconds; with
-// every line in flight they add up to more than L2 (136 MB at 65x512x512), so they are stored with an
-// evict-last L2 policy where that keeps them on chip.
-// IX: the index type of the voxel, line and coefficient-block arithmetic (int32_t when the grid and its stencil
-// blocks have fewer than 2^31 elements, which makes the line -> (k, j) division a 32-bit one).
-template <bool HAS_Q, typename IX = int64_t>
-__device__ __forceinline__ double stencil_x(const Dims& d, const double* __restrict__ T, const Coeffs& c,
-                                            const uint8_t* __restrict__ vclass, const double* __restrict__ qdense,
-                                            const double* __restrict__ qshape, const double* sq, IX L, int ch,
-                                            int lane) {
-  const IX nx = (IX)d.nx, ny = (IX)d.ny, nz = (IX)d.nz;
-  const IX i = (IX)ch * 32 + lane;
-  const IX k = L / ny, j = L - k * ny;
-  const IX p = L * nx + i;
-  const IX nxy = nx * ny;
-  const double* __restrict__ w = c.xb + ((L * (IX)c.nchunks + ch) * kXBlockCoeffs) * 32 + lane;
-  const double t = T[p];
-  const double txl = i > 0 ? T[p - 1] : t;
-  const double txh = i + 1 < nx ? T[p + 1] : t;
-  const double tyl = j > 0 ? T[p - nx] : t;
-  const double tyh = j + 1 < ny ? T[p + nx] : t;
-  const double tzl = k > 0 ? T[p - nxy] : t;
-  const double tzh = k + 1 < nz ? T[p + nxy] : t;
-  double r = w[kWc * 32] * t;
-  r = fma(w[kWxl * 32], txl, r);
-  r = fma(w[kWxh * 32], txh, r);
-  r = fma(w[kWyl * 32], tyl, r);
-  r = fma(w[kWyh * 32], tyh, r);
-  r = fma(w[kWzl * 32], tzl, r);
-  r = fma(w[kWzh * 32], tzh, r);
-  if (HAS_Q) {
-    double q = sq[vclass[p]];
-    if (qshape) q *= qshape[p];
-    if (qdense) q += qdense[p];
-    r = fma(w[kWq * 32], q, r);
-  }
-  return r;
-}
-
-// RANGED: the launch covers x-lines [line_begin, line_end) (the overlapped host-buffer step); otherwise all
-// nz*ny lines, with the arguments unused -- the two are separate instances so that the whole-grid kernel keeps
-// its own register allocation.  LINES x-lines per CTA: 32 for the whole grid; the host-buffer step's later,
-// smaller slabs take 16 or 8, whose CTAs finish sooner (a CTA's chunk loop, not the GPU's throughput, sets
-// how long a small launch takes).
-// PITCH 0: W0 shares T's row pitch nx; 1: one pad column (odd nx: pitch nx + 1, so the W0 index of voxel (L, i)
-// is its T index plus L); 2: any other pitch c.px (padding for tests).
-template <int PITCH, typename IX = int64_t>
-__device__ __forceinline__ IX w0_index(const Dims& d, const Coeffs& c, IX L, IX i) {
-  if (PITCH == 0) return L * (IX)d.nx + i;
-  if (PITCH == 1) return L * (IX)d.nx + i + L;
-  return L * (IX)c.px + i;
-}
-
-// The class source values come from the kernel's parameter table qt, or (QROW) from the global row qrow.  The
-// kernel owns the shared arrays: sr, sa [LINES][kXChunk + 1] and sq [HS2G_MAX_CLASSES when HAS_Q].
-template <bool HAS_Q, bool RANGED, int LINES, int PITCHED, bool QROW = false, typename QT = QTable,
-          typename IX = int64_t>
-__device__ __forceinline__ void sweep_x_body(const Dims& d, const double* __restrict__ T, const Coeffs& c,
-                                             const uint8_t* __restrict__ vclass, const double* __restrict__ qdense,
-                                             const double* __restrict__ qshape, const QT& qt,
-                                             const double* __restrict__ qrow, double* __restrict__ W0,
-                                             int64_t line_begin, int64_t line_end, double (*sr)[kXChunk + 1],
-                                             double (*sa)[kXChunk + 1], double* sq) {
-  constexpr int kPerWarp = LINES / kXWarps;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if constexpr (HAS_Q) {
-    for (int e = threadIdx.x; e < HS2G_MAX_CLASSES; e += kXThreads) {
-      if constexpr (QROW)
-        sq[e] = qrow[e];
-      else
-        sq[e] = qt.q[e];
-    }
-  }
-  const IX nx = (IX)d.nx;
-  const IX nlines = RANGED ? (IX)line_end : (IX)(d.nz * d.ny);
-  const IX L0 = (RANGED ? (IX)line_begin : 0) + (IX)blockIdx.x * LINES;
-  const int nchunks = (int)((d.nx + kXChunk - 1) / kXChunk);
-  wait_prior_grid();  // T comes from the previous step's z sweep, which used W0 as its scratch
-  __syncthreads();
-
-  // forward: z_i = R'_i - a0_i * z_{i-1}
-  double carry = 0.0;
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const IX i = (IX)ch * kXChunk + lane;
-#pragma unroll
-    for (int ll = 0; ll < kPerWarp; ++ll) {
-      const int l = warp * kPerWarp + ll;
-      const IX L = L0 + l;
-      double r = 0.0, a = 0.0;
-      if (L < nlines && i < nx) {
-        r = stencil_x<HAS_Q, IX>(d, T, c, vclass, qdense, qshape, sq, L, ch, lane);
-        a = c.a0[L * nx + i];
-      }
-      sr[l][lane] = r;
-      sa[l][lane] = a;
-    }
-    __syncthreads();
-    if (warp * 32 + lane < LINES) {  // lane = line of the recurrence
-      const int l = warp * 32 + lane;
-      const int cw = (int)min((int64_t)kXChunk, d.nx - (int64_t)ch * kXChunk);
-      double z = carry;
-      if (cw == kXChunk) {  // full chunks unrolled: the shared loads of later rows issue ahead of the chain
-#pragma unroll 4
-        for (int cc = 0; cc < kXChunk; ++cc) {
-          z = fma(-sa[l][cc], z, sr[l][cc]);
-          sr[l][cc] = z;
-        }
-      } else {
-        for (int cc = 0; cc < cw; ++cc) {
-          z = fma(-sa[l][cc], z, sr[l][cc]);
-          sr[l][cc] = z;
-        }
-      }
-      carry = z;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int ll = 0; ll < kPerWarp; ++ll) {
-      const int l = warp * kPerWarp + ll;
-      const IX L = L0 + l;
-      if (L < nlines && i < nx) W0[w0_index<PITCHED, IX>(d, c, L, i)] = sr[l][lane];
-    }
-    __syncthreads();
-  }
-
-  // back substitution: W0_i = z_i - b0_i * W0_{i+1}
-  carry = 0.0;
-  for (int ch = nchunks - 1; ch >= 0; --ch) {
-    const IX i = (IX)ch * kXChunk + lane;
-#pragma unroll
-    for (int ll = 0; ll < kPerWarp; ++ll) {
-      const int l = warp * kPerWarp + ll;
-      const IX L = L0 + l;
-      double z = 0.0, b = 0.0;
-      if (L < nlines && i < nx) {
-        const IX p = L * nx + i;
-        z = W0[w0_index<PITCHED, IX>(d, c, L, i)];
-        b = c.b0[p];
-      }
-      sr[l][lane] = z;
-      sa[l][lane] = b;
-    }
-    __syncthreads();
-    if (warp * 32 + lane < LINES) {
-      const int l = warp * 32 + lane;
-      const int cw = (int)min((int64_t)kXChunk, d.nx - (int64_t)ch * kXChunk);
-      double x = carry;
-      if (cw == kXChunk) {
-#pragma unroll 4
-        for (int cc = kXChunk - 1; cc >= 0; --cc) {
-          x = fma(-sa[l][cc], x, sr[l][cc]);
-          sr[l][cc] = x;
-        }
-      } else {
-        for (int cc = cw - 1; cc >= 0; --cc) {
-          x = fma(-sa[l][cc], x, sr[l][cc]);
-          sr[l][cc] = x;
-        }
-      }
-      carry = x;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int ll = 0; ll < kPerWarp; ++ll) {
-      const int l = warp * kPerWarp + ll;
-      const IX L = L0 + l;
-      if (L < nlines && i < nx) W0[w0_index<PITCHED, IX>(d, c, L, i)] = sr[l][lane];
-    }
-    __syncthreads();
-  }
-}
-
-// The x sweep over the whole grid: the register budget is set to 72, which keeps 7 CTAs of 128 threads per SM, so
-// the 1040 CTAs of a 65x512-line grid run in one wave (332 us at 65x512x512; under a bound of 6 blocks the
-// instance without a source also gets 72 registers and takes 334 us, while the instances with a source term or
-// padded W0 rows take 78-80 registers there, 6 CTAs per SM, two waves: 694 us for a source step).  Padded rows
-// of an odd nx use the one-column index (349 us at 65x512x511; with a general pitch 362 us).
-// The class table is a kernel parameter only in the instances with a source (2 KB that the others would copy at
-// every launch for nothing).
-template <bool HAS_Q>
-using XTable = typename std::conditional<HAS_Q, QTable, int>::type;
-template <bool HAS_Q, bool RANGED, int LINES, int PITCH, typename IX = int64_t>
-__global__ void __maxnreg__(72) sweep_x_lean_kernel(Dims d, const double* __restrict__ T, Coeffs c,
-                                                    const uint8_t* __restrict__ vclass,
-                                                    const double* __restrict__ qdense,
-                                                    const double* __restrict__ qshape, XTable<HAS_Q> qt,
-                                                    double* __restrict__ W0, int64_t line_begin, int64_t line_end) {
-  __shared__ double sr[LINES][kXChunk + 1];
-  __shared__ double sa[LINES][kXChunk + 1];
-  __shared__ double sq[HAS_Q ? HS2G_MAX_CLASSES : 1];
-  sweep_x_body<HAS_Q, RANGED, LINES, PITCH, false, XTable<HAS_Q>, IX>(d, T, c, vclass, qdense, qshape, qt, nullptr,
-                                                                      W0, line_begin, line_end, sr, sa, sq);
-}
-// The line ranges of the host-buffer step on unpadded rows keep the 6-block bound (80 registers at 32 lines per
-// CTA): measured against the 72-register build there, 9.62e9 against 9.39e9 voxel-steps/s end to end.
-template <bool HAS_Q, bool RANGED, int LINES = kXLines>
-__global__ void __launch_bounds__(kXThreads, kXMinBlocks) sweep_x_kernel(Dims d, const double* __restrict__ T, Coeffs c,
-                                                             const uint8_t* __restrict__ vclass,
-                                                             const double* __restrict__ qdense,
-                                                             const double* __restrict__ qshape, XTable<HAS_Q> qt,
-                                                             double* __restrict__ W0, int64_t line_begin,
-                                                             int64_t line_end) {
-  __shared__ double sr[LINES][kXChunk + 1];
-  __shared__ double sa[LINES][kXChunk + 1];
-  __shared__ double sq[HAS_Q ? HS2G_MAX_CLASSES : 1];
-  sweep_x_body<HAS_Q, RANGED, LINES, 0>(d, T, c, vclass, qdense, qshape, qt, nullptr, W0, line_begin, line_end, sr,
-                                        sa, sq);
-}
-
-// The x sweep of a step whose class table is row ds->step of the handle's device schedule (the steps with a
-// source in the captured step graphs of hs2g_run): thread 0 reads the row's address once for the CTA; an
-// inactive row or one past the schedule's end gives the zero table.  Only the source body is compiled here:
-// the steps without a source run sweep_x_lean_kernel, whose code a second body in the same kernel would slow
-// (measured 3 us per step at 65x512x512).
-__device__ const double kZeroRow[HS2G_MAX_CLASSES] = {};
-template <int PITCH>
-__global__ void __maxnreg__(72) sweep_x_row_kernel(Dims d, const double* __restrict__ T, Coeffs c,
-                                                   const uint8_t* __restrict__ vclass,
-                                                   const DevSchedule* __restrict__ ds, double* __restrict__ W0) {
-  __shared__ double sr[kXLines][kXChunk + 1];
-  __shared__ double sa[kXLines][kXChunk + 1];
-  __shared__ double sq[HS2G_MAX_CLASSES];
-  __shared__ const double* s_row;
-  if (threadIdx.x == 0) {
+// the class source values of the launch into shared memory (SRC), before the kernel waits for the previous one
+template <int SRC>
+__device__ __forceinline__ void x_sources(XProblem<double>& P, const XTable<SRC>& qt, const DevSchedule* ds, double* sq) {
+  if constexpr (SRC == kTable)
+    for (int e = threadIdx.x; e < HS2G_MAX_CLASSES; e += blockDim.x) sq[e] = qt.q[e];
+  if constexpr (SRC == kRow) {
     const int64_t st = ds->step;
-    s_row = st >= 0 && st < ds->n && ds->active[st] ? ds->q + st * HS2G_MAX_CLASSES : kZeroRow;
+    const bool on = st >= 0 && st < ds->n && ds->active[st];
+    for (int e = threadIdx.x; e < HS2G_MAX_CLASSES; e += blockDim.x) sq[e] = on ? ds->q[st * HS2G_MAX_CLASSES + e] : 0.0;
+    P.qshape = ds->shape;
   }
-  __syncthreads();
-  const int no_table = 0;  // the table comes from the row
-  sweep_x_body<true, false, kXLines, PITCH, true>(d, T, c, vclass, nullptr, ds->shape, no_table, s_row, W0, 0, 0, sr,
-                                                  sa, sq);
+}
+// The stencil of the x-lines [begin, end): a CTA per kXStencilLines lines and per gridDim.y-th chunk of columns.
+template <int SRC, typename IX>
+__global__ void __launch_bounds__(32 * kXStencilWarps, kXStencilCtas) x_stencil_kernel(XProblem<double> P, XTable<SRC> qt,
+                                                                           const DevSchedule* ds, int64_t begin,
+                                                                           int64_t end) {
+  __shared__ XLine<IX> lines[kXStencilLines];
+  __shared__ double sq[SRC == kNoSource ? 1 : HS2G_MAX_CLASSES];
+  x_sources<SRC>(P, qt, ds, sq);
+  wait_prior_grid();  // T comes from the previous step's z sweep, which used W0 as its scratch
+  x_stencil_lines<double, SRC != kNoSource, IX>(P, begin + blockIdx.x * (int64_t)kXStencilLines, end, blockIdx.y,
+                                                gridDim.y, lines, sq);
+}
+// The whole x sweep of [begin, end), 16 lines per CTA.
+template <int SRC, typename IX>
+__global__ void __launch_bounds__(kXFusedThreads, 3) x_fused_kernel(XProblem<double> P, XTable<SRC> qt,
+                                                                    const DevSchedule* ds, int64_t begin, int64_t end) {
+  extern __shared__ __align__(16) unsigned char x_sm[];
+  x_sources<SRC>(P, qt, ds, reinterpret_cast<double*>(x_sm));
+  wait_prior_grid();
+  x_fused_lines<SRC != kNoSource, IX>(P, begin + blockIdx.x * (int64_t)16, end, x_sm);
+}
+// The x line solves of [begin, end) in W0, 16 lines per warp.
+template <bool TABLE, bool KEEP>
+__global__ void __launch_bounds__(32 * kPairMaxWarps) x_solve_kernel(XProblem<double> P, int64_t begin, int64_t end,
+                                                                     int64_t smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char x_sm[];
+  const int64_t L0 = begin + (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * x_lines<true>();
+  if (L0 >= end) return;
+  wait_prior_grid();
+  x_solve_lines<double, true, TABLE, KEEP>(P, L0, (int)min((int64_t)x_lines<true>(), end - L0),
+                                           reinterpret_cast<double*>(x_sm + (threadIdx.x >> 5) * smem_per_warp));
 }
 
-// Whether the whole-grid x sweep may index in 32 bits: every voxel index (with the pad column of an odd nx) and
-// every stencil-block element below 2^31.  HS2G_X_INDEX=64 keeps 64-bit indices.
-bool x_index32(const Dims& d, const Coeffs& c) {
-  static const bool off = [] {
-    const char* e = getenv("HS2G_X_INDEX");
-    return e && strcmp(e, "64") == 0;
-  }();
-  const int64_t lim = (int64_t)1 << 31;
-  return !off && d.nvox() + d.nz * d.ny < lim && d.nz * d.ny * c.nchunks * kXBlockCoeffs * 32 < lim;
-}
+// 32-bit index arithmetic when every voxel index, with the pad column of an odd nx, is below 2^31
+bool x_index32(const Dims& d, const Coeffs& c) { return d.nz * d.ny * c.px < ((int64_t)1 << 31); }
 
-// x sweep over all lines (RANGED false) or the lines [line_begin, line_end) of the host-buffer step
-template <bool RANGED, int LINES>
-void launch_x(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t line_begin, int64_t line_end,
-              cudaStream_t s) {
-  const Dims& d = a.d;
-  const unsigned gx = (unsigned)(((RANGED ? line_end - line_begin : d.nz * d.ny) + LINES - 1) / LINES);
-  const bool has_q = a.has_qtab || a.qdense != nullptr;
-  const int pitch = c.px == d.nx ? 0 : c.px == d.nx + 1 ? 1 : 2;
-#define HS2G_X(KERNEL, TABLE, ...)                                                                             \
-  launch_kernel(KERNEL<__VA_ARGS__>, dim3(gx), dim3(kXThreads), 0, s, a.pdl_x, d, a.T_in, c, a.vclass, a.qdense, \
-                a.qshape, TABLE, a.W0, line_begin, line_end)
-  if constexpr (!RANGED) {
-    if (pitch < 2 && x_index32(d, c)) {
-      if (pitch == 0) {
-        if (has_q)
-          HS2G_X(sweep_x_lean_kernel, q, true, false, LINES, 0, int32_t);
-        else
-          HS2G_X(sweep_x_lean_kernel, 0, false, false, LINES, 0, int32_t);
-      } else {
-        if (has_q)
-          HS2G_X(sweep_x_lean_kernel, q, true, false, LINES, 1, int32_t);
-        else
-          HS2G_X(sweep_x_lean_kernel, 0, false, false, LINES, 1, int32_t);
-      }
-      return;
-    }
-  }
-  if (RANGED && pitch == 0) {
-    if (has_q)
-      HS2G_X(sweep_x_kernel, q, true, RANGED, LINES);
-    else
-      HS2G_X(sweep_x_kernel, 0, false, RANGED, LINES);
-  } else if (pitch == 0) {
-    if (has_q)
-      HS2G_X(sweep_x_lean_kernel, q, true, RANGED, LINES, 0);
-    else
-      HS2G_X(sweep_x_lean_kernel, 0, false, RANGED, LINES, 0);
-  } else if (pitch == 1) {
-    if (has_q)
-      HS2G_X(sweep_x_lean_kernel, q, true, RANGED, LINES, 1);
-    else
-      HS2G_X(sweep_x_lean_kernel, 0, false, RANGED, LINES, 1);
-  } else {
-    if (has_q)
-      HS2G_X(sweep_x_lean_kernel, q, true, RANGED, LINES, 2);
-    else
-      HS2G_X(sweep_x_lean_kernel, 0, false, RANGED, LINES, 2);
-  }
-#undef HS2G_X
+using XSolveKernel = void (*)(XProblem<double>, int64_t, int64_t, int64_t);
+XSolveKernel x_solve_for(bool table, bool keep) {
+  return table ? (keep ? x_solve_kernel<true, true> : x_solve_kernel<true, false>)
+               : (keep ? x_solve_kernel<false, true> : x_solve_kernel<false, false>);
 }
-
-void launch_x_row(const StepArgs& a, const Coeffs& c, const DevSchedule* ds, cudaStream_t s) {
-  const Dims& d = a.d;
-  const unsigned gx = (unsigned)((d.nz * d.ny + kXLines - 1) / kXLines);
-  const int pitch = c.px == d.nx ? 0 : c.px == d.nx + 1 ? 1 : 2;
-  if (pitch == 0)
-    launch_kernel(sweep_x_row_kernel<0>, dim3(gx), dim3(kXThreads), 0, s, a.pdl_x, d, a.T_in, c, a.vclass, ds, a.W0);
-  else if (pitch == 1)
-    launch_kernel(sweep_x_row_kernel<1>, dim3(gx), dim3(kXThreads), 0, s, a.pdl_x, d, a.T_in, c, a.vclass, ds, a.W0);
-  else
-    launch_kernel(sweep_x_row_kernel<2>, dim3(gx), dim3(kXThreads), 0, s, a.pdl_x, d, a.T_in, c, a.vclass, ds, a.W0);
+template <int SRC>
+cudaError_t launch_x(const StepArgs& a, const Coeffs& c, const XTable<SRC>& q, const DevSchedule* ds, int64_t begin,
+                     int64_t end, cudaStream_t s) {
+  if (end <= begin) return cudaSuccess;
+  const XProblem<double> P{a.d.nz, a.d.ny, a.d.nx, a.T_in, c.xb, c.bidx, c.nchunks, c.a0, c.b0, c.cls0,
+                           a.vclass, a.qdense, a.qshape, a.W0, c.px};
+  if (c.cls0 && (x_index32(a.d, c) ? x_fused<int32_t>(a.d.nx, end - begin) : x_fused<int64_t>(a.d.nx, end - begin))) {
+    const dim3 grid((unsigned)((end - begin + 15) / 16)), block(kXFusedThreads);
+    if (x_index32(a.d, c))
+      return launch_kernel(x_fused_kernel<SRC, int32_t>, grid, block, x_fused_smem<int32_t>(a.d.nx), s, a.pdl_x, P, q, ds,
+                           begin, end);
+    return launch_kernel(x_fused_kernel<SRC, int64_t>, grid, block, x_fused_smem<int64_t>(a.d.nx), s, a.pdl_x, P, q, ds,
+                         begin, end);
+  }
+  // a CTA walks its lines' chunks, or takes every second, fourth ... of them until there are CTAs enough for the GPU
+  const int64_t ctas = (end - begin + kXStencilLines - 1) / kXStencilLines;
+  unsigned split = 1;
+  while (split < c.nchunks && split < 32768 && ctas * split < 152 * 8) split *= 2;
+  const dim3 grid((unsigned)ctas, split), block(32 * kXStencilWarps);
+  cudaError_t e = x_index32(a.d, c)
+                      ? launch_kernel(x_stencil_kernel<SRC, int32_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end)
+                      : launch_kernel(x_stencil_kernel<SRC, int64_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end);
+  if (e != cudaSuccess) return e;
+  const int64_t groups = (end - begin + x_lines<true>() - 1) / x_lines<true>();
+  const PairShape sh = c.cls0 ? x_solve_shape<double, true, true>(a.d.nx, groups)
+                              : x_solve_shape<double, true, false>(a.d.nx, groups);
+  return launch_kernel(x_solve_for(c.cls0 != nullptr, sh.keep), dim3((unsigned)((groups + sh.warps - 1) / sh.warps)),
+                       dim3(32 * sh.warps), sh.smem, s, a.pdl, P, begin, end, (int64_t)(sh.smem / sh.warps));
+}
+cudaError_t launch_x_any(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t begin, int64_t end,
+                         cudaStream_t s) {
+  if (a.has_qtab || a.qdense) return launch_x<kTable>(a, c, q, nullptr, begin, end, s);
+  return launch_x<kNoSource>(a, c, 0, nullptr, begin, end, s);
 }
 
 // The y sweep (ADD_T false: W1 = s2 * dT1 from W0 = sigma * dT0; rows of lines k) and the z sweep (ADD_T: T_out =
@@ -524,20 +289,38 @@ cudaError_t launch_yz(const StepArgs& a, const Coeffs& c, cudaStream_t s, cudaEv
 }
 }  // namespace
 
-cudaError_t sweeps_prepare() {
+cudaError_t sweeps_prepare(const Dims& d, const Coeffs& c) {
+  constexpr size_t kDefault = 48 * 1024, kMost = 226 * 1024;
   cudaError_t e = cudaSuccess;
-  for (int v = 0; v < 16 && e == cudaSuccess; ++v) {
-    const bool keep = v & 1, table = v & 2, t16 = v & 4;
-    const void* k = v & 8 ? (const void*)pair_kernel<true>(keep, table, t16) : (const void*)pair_kernel<false>(keep, table, t16);
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  auto allow = [&](const void* kernel, size_t smem) {  // a CTA has up to kPairMaxWarps warps' shares, at most kMost
+    if (smem > kDefault && e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min(smem, kMost));
+  };
+  const bool tx = c.cls0 != nullptr, ty = c.cls1 != nullptr, tz = c.cls2 != nullptr;
+  auto most = [](size_t keep, size_t ring) { return kPairMaxWarps * std::max(keep, ring); };
+  for (int keep = 0; keep < 2; ++keep) {
+    allow((const void*)x_solve_for(tx, keep), most(tx ? x_solve_smem<double, true, true, true>(d.nx) : x_solve_smem<double, true, false, true>(d.nx),
+                                                   x_solve_smem<double, true, false, false>(d.nx)));
+    allow((const void*)pair_kernel<false>(keep, ty, true),
+          most(ty ? pair_smem<double, true, false, true, true>(d.ny) : pair_smem<double, true, false, true, false>(d.ny),
+               pair_smem<double, true, false, false, false>(d.ny)));
+    for (int t16 = 0; t16 < 2; ++t16)
+      allow((const void*)pair_kernel<true>(keep, tz, t16),
+            most(tz ? pair_smem<double, true, true, true, true>(d.nz) : pair_smem<double, true, true, true, false>(d.nz),
+                 pair_smem<double, true, true, false, false>(d.nz)));
   }
+  const void* fused[] = {(const void*)x_fused_kernel<kNoSource, int32_t>, (const void*)x_fused_kernel<kTable, int32_t>,
+                         (const void*)x_fused_kernel<kRow, int32_t>,      (const void*)x_fused_kernel<kNoSource, int64_t>,
+                         (const void*)x_fused_kernel<kTable, int64_t>,    (const void*)x_fused_kernel<kRow, int64_t>};
+  for (const void* k : fused) allow(k, x_fused_smem<int64_t>(d.nx));
   return e;
 }
 
 cudaError_t launch_step_events(const StepArgs& a, const Coeffs& c, const QTable& q, cudaStream_t s,
                                cudaEvent_t ev[4]) {
   if (ev) cudaEventRecord(ev[0], s);
-  launch_x<false, kXLines>(a, c, q, 0, 0, s);
+  const cudaError_t e = launch_x_any(a, c, q, 0, a.d.nz * a.d.ny, s);
+  if (e != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[1], s);
   return launch_yz(a, c, s, ev);
 }
@@ -547,7 +330,8 @@ cudaError_t launch_step(const StepArgs& a, const Coeffs& c, const QTable& q, cud
 }
 
 cudaError_t launch_step_row(const StepArgs& a, const Coeffs& c, const DevSchedule* ds, cudaStream_t s) {
-  launch_x_row(a, c, ds, s);
+  const cudaError_t e = launch_x<kRow>(a, c, 0, ds, 0, a.d.nz * a.d.ny, s);
+  if (e != cudaSuccess) return e;
   return launch_yz(a, c, s, nullptr);
 }
 
@@ -570,22 +354,9 @@ double surface_dz2(double dz) {
   return std::pow(dz, (double)two);
 }
 
-template <int LINES>
-void launch_x_lines(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t line_begin, int64_t line_end,
-                    cudaStream_t s) {
-  launch_x<true, LINES>(a, c, q, line_begin, line_end, s);
-}
-
 cudaError_t launch_x_range(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t line_begin,
-                           int64_t line_end, int lines_per_cta, cudaStream_t s) {
-  if (line_end <= line_begin) return cudaSuccess;
-  if (lines_per_cta == 8)
-    launch_x_lines<8>(a, c, q, line_begin, line_end, s);
-  else if (lines_per_cta == 16)
-    launch_x_lines<16>(a, c, q, line_begin, line_end, s);
-  else
-    launch_x_lines<kXLines>(a, c, q, line_begin, line_end, s);
-  return cudaGetLastError();
+                           int64_t line_end, cudaStream_t s) {
+  return launch_x_any(a, c, q, line_begin, line_end, s);
 }
 
 cudaError_t launch_y(const StepArgs& a, const Coeffs& c, cudaStream_t s) {

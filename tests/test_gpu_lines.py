@@ -34,8 +34,33 @@ def _spec(shape, random_faces):
     return spec
 
 
-def _field(shape):
-    return 293.0 + np.random.default_rng(4).random(shape)
+def _field(shape, kind="kelvin"):
+    T = 293.0 + np.random.default_rng(4).random(shape)
+    if kind == "mixed":       # signs, binary exponents and zeros side by side: the stencil's FP64 chain, voxel by voxel
+        rng = np.random.default_rng(5)
+        T = np.where(rng.random(shape) < 0.5, T - 293.5, rng.choice([0.0, -0.0, 250.0, 260.0, 1e-300, -7.0], size=shape))
+    elif kind == "negative":  # one sign and exponent
+        T = -T
+    return T
+
+
+@pytest.mark.parametrize("kind", ["kelvin", "mixed", "negative"])
+@pytest.mark.parametrize("shape", [(9, 20, 70), (5, 130, 37)])
+def test_stencil_of_any_temperatures_vs_oracle(cuda_ok, shape, kind):
+    """The stencil in integers and in FP64, for all voxels and for some of a warp's, and through the two layouts of the
+    x sweep (the batch takes it in two kernels, the small problem in one): the same bits, within the parity bar."""
+    spec = _spec(shape, False)
+    vol = W.volumetric_tuple(hs, spec)
+    P, S = hs.setup(*W.setup_args(hs, spec))
+    Po, _ = oracle.setup(*W.setup_args(HS, spec))
+    T0 = _field(shape, kind)
+    T = hs.run_adi_steps(P, S, 0.0, spec["dt"], T0, spec["arrays"]["volumetric"], vol)
+    assert rel_err(T, oracle.run_adi_steps(Po, None, 0.0, spec["dt"], T0, spec["arrays"]["volumetric"], vol)) <= 1e-12
+    b = Batch([W.setup_args(hs, spec)], precision=64)
+    b.set_temperature([T0])
+    b.set_sources([0.0], spec["dt"])
+    b.run(1)
+    np.testing.assert_array_equal(b.get_temperature()[0], T)
 
 
 @pytest.mark.parametrize("random_faces", [False, True])
