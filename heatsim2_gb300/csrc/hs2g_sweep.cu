@@ -292,9 +292,11 @@ cudaError_t launch_yz(const StepArgs& a, const Coeffs& c, cudaStream_t s, cudaEv
 cudaError_t sweeps_prepare(const Dims& d, const Coeffs& c) {
   constexpr size_t kDefault = 48 * 1024, kMost = 226 * 1024;
   cudaError_t e = cudaSuccess;
-  auto allow = [&](const void* kernel, size_t smem) {  // a CTA has up to kPairMaxWarps warps' shares, at most kMost
+  // A CTA has up to kPairMaxWarps warps' shares, at most kMost.  The limit belongs to the kernel, not to the problem:
+  // always the same value, so that a small problem never takes from what an earlier one needs.
+  auto allow = [&](const void* kernel, size_t smem) {
     if (smem > kDefault && e == cudaSuccess)
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min(smem, kMost));
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
   };
   const bool tx = c.cls0 != nullptr, ty = c.cls1 != nullptr, tz = c.cls2 != nullptr;
   auto most = [](size_t keep, size_t ring) { return kPairMaxWarps * std::max(keep, ring); };

@@ -82,3 +82,21 @@ def test_line_solves_vs_oracle(cuda_ok, shape, random_faces):
         b.run(2)
         got = b.get_temperature()[0]
         assert rel_err(got, T) <= tol, precision
+
+
+def test_problems_of_several_sizes_side_by_side(cuda_ok):
+    """What a problem's setup allows its kernels (shared memory) never takes from an earlier, larger problem."""
+    made = []
+    for shape in [(3, 3, 1000), (3, 700, 40), (3, 3, 400), (3, 300, 40)]:
+        spec = _spec(shape, False)
+        P, S = hs.setup(*W.setup_args(hs, spec))
+        made.append((P, S, spec, shape))
+
+    def step(P, S, spec, shape):
+        return hs.run_adi_steps(P, S, 0.0, spec["dt"], _field(shape), spec["arrays"]["volumetric"],
+                                W.volumetric_tuple(hs, spec))
+    for P, S, spec, shape in made:
+        alone, _ = oracle.setup(*W.setup_args(HS, spec))
+        ref = oracle.run_adi_steps(alone, None, 0.0, spec["dt"], _field(shape), spec["arrays"]["volumetric"],
+                                   W.volumetric_tuple(hs, spec))
+        assert rel_err(step(P, S, spec, shape), ref) <= 1e-12
