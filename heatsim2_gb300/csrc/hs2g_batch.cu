@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(32 * kPairMaxWarps) batch_pair_kernel(BatchVie
   const int64_t w = ADD_T ? row * I.px + i0 : row * ny * I.px + i0, wst = ADD_T ? ny * I.px : I.px;
   constexpr int AX = ADD_T ? 2 : 1;
   const int32_t* cls = I.cls[AX];
-  PairLines<R> p;
+  PairLines<R> p{};
   p.W = (ADD_T ? v.W1 : v.W0) + I.woff + w;
   p.wst = p.cst = p.zst = wst;
   p.a = (const R*)I.a[AX] + (cls ? 0 : w);

@@ -66,21 +66,23 @@ struct PairLines {
   int64_t st;
   R* Z;
   int64_t zst;
+  const R* sc;  // SCALE: the right-hand sides are W * sc, laid out like W
+  R* X;         // SCALE, ADD_T: x itself is stored here too, unless null (laid out like W; may be Z)
 };
 
 // rows of 32 elements a warp holds in shared memory, in whole blocks: with KEEP its half lines' values and (ADD_T) room
 // for the temperatures copied ahead, otherwise rings of right-hand sides (forward) or forward values and temperatures
-// (back); a ring of coefficients when they come row by row (TABLE false)
-template <bool TWO, bool ADD_T, bool KEEP, bool TABLE>
+// (back); a ring of coefficients when they come row by row (TABLE false), one of the scale (SCALE)
+template <bool TWO, bool ADD_T, bool KEEP, bool TABLE, bool SCALE = false>
 __host__ __device__ constexpr int64_t pair_rows_held(int64_t n) {
   return kPairRows *
-         ((TABLE ? 0 : pair_ahead<ADD_T>() + 1) +
+         (((TABLE ? 0 : 1) + (SCALE ? 1 : 0)) * (pair_ahead<ADD_T>() + 1) +
           (KEEP ? ((TWO ? n / 2 : n) + kPairRows - 1) / kPairRows + (ADD_T ? pair_ahead<ADD_T>() : 0)
                 : (pair_ahead<ADD_T>() + 1) * (ADD_T ? 2 : 1)));
 }
-template <typename R, bool TWO, bool ADD_T, bool KEEP, bool TABLE>
+template <typename R, bool TWO, bool ADD_T, bool KEEP, bool TABLE, bool SCALE = false>
 __host__ __device__ constexpr size_t pair_smem(int64_t max_len) {  // per warp
-  return sizeof(R) * 32 * (size_t)pair_rows_held<TWO, ADD_T, KEEP, TABLE>(max_len);
+  return sizeof(R) * 32 * (size_t)pair_rows_held<TWO, ADD_T, KEEP, TABLE, SCALE>(max_len);
 }
 
 // Copies rows of a warp's lines to shared memory, VEC elements per lane and instruction: a half warp (a warp when
@@ -132,7 +134,7 @@ struct RowCopy {
 // chain, so the rows are copied ahead with cp.async and each block's table coefficients are loaded a block ahead.
 // KEEP: the right-hand sides land where the forward values replace them and stay until the back pass (the
 // temperatures follow into rows the back pass has left); otherwise the forward values go to Z and come back.
-template <typename R, bool TWO, bool ADD_T, bool KEEP, bool TABLE, int VEC, int TVEC>
+template <typename R, bool TWO, bool ADD_T, bool KEEP, bool TABLE, int VEC, int TVEC, bool SCALE = false>
 __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int width, R* smem) {
   constexpr int RB = kPairRows, LA = pair_ahead<ADD_T>();
   constexpr int kRing = LA + 1;  // ring blocks
@@ -156,27 +158,33 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
   R wm = 0, am = 0, bm = 0, tm = 0;  // the middle row
   if (TWO) {
     wm = p.W[m * p.wst + mine];
+    if (SCALE) wm *= p.sc[m * p.wst + mine];
     am = A[m * cst];
     bm = B[m * cst];
     if (ADD_T) tm = p.T[m * p.st + mine];
   }
-  R* col = smem + (TABLE ? 0 : kRing * RB * 32) + lane;  // this lane's column of the rows
-  const R* ccol = smem + lane;                           // and of the coefficient ring
+  constexpr int kRings = (TABLE ? 0 : 1) + (SCALE ? 1 : 0);
+  R* col = smem + kRings * kRing * RB * 32 + lane;                           // this lane's column of the rows,
+  const R* ccol = smem + lane;                                              // of the coefficient ring
+  const R* scol = smem + (kRings - 1) * kRing * RB * 32 + lane;              // and of the scale's
   const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(smem);
-  const uint32_t col_s = ring_s + (TABLE ? 0 : kRing * kBlk);
+  const uint32_t scale_s = ring_s + (kRings - 1) * kRing * kBlk;
+  const uint32_t col_s = ring_s + kRings * kRing * kBlk;
   auto slot = [&](int q) { return KEEP ? q : q % kRing; };
   auto tslot = [&](int q) { return KEEP ? q + LA : kRing + q % kRing; };
-  RowCopy<R, TWO, VEC> cw, ca;   // right-hand sides (then forward values), coefficients
-  RowCopy<R, TWO, TVEC> ct;      // temperatures
+  RowCopy<R, TWO, VEC> cw, ca, cs;  // right-hand sides (then forward values), coefficients, scale
+  RowCopy<R, TWO, TVEC> ct;         // temperatures
   const int back0 = (nb - 1) * RB;
   cw.init(p.W, p.wst, n, upper, lane, width, 0, 1);
   if (!TABLE) ca.init(p.a, p.cst, n, upper, lane, width, 0, 1);
+  if (SCALE) cs.init(p.sc, p.wst, n, upper, lane, width, 0, 1);
   if (ADD_T) ct.init(p.T, p.st, n, upper, lane, width, back0 + RB - TVEC, -1);
   // item i of the copy sequence: i < nb the forward blocks, then the back blocks from the last
   auto issue = [&](int i, bool may_turn) {
     if (i < nb) {
       cw.template block<false>(col_s + slot(i) * kBlk, i, rows, i < nfull);
       if (!TABLE) ca.template block<false>(ring_s + (i % kRing) * kBlk, i, rows, i < nfull);
+      if (SCALE) cs.template block<false>(scale_s + (i % kRing) * kBlk, i, rows, i < nfull);
     } else if (may_turn && i < 2 * nb) {
       const int q = 2 * nb - 1 - i;
       if (i == nb) {
@@ -221,7 +229,7 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
 #pragma unroll
     for (int k = 0; k < RB; ++k) {
       a[k] = TABLE ? next[k] : cc[k * 32];
-      w[k] = c[k * 32];
+      w[k] = SCALE ? c[k * 32] * scol[((q % kRing) * RB + k) * 32] : c[k * 32];
     }
     if (TABLE) load(q + 1 < nb ? A : B, q + 1 < nb ? q + 1 : nb - 1);
     __syncwarp();
@@ -253,7 +261,10 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
   if (TWO) {
     const R other = __shfl_xor_sync(0xffffffffu, z, 16);
     x = fma(bm, upper ? z : other, fma(am, upper ? other : z, wm));  // the same value in both halves
-    if (!upper && live) p.out[m * p.st + mine] = ADD_T ? tm + x : x;
+    if (!upper && live) {
+      p.out[m * p.st + mine] = ADD_T ? tm + x : x;
+      if (SCALE && ADD_T && p.X) p.X[m * p.wst + mine] = x;
+    }
   }
   if (!KEEP) {
     cp_async_wait_pending<0>();
@@ -264,6 +275,8 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
   }
   const int64_t dT = (upper ? -p.st : p.st) * (int64_t)sizeof(R);
   R* oc = step_bytes(p.out + s * p.st + mine, (rows - 1) * dT);
+  const int64_t dX = (upper ? -p.wst : p.wst) * (int64_t)sizeof(R);
+  R* xc = SCALE && ADD_T && p.X ? step_bytes(p.X + s * p.wst + mine, (rows - 1) * dX) : nullptr;
 #pragma unroll 1
   for (int i = nb; i < 2 * nb; ++i) {
     cp_async_wait_pending<LA - 1>();
@@ -283,6 +296,10 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
     auto put = [&](int k) {
       if (live) *oc = ADD_T ? tt[k] + x : x;
       oc = step_bytes(oc, -dT);
+      if (SCALE && ADD_T && xc) {
+        if (live) *xc = x;
+        xc = step_bytes(xc, -dX);
+      }
     };
     if (q < nfull) {
 #pragma unroll
@@ -309,14 +326,14 @@ struct PairShape {
   int warps;
   size_t smem;
 };
-template <typename R, bool TWO, bool ADD_T, bool TABLE>
+template <typename R, bool TWO, bool ADD_T, bool TABLE, bool SCALE = false>
 inline PairShape pair_shape(int64_t max_len, int64_t groups, int force_keep = -1) {
   constexpr size_t kSmem = 227 * 1024, kReserved = 1024;  // per SM, and what a CTA takes beside its own
-  const size_t held = pair_smem<R, TWO, ADD_T, true, TABLE>(max_len);
+  const size_t held = pair_smem<R, TWO, ADD_T, true, TABLE, SCALE>(max_len);
   const int64_t per = (int64_t)(kSmem / (held + kReserved));
   PairShape sh;
   sh.keep = per > 0 && (force_keep >= 0 ? force_keep != 0 : per >= 8 || groups <= 152 * per);
-  const size_t each = sh.keep ? held : pair_smem<R, TWO, ADD_T, false, TABLE>(max_len);
+  const size_t each = sh.keep ? held : pair_smem<R, TWO, ADD_T, false, TABLE, SCALE>(max_len);
   sh.warps = 1;
   while (sh.warps < kPairMaxWarps && groups >= 152 * 8 * sh.warps && 2 * sh.warps * each <= 64 * 1024) sh.warps *= 2;
   sh.smem = each * sh.warps;

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(32 * kPairMaxWarps) pair_sweep_kernel(PairArgs
   const int64_t grp = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t row = g.begin + grp / gpr, i0 = (grp % gpr) * 16;
   if (row >= g.end) return;
-  PairLines<double> p;
+  PairLines<double> p{};
   const int64_t w = ADD_T ? row * g.px + i0 : row * g.d.ny * g.px + i0;  // first line's first row in the padded arrays
   const int64_t wst = ADD_T ? g.d.ny * g.px : g.px;
   p.W = g.W + w;

@@ -157,6 +157,8 @@ struct XProblem {
   const double* qshape;
   R* W0;                 // row pitch px
   int64_t px;
+  const R* in;           // x_solve_lines with SCALE: the right-hand sides are in * sc (row pitch px), the solution W0
+  const R* sc;
 };
 
 // What the stencil knows of an x-line of its CTA (in shared memory): its first voxel, its first entry of the block
@@ -318,13 +320,13 @@ template <typename R>
 __host__ __device__ constexpr int x_coef_elems() {
   return (kXAhead + 1) * kXCols + x_pad<R>();
 }
-template <typename R, bool TWO, bool TABLE, bool KEEP>
+template <typename R, bool TWO, bool TABLE, bool KEEP, bool SCALE = false>
 __host__ __device__ constexpr size_t x_solve_smem(int64_t max_nx) {  // per warp
-  return sizeof(R) * 32 * (size_t)(x_row_elems<R, TWO, KEEP>(max_nx) + (TABLE ? 0 : x_coef_elems<R>()));
+  return sizeof(R) * 32 * (size_t)(x_row_elems<R, TWO, KEEP>(max_nx) + ((TABLE ? 0 : 1) + (SCALE ? 1 : 0)) * x_coef_elems<R>());
 }
 
 // The x-lines [L0, L0 + count) of W0 (count <= x_lines), in place.  One warp; smem: its own.
-template <typename R, bool TWO, bool TABLE, bool KEEP>
+template <typename R, bool TWO, bool TABLE, bool KEEP, bool SCALE = false>
 __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, int count, R* smem) {
   constexpr int RB = kXCols, LA = kXAhead, VEC = 16 / (int)sizeof(R), LPB = RB / VEC;  // pieces per line and block
   const int lane = threadIdx.x & 31, n = (int)P.nx;
@@ -342,8 +344,11 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
   const int rw = x_row_elems<R, TWO, KEEP>(P.nx);
   R* row = smem + lane * rw;
   R* crow = smem + 32 * rw + lane * x_coef_elems<R>();
+  const R* srow = crow + (TABLE ? 0 : 32 * x_coef_elems<R>());  // SCALE: the ring of the scale
+  const R* in = SCALE ? P.in : P.W0;
   const uint32_t rows_s = (uint32_t)__cvta_generic_to_shared(smem);
   const uint32_t coef_s = rows_s + 32 * rw * (uint32_t)sizeof(R);
+  const uint32_t scale_s = coef_s + (TABLE ? 0 : 32 * x_coef_elems<R>() * (uint32_t)sizeof(R));
   // position of block q in a row.  Right ends hold a block's columns in ascending order, so slot t of the block is at
   // RB - 1 - t
   auto slot = [&](int q) { return (KEEP ? q : q % (LA + 1)) * RB; };
@@ -394,14 +399,16 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
   auto tab = [&](int c) { return TABLE && c > m ? m + n - c : c; };  // table position of a column
   R wm = 0, am = 0, bm = 0;  // the middle column
   if (TWO) {
-    wm = P.W0[L * P.px + m];
+    wm = in[L * P.px + m];
+    if (SCALE) wm *= P.sc[L * P.px + m];
     am = A[tab(m)];
     bm = B[tab(m)];
   }
   const int start = upper ? m + 1 - skip : 0;  // table position of slot 0
   auto issue = [&](int i, bool may_turn) {
     if (i < nb) {
-      copy(P.W0, P.px, rows_s, rw, slot(i), i);
+      copy(in, P.px, rows_s, rw, slot(i), i);
+      if (SCALE) copy(P.sc, P.px, scale_s, x_coef_elems<R>(), cslot(i), i);
       if (!TABLE) copy(P.a0, P.px, coef_s, x_coef_elems<R>(), cslot(i), i);
     } else if (may_turn && i < 2 * nb) {
       const int q = 2 * nb - 1 - i;
@@ -433,12 +440,12 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
     cp_async_wait_pending<LA - 1>();
     __syncwarp();
     R* at = row + slot(q) + o;
-    const R* cat = crow + cslot(q) + o;
+    const R *cat = crow + cslot(q) + o, *sat = srow + cslot(q) + o;
     R a[RB], w[RB];
 #pragma unroll
     for (int k = 0; k < RB; ++k) {
       a[k] = TABLE ? next[k] : cat[d * k];
-      w[k] = at[d * k];
+      w[k] = SCALE ? at[d * k] * sat[d * k] : at[d * k];
     }
     if (TABLE) load(q + 1 < nb ? A : B, q + 1 < nb ? q + 1 : nb - 1);
     issue(q + LA, KEEP);
@@ -686,14 +693,14 @@ inline bool x_fused(int64_t nx, int64_t lines) {
 }
 
 // How a launch of the line solves over `groups` warps runs (as pair_shape)
-template <typename R, bool TWO, bool TABLE>
+template <typename R, bool TWO, bool TABLE, bool SCALE = false>
 inline PairShape x_solve_shape(int64_t max_nx, int64_t groups, int force_keep = -1) {
   constexpr size_t kSmem = 227 * 1024, kReserved = 1024;
-  const size_t held = x_solve_smem<R, TWO, TABLE, true>(max_nx);
+  const size_t held = x_solve_smem<R, TWO, TABLE, true, SCALE>(max_nx);
   const int64_t per = (int64_t)(kSmem / (held + kReserved));
   PairShape sh;
   sh.keep = per > 0 && (force_keep >= 0 ? force_keep != 0 : per >= 8 || groups <= 152 * per);
-  const size_t each = sh.keep ? held : x_solve_smem<R, TWO, TABLE, false>(max_nx);
+  const size_t each = sh.keep ? held : x_solve_smem<R, TWO, TABLE, false, SCALE>(max_nx);
   sh.warps = 1;
   while (sh.warps < kPairMaxWarps && groups >= 152 * 8 * sh.warps && 2 * sh.warps * each <= 64 * 1024) sh.warps *= 2;
   sh.smem = each * sh.warps;

@@ -410,3 +410,43 @@ def test_errors(cuda_ok):
         a.set_parameters(np.ones((2, 3, 4)), -np.ones((2, 3, 4)), np.zeros((2, 3, 4)))
     with pytest.raises(ValueError):
         a.set_parameters(np.ones((2, 3, 5)), np.ones((2, 3, 4)), np.zeros((2, 3, 4)))
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 16), (2, 1, 15), (3, 3, 17), (15, 18, 33), (16, 17, 1), (17, 16, 31),
+                                   (33, 15, 16), (18, 33, 47), (2, 3, 130), (2, 130, 3), (130, 2, 3)])
+def test_line_solves_at_their_edges(cuda_ok, shape):
+    """Lines around the blocks of eight rows of a half line, rows around the warps' 16 lines and the pads of odd rows:
+    state, loss and gradients as above against autograd."""
+    dt, N = 0.01, 5
+    p = _problem(6, shape, N)
+    a, (loss, T) = _adjoint(p, dt, 2, return_state=True)
+    g = a.backward()
+    states = TA.run(torch.tensor(p["T0"]), torch.tensor(p["k"]), torch.tensor(p["C"]), torch.tensor(p["q"]),
+                    p["schedule"], dt, p["spacing"])
+    assert rel_err(T, states[-1].numpy()) <= 1e-12
+    tk = [torch.tensor(p[n], requires_grad=True) for n in ("k", "C", "q", "T0")]
+    J = TA.misfit(tk[3], tk[0], tk[1], tk[2], p["schedule"], torch.tensor(p["obs"]), dt, p["spacing"])
+    J.backward()
+    assert abs(loss[0] - J.item()) <= 1e-12 * J.item()
+    for name, mine, t in zip(("k", "C", "q", "T0"), g, tk):
+        assert rel_err(mine, t.grad.numpy()) <= 1e-10, name
+
+
+@pytest.mark.parametrize("shape", [(4, 700, 160), (700, 4, 160), (4, 100, 1000)])
+def test_long_lines_through_shared_and_global_memory(cuda_ok, shape):
+    """Forward values of long lines stay in shared memory in a single instance and go through global memory in a batch
+    (more warps than that leaves room for): the same bits."""
+    dt, N = 0.005, 3
+    probs = [_problem(60 + i, shape, N) for i in range(8)]
+    for p in probs[1:]:
+        p["schedule"] = probs[0]["schedule"]
+    b = Adjoint([(p["shape"], p["spacing"]) for p in probs], dt)
+    b.set_parameters([p["k"] for p in probs], [p["C"] for p in probs], [p["q"] for p in probs])
+    lb = b.forward([p["T0"] for p in probs], [p["obs"] for p in probs], probs[0]["schedule"], 2)
+    gb = b.backward()
+    for i in (0, 7):
+        a, la = _adjoint(probs[i], dt, 2)
+        ga = a.backward()
+        assert lb[i] == la[0]
+        for x, y in zip(gb, ga):
+            np.testing.assert_array_equal(x[i], y)
