@@ -84,7 +84,7 @@ __device__ __forceinline__ Line line_at(const AView& v, int axis, int64_t t) {
 }
 
 struct Vox {
-  int64_t i, j, k, nx, ny, nz, px, nxy;  // nxy: voxels from one layer to the next
+  int i, j, k, nx, ny, nz, px, nxy;  // nxy: voxels from one layer to the next
   int inst;
   bool in;  // false: a pad of its row
 };
@@ -96,7 +96,7 @@ __device__ __forceinline__ Vox vox_at(const AView& v, int64_t p) {
   const uint32_t row = l / px, k = row / ny;
   Vox r;
   r.inst = n;
-  r.nx = in.nx; r.ny = in.ny; r.nz = in.nz; r.px = in.px; r.nxy = in.px * in.ny;
+  r.nx = (int)in.nx; r.ny = (int)in.ny; r.nz = (int)in.nz; r.px = (int)in.px; r.nxy = (int)(in.px * in.ny);
   r.i = l - row * px; r.j = row - k * ny; r.k = k;
   r.in = r.i < r.nx;
   return r;
@@ -142,6 +142,20 @@ __global__ void adj_setup_kernel(AView v, const double* __restrict__ k, const do
 // identity rows with couplings from computed neighbours are not), so the adjoint's transposed solves remain
 // the forward solves.
 constexpr double kFixedCapacity = 1e300;
+
+// Whether s v is more than a zero: without the FP64 unit, whose instructions are what the voxel kernels wait for.  (A
+// product with zero is NaN when v is infinite or NaN.)
+__device__ __forceinline__ bool adds_something(double s, double v) {
+  return ((uint64_t)__double_as_longlong(s) << 1) != 0 ||
+         ((uint64_t)__double_as_longlong(v) << 1) >= (uint64_t(0x7ff) << 53);
+}
+// false, unknown to the compiler: `while (again) { ...; again = never(); }` is a branch that stays one, where the FP64
+// instructions of an `if` would be issued with a predicate, whether or not it holds
+__device__ __forceinline__ bool never() {
+  unsigned zero;
+  asm volatile("mov.u32 %0, 0;" : "=r"(zero));
+  return zero != 0;
+}
 
 // The same with face classes and fixed voxels: the conductance of a face of class c on axis a is the class's
 // affine form f0 + flo k_lo + fhi k_hi, the k of a fixed side replaced by its computed neighbour's
@@ -201,8 +215,10 @@ __global__ void adj_diag_kernel(AView v, const double* __restrict__ gx, const do
 // conductance towards the middle,
 //     z_r = W_r - a_r z_{r -+ 1},   x_r = z_r - b_r x_{r +- 1}   (lower, upper end),
 //     x_m = W_m - a_m z_{m-1} - b_m z_{m+1},   W = rhs scale.
-// Kept: -a = G / (2 p) of the face away from the middle, -b = G / (2 p) of the face towards it, ip = 1 / p and
-// mip = M / p, the scale of b = rhs and of b = M rhs.  A pair of lanes takes a line, one end each.
+// Kept: -a = G / (2 p) of the face away from the middle, -b = G / (2 p) of the face towards it, ip = 1 / p (x: half of
+// it, see adj_update_kernel) and mip = M / p, the scale of b = rhs and of b = M rhs.  A pair of lanes takes a line, one
+// end each.  FP64 arithmetic bounds the kernel on many lines: one reciprocal per row and quotients from it by one
+// correction step, 5.86 million voxels 688 us on the three axes against 865 with two divisions.
 __global__ void adj_factor_kernel(AView v, int axis, int64_t nlines, const double* __restrict__ M,
                                   const double* __restrict__ g, double* __restrict__ a, double* __restrict__ b,
                                   double* __restrict__ ip, double* __restrict__ mip) {
@@ -213,15 +229,18 @@ __global__ void adj_factor_kernel(AView v, int axis, int64_t nlines, const doubl
   const int64_t rows = upper ? ln.len - 1 - m : m;
   const int64_t d = upper ? -ln.stride : ln.stride;
   int64_t p = ln.base + (upper ? (ln.len - 1) * ln.stride : 0);
+  const double one = axis == 0 ? 0.5 : 1.0;
   double away = 0.0, drop = 0.0;  // half the conductance away from the middle, and what it takes from the pivot
   for (int64_t r = 0; r < rows; ++r, p += d) {
     const double in = 0.5 * g[upper ? p : p + ln.stride];
     const double m0 = M[p], piv = m0 + (away + in) - drop, inv = 1.0 / piv;
+    double bb = __dmul_rn(in, inv);
+    bb = __fma_rn(__fma_rn(-bb, piv, in), inv, bb);  // in / piv
     a[p] = away * inv;
-    b[p] = in / piv;
-    ip[p] = inv;
+    b[p] = bb;
+    ip[p] = one * inv;
     mip[p] = __dmul_rn(m0, inv);
-    drop = in * (in / piv);
+    drop = in * bb;
     away = in;
   }
   const double away_up = __shfl_xor_sync(0xffffffffu, away, 1), drop_up = __shfl_xor_sync(0xffffffffu, drop, 1);
@@ -229,13 +248,14 @@ __global__ void adj_factor_kernel(AView v, int axis, int64_t nlines, const doubl
     const double m0 = M[p], piv = m0 + (away + away_up) - drop - drop_up, inv = 1.0 / piv;
     a[p] = away * inv;
     b[p] = away_up * inv;
-    ip[p] = inv;
+    ip[p] = one * inv;
     mip[p] = __dmul_rn(m0, inv);
   }
 }
 
 // r0 = s q - D T_p + sum over faces of G T_nbr at voxel p = (k, j, i) of an (nz, ny, nx) instance (D = the sum
-// of the six G): 8 FP64 operations against 13 for the face-by-face differences; temperatures are offsets
+// of the six G): 8 FP64 operations against 13 for the face-by-face differences (skipping the source where s = 0, as
+// adj_update_kernel does, made it slower: 110 us against 97 for 5.86 million voxels); temperatures are offsets
 // from their initial mean, so the cancellation in -D T_p + sum G T_nbr stays at the rounding of the increments
 __device__ __forceinline__ double residual_at(const double* __restrict__ T, const double* __restrict__ gx,
                                               const double* __restrict__ gy, const double* __restrict__ gz,
@@ -251,7 +271,8 @@ __device__ __forceinline__ double residual_at(const double* __restrict__ T, cons
   return r;
 }
 
-// the right-hand sides of the forward x stage, W = r0 ip
+// the right-hand sides of the forward x stage, W = r0 ip (half of them, as ip is halved).  FP64 arithmetic bounds it:
+// 5.86 million voxels 97 us.
 __global__ void adj_resid_kernel(AView v, const double* __restrict__ T, const double* __restrict__ gx,
                                  const double* __restrict__ gy, const double* __restrict__ gz,
                                  const double* __restrict__ D, const double* __restrict__ q, double s,
@@ -301,7 +322,7 @@ __global__ void __launch_bounds__(32 * kPairMaxWarps) adj_x_kernel(AView v, int6
 }
 // y (axis 1) or z (axis 2) lines, y = A_a^-1 (scale rhs); ADD_T: T_out = T_in + y (which may be the same), y itself
 // only when given, Z the scratch of the forward values, and with obs the top layer's T_out - obs of step obs_step in
-// obs's place
+// obs's place (y is half the increment: T_out = T_in + 2 y)
 template <bool ADD_T, bool KEEP>
 __global__ void __launch_bounds__(32 * kPairMaxWarps) adj_pair_kernel(AView v, int axis, int64_t ngroups,
                                                                       const double* rhs, const double* __restrict__ a,
@@ -358,54 +379,85 @@ __global__ void adj_seed_kernel(AView v, const double* __restrict__ diff, int64_
 }
 
 // lambda += L mu0 (+ the misfit gradient of observation obs_step, from diff, when obs_step >= 0), and the
-// gradient accumulation of one step; one thread per voxel, each voxel owning its three low faces
-__global__ void adj_update_kernel(AView v, const double* __restrict__ gx, const double* __restrict__ gy,
-                                  const double* __restrict__ gz, const double* __restrict__ T,
-                                  const double* __restrict__ y0, const double* __restrict__ y1,
-                                  const double* __restrict__ y2, const double* __restrict__ mu0,
-                                  const double* __restrict__ mu1, const double* __restrict__ mu2, double s,
-                                  const double* __restrict__ diff, int64_t obs_step, double* __restrict__ lam,
-                                  double* __restrict__ ggx, double* __restrict__ ggy, double* __restrict__ ggz,
-                                  double* __restrict__ gM, double* __restrict__ gq) {
+// gradient accumulation of one step; one thread per voxel, each voxel owning its three low faces.
+// FP64 arithmetic bounds it, so what can be had without is: the increments h = y / 2 are halved (the x stage's scale
+// is, exactly, and with it what follows), which takes the factors 1/2 out of the face gradients; a voxel's
+// T + h0 and its difference of mu0 to the left are formed once and shared through shared memory with the
+// neighbour that needs them; the source gradient is skipped where s = 0.  gM accumulates half its value.
+// 29 operations (30 with a source) against 34, five CTAs to an SM (48 registers): 5.86 million voxels 323 us
+// against 375 (the FP64 unit 84% busy; 22 fields of 8 bytes take 154).
+constexpr int kUpdateThreads = 256;
+__global__ void __launch_bounds__(kUpdateThreads, 5) adj_update_kernel(
+    AView v, const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
+    const double* __restrict__ T, const double* __restrict__ h0, const double* __restrict__ h1,
+    const double* __restrict__ h2, const double* __restrict__ mu0, const double* __restrict__ mu1,
+    const double* __restrict__ mu2, double s, const double* __restrict__ diff, int64_t obs_step,
+    double* __restrict__ lam, double* __restrict__ ggx, double* __restrict__ ggy, double* __restrict__ ggz,
+    double* __restrict__ gM, double* __restrict__ gq) {
+  __shared__ double sw[kUpdateThreads + 1], sd[kUpdateThreads + 1];
+  const int t = threadIdx.x;
+  const int64_t p0 = blockIdx.x * (int64_t)kUpdateThreads, p = p0 + t;
+  Vox x{};
+  if (p < v.nvox) x = vox_at(v, p);
   wait_prior_grid();  // the previous kernel on the stream (programmatic dependent launch)
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= v.nvox) return;
-  const Vox x = vox_at(v, p);
+  double m0 = 0.0, Tp = 0.0, a0 = 0.0, d0x = 0.0, w = 0.0;
+  if (x.in) {
+    m0 = mu0[p];
+    Tp = T[p];
+    a0 = h0[p];
+    w = Tp + a0;
+    if (x.i > 0) d0x = m0 - mu0[p - 1];
+  }
+  sw[t + 1] = w;
+  sd[t] = d0x;
+  // the neighbours beyond the block (read by voxels of their row alone): T + h0 on the left, mu0's difference on the right
+  if (t < 2) {
+    const int64_t r = p0 + kUpdateThreads;
+    const double *b0 = t ? mu0 + r : T + p0 - 1, *b1 = t ? mu0 + r - 1 : h0 + p0 - 1;
+    double e0 = 0.0, e1 = 0.0;
+    if (t ? r < v.nvox : p0 > 0) {
+      e0 = *b0;
+      e1 = *b1;
+    }
+    if (t) e1 = -e1;
+    (t ? sd[kUpdateThreads] : sw[0]) = e0 + e1;
+  }
+  __syncthreads();
   if (!x.in) return;
-  const double m0 = mu0[p], Tp = T[p];
-  const double m1 = mu1[p], m2 = mu2[p];
-  const double a0 = y0[p], a1 = y1[p], a2 = y2[p];
-  // each low-face difference of mu0 serves both lambda's update (L mu0) and that face's gradient
+  const double m1 = mu1[p], m2 = mu2[p], a1 = h1[p], a2 = h2[p];
   double l = lam[p];
   if (x.i > 0) {
-    const int64_t q = p - 1;
-    const double d0 = m0 - mu0[q];
-    l = fma(-gx[p], d0, l);
-    ggx[p] = fma(-d0, fma(0.5, a0 - y0[q], Tp - T[q]), ggx[p]);
+    l = fma(-gx[p], d0x, l);
+    ggx[p] = fma(-d0x, w - sw[t], ggx[p]);
   }
   if (x.j > 0) {
     const int64_t q = p - x.px;
     const double d0 = m0 - mu0[q];
     l = fma(-gy[p], d0, l);
-    ggy[p] = fma(-0.5 * (m1 - mu1[q]), a1 - y1[q], fma(-d0, Tp - T[q], ggy[p]));
+    ggy[p] = fma(-(m1 - mu1[q]), a1 - h1[q], fma(-d0, Tp - T[q], ggy[p]));
   }
   if (x.k > 0) {
     const int64_t q = p - x.nxy;
     const double d0 = m0 - mu0[q];
     l = fma(-gz[p], d0, l);
-    ggz[p] = fma(-0.5 * (m2 - mu2[q]), a2 - y2[q], fma(-d0, Tp - T[q], ggz[p]));
+    ggz[p] = fma(-(m2 - mu2[q]), a2 - h2[q], fma(-d0, Tp - T[q], ggz[p]));
   }
-  if (x.i + 1 < x.nx) l = fma(gx[p + 1], mu0[p + 1] - m0, l);
+  if (x.i + 1 < x.nx) l = fma(gx[p + 1], sd[t + 1], l);
   if (x.j + 1 < x.ny) l = fma(gy[p + x.px], mu0[p + x.px] - m0, l);
   if (x.k + 1 < x.nz) l = fma(gz[p + x.nxy], mu0[p + x.nxy] - m0, l);
-  if (obs_step >= 0 && x.k == 0) {
-    const AInst& in = v.inst[x.inst];
-    l += 2.0 * diff[in.obs_off + (obs_step * x.ny + x.j) * x.nx + x.i];
+  bool again = obs_step >= 0 && x.k == 0;
+  while (again) {
+    l += 2.0 * diff[v.inst[x.inst].obs_off + (obs_step * x.ny + x.j) * x.nx + x.i];
+    again = never();
   }
   lam[p] = l;
-  // mu2 y1 + mu1 y0 - mu0 y0 - mu1 y1 - mu2 y2 = mu2 (y1 - y2) + mu1 (y0 - y1) - mu0 y0
+  // half of mu2 y1 + mu1 y0 - mu0 y0 - mu1 y1 - mu2 y2 = mu2 (y1 - y2) + mu1 (y0 - y1) - mu0 y0
   gM[p] = fma(m2, a1 - a2, fma(m1, a0 - a1, fma(-m0, a0, gM[p])));
-  gq[p] = fma(s, m0, gq[p]);
+  again = adds_something(s, m0);
+  while (again) {
+    gq[p] = fma(s, m0, gq[p]);
+    again = never();
+  }
 }
 
 // s + v as an unevaluated pair: returns the rounded sum, err receives its exact rounding error (Knuth's TwoSum)
@@ -454,9 +506,9 @@ __global__ void adj_misfit_kernel(AView v, const double* __restrict__ diff, int6
   }
 }
 
-// chain to the parameters: gk from the face gradients (G = (k_lo + k_hi) / (2 d^2)), gC = gM / dt
+// chain to the parameters: gk from the face gradients (G = (k_lo + k_hi) / (2 d^2)), gC = 2 gM / dt (gM is half)
 __global__ void adj_chain_kernel(AView v, const double* __restrict__ ggx, const double* __restrict__ ggy,
-                                 const double* __restrict__ ggz, const double* __restrict__ gM, double inv_dt,
+                                 const double* __restrict__ ggz, const double* __restrict__ gM, double two_inv_dt,
                                  double* __restrict__ gk, double* __restrict__ gC) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= v.nvox) return;
@@ -471,13 +523,13 @@ __global__ void adj_chain_kernel(AView v, const double* __restrict__ ggx, const 
   if (x.k > 0) fz += ggz[p];
   if (x.k + 1 < x.nz) fz += ggz[p + x.nxy];
   gk[p] = 0.5 * (in.idx2 * fx + in.idy2 * fy + in.idz2 * fz);
-  gC[p] = gM[p] * inv_dt;
+  gC[p] = gM[p] * two_inv_dt;
 }
 
 // The chain with face classes: d G_f / d k of each side from the face's affine form (both coefficients to the
 // computed side of a face with a fixed neighbour); no gradient for fixed voxels' k, C and q.
 __global__ void adj_chain_faces_kernel(AView v, const double* __restrict__ ggx, const double* __restrict__ ggy,
-                                       const double* __restrict__ ggz, const double* __restrict__ gM, double inv_dt,
+                                       const double* __restrict__ ggz, const double* __restrict__ gM, double two_inv_dt,
                                        const uint8_t* __restrict__ fcls, int nclass, const double* __restrict__ forms,
                                        const uint8_t* __restrict__ fixed, double* __restrict__ gk,
                                        double* __restrict__ gC, double* __restrict__ gq) {
@@ -512,7 +564,7 @@ __global__ void adj_chain_faces_kernel(AView v, const double* __restrict__ ggx, 
     }
   }
   gk[p] = acc;
-  gC[p] = gM[p] * inv_dt;
+  gC[p] = gM[p] * two_inv_dt;
 }
 
 }  // namespace
@@ -691,7 +743,9 @@ cudaError_t bwd_step(hs2g_adjoint* a, const double* Tn, const double* y0, const 
   if (e == cudaSuccess) e = ysolve(a, st, 1, true, a->mu[2], a->mu[1]);
   if (e == cudaSuccess) e = xsolve<true>(a, st, a->mu[1], a->mu[0]);
   if (e == cudaSuccess)
-    e = launch_kernel(hs2g::adj_update_kernel, dim3(nblk(a->n)), dim3(kTh), 0, st, adj_pdl(), view(a), a->g[0], a->g[1],
+    e = launch_kernel(hs2g::adj_update_kernel,
+                      dim3((unsigned)((a->n + hs2g::kUpdateThreads - 1) / hs2g::kUpdateThreads)),
+                      dim3(hs2g::kUpdateThreads), 0, st, adj_pdl(), view(a), a->g[0], a->g[1],
                       a->g[2], Tn, y0, y1, y2, a->mu[0], a->mu[1], a->mu[2], s, a->obs, obs_step, a->lam, a->gg[0],
                       a->gg[1], a->gg[2], a->gM, a->gq);
   return e;
@@ -1113,11 +1167,11 @@ int hs2g_adjoint_backward(hs2g_adjoint* a, double* gk, double* gC, double* gq, d
   }
   if (e == cudaSuccess) {
     if (a->forms)
-      hs2g::adj_chain_faces_kernel<<<nblk(n), kTh, 0, st>>>(v, a->gg[0], a->gg[1], a->gg[2], a->gM, 1.0 / a->dt,
+      hs2g::adj_chain_faces_kernel<<<nblk(n), kTh, 0, st>>>(v, a->gg[0], a->gg[1], a->gg[2], a->gM, 2.0 / a->dt,
                                                             a->fcls, a->nclass, a->forms, a->fixed, a->mu[0],
                                                             a->mu[1], a->gq);
     else
-      hs2g::adj_chain_kernel<<<nblk(n), kTh, 0, st>>>(v, a->gg[0], a->gg[1], a->gg[2], a->gM, 1.0 / a->dt,
+      hs2g::adj_chain_kernel<<<nblk(n), kTh, 0, st>>>(v, a->gg[0], a->gg[1], a->gg[2], a->gM, 2.0 / a->dt,
                                                       a->mu[0], a->mu[1]);
     e = cudaGetLastError();
   }

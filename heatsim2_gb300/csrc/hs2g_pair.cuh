@@ -66,7 +66,7 @@ struct PairLines {
   int64_t st;
   R* Z;
   int64_t zst;
-  const R* sc;  // SCALE: the right-hand sides are W * sc, laid out like W
+  const R* sc;  // SCALE: the right-hand sides are W * sc, laid out like W; ADD_T then adds 2 x to T
   R* X;         // SCALE, ADD_T: x itself is stored here too, unless null (laid out like W; may be Z)
 };
 
@@ -257,12 +257,13 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
         }
     }
   }
+  auto plus = [](R t, R x) { return SCALE ? fma(R(2), x, t) : t + x; };
   R x = 0;
   if (TWO) {
     const R other = __shfl_xor_sync(0xffffffffu, z, 16);
     x = fma(bm, upper ? z : other, fma(am, upper ? other : z, wm));  // the same value in both halves
     if (!upper && live) {
-      p.out[m * p.st + mine] = ADD_T ? tm + x : x;
+      p.out[m * p.st + mine] = ADD_T ? plus(tm, x) : x;
       if (SCALE && ADD_T && p.X) p.X[m * p.wst + mine] = x;
     }
   }
@@ -294,7 +295,7 @@ __device__ __forceinline__ void pair_solve(const PairLines<R>& p, int n, int wid
     __syncwarp();
     issue(i + LA, true);
     auto put = [&](int k) {
-      if (live) *oc = ADD_T ? tt[k] + x : x;
+      if (live) *oc = ADD_T ? plus(tt[k], x) : x;
       oc = step_bytes(oc, -dT);
       if (SCALE && ADD_T && xc) {
         if (live) *xc = x;
