@@ -607,7 +607,7 @@ struct hs2g_adjoint {
   double* ckpts = nullptr;  // ceil(nsteps / ckpt) * n
   double* seg = nullptr;    // ckpt * 4 * n: T, y0, y1, y2 of each step of a segment
   double* seg2 = nullptr;   // a second segment store: the next segment is recomputed while this one is swept
-  int stored_seg = -1;      // the segment whose states the last forward pass left in its store (-1: none)
+  int stored_from = -1;     // the last forward pass left the states of the segments from here on in the stores (-1: none)
   cudaStream_t rec_stream = nullptr;  // the recompute stream
   cudaEvent_t ev_rec[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr}, ev_start = nullptr;
   double* T = nullptr;      // forward state
@@ -931,7 +931,7 @@ int hs2g_adjoint_set_parameters(hs2g_adjoint* a, const double* k, const double* 
   const cudaMemcpyKind kind = in_kind(flags);
   a->have_params = false;
   a->nsteps = 0;
-  a->stored_seg = -1;
+  a->stored_from = -1;
   cudaError_t e = copy_in(a, a->k, k, kind, a->mu[0], st);
   if (e == cudaSuccess) e = copy_in(a, a->C, C, kind, a->mu[1], st);
   if (e == cudaSuccess) e = copy_in(a, a->q, q, kind, a->mu[2], st);
@@ -975,7 +975,7 @@ int hs2g_adjoint_set_faces(hs2g_adjoint* a, int nclass, const double* forms, con
     a->nclass = 0;
     a->have_params = false;
     a->nsteps = 0;
-    a->stored_seg = -1;
+    a->stored_from = -1;
     return HS2G_OK;
   }
   if (!a || nclass < 1 || nclass > HS2G_MAX_CLASSES || !forms || !face_z || !face_y || !face_x)
@@ -1015,7 +1015,7 @@ int hs2g_adjoint_set_faces(hs2g_adjoint* a, int nclass, const double* forms, con
   if (e != cudaSuccess) return acuda(e, "hs2g_adjoint_set_faces");
   a->have_params = false;  // the faces apply from the next hs2g_adjoint_set_parameters
   a->nsteps = 0;
-  a->stored_seg = -1;
+  a->stored_from = -1;
   return HS2G_OK;
 }
 
@@ -1044,31 +1044,32 @@ int hs2g_adjoint_forward(hs2g_adjoint* a, int nsteps, const double* schedule, co
   if (e == cudaSuccess) e = copy_in(a, a->T, T0, in_kind(flags), a->mu[0], st);
   if (e == cudaSuccess) e = cudaEventRecord(a->ev0, st);
   a->sched.assign(schedule, schedule + nsteps);
-  a->stored_seg = -1;
-  // The last segment's states (T, y0, y1, y2 of each step, the layout the recompute writes) go straight into
-  // the segment store the backward pass sweeps first, when the stores already exist from an earlier backward
-  // pass: that pass then skips its first recompute, the one nothing overlaps.  The same kernels compute the
-  // same states, so the gradients do not change.
+  a->stored_from = -1;
+  // The states of the last two segments (T, y0, y1, y2 of each step, the layout the recompute writes) go straight into
+  // the two stores, which the backward pass sweeps first, when the stores already exist from an earlier backward pass:
+  // that pass then recomputes neither.  The same kernels compute the same states, so the gradients do not change.
+  // (With the last segment alone, six instances of 5.86 million voxels, 40 steps in segments of 10: 41.3 ms; with both
+  // 39.2.)
   const int64_t seg_need = (int64_t)ckpt * 4 * n;
-  double* store = nullptr;
+  double* stores[2] = {a->seg, a->seg2};
+  int64_t from = nck;
   if (a->seg && a->seg_cap >= seg_need && (nck == 1 || (a->seg2 && a->seg2_cap >= seg_need)))
-    store = ((nck - 1) & 1) ? a->seg2 : a->seg;
-  const int s_store = store ? (int)((nck - 1) * ckpt) : nsteps;
+    from = std::max<int64_t>(0, nck - 2);
   const hs2g::AView v = view(a);
   for (int s = 0; s < nsteps && e == cudaSuccess; ++s) {
-    if (s % ckpt == 0)
-      e = cudaMemcpyAsync(a->ckpts + (int64_t)(s / ckpt) * n, a->T, sizeof(double) * n, cudaMemcpyDeviceToDevice,
-                          st);
-    if (s < s_store) {
-      // the adjoint buffers are free during the forward pass and hold the increments
-      if (e == cudaSuccess) e = fwd_step(a, st, a->T, a->T, a->mu[0], a->mu[1], a->mu[2], false, a->sched[s], s);
-    } else {
-      double* slot = store + (int64_t)(s - s_store) * 4 * n;
-      if (s == s_store && e == cudaSuccess)
-        e = cudaMemcpyAsync(slot, a->T, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
-      double* out = s + 1 < nsteps ? slot + 4 * n : a->T;
-      if (e == cudaSuccess) e = fwd_step(a, st, slot, out, slot + n, slot + 2 * n, slot + 3 * n, true, a->sched[s], s);
+    const int sg = s / ckpt, j = s - sg * ckpt;
+    const bool kept = sg >= from;
+    double* slot = kept ? stores[sg & 1] + (int64_t)j * 4 * n : nullptr;
+    if (j == 0) {
+      e = cudaMemcpyAsync(a->ckpts + (int64_t)sg * n, a->T, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
+      if (kept && e == cudaSuccess) e = cudaMemcpyAsync(slot, a->T, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
     }
+    if (e != cudaSuccess) break;
+    if (kept)  // a segment's last state goes back to T
+      e = fwd_step(a, st, slot, j + 1 < ckpt && s + 1 < nsteps ? slot + 4 * n : a->T, slot + n, slot + 2 * n,
+                   slot + 3 * n, true, a->sched[s], s);
+    else       // the adjoint buffers are free during the forward pass and hold the increments
+      e = fwd_step(a, st, a->T, a->T, a->mu[0], a->mu[1], a->mu[2], false, a->sched[s], s);
   }
   for (int s = 0; s < nsteps && e == cudaSuccess; s += 65535) {  // a launch's limit on z
     hs2g::adj_misfit_kernel<<<dim3(hs2g::kMisfitBlocks, a->ninst, std::min(nsteps - s, 65535)), 256, 0, st>>>(
@@ -1096,7 +1097,7 @@ int hs2g_adjoint_forward(hs2g_adjoint* a, int nsteps, const double* schedule, co
   }
   a->nsteps = nsteps;
   a->ckpt = ckpt;
-  a->stored_seg = store ? (int)(nck - 1) : -1;
+  a->stored_from = from < nck ? (int)from : -1;
   return HS2G_OK;
 }
 
@@ -1120,9 +1121,9 @@ int hs2g_adjoint_backward(hs2g_adjoint* a, double* gk, double* gC, double* gq, d
     if (!dbl) cudaGetLastError();  // out of memory for the second store: recompute and sweep in turn
   }
   double* bufs[2] = {a->seg, dbl ? a->seg2 : a->seg};
-  // the last forward pass may have left the last segment in its store (see hs2g_adjoint_forward)
-  const bool stored = a->stored_seg == nseg - 1 && (nseg == 1 || dbl);
-  a->stored_seg = -1;
+  // the last forward pass may have left the last segments in the stores (see hs2g_adjoint_forward)
+  const int from = a->stored_from >= 0 && (nseg == 1 || dbl) ? a->stored_from : nseg;
+  a->stored_from = -1;
   e = cudaEventRecord(a->ev0, st);
   double* zero_list[] = {a->gg[0], a->gg[1], a->gg[2], a->gM, a->gq};
   for (double* p : zero_list)
@@ -1147,14 +1148,14 @@ int hs2g_adjoint_backward(hs2g_adjoint* a, double* gk, double* gC, double* gq, d
     if (r == cudaSuccess && dbl) r = cudaEventRecord(a->ev_rec[sg & 1], rs);
     return r;
   };
-  if (e == cudaSuccess && !stored) e = recompute(nseg - 1);
+  if (e == cudaSuccess && from == nseg) e = recompute(nseg - 1);
   for (int sg = nseg - 1; sg >= 0 && e == cudaSuccess; --sg) {
-    if (dbl && sg >= 1) {
+    if (dbl && sg >= 1 && sg - 1 < from) {
       // store (sg-1)&1 was last read by the sweep of segment sg+1
       e = cudaStreamWaitEvent(rs, a->ev_done[(sg - 1) & 1], 0);
       if (e == cudaSuccess) e = recompute(sg - 1);
     }
-    if (e == cudaSuccess && dbl && !(stored && sg == nseg - 1)) e = cudaStreamWaitEvent(st, a->ev_rec[sg & 1], 0);
+    if (e == cudaSuccess && dbl && sg < from) e = cudaStreamWaitEvent(st, a->ev_rec[sg & 1], 0);
     const int s0 = sg * C, s1 = std::min(N, s0 + C);
     const double* buf = bufs[sg & 1];
     for (int s = s1 - 1; s >= s0 && e == cudaSuccess; --s) {
