@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "hs2g_internal.cuh"
+#include "hs2g_few.cuh"
 #include "hs2g_pair.cuh"
 #include "hs2g_x.cuh"
 
@@ -320,52 +321,97 @@ __global__ void __launch_bounds__(32 * kPairMaxWarps) adj_x_kernel(AView v, int6
   x_solve_lines<double, true, false, KEEP, SCALE>(P, L0, (int)min((int64_t)16, in.nz * in.ny - L0),
                                                   reinterpret_cast<double*>(adj_sm + warp * smem_per_warp));
 }
-// y (axis 1) or z (axis 2) lines, y = A_a^-1 (scale rhs); ADD_T: T_out = T_in + y (which may be the same), y itself
-// only when given, Z the scratch of the forward values, and with obs the top layer's T_out - obs of step obs_step in
-// obs's place (y is half the increment: T_out = T_in + 2 y)
-template <bool ADD_T, bool KEEP>
-__global__ void __launch_bounds__(32 * kPairMaxWarps) adj_pair_kernel(AView v, int axis, int64_t ngroups,
-                                                                      const double* rhs, const double* __restrict__ a,
-                                                                      const double* __restrict__ b,
-                                                                      const double* __restrict__ scale, double* y,
-                                                                      double* Z, const double* T_in, double* T_out,
-                                                                      double* obs, int64_t obs_step,
-                                                                      int64_t smem_per_warp) {
+template <bool SCALE>
+__global__ void __launch_bounds__(kFewThreads, 4) adj_few_x_kernel(AView v, const double* rhs,
+                                                                   const double* __restrict__ a,
+                                                                   const double* __restrict__ b,
+                                                                   const double* __restrict__ scale, double* y) {
   extern __shared__ __align__(16) unsigned char adj_sm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t grp = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp;
-  if (grp >= ngroups) return;
-  const int64_t* pre = v.grp_off + axis * (v.ninst + 1);
+  const int i = find_inst(v.grp_off, v.ninst, blockIdx.x);
+  const AInst& in = v.inst[i];
+  const int64_t L0 = (blockIdx.x - v.grp_off[i]) * 16, at = in.off + L0 * in.px;
+  few_x_solve<SCALE>(rhs + at, scale + at, a + at, b + at, y + at, in.px, (int)in.nx,
+                     (int)min((int64_t)16, in.nz * in.ny - L0), reinterpret_cast<double*>(adj_sm),
+                     [] { wait_prior_grid(); });
+}
+
+// y (axis 1) or z (axis 2) lines, y = A_a^-1 (scale rhs); with T_out, T_out = T_in + 2 y (which may be the same; y is
+// half the increment), y itself only when given, Z the scratch of the forward values, and with obs the top layer's
+// T_out - obs of step obs_step in obs's place
+struct APair {
+  int axis;
+  const double *rhs, *a, *b, *scale;
+  double *y, *Z;
+  const double* T_in;
+  double *T_out, *obs;
+  int64_t obs_step;
+};
+// the 16 lines of group grp: their rows and number, and this lane's observation (null: none)
+template <bool ADD_T>
+__device__ __forceinline__ void apair_lines(const AView& v, const APair& g, int64_t grp, PairLines<double>& p, int& n,
+                                            int& width, double*& ob) {
+  const int lane = threadIdx.x & 31;
+  const int64_t* pre = v.grp_off + g.axis * (v.ninst + 1);
   const int i = find_inst(pre, v.ninst, grp);
   const AInst& in = v.inst[i];
   const int64_t l = grp - pre[i], px = in.px, nxy = in.ny * px;
   // y: 16 of a layer's px lines, z: 16 of all ny px (the pads' among them)
   const int64_t gpr = (px + 15) / 16;
-  const int64_t first = axis == 1 ? (l % gpr) * 16 : l * 16;
-  const int width = (int)min((int64_t)16, (axis == 1 ? px : nxy) - first);
-  const int64_t base = in.off + (axis == 1 ? (l / gpr) * nxy : 0) + first;
-  PairLines<double> p{};
-  p.W = rhs + base;
-  p.a = a + base;
-  p.b = b + base;
-  p.sc = scale + base;
-  p.wst = p.cst = p.st = p.zst = axis == 1 ? px : nxy;
-  p.out = (ADD_T ? T_out : y) + base;
+  const int64_t first = g.axis == 1 ? (l % gpr) * 16 : l * 16;
+  width = (int)min((int64_t)16, (g.axis == 1 ? px : nxy) - first);
+  n = (int)(g.axis == 1 ? in.ny : in.nz);
+  const int64_t base = in.off + (g.axis == 1 ? (l / gpr) * nxy : 0) + first;
+  p.W = g.rhs + base;
+  p.a = g.a + base;
+  p.b = g.b + base;
+  p.sc = g.scale + base;
+  p.wst = p.cst = p.st = p.zst = g.axis == 1 ? px : nxy;
+  p.out = (ADD_T ? g.T_out : g.y) + base;
   if (ADD_T) {
-    p.T = T_in + base;
-    p.X = y ? y + base : nullptr;
+    p.T = g.T_in + base;
+    p.X = g.y ? g.y + base : nullptr;
   }
-  p.Z = (ADD_T ? Z : y) + base;
-  double* ob = nullptr;
-  if (ADD_T && obs && lane < width) {
+  p.Z = (ADD_T ? g.Z : g.y) + base;
+  ob = nullptr;
+  if (ADD_T && g.obs && lane < width) {
     const uint32_t at = (uint32_t)first + lane, j = at / (uint32_t)px, c = at - j * (uint32_t)px;
-    if (c < in.nx) ob = obs + in.obs_off + obs_step * in.ny * in.nx + j * in.nx + c;
+    if (c < in.nx) ob = g.obs + in.obs_off + g.obs_step * in.ny * in.nx + j * in.nx + c;
   }
+}
+template <bool ADD_T, bool KEEP>
+__global__ void __launch_bounds__(32 * kPairMaxWarps) adj_pair_kernel(AView v, APair g, int64_t ngroups,
+                                                                      int64_t smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char adj_sm[];
+  const int warp = threadIdx.x >> 5;
+  const int64_t grp = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp;
+  if (grp >= ngroups) return;
+  PairLines<double> p{};
+  int n, width;
+  double* ob;
+  apair_lines<ADD_T>(v, g, grp, p, n, width, ob);
   wait_prior_grid();  // the previous kernel on the stream (programmatic dependent launch)
   const double seen = ob ? *ob : 0.0;
-  pair_solve<double, true, ADD_T, KEEP, false, 2, 2, true>(p, (int)(axis == 1 ? in.ny : in.nz), width,
+  pair_solve<double, true, ADD_T, KEEP, false, 2, 2, true>(p, n, width,
                                                             reinterpret_cast<double*>(adj_sm + warp * smem_per_warp));
-  if (ob) *ob = p.out[lane] - seen;  // row 0 is stored by the lower end's lane
+  if (ob) *ob = p.out[threadIdx.x & 31] - seen;  // row 0 is stored by the lower end's lane
+}
+template <bool ADD_T>
+__global__ void __launch_bounds__(kFewThreads, 4) adj_few_pair_kernel(AView v, APair g) {
+  extern __shared__ __align__(16) unsigned char adj_sm[];
+  PairLines<double> p{};
+  int n, width;
+  double* ob;
+  apair_lines<ADD_T>(v, g, blockIdx.x, p, n, width, ob);
+  if (threadIdx.x >= 32) ob = nullptr;
+  double seen = 0.0;
+  few_solve<ADD_T>(p, n, width, reinterpret_cast<double*>(adj_sm), [&] {
+    wait_prior_grid();  // the previous kernel on the stream (programmatic dependent launch)
+    if (ob) seen = *ob;
+  });
+  if (ADD_T && g.obs) {
+    __syncthreads();  // row 0 is another warp's store
+    if (ob) *ob = p.out[threadIdx.x] - seen;
+  }
 }
 
 // lambda = misfit gradient of the last observation, 2 (T_N - d_{N-1}) on the top layer, 0 below; diff: the forward
@@ -693,32 +739,45 @@ cudaError_t copy_out(const hs2g_adjoint* a, double* dst, const double* src, cuda
 template <bool SCALE>
 cudaError_t xsolve(const hs2g_adjoint* a, cudaStream_t st, const double* rhs, double* y) {
   const int64_t groups = a->ngroups[0];
+  const size_t few = hs2g::few_x_smem<SCALE>(a->max_len[0]);
+  if (hs2g::few_lines(groups, few))
+    return launch_kernel(hs2g::adj_few_x_kernel<SCALE>, dim3((unsigned)groups), dim3(hs2g::kFewThreads), few, st,
+                         adj_pdl(), view(a), SCALE ? rhs : y, a->ca[0], a->cb[0], a->mip[0], y);
   const hs2g::PairShape sh = hs2g::x_solve_shape<double, true, false, SCALE>(a->max_len[0], groups);
   return launch_kernel(sh.keep ? hs2g::adj_x_kernel<SCALE, true> : hs2g::adj_x_kernel<SCALE, false>,
                        dim3((unsigned)((groups + sh.warps - 1) / sh.warps)), dim3(32 * sh.warps), sh.smem, st,
                        adj_pdl(), view(a), groups, SCALE ? rhs : y, a->ca[0], a->cb[0], a->mip[0], y,
                        (int64_t)(sh.smem / sh.warps));
 }
+template <bool ADD_T>
+cudaError_t pair_launch(const hs2g_adjoint* a, cudaStream_t st, const hs2g::APair& g) {
+  const int64_t groups = a->ngroups[g.axis];
+  const size_t few = hs2g::few_smem(a->max_len[g.axis]);
+  if (hs2g::few_lines(groups, few))
+    return launch_kernel(hs2g::adj_few_pair_kernel<ADD_T>, dim3((unsigned)groups), dim3(hs2g::kFewThreads), few, st,
+                         adj_pdl(), view(a), g);
+  const hs2g::PairShape sh = hs2g::pair_shape<double, true, ADD_T, false, true>(a->max_len[g.axis], groups);
+  return launch_kernel(sh.keep ? hs2g::adj_pair_kernel<ADD_T, true> : hs2g::adj_pair_kernel<ADD_T, false>,
+                       dim3((unsigned)((groups + sh.warps - 1) / sh.warps)), dim3(32 * sh.warps), sh.smem, st,
+                       adj_pdl(), view(a), g, groups, (int64_t)(sh.smem / sh.warps));
+}
 // y = A_a^-1 (M rhs) on the y or z lines (weighted false: A_a^-1 rhs)
 cudaError_t ysolve(const hs2g_adjoint* a, cudaStream_t st, int axis, bool weighted, const double* rhs, double* y) {
-  const int64_t groups = a->ngroups[axis];
-  const hs2g::PairShape sh = hs2g::pair_shape<double, true, false, false, true>(a->max_len[axis], groups);
-  return launch_kernel(sh.keep ? hs2g::adj_pair_kernel<false, true> : hs2g::adj_pair_kernel<false, false>,
-                       dim3((unsigned)((groups + sh.warps - 1) / sh.warps)), dim3(32 * sh.warps), sh.smem, st,
-                       adj_pdl(), view(a), axis, groups, rhs, a->ca[axis], a->cb[axis],
-                       weighted ? a->mip[axis] : a->ip[axis], y, nullptr, nullptr, nullptr, nullptr, (int64_t)0,
-                       (int64_t)(sh.smem / sh.warps));
+  hs2g::APair g{};
+  g.axis = axis;
+  g.rhs = rhs;
+  g.a = a->ca[axis];
+  g.b = a->cb[axis];
+  g.scale = weighted ? a->mip[axis] : a->ip[axis];
+  g.y = y;
+  return pair_launch<false>(a, st, g);
 }
-// the forward z stage: y2 = A_z^-1 (M y1) (stored when keep_y), T_out = T_in + y2, and T_out - obs of step obs_step
+// the forward z stage: y2 = A_z^-1 (M y1) (stored when keep_y), T_out = T_in + 2 y2, and T_out - obs of step obs_step
 // >= 0 in obs's place
 cudaError_t zstep(const hs2g_adjoint* a, cudaStream_t st, const double* y1, double* y2, bool keep_y, const double* T_in,
                   double* T_out, int64_t obs_step) {
-  const int64_t groups = a->ngroups[2];
-  const hs2g::PairShape sh = hs2g::pair_shape<double, true, true, false, true>(a->max_len[2], groups);
-  return launch_kernel(sh.keep ? hs2g::adj_pair_kernel<true, true> : hs2g::adj_pair_kernel<true, false>,
-                       dim3((unsigned)((groups + sh.warps - 1) / sh.warps)), dim3(32 * sh.warps), sh.smem, st,
-                       adj_pdl(), view(a), 2, groups, y1, a->ca[2], a->cb[2], a->mip[2], keep_y ? y2 : nullptr, y2,
-                       T_in, T_out, obs_step >= 0 ? a->obs : nullptr, obs_step, (int64_t)(sh.smem / sh.warps));
+  return pair_launch<true>(a, st, hs2g::APair{2, y1, a->ca[2], a->cb[2], a->mip[2], keep_y ? y2 : nullptr, y2, T_in,
+                                              T_out, obs_step >= 0 ? a->obs : nullptr, obs_step});
 }
 
 // one forward step T_in -> T_out on stream st (T_out may alias T_in; NULL skips it), y0, y1 and with keep_y y2 left in
@@ -856,7 +915,9 @@ int hs2g_adjoint_create(int n, const hs2g_adjoint_grid* grids, double dt, int de
   const void* solves[] = {(const void*)hs2g::adj_pair_kernel<false, false>, (const void*)hs2g::adj_pair_kernel<false, true>,
                           (const void*)hs2g::adj_pair_kernel<true, false>,  (const void*)hs2g::adj_pair_kernel<true, true>,
                           (const void*)hs2g::adj_x_kernel<false, false>,    (const void*)hs2g::adj_x_kernel<false, true>,
-                          (const void*)hs2g::adj_x_kernel<true, false>,     (const void*)hs2g::adj_x_kernel<true, true>};
+                          (const void*)hs2g::adj_x_kernel<true, false>,     (const void*)hs2g::adj_x_kernel<true, true>,
+                          (const void*)hs2g::adj_few_pair_kernel<false>,    (const void*)hs2g::adj_few_pair_kernel<true>,
+                          (const void*)hs2g::adj_few_x_kernel<false>,       (const void*)hs2g::adj_few_x_kernel<true>};
   for (const void* f : solves)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
   if (e == cudaSuccess) e = cudaMalloc(&a->inst, sizeof(hs2g::AInst) * n);

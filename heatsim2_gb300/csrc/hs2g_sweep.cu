@@ -129,14 +129,12 @@ struct PairArgs {
   double* Z;
   int64_t begin, end;
 };
-template <bool ADD_T, bool KEEP, bool TABLE, int TVEC>
-__global__ void __launch_bounds__(32 * kPairMaxWarps) pair_sweep_kernel(PairArgs g, int64_t smem_per_warp) {
-  extern __shared__ __align__(16) unsigned char pair_sm[];
+// the 16 lines of group grp; their number, 0 past the last group
+template <bool ADD_T, bool TABLE>
+__device__ __forceinline__ int pair_group(const PairArgs& g, int64_t grp, PairLines<double>& p) {
   const int64_t nx = g.d.nx, gpr = (nx + 15) / 16;  // groups per row of lines
-  const int64_t grp = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t row = g.begin + grp / gpr, i0 = (grp % gpr) * 16;
-  if (row >= g.end) return;
-  PairLines<double> p{};
+  if (row >= g.end) return 0;
   const int64_t w = ADD_T ? row * g.px + i0 : row * g.d.ny * g.px + i0;  // first line's first row in the padded arrays
   const int64_t wst = ADD_T ? g.d.ny * g.px : g.px;
   p.W = g.W + w;
@@ -148,12 +146,18 @@ __global__ void __launch_bounds__(32 * kPairMaxWarps) pair_sweep_kernel(PairArgs
   p.out = g.out + (ADD_T ? row * nx + i0 : w);
   p.st = ADD_T ? g.d.nxy() : wst;
   p.Z = g.Z + w;
+  return (int)min((int64_t)16, nx - i0);
+}
+template <bool ADD_T, bool KEEP, bool TABLE, int TVEC>
+__global__ void __launch_bounds__(32 * kPairMaxWarps) pair_sweep_kernel(PairArgs g, int64_t smem_per_warp) {
+  extern __shared__ __align__(16) unsigned char pair_sm[];
+  PairLines<double> p{};
+  const int width = pair_group<ADD_T, TABLE>(g, blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5), p);
+  if (!width) return;
   wait_prior_grid();
   pair_solve<double, true, ADD_T, KEEP, TABLE, 2, TVEC>(
-      p, (int)(ADD_T ? g.d.nz : g.d.ny), (int)min((int64_t)16, nx - i0),
-      reinterpret_cast<double*>(pair_sm + (threadIdx.x >> 5) * smem_per_warp));
+      p, (int)(ADD_T ? g.d.nz : g.d.ny), width, reinterpret_cast<double*>(pair_sm + (threadIdx.x >> 5) * smem_per_warp));
 }
-
 __global__ void copy_layer_kernel(Dims d, const double* __restrict__ T, int layer, double* __restrict__ dst) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t < d.nxy()) dst[t] = T[(int64_t)layer * d.nxy() + t];

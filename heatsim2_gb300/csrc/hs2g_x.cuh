@@ -450,11 +450,12 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
     if (TABLE) load(q + 1 < nb ? A : B, q + 1 < nb ? q + 1 : nb - 1);
     issue(q + LA, KEEP);
     if (q >= first_full && q < least) {
+      R v[RB];
 #pragma unroll
-      for (int k = 0; k < RB; ++k) {
-        z = fma(a[k], z, w[k]);
-        at[d * k] = z;
-      }
+      for (int k = 0; k < RB; ++k) v[k] = z = chain_fma(a[k], z, w[k]);
+      chain_order();
+#pragma unroll
+      for (int k = 0; k < RB; ++k) at[d * k] = v[k];
     } else {
       const int lo = skip - q * RB, hi = rows - q * RB;
 #pragma unroll
@@ -501,11 +502,12 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
     if (TABLE && q > 0) load(B, q - 1);
     issue(i + LA, true);
     if (q >= first_full && q < least) {
+      R v[RB];
 #pragma unroll
-      for (int k = RB - 1; k >= 0; --k) {
-        x = fma(b[k], x, w[k]);
-        at[d * k] = x;
-      }
+      for (int k = RB - 1; k >= 0; --k) v[k] = x = chain_fma(b[k], x, w[k]);
+      chain_order();
+#pragma unroll
+      for (int k = RB - 1; k >= 0; --k) at[d * k] = v[k];
     } else {
       const int lo = skip - q * RB, hi = rows - q * RB;
 #pragma unroll
@@ -620,11 +622,12 @@ __device__ __forceinline__ void x_fused_lines(const XProblem<double>& P, int64_t
           for (int u = 0; u < 8; ++u) a[u] = t0 + 8 + u < cnt ? arow[t0 + 8 + u] : 0.0;
         }
         if (t0 + 8 <= least) {
+          double v[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            z = fma(c[u], z, r[u]);
-            row[t0 + u] = z;
-          }
+          for (int u = 0; u < 8; ++u) v[u] = z = chain_fma(c[u], z, r[u]);
+          chain_order();
+#pragma unroll
+          for (int u = 0; u < 8; ++u) row[t0 + u] = v[u];
         } else {
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
@@ -662,11 +665,12 @@ __device__ __forceinline__ void x_fused_lines(const XProblem<double>& P, int64_t
           for (int u = 0; u < 8; ++u) b[u] = brow[t0 - 8 + u];
         }
         if (t0 + 8 <= least) {
+          double v[8];
 #pragma unroll
-          for (int u = 7; u >= 0; --u) {
-            x = fma(c[u], x, r[u]);
-            row[t0 + u] = x;
-          }
+          for (int u = 7; u >= 0; --u) v[u] = x = chain_fma(c[u], x, r[u]);
+          chain_order();
+#pragma unroll
+          for (int u = 7; u >= 0; --u) row[t0 + u] = v[u];
         } else {
 #pragma unroll
           for (int u = 7; u >= 0; --u) {
