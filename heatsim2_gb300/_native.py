@@ -25,7 +25,7 @@ MAX_ZERO_FORMS = 24
 MAX_CLASSES = 256
 
 EXPORTED = ("hs2g_abi_version", "hs2g_last_error", "hs2g_create_classes", "hs2g_create_dense", "hs2g_destroy",
-            "hs2g_set_stream", "hs2g_shape", "hs2g_step", "hs2g_run", "hs2g_source_table", "hs2g_get_faces",
+            "hs2g_set_stream", "hs2g_shape", "hs2g_step", "hs2g_run", "hs2g_source_table", "hs2g_source_tables", "hs2g_get_faces",
             "hs2g_device_bytes", "hs2g_run_timed", "hs2g_fp64_fma_rate", "hs2g_step_static",
             "hs2g_batch_create", "hs2g_batch_destroy", "hs2g_batch_layout", "hs2g_batch_device_bytes",
             "hs2g_batch_set_temperature", "hs2g_batch_get_temperature", "hs2g_batch_set_sources",
@@ -132,6 +132,8 @@ def load():
         L.hs2g_surface_temperature.restype = i32
         L.hs2g_source_table.argtypes = [i32, vp, vp, dp, dp, dp, vp]
         L.hs2g_source_table.restype = i32
+        L.hs2g_source_tables.argtypes = [i32, vp, vp, ctypes.c_int64, vp, dp, dp, vp]
+        L.hs2g_source_tables.restype = i32
         L.hs2g_set_source_classes.argtypes = [vp, vp, i32]
         L.hs2g_set_source_classes.restype = i32
         L.hs2g_set_schedule.argtypes = [vp, ctypes.c_int64, vp, i32]

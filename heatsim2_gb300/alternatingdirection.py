@@ -202,6 +202,17 @@ def source_table(sources, t, dt, volume):
     return qtab, active > 0
 
 
+def source_tables(sources, times, dt, volume):
+    """(qtabs ndarray[len(times), 256], any_active): source_table for every time, in one native call."""
+    times = np.array([float(t) for t in times])
+    qtabs = np.empty((times.size, _native.MAX_CLASSES))
+    vol = float(volume) if np.ndim(volume) == 0 else 1.0
+    active = _native.check(_native.load().hs2g_source_tables(sources.n, sources.kind.ctypes.data,
+                                                             sources.params.ctypes.data, times.size, times.ctypes.data,
+                                                             float(dt), vol, qtabs.ctypes.data))
+    return qtabs, active > 0
+
+
 # --------------------------------------------------------------------------------------------------------
 # stepping
 # --------------------------------------------------------------------------------------------------------
@@ -314,11 +325,7 @@ def run(ADI_params, Tarray, times, dt, volumetric_elements, volumetric, record_l
         _native.check(L.hs2g_set_stream(P.handle.ptr, None))
         ptr = T.ctypes.data
         flags = 0
-    qtabs = np.zeros((n, _native.MAX_CLASSES))
-    any_active = False
-    for s, t in enumerate(times):
-        qtabs[s], act = source_table(sources, t, dt, P.volume_array)
-        any_active |= act
+    qtabs, any_active = source_tables(sources, times, dt, P.volume_array)
     if any_active:
         # a changed source-class map and the shapes of the shaped classes that fire within the run are set on
         # the device first; the steps then run in one native call, firing steps included

@@ -13,7 +13,7 @@ import numpy as np
 
 from . import _native
 from .crank_nicolson import ClassProblem, raise_compile_error, current_device
-from .alternatingdirection import _ClassSources, source_table
+from .alternatingdirection import _ClassSources, source_tables
 
 
 def shard(sizes, world, rank):
@@ -112,11 +112,9 @@ class Batch(object):
                                       "not provided in the batched form")
         nclass = max(1, max(len(p.volumetric) for p in self.problems))
         q = np.zeros((len(times), self.n, nclass))
-        for s, t in enumerate(times):
-            for i, (src, p) in enumerate(zip(srcs, self.problems)):
-                dz, dy, dx = p.spacing
-                tab, _ = source_table(src, t, dt, dz * dy * dx)
-                q[s, i, :] = tab[:nclass]
+        for i, (src, p) in enumerate(zip(srcs, self.problems)):
+            dz, dy, dx = p.spacing
+            q[:, i, :] = source_tables(src, times, dt, dz * dy * dx)[0][:, :nclass]
         _native.check(_native.load().hs2g_batch_set_sources(self._h, len(times), nclass, q.ctypes.data))
 
     def run(self, nsteps, sync=True):

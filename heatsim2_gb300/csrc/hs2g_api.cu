@@ -747,6 +747,19 @@ int hs2g_source_table(int nsrc, const int32_t* kind, const double* params, doubl
   return active;
 }
 
+int hs2g_source_tables(int nsrc, const int32_t* kind, const double* params, int64_t ntimes, const double* times, double dt,
+                       double volume, double* qtabs) {
+  if (ntimes < 0 || ntimes > INT32_MAX || (ntimes > 0 && (!times || !qtabs)))
+    return fail(HS2G_ERR_ARG, "bad source table arguments");
+  int active = 0;
+  for (int64_t s = 0; s < ntimes; ++s) {
+    const int n = hs2g_source_table(nsrc, kind, params, times[s], dt, volume, qtabs + s * HS2G_MAX_CLASSES);
+    if (n < 0) return n;
+    active += n > 0;
+  }
+  return active;
+}
+
 int hs2g_step(hs2g_handle* h, const double* T_in, double* T_out, const double* qtab, const double* qdense,
               const uint8_t* volumetric, int flags) {
   if (!h || !T_in || !T_out) return fail(HS2G_ERR_ARG, "null argument");

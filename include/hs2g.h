@@ -220,6 +220,11 @@ int hs2g_fp64_fma_rate(int device, double* fma_per_s);
 int hs2g_source_table(int nsrc, const int32_t* kind, const double* params, double t, double dt, double volume,
                       double* qtab);
 
+/* hs2g_source_table for each of times[0 .. ntimes-1] into the rows of qtabs[ntimes][HS2G_MAX_CLASSES]; returns the
+   number of times with a non-zero value (>= 0) or an error. */
+int hs2g_source_tables(int nsrc, const int32_t* kind, const double* params, int64_t ntimes, const double* times, double dt,
+                       double volume, double* qtabs);
+
 /*
  * Device-resident source schedule of a handle (the batched form's hs2g_batch_set_sources for one problem):
  * qtabs[nsteps][HS2G_MAX_CLASSES] class source values (W/m^3) for steps 0 .. nsteps-1, a host array or, with

@@ -80,3 +80,25 @@ def test_source_table_rejects_per_voxel_kinds(lib):
     q = np.zeros(256)
     assert lib.hs2g_source_table(1, kind.ctypes.data, params.ctypes.data, 0.0, 0.01, 1.0, q.ctypes.data) == \
         _native.ERR_ARG
+
+
+def test_source_tables_are_the_tables_of_the_times(lib):
+    kind = np.array([k for k, _ in SOURCES], dtype=np.int32)
+    params = np.zeros((len(SOURCES), 4))
+    for c, (_, p) in enumerate(SOURCES):
+        params[c, :len(p)] = p
+    times = np.array([0.0, 0.005, 0.01, 0.02, 0.030000000000000002, 0.04])
+    got, one, active = np.full((times.size, 256), np.nan), np.zeros(256), 0
+    for s, t in enumerate(times):
+        active += lib.hs2g_source_table(len(SOURCES), kind.ctypes.data, params.ctypes.data, t, 0.01, 1e-9,
+                                        one.ctypes.data) > 0
+        if s == 0:
+            assert lib.hs2g_source_tables(len(SOURCES), kind.ctypes.data, params.ctypes.data, times.size,
+                                          times.ctypes.data, 0.01, 1e-9, got.ctypes.data) >= 0
+        np.testing.assert_array_equal(got[s], one)
+    assert lib.hs2g_source_tables(len(SOURCES), kind.ctypes.data, params.ctypes.data, times.size, times.ctypes.data,
+                                  0.01, 1e-9, got.ctypes.data) == active
+    assert lib.hs2g_source_tables(0, None, None, 0, None, 0.01, 1e-9, None) == 0
+    kind[0] = 4
+    assert lib.hs2g_source_tables(len(SOURCES), kind.ctypes.data, params.ctypes.data, times.size, times.ctypes.data,
+                                  0.01, 1e-9, got.ctypes.data) == _native.ERR_ARG
