@@ -38,31 +38,31 @@ for _p in (ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests")):
 
 METRIC = "voxel-steps/s"
 SEED = 1
-# algorithmic bytes and FP64 operations per grid voxel, per kernel (dense coefficient layout, no source active):
-#   sweep_x  reads T and 9 coefficient arrays (wc wxl wxh wyl wyh wzl wzh a0 b0), writes W0
-#   sweep_y  reads W0, a1, b1, writes W1
-#   sweep_z  reads W1, a2, b2, T, writes T'
-BYTES_PER_VOXEL = {"sweep_x": 8 + 9 * 8 + 8, "sweep_y": 4 * 8, "sweep_z": 5 * 8}
+# algorithmic bytes and FP64 operations per grid voxel, per sweep (a class problem, whose coefficients come from tables
+# of distinct blocks and lines that stay in cache; no source active; the x stencil is formed in integers):
+#   sweep_x  reads T, writes the right-hand sides, reads them for the line solves, writes W0
+#   sweep_y  reads W0, writes W1
+#   sweep_z  reads W1, T, writes T'
+BYTES_PER_VOXEL = {"sweep_x": 4 * 8, "sweep_y": 2 * 8, "sweep_z": 3 * 8}
 # the algorithmic bytes the roofline is reported on: each sweep touching each array it needs once, with the face
 # conductances and capacities re-read in every sweep (136 B per voxel and step):
 #   sweep_x  reads T, M, Gx, Gy, Gz, Q, writes T*0 (7 arrays)
 #   sweep_y  reads T, T*0, M, Gy, writes T*1 (5)
 #   sweep_z  reads T, T*1, M, Gz, writes T' (5)
 ROOFLINE_BYTES_PER_VOXEL = {"sweep_x": 7 * 8, "sweep_y": 5 * 8, "sweep_z": 5 * 8}
-FP64_OPS_PER_VOXEL = {"sweep_x": 9, "sweep_y": 2, "sweep_z": 3}
+FP64_OPS_PER_VOXEL = {"sweep_x": 2, "sweep_y": 2, "sweep_z": 3}
 KERNELS = ("sweep_x", "sweep_y", "sweep_z")
 # adjoint: arrays touched per voxel and step (8 B each), from the kernels of hs2g_adjoint.cu
-#   forward step (forward pass, and again as the recompute of the backward pass): x stage reads T, gx, gy, gz,
-#   D, q, lo0, ip0, u0 and writes y0 (10); y stage reads y0, lo1, mip1, u1 (mip = M / piv), writes y1 (5); z stage
-#   reads y1, lo2, mip2, u2, T, writes y2, T' (7)                                             -> 22 arrays
-#   reverse step: transposed z reads lambda, u2, lo2, ip2, writes mu2 (5); transposed y reads mu2, u1, lo1,
-#   mip1, writes mu1 (5); transposed x the same for mu0 (5); update reads gx, gy, gz, T, y0, y1, y2, mu0, mu1,
+#   forward step (forward pass, and again as the recompute of the backward pass): residual reads T, gx, gy, gz, D, q,
+#   ip0 and writes W (8); x stage reads W, a0, b0, writes y0 (4); y stage reads y0, a1, mip1, b1 (mip = M / piv), writes
+#   y1 (5); z stage reads y1, a2, mip2, b2, T, writes y2, T' (7)                              -> 24 arrays
+#   reverse step: transposed z reads lambda, a2, ip2, b2, writes mu2 (5); transposed y reads mu2, a1, mip1, b1,
+#   writes mu1 (5); transposed x the same for mu0 (5); update reads gx, gy, gz, T, y0, y1, y2, mu0, mu1,
 #   mu2, lambda and the five accumulators and writes lambda and the accumulators (22)          -> 37 arrays
-# so one gradient evaluation moves (22 + 22 + 37) * 8 = 648 B (the x stage also reads the diagonal D) and does
-# about 18 + 18 + (3 + 3 + 3 + 34) = 79 FP64 operations per voxel and step (forward step, recompute,
-# transposed solves and update).
-ADJ_BYTES_PER_VOXEL_STEP = (22 + 22 + 37) * 8
-ADJ_FP64_OPS_PER_VOXEL_STEP = 79
+# so one gradient evaluation moves (24 + 24 + 37) * 8 = 680 B and does about 18 + 18 + (3 + 3 + 3 + 29) = 74 FP64
+# operations per voxel and step (forward step, recompute, transposed solves and update).
+ADJ_BYTES_PER_VOXEL_STEP = (24 + 24 + 37) * 8
+ADJ_FP64_OPS_PER_VOXEL_STEP = 74
 
 
 def parse_args():
@@ -663,7 +663,7 @@ def gpu_arm(args, world, rank, local_rank):
                        "grid": [nz, ny, nx], "computed_voxels": compute_vox, "seed": SEED,
                        "l2": "inputs larger than L2 (T %.0f MB, device state %.0f MB)"
                              % (grid_vox * 8 / 1e6, state_bytes / 1e6),
-                       "kernels": "x: CTA-staged stencil + warp recurrence; y: TMA tensor-tile ring; z: per-line; "
+                       "kernels": "x: integer stencil, then lines from both ends; y, z: lines from both ends; "
                                   "timed as hs2g_run: schedule rows on the device, one step-graph replay per step",
                        "parallelism": "replicas" if world > 1 else "single"},
             "roofline": roofline, "fp64_roofline": fp64, "step_hbm": step_hbm,
@@ -671,7 +671,9 @@ def gpu_arm(args, world, rank, local_rank):
             "kernel_hbm_frac": per_kernel_hbm, "kernel_hbm_frac_implementation_bytes": per_kernel_hbm_impl,
             "kernel_dram_frac_measured_traffic": per_kernel_traffic,
             "host_launched_ms_per_step": host_launched_ms / K,
-            "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": 3 * K, "clocks": clk, "setup_s": setup_s,
+            "cpu_baseline": cpu, "e2e": e2e,
+            # the x sweep of more lines than fit at once is two kernels (hs2g_x.cuh)
+            "gpu_launches": (4 if nz * ny > 152 * 3 * 16 else 3) * K, "clocks": clk, "setup_s": setup_s,
             "device_bytes": state_bytes, "batched": batched, "adjoint": adjoint, "curved": curved,
         }
         print(json.dumps(line), flush=True)

@@ -2,8 +2,8 @@
 
 The reference advances one problem per ``run_adi_steps`` call; a user with many specimens loops over them.
 ``Batch`` takes a list of problems given as ``heatsim2.setup`` argument tuples, compiles them into one
-concatenated device state (libhs2g ``hs2g_batch_create``) and advances all of them per step with three
-persistent sweep kernels captured in one CUDA graph.  ``precision=64`` gives, per instance, exactly the
+concatenated device state (libhs2g ``hs2g_batch_create``) and advances all of them per step with four
+sweep kernels captured in one CUDA graph.  ``precision=64`` gives, per instance, exactly the
 result of ``setup`` + ``run_adi_steps``; ``precision=32`` stores and sweeps in float (coefficients compiled in
 double) for throughput, with its error against double left to the caller to measure.
 """

@@ -196,7 +196,7 @@ int check_kernel_error(hs2g_handle* h) {
               (long long)i);
 }
 
-// Row pitch of the y sweep's arrays: nx rounded up to an even count, so that TMA tile rows start on 16-byte
+// Row pitch of the y sweep's arrays: nx rounded up to an even count, so that its rows start on 16-byte
 // boundaries whatever nx is (HS2G_ROW_PITCH=<multiple> pads further, for tests of the padded layout).
 int64_t y_pitch(int64_t nx) {
   int64_t m = 2;
