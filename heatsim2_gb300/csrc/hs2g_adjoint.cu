@@ -292,7 +292,7 @@ __global__ void adj_resid_kernel(AView v, const double* __restrict__ T, const do
 // instance's results do not depend on what it is solved with.
 // A few lines are bound by the latency of a half line's chain, many by memory (32 to 56 bytes per voxel).  Against one
 // thread per line, or one warp per 32 lines with a second one copying: y lines of six instances of 0.4 to 1.8 million
-// voxels 138 -> 55 us, of 32x128x128 26 -> 16 us; x with its residual 177 -> 160 us and 33 -> 27 us; z of 32 rows alike.
+// voxels 138 -> 55 us, of 32x128x128 26 -> 16 us; x with its residual 177 -> 152 us and 33 -> 27 us; z of 32 rows alike.
 // x lines, y = A_x^-1 (M rhs); SCALE false: in place from y = W
 template <bool SCALE, bool KEEP>
 __global__ void __launch_bounds__(32 * kPairMaxWarps) adj_x_kernel(AView v, int64_t ngroups, const double* rhs,

@@ -10,7 +10,7 @@
 // with a neighbour of another sign or exponent, with zero, infinite or NaN temperatures, or with weights that are
 // negative or out of range take the chain, each voxel by itself.
 //
-// 65x512x512: 120 us for the stencil (its integer instructions' latency, 16 warps to an SM) and 115 us for the line
+// 65x512x512: 120 us for the stencil (its integer instructions' latency, 16 warps to an SM) and 103 us for the line
 // solves (16 bytes of HBM traffic per voxel, 54 us of FMAs), against 324 us for the chain with coefficients read per
 // voxel; a field of white noise, every voxel in the chain, 346 us.  37x187x211: 34 us against 94.
 #pragma once
@@ -304,21 +304,32 @@ __device__ __forceinline__ void x_stencil_lines(const XProblem<R>& P, int64_t L0
 // A warp takes 16 x-lines from both ends (FP32: 32, one way) as pair_solve takes the y and z lines, lane = line; but a
 // line's columns lie side by side in memory, so its blocks of eight columns are copied to shared memory in 16-byte
 // pieces of a line, each lane's columns in a row of its own, and leave it the same way.  The right ends' windows are
-// mirrored in address only: a lane walks down its row there.
+// mirrored in a lane's registers.
 constexpr int kXCols = 8;   // columns per block
 constexpr int kXAhead = 3;  // blocks in flight ahead of the one in use
+// FP64: the rows are whole groups of eight 16-byte pieces, and a row's pieces are permuted within their groups by its
+// number, so that neither the copies (a block's pieces of a few rows) nor the lanes (one piece of eight rows) meet in a
+// bank; with the pieces in order and rows one piece of pad apart, 8-byte accesses met twice everywhere.  65x512x512: 118
+// -> 103 us, 12 uneven instances of 14 million voxels 107 -> 95 us.  FP32 keeps rows with a pad and 4-byte accesses
+// (its batch took 59.6 ms with permuted pieces, 51.3 ms so).
 template <typename R>
-__host__ __device__ constexpr int x_pad() {
-  return 16 / (int)sizeof(R);  // elements between the rows, which keeps their pieces on 16-byte boundaries
+__host__ __device__ constexpr int x_row_round(int64_t elems) {
+  return sizeof(R) == 8 ? (int)((elems + 15) / 16 * 16) : (int)elems + 4;
 }
 // elements of a lane's row: with KEEP its whole half line, else a ring of blocks; and a ring of coefficients (not TABLE)
 template <typename R, bool TWO, bool KEEP>
 __host__ __device__ constexpr int x_row_elems(int64_t n) {
-  return (KEEP ? (int)(((TWO ? n / 2 + 2 : n) + kXCols - 1) / kXCols) : kXAhead + 1) * kXCols + x_pad<R>();
+  return x_row_round<R>((KEEP ? ((TWO ? n / 2 + 2 : n) + kXCols - 1) / kXCols : kXAhead + 1) * kXCols);
 }
 template <typename R>
 __host__ __device__ constexpr int x_coef_elems() {
-  return (kXAhead + 1) * kXCols + x_pad<R>();
+  return x_row_round<R>((kXAhead + 1) * kXCols);
+}
+// place (in elements) of piece p of row r in its row
+template <typename R>
+__device__ __forceinline__ int x_piece(int p, int r) {
+  if constexpr (sizeof(R) == 4) return p * 4;
+  return ((p & ~7) | ((p & 7) ^ ((r & 1) << 2 | (r >> 1 & 3)))) * 2;
 }
 template <typename R, bool TWO, bool TABLE, bool KEEP, bool SCALE = false>
 __host__ __device__ constexpr size_t x_solve_smem(int64_t max_nx) {  // per warp
@@ -363,7 +374,8 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
       const bool up = TWO && r >= 16;
       const int l = TWO ? r & 15 : r, c = column0(q, up) + v;
       if (l < count && c >= 0 && c < E)
-        cp_async_bytes<16>(dst + (uint32_t)((r * row_elems + at + v) * sizeof(R)), base + (L0 + l) * pitch + c);
+        cp_async_bytes<16>(dst + (uint32_t)((r * row_elems + x_piece<R>(at / VEC + e % LPB, r)) * sizeof(R)),
+                           base + (L0 + l) * pitch + c);
     }
   };
   // a block's values to W0: whole pieces inside the side's columns, single elements at its inner end
@@ -375,7 +387,7 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
       const int l = TWO ? r & 15 : r, c = column0(q, up) + v;
       const int lo = up ? m + 1 : 0, hi = up ? n : (TWO ? m + (back ? 1 : 0) : n);  // columns of the side
       if (l < count) {
-        const R* src = smem + r * rw + slot(q) + v;
+        const R* src = smem + r * rw + x_piece<R>(slot(q) / VEC + e % LPB, r);
         R* dst = P.W0 + (L0 + l) * P.px + c;
         if (c >= lo && c + VEC <= hi) {
           *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
@@ -433,40 +445,66 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
   if (TABLE) load(A, 0);
 #pragma unroll 1
   for (int i = 0; i < LA; ++i) issue(i, KEEP);
-  const int d = upper ? -1 : 1, o = upper ? RB - 1 : 0;  // slot t of a block at o + d t
+  // this lane's values of the block at element `at` of its row, slot 0 first (the last column on the right)
+  auto take = [&](const R* r, int at, R (&w)[RB]) {
+    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+      for (int k = 0; k < RB; ++k) w[k] = r[at + k];
+    } else {
+      R e[RB];
+#pragma unroll
+      for (int j = 0; j < LPB; ++j)
+        *reinterpret_cast<double2*>(e + j * VEC) = *reinterpret_cast<const double2*>(r + x_piece<R>(at / VEC + j, lane));
+#pragma unroll
+      for (int k = 0; k < RB; ++k) w[k] = upper ? e[RB - 1 - k] : e[k];
+    }
+  };
+  auto put = [&](int at, const R (&w)[RB]) {
+    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+      for (int k = 0; k < RB; ++k) row[at + k] = w[k];
+    } else {
+      R e[RB];
+#pragma unroll
+      for (int k = 0; k < RB; ++k) e[k] = upper ? w[RB - 1 - k] : w[k];
+#pragma unroll
+      for (int j = 0; j < LPB; ++j)
+        *reinterpret_cast<double2*>(row + x_piece<R>(at / VEC + j, lane)) = *reinterpret_cast<double2*>(e + j * VEC);
+    }
+  };
   R z = 0;
 #pragma unroll 1
   for (int q = 0; q < nb; ++q) {
     cp_async_wait_pending<LA - 1>();
     __syncwarp();
-    R* at = row + slot(q) + o;
-    const R *cat = crow + cslot(q) + o, *sat = srow + cslot(q) + o;
     R a[RB], w[RB];
+    take(row, slot(q), w);
+    if (!TABLE) take(crow, cslot(q), a);
+    if (SCALE) {
+      R sc[RB];
+      take(srow, cslot(q), sc);
 #pragma unroll
-    for (int k = 0; k < RB; ++k) {
-      a[k] = TABLE ? next[k] : cat[d * k];
-      w[k] = SCALE ? at[d * k] * sat[d * k] : at[d * k];
+      for (int k = 0; k < RB; ++k) w[k] *= sc[k];
+    }
+    if (TABLE) {
+#pragma unroll
+      for (int k = 0; k < RB; ++k) a[k] = next[k];
     }
     if (TABLE) load(q + 1 < nb ? A : B, q + 1 < nb ? q + 1 : nb - 1);
     issue(q + LA, KEEP);
     if (q >= first_full && q < least) {
-      R v[RB];
 #pragma unroll
-      for (int k = 0; k < RB; ++k) v[k] = z = chain_fma(a[k], z, w[k]);
-      chain_order();
-#pragma unroll
-      for (int k = 0; k < RB; ++k) at[d * k] = v[k];
+      for (int k = 0; k < RB; ++k) w[k] = z = chain_fma(a[k], z, w[k]);
     } else {
       const int lo = skip - q * RB, hi = rows - q * RB;
 #pragma unroll
       for (int k = 0; k < RB; ++k) {
         const R f = fma(a[k], z, w[k]);
-        if (k >= lo && k < hi) {
-          z = f;
-          at[d * k] = f;
-        }
+        if (k >= lo && k < hi) w[k] = z = f;
       }
     }
+    chain_order();
+    put(slot(q), w);
     if (!KEEP) {
       __syncwarp();
       store(q, false);
@@ -491,34 +529,29 @@ __device__ __forceinline__ void x_solve_lines(const XProblem<R>& P, int64_t L0, 
     cp_async_wait_pending<LA - 1>();
     __syncwarp();
     const int q = 2 * nb - 1 - i;
-    R* at = row + slot(q) + o;
-    const R* cat = crow + cslot(i) + o;
     R b[RB], w[RB];
+    take(row, slot(q), w);
+    if (TABLE) {
 #pragma unroll
-    for (int k = 0; k < RB; ++k) {
-      b[k] = TABLE ? next[k] : cat[d * k];
-      w[k] = at[d * k];
+      for (int k = 0; k < RB; ++k) b[k] = next[k];
+    } else {
+      take(crow, cslot(i), b);
     }
     if (TABLE && q > 0) load(B, q - 1);
     issue(i + LA, true);
     if (q >= first_full && q < least) {
-      R v[RB];
 #pragma unroll
-      for (int k = RB - 1; k >= 0; --k) v[k] = x = chain_fma(b[k], x, w[k]);
-      chain_order();
-#pragma unroll
-      for (int k = RB - 1; k >= 0; --k) at[d * k] = v[k];
+      for (int k = RB - 1; k >= 0; --k) w[k] = x = chain_fma(b[k], x, w[k]);
     } else {
       const int lo = skip - q * RB, hi = rows - q * RB;
 #pragma unroll
       for (int k = RB - 1; k >= 0; --k) {
         const R f = fma(b[k], x, w[k]);
-        if (k >= lo && k < hi) {
-          x = f;
-          at[d * k] = f;
-        }
+        if (k >= lo && k < hi) w[k] = x = f;
       }
     }
+    chain_order();
+    put(slot(q), w);
     __syncwarp();
     store(q, false);
     __syncwarp();
