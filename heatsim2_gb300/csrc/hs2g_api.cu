@@ -280,12 +280,26 @@ int factor(hs2g_handle* h, const hs2g::Faces& faces) {
   const Dims& d = h->d;
   Coeffs& c = h->c;
   const int64_t n = d.nvox(), np = d.nz * d.ny * c.px;
-  double* sc = nullptr;  // s2, sigma and the scratch of the search for equal lines and blocks
-  const int64_t len = 2 * n + (int64_t)(hs2g::compress_scratch(d) + 7) / 8;
+  // s2 and sigma, and the scratch of the search for equal lines and blocks: without room for that everything stays in
+  // voxel order
+  double* sc = nullptr;
+  const int64_t wanted = 2 * n + (int64_t)(hs2g::compress_scratch(d) + 7) / 8;
+  int64_t len = wanted;
   int rc;
-  if ((rc = dalloc(h, &sc, len, "factor scratch"))) return rc;
+  if (dalloc(h, &sc, len, "factor scratch") && (rc = dalloc(h, &sc, len = 2 * n, "factor scratch"))) return rc;
   cudaError_t e = hs2g::launch_factor(d, faces, h->M, h->compute, sc, sc + n, c, h->stream, true);
-  if (e == cudaSuccess) e = hs2g::compress_coeffs(d, faces, h->compute, sc, c, 64, (unsigned char*)(sc + 2 * n), &h->kept, h->stream);
+  auto compress = [&](unsigned char* scratch) {
+    return hs2g::compress_coeffs(d, faces, h->compute, sc, c, 64, scratch, &h->kept, h->stream);
+  };
+  if (e == cudaSuccess) e = compress(len == wanted ? (unsigned char*)(sc + 2 * n) : nullptr);
+  if (e == cudaErrorMemoryAllocation && len == wanted) {  // the blocks did not fit beside the scratch
+    cudaGetLastError();
+    cudaStreamSynchronize(h->stream);
+    dfree(h, sc, len);
+    if ((rc = dalloc(h, &sc, len = 2 * n, "factor scratch"))) return rc;
+    e = hs2g::launch_factor(d, faces, h->M, h->compute, sc, sc + n, c, h->stream, true);
+    if (e == cudaSuccess) e = compress(nullptr);
+  }
   cudaError_t e2 = cudaStreamSynchronize(h->stream);
   dfree(h, sc, len);
   if (e == cudaErrorMemoryAllocation) {

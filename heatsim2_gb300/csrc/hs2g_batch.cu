@@ -77,9 +77,9 @@ __device__ __forceinline__ XProblem<R> x_problem(const BatchView<R>& v, const In
 }
 // x sweep: a work item is kXItemLines consecutive x-lines of one instance.  The stencil takes a CTA per item and
 // gridDim.y-th chunk of columns (IX = int32_t when every instance has fewer than 2^31 voxels); the line solves a warp
-// per 16 (FP64) or 32 (FP32) lines of an item.  DENSE: some instance keeps its coefficients in voxel order.
+// per 16 (FP64) or 32 (FP32) lines of an item.  DENSE: some instance keeps its blocks, or line coefficients, in voxel order.
 constexpr int kXItemLines = 64;
-template <typename R, typename IX>
+template <typename R, bool DENSE, typename IX>
 __global__ void __launch_bounds__(32 * kXStencilWarps, kXStencilCtas) batch_stencil_kernel(BatchView<R> v) {
   __shared__ XLine<IX> lines[kXStencilLines];
   __shared__ R sq[HS2G_MAX_CLASSES];
@@ -93,9 +93,15 @@ __global__ void __launch_bounds__(32 * kXStencilWarps, kXStencilCtas) batch_sten
   if (step < v.nsched && v.active[(int64_t)step * v.ninst + item.inst]) {
     const R* q = v.qtabs + ((int64_t)step * v.ninst + item.inst) * v.nclass;
     for (int c = threadIdx.x; c < HS2G_MAX_CLASSES; c += 32 * kXStencilWarps) sq[c] = c < v.nclass ? q[c] : R(0);
-    x_stencil_lines<R, true, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
+    if (!DENSE || P.bidx)
+      x_stencil_lines<R, true, true, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
+    else
+      x_stencil_lines<R, true, false, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
   } else {
-    x_stencil_lines<R, false, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
+    if (!DENSE || P.bidx)
+      x_stencil_lines<R, false, true, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
+    else
+      x_stencil_lines<R, false, false, IX>(P, L0, end, blockIdx.y, gridDim.y, lines, sq);
   }
 }
 template <typename R, bool KEEP, bool DENSE>
@@ -208,6 +214,7 @@ struct Batch {
   Tuning tune{1, true, true, true};
   int64_t max_nx = 0, max_ny = 0, max_nz = 0;  // longest x, y and z line
   bool dense[3] = {false, false, false};  // some instance keeps its x / y / z coefficients in voxel order
+  bool dense_blocks = false;              // and its stencil blocks
   bool ix32 = false;  // every instance's voxels and stencil blocks below 2^31 elements: 32-bit x-sweep indices
   cudaGraphExec_t graph = nullptr;
   int64_t bytes = 0;
@@ -306,10 +313,9 @@ cudaError_t launch_axis(const Batch& b, int axis, const Tuning& t, cudaStream_t 
   BatchView<R> v = view<R>(b);
   if (axis == 0) {
     const dim3 grid((unsigned)(b.nxw * (kXItemLines / kXStencilLines)), (unsigned)t.x_split);
-    if (b.ix32)
-      batch_stencil_kernel<R, int32_t><<<grid, 32 * kXStencilWarps, 0, s>>>(v);
-    else
-      batch_stencil_kernel<R, int64_t><<<grid, 32 * kXStencilWarps, 0, s>>>(v);
+    const auto stencil = b.dense_blocks ? (b.ix32 ? batch_stencil_kernel<R, true, int32_t> : batch_stencil_kernel<R, true, int64_t>)
+                                        : (b.ix32 ? batch_stencil_kernel<R, false, int32_t> : batch_stencil_kernel<R, false, int64_t>);
+    stencil<<<grid, 32 * kXStencilWarps, 0, s>>>(v);
     const PairShape sh = batch_x_shape<R>(b, t.x_keep ? 1 : 0);
     batch_x_solve_for<R>(sh.keep, b.dense[0])<<<(unsigned)b.nxw, 32 * sh.warps, sh.smem, s>>>(
         v, (int64_t)(sh.smem / sh.warps));
@@ -588,6 +594,7 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   b.coef_mem.push_back(kept.blocks.pool);
   I.pool = kept.blocks.pool;
   I.bidx = kept.blocks.bidx;
+  if (!I.bidx) b.dense_blocks = true;
   b.bytes += (int64_t)kept.blocks.bytes;
   const double* coeffs[3][2] = {{c.a0, c.b0}, {c.a1, c.b1}, {c.a2, c.b2}};
   for (int ax = 0; ax < 3; ++ax) {

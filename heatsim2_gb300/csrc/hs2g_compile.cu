@@ -378,12 +378,32 @@ __device__ __forceinline__ int exterior_faces(const Dims& d, int64_t t, int64_t 
   return (i == 0) | (i + 1 == d.nx) << 1 | (j == 0) << 2 | (j + 1 == d.ny) << 3 | (k == 0) << 4 | (k + 1 == d.nz) << 5;
 }
 // writes a block (one warp); true when two products do for each of its voxels (kXTwoWeights)
-template <typename R>
+template <typename R, bool SHARED>
 __device__ __forceinline__ bool store_block(R* blk, int lane, const double (&v)[8], int exterior) {
+  bool two = false;
+  if constexpr (sizeof(R) == 8 && !SHARED) {
+    const double w[6] = {v[1], v[2], v[3], v[4], v[5], v[6]};
+    const bool fine = x_own_fine(v[0], w);
+    const int hi = __double2hiint(v[0]);
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      const long long i = llrint(ldexp(w[f], 62 - (x_own_exponent(hi) - 4)));
+      const int lo = (int)(unsigned)i;
+      const uint2 wi = make_uint2((unsigned)lo, (unsigned)((i - lo) >> 32));
+      if (fine)
+        reinterpret_cast<uint2*>(blk)[f * 32 + lane] = wi;
+      else
+        blk[f * 32 + lane] = w[f];
+    }
+    int* words = reinterpret_cast<int*>(blk + 6 * 32);
+    words[lane] = fine ? hi : kXOwnDoubles;
+    words[32 + lane] = __double2loint(v[0]);
+    blk[7 * 32 + lane] = v[7];
+    return false;
+  }
 #pragma unroll
   for (int c = 0; c < 8; ++c) blk[c * 32 + lane] = (R)v[c];
-  bool two = false;
-  if constexpr (sizeof(R) == 8) {
+  if constexpr (sizeof(R) == 8 && SHARED) {
     double w[6];
 #pragma unroll
     for (int f = 0; f < 6; ++f) w[f] = exterior >> f & 1 ? (exterior >> (f ^ 1) & 1 ? 0.0 : v[1 + (f ^ 1)]) : v[1 + f];
@@ -433,20 +453,20 @@ __global__ void number_blocks_kernel(int64_t blocks, const int* owner, const int
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b < blocks && owner[slot[b]] == (int)b) id[slot[b]] = atomicAdd(count, 1);
 }
-// writes the owners' blocks (slot null: every block at its own place)
-template <typename R, class F>
+// writes the owners' blocks, or (SHARED false) every block at its own place
+template <typename R, bool SHARED, class F>
 __global__ void write_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
                                     int64_t nchunks, const int* owner, const int* slot, int* id, R* pool) {
   const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= d.nz * d.ny * nchunks) return;
-  if (slot && owner[slot[b]] != (int)b) return;
+  if (SHARED && owner[slot[b]] != (int)b) return;
   double v[8];
   block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31), v);
-  const int64_t at = slot ? (int64_t)id[slot[b]] : b;
-  const bool two = store_block(pool + at * x_block_elems<R>(), threadIdx.x & 31, v,
-                               exterior_faces(d, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31)));
+  const int64_t at = SHARED ? (int64_t)id[slot[b]] : b;
+  const bool two = store_block<R, SHARED>(pool + at * x_block_elems<R, SHARED>(), threadIdx.x & 31, v,
+                                          exterior_faces(d, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31)));
   __syncwarp();
-  if (two && slot && (threadIdx.x & 31) == 0) id[slot[b]] = (int)at | kXTwoWeights;
+  if (SHARED && two && (threadIdx.x & 31) == 0) id[slot[b]] = (int)at | kXTwoWeights;
 }
 template <class F>
 __global__ void index_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
@@ -475,7 +495,7 @@ cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const doub
                           unsigned char* scratch, Compressed* out, cudaStream_t s) {
   const int64_t nch = (d.nx + 31) / 32, blocks = block_count(d);
   const unsigned wgrid = (unsigned)((blocks + 7) / 8), tgrid = (unsigned)((blocks + 255) / 256);
-  const size_t bytes = sizeof(R) * x_block_elems<R>();
+  const size_t bytes = sizeof(R) * x_block_elems<R, true>(), own_bytes = sizeof(R) * x_block_elems<R, false>();
   LineJob job[3];
   job[0].grid = {c.a0, c.b0, d.nz * d.ny, 1, c.px, d.nx, 1};
   job[0].mid = two_ended ? x_mid(d.nx) : -1;
@@ -483,10 +503,10 @@ cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const doub
   job[2].grid = {c.a2, c.b2, d.ny, d.nx, c.px, d.nz, d.ny * c.px};
   // all four searches are queued, then their counts read at once, and the checks' outcomes likewise
   unsigned char* at = scratch;
-  bool on[4] = {};
+  bool on[4] = {};  // (without scratch none is)
   int host[4][2] = {};
   cudaError_t e = cudaSuccess;
-  for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
+  for (int a = 0; a < 3 && scratch && e == cudaSuccess; ++a) {
     const int64_t lines = job[a].grid.lines();
     if (lines >= ((int64_t)1 << 29)) continue;
     on[a] = true;
@@ -496,7 +516,7 @@ cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const doub
       e = cudaMemcpyAsync(host[a], job[a].table.count, sizeof(int), cudaMemcpyDeviceToHost, s);
   }
   ClassTable t(blocks_countable(d) ? blocks : 0);
-  if (e == cudaSuccess && blocks_countable(d)) {
+  if (e == cudaSuccess && scratch && blocks_countable(d)) {
     on[3] = true;
     t.place(at);
     e = t.clear(s);
@@ -525,7 +545,7 @@ cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const doub
     e = cudaMalloc(&x.pool, x.bytes);
     if (e == cudaSuccess) {
       x.bidx = reinterpret_cast<int32_t*>((unsigned char*)x.pool + bytes * x.count);
-      write_blocks_kernel<R><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, (R*)x.pool);
+      write_blocks_kernel<R, true><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, (R*)x.pool);
       index_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, x.bidx, t.count + 1);
       e = cudaGetLastError();
     }
@@ -544,10 +564,10 @@ cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const doub
   }
   if (e == cudaSuccess && !shared) {  // every block for itself
     x.count = blocks;
-    x.bytes = bytes * blocks;
+    x.bytes = own_bytes * blocks;
     e = cudaMalloc(&x.pool, x.bytes);
     if (e == cudaSuccess) {
-      write_blocks_kernel<R><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, nullptr, nullptr, nullptr, (R*)x.pool);
+      write_blocks_kernel<R, false><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, nullptr, nullptr, nullptr, (R*)x.pool);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -14,8 +14,6 @@ struct Dims {
   __host__ __device__ int64_t nxy() const { return ny * nx; }
 };
 
-constexpr int kXBlockDoubles = (8 + 6) * 32 + 16;  // an FP64 stencil block (hs2g_x.cuh)
-
 // middle column of the two-ended x elimination
 __host__ __device__ inline int64_t x_mid(int64_t nx) { return (nx - 1) / 2; }
 
@@ -214,8 +212,8 @@ struct Faces {
 cudaError_t launch_factor(const Dims& d, const Faces& f, const double* M, const uint8_t* compute, double* s2,
                           double* sigma, const Coeffs& c, cudaStream_t s, bool two_ended);
 // What the step keeps of the factors (hs2g_compile.cu): the stencil blocks, and the x, y and z line tables where the
-// lines have few classes (lines[a].cls null: c's arrays stay).  scratch: compress_scratch(d) bytes.  Waits for the
-// stream.
+// lines have few classes (lines[a].cls null: c's arrays stay).  scratch: compress_scratch(d) bytes, or null: no search,
+// everything in voxel order.  Waits for the stream.
 struct Compressed {
   XBlocks blocks;
   LineTables lines[3];

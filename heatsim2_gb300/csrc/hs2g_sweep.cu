@@ -39,7 +39,7 @@ __device__ __forceinline__ void x_sources(XProblem<double>& P, const XTable<SRC>
   }
 }
 // The stencil of the x-lines [begin, end): a CTA per kXStencilLines lines and per gridDim.y-th chunk of columns.
-template <int SRC, typename IX>
+template <int SRC, bool SHARED, typename IX>
 __global__ void __launch_bounds__(32 * kXStencilWarps, kXStencilCtas) x_stencil_kernel(XProblem<double> P, XTable<SRC> qt,
                                                                            const DevSchedule* ds, int64_t begin,
                                                                            int64_t end) {
@@ -47,17 +47,17 @@ __global__ void __launch_bounds__(32 * kXStencilWarps, kXStencilCtas) x_stencil_
   __shared__ double sq[SRC == kNoSource ? 1 : HS2G_MAX_CLASSES];
   x_sources<SRC>(P, qt, ds, sq);
   wait_prior_grid();  // T comes from the previous step's z sweep, which used W0 as its scratch
-  x_stencil_lines<double, SRC != kNoSource, IX>(P, begin + blockIdx.x * (int64_t)kXStencilLines, end, blockIdx.y,
+  x_stencil_lines<double, SRC != kNoSource, SHARED, IX>(P, begin + blockIdx.x * (int64_t)kXStencilLines, end, blockIdx.y,
                                                 gridDim.y, lines, sq);
 }
 // The whole x sweep of [begin, end), 16 lines per CTA.
-template <int SRC, typename IX>
+template <int SRC, bool SHARED, typename IX>
 __global__ void __launch_bounds__(kXFusedThreads, 3) x_fused_kernel(XProblem<double> P, XTable<SRC> qt,
                                                                     const DevSchedule* ds, int64_t begin, int64_t end) {
   extern __shared__ __align__(16) unsigned char x_sm[];
   x_sources<SRC>(P, qt, ds, reinterpret_cast<double*>(x_sm));
   wait_prior_grid();
-  x_fused_lines<SRC != kNoSource, IX>(P, begin + blockIdx.x * (int64_t)16, end, x_sm);
+  x_fused_lines<SRC != kNoSource, SHARED, IX>(P, begin + blockIdx.x * (int64_t)16, end, x_sm);
 }
 // The x line solves of [begin, end) in W0, 16 lines per warp.
 template <bool TABLE, bool KEEP>
@@ -79,7 +79,7 @@ XSolveKernel x_solve_for(bool table, bool keep) {
   return table ? (keep ? x_solve_kernel<true, true> : x_solve_kernel<true, false>)
                : (keep ? x_solve_kernel<false, true> : x_solve_kernel<false, false>);
 }
-template <int SRC>
+template <int SRC, bool SHARED>
 cudaError_t launch_x(const StepArgs& a, const Coeffs& c, const XTable<SRC>& q, const DevSchedule* ds, int64_t begin,
                      int64_t end, cudaStream_t s) {
   if (end <= begin) return cudaSuccess;
@@ -88,9 +88,9 @@ cudaError_t launch_x(const StepArgs& a, const Coeffs& c, const XTable<SRC>& q, c
   if (c.cls0 && (x_index32(a.d, c) ? x_fused<int32_t>(a.d.nx, end - begin) : x_fused<int64_t>(a.d.nx, end - begin))) {
     const dim3 grid((unsigned)((end - begin + 15) / 16)), block(kXFusedThreads);
     if (x_index32(a.d, c))
-      return launch_kernel(x_fused_kernel<SRC, int32_t>, grid, block, x_fused_smem<int32_t>(a.d.nx), s, a.pdl_x, P, q, ds,
+      return launch_kernel(x_fused_kernel<SRC, SHARED, int32_t>, grid, block, x_fused_smem<int32_t>(a.d.nx), s, a.pdl_x, P, q, ds,
                            begin, end);
-    return launch_kernel(x_fused_kernel<SRC, int64_t>, grid, block, x_fused_smem<int64_t>(a.d.nx), s, a.pdl_x, P, q, ds,
+    return launch_kernel(x_fused_kernel<SRC, SHARED, int64_t>, grid, block, x_fused_smem<int64_t>(a.d.nx), s, a.pdl_x, P, q, ds,
                          begin, end);
   }
   // a CTA walks its lines' chunks, or takes every second, fourth ... of them until there are CTAs enough for the GPU
@@ -99,8 +99,8 @@ cudaError_t launch_x(const StepArgs& a, const Coeffs& c, const XTable<SRC>& q, c
   while (split < c.nchunks && split < 32768 && ctas * split < 152 * 8) split *= 2;
   const dim3 grid((unsigned)ctas, split), block(32 * kXStencilWarps);
   cudaError_t e = x_index32(a.d, c)
-                      ? launch_kernel(x_stencil_kernel<SRC, int32_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end)
-                      : launch_kernel(x_stencil_kernel<SRC, int64_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end);
+                      ? launch_kernel(x_stencil_kernel<SRC, SHARED, int32_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end)
+                      : launch_kernel(x_stencil_kernel<SRC, SHARED, int64_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end);
   if (e != cudaSuccess) return e;
   const int64_t groups = (end - begin + x_lines<true>() - 1) / x_lines<true>();
   const PairShape sh = c.cls0 ? x_solve_shape<double, true, true>(a.d.nx, groups)
@@ -110,8 +110,11 @@ cudaError_t launch_x(const StepArgs& a, const Coeffs& c, const XTable<SRC>& q, c
 }
 cudaError_t launch_x_any(const StepArgs& a, const Coeffs& c, const QTable& q, int64_t begin, int64_t end,
                          cudaStream_t s) {
-  if (a.has_qtab || a.qdense) return launch_x<kTable>(a, c, q, nullptr, begin, end, s);
-  return launch_x<kNoSource>(a, c, 0, nullptr, begin, end, s);
+  if (a.has_qtab || a.qdense)
+    return c.bidx ? launch_x<kTable, true>(a, c, q, nullptr, begin, end, s)
+                  : launch_x<kTable, false>(a, c, q, nullptr, begin, end, s);
+  return c.bidx ? launch_x<kNoSource, true>(a, c, 0, nullptr, begin, end, s)
+                : launch_x<kNoSource, false>(a, c, 0, nullptr, begin, end, s);
 }
 
 // The y sweep (ADD_T false: W1 = s2 * dT1 from W0 = sigma * dT0; rows of lines k) and the z sweep (ADD_T: T_out =
@@ -315,10 +318,17 @@ cudaError_t sweeps_prepare(const Dims& d, const Coeffs& c) {
             most(tz ? pair_smem<double, true, true, true, true>(d.nz) : pair_smem<double, true, true, true, false>(d.nz),
                  pair_smem<double, true, true, false, false>(d.nz)));
   }
-  const void* fused[] = {(const void*)x_fused_kernel<kNoSource, int32_t>, (const void*)x_fused_kernel<kTable, int32_t>,
-                         (const void*)x_fused_kernel<kRow, int32_t>,      (const void*)x_fused_kernel<kNoSource, int64_t>,
-                         (const void*)x_fused_kernel<kTable, int64_t>,    (const void*)x_fused_kernel<kRow, int64_t>};
-  for (const void* k : fused) allow(k, x_fused_smem<int64_t>(d.nx));
+  auto allow_fused = [&](auto shared) {
+    constexpr bool S = decltype(shared)::value;
+    for (const void* k : {(const void*)x_fused_kernel<kNoSource, S, int32_t>, (const void*)x_fused_kernel<kTable, S, int32_t>,
+                          (const void*)x_fused_kernel<kRow, S, int32_t>, (const void*)x_fused_kernel<kNoSource, S, int64_t>,
+                          (const void*)x_fused_kernel<kTable, S, int64_t>, (const void*)x_fused_kernel<kRow, S, int64_t>})
+      allow(k, x_fused_smem<int64_t>(d.nx));
+  };
+  if (c.bidx)
+    allow_fused(std::true_type());
+  else
+    allow_fused(std::false_type());
   return e;
 }
 
@@ -336,7 +346,8 @@ cudaError_t launch_step(const StepArgs& a, const Coeffs& c, const QTable& q, cud
 }
 
 cudaError_t launch_step_row(const StepArgs& a, const Coeffs& c, const DevSchedule* ds, cudaStream_t s) {
-  const cudaError_t e = launch_x<kRow>(a, c, 0, ds, 0, a.d.nz * a.d.ny, s);
+  const cudaError_t e = c.bidx ? launch_x<kRow, true>(a, c, 0, ds, 0, a.d.nz * a.d.ny, s)
+                               : launch_x<kRow, false>(a, c, 0, ds, 0, a.d.nz * a.d.ny, s);
   if (e != cudaSuccess) return e;
   return launch_yz(a, c, s, nullptr);
 }

@@ -32,15 +32,23 @@ __host__ __device__ constexpr int x_lines() {
   return TWO ? 16 : 32;
 }
 
-// Stencil block of 32 columns of an x-line: [wc, wxl, wxh, wyl, wyh, wzl, wzh, wq] x 32 and, in FP64, the six face
-// weights as integers x 32 (low word signed, high word below 2^31) and their exponents (int32 x 32).  A face on the
-// grid's exterior has no neighbour, the voxel itself stands in for it, and its integer weight may be anything: it is
-// set to the opposite face's.  Where a voxel's four x and y weights are then equal and its two z weights too, two
-// products do (x_int_stencil2); a block of such voxels has kXTwoWeights set in its index.
+// Stencil block of 32 columns of an x-line: [wc, wxl, wxh, wyl, wyh, wzl, wzh, wq] x 32 and, in FP64 where the blocks
+// repeat (SHARED, an index names the block of a line's columns), the six face weights as integers x 32 (low word signed,
+// high word below 2^31) and their exponents (int32 x 32).  A face on the grid's exterior has no neighbour, the voxel
+// itself stands in for it, and its integer weight may be anything: it is set to the opposite face's.  Where a voxel's
+// four x and y weights are then equal and its two z weights too, two products do (x_int_stencil2); a block of such voxels
+// has kXTwoWeights set in its index.
+// Where the blocks do not repeat every column has its own and keeps each weight once, as an integer, in 64 bytes per voxel
+// (both forms take 116, and a quarter fewer voxels fit the device): the six weights x 32, the high words of wc x 32 (its
+// exponent is the weights'), the low words x 32, wq x 32.  A voxel whose weights no integers stand for (x_own_fine) has
+// them as doubles in the integers' place and kXOwnDoubles for wc's high word.  64x256x512, no two blocks alike: as fast as
+// with both forms (309 us per step against 310; 340 against 339 where the temperatures need the chain); with doubles kept
+// and made integers on reading 348.
 constexpr int32_t kXTwoWeights = 1 << 30;
-template <typename R>
+constexpr int kXOwnDoubles = 0x7ff80000;
+template <typename R, bool SHARED>
 __host__ __device__ constexpr int x_block_elems() {
-  return sizeof(R) == 8 ? (8 + 6) * 32 + 16 : 8 * 32;
+  return sizeof(R) == 8 && SHARED ? (8 + 6) * 32 + 16 : 8 * 32;
 }
 
 // The exact integers' part of a block: w_f = wi_f * 2^(E - 62) with E the exponent of the weights' sum.  Returns E + 4,
@@ -64,7 +72,6 @@ __device__ __forceinline__ int x_int_weights(const double (&w)[6], uint2 (&wi)[6
   }
   return fine ? E + 4 : -100000;
 }
-
 // s * 2^(x0 - 1086) rounded to nearest, negated for negative temperatures (hp: the sign); |s| < 2^61, and x0 leaves no
 // result out of range.  In integers too: a conversion instruction takes the FP64 unit as long as an FMA of the
 // recurrences, which it would hold up.
@@ -80,6 +87,27 @@ __device__ __forceinline__ double x_scaled(long long s, int hp, int x0) {
 // exponent, neither zero nor infinite nor NaN, and a result whose exponent is in range for every sum
 __device__ __forceinline__ bool x_representable(unsigned diff, int hp, int x0) {
   return diff < (1u << 20) && (unsigned)(((hp >> 20) & 0x7ff) - 1) < 2046u && (unsigned)(x0 - 64) < 1981u;
+}
+
+// A column's own block: whether integers stand for its weights w with wc their negative sum (the exponents leave room for
+// every weight as a normal number), their exponent as x_int_weights returns it, from wc's high word, and a weight back.
+__device__ __forceinline__ bool x_own_fine(double wc, const double (&w)[6]) {
+  const int ec = (__double2hiint(wc) >> 20) & 0x7ff;
+  bool fine = wc == 0.0 || (wc < 0.0 && ec > 123 && ec < 2047);
+#pragma unroll
+  for (int f = 0; f < 6; ++f) fine &= w[f] >= 0.0 && w[f] <= -wc * (1.0 + 0x1p-40);
+  return fine;
+}
+__device__ __forceinline__ int x_own_exponent(int hi) {
+  const int ec = (hi >> 20) & 0x7ff;
+  return ec == 0 ? 4 : ec == 2047 ? -100000 : ec - 1022 + 4;
+}
+// (the integer has at most the double's 53 significant bits: as x_scaled, with nothing to round)
+__device__ __forceinline__ double x_own_weight(uint2 wi, int e4) {
+  const unsigned long long v = ((unsigned long long)wi.y << 32) + (unsigned long long)(long long)(int)wi.x;
+  const int lz = __clzll((long long)v);
+  const unsigned long long q = (v << ((lz - 1) & 63)) >> 10;  // top bit at 52
+  return __hiloint2double(v ? ((e4 + 1019 - lz) << 20) + (int)(q >> 32) : 0, (int)(unsigned)q);
 }
 
 // sum of wi_f (T_f - T_p) as a double; t: the six neighbours' temperatures; ok false: not representable, use FP64.  two:
@@ -147,7 +175,7 @@ struct XProblem {
   int64_t nz, ny, nx;
   const R* T;
   const R* pool;         // stencil blocks
-  const int32_t* bidx;   // block of (line, chunk), or null: one block each, in order
+  const int32_t* bidx;   // block of (line, chunk) (SHARED), or null: one block each, in order
   int64_t nchunks;
   const R* a0;           // row pitch px, or with cls tables per line class (last first right of the middle column)
   const R* b0;
@@ -189,25 +217,66 @@ __device__ __forceinline__ R x_chain(const R* __restrict__ w, R t, const R (&n)[
   return r;
 }
 
+// the chain for a column with a block of its own; every lane of the warp calls it
+__device__ __forceinline__ double x_chain_own(const double* __restrict__ blk, int slot, double t, const double (&n)[6]) {
+  const int* words = reinterpret_cast<const int*>(blk + 6 * 32);
+  const int hi = words[slot], e4 = x_own_exponent(hi);
+  double w[6], wc = __hiloint2double(hi, words[32 + slot]);
+#pragma unroll
+  for (int f = 0; f < 6; ++f) w[f] = x_own_weight(reinterpret_cast<const uint2*>(blk)[f * 32 + slot], e4);
+  const bool doubles = hi == kXOwnDoubles;
+  int some = __any_sync(0xffffffffu, doubles);
+  while (some) {  // (a branch that stays one, as in x_stencil_values)
+#pragma unroll
+    for (int f = 0; f < 6; ++f) w[f] = doubles ? blk[f * 32 + slot] : w[f];
+    wc = doubles ? -(((w[0] + w[1]) + (w[2] + w[3])) + (w[4] + w[5])) : wc;
+    asm volatile("mov.u32 %0, 0;" : "=r"(some));
+  }
+  double r = wc * t;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) r = fma(w[f], n[f], r);
+  return r;
+}
+
 // Right-hand sides of column c (a lane's own) of the PER lines at own.  Every lane of the warp calls it.
-template <typename R, bool HAS_Q, int PER, typename IX>
+template <typename R, bool HAS_Q, bool SHARED, int PER, typename IX>
 __device__ __forceinline__ void x_stencil_values(const XProblem<R>& P, const XLine<IX>* own, const R* sq, int c,
                                                  R (&r)[PER]) {
   const int slot = c & 31;
   const IX dxl = c > 0 ? -1 : 0, dxh = c + 1 < (int)P.nx ? 1 : 0;
   int32_t blk[PER];
   int32_t two = kXTwoWeights;
+  if constexpr (SHARED) {
 #pragma unroll
-  for (int l = 0; l < PER; ++l) {
-    const IX at = own[l].blk + (c >> 5);
-    blk[l] = P.bidx ? P.bidx[at] : (int32_t)at;
-    two &= blk[l];
+    for (int l = 0; l < PER; ++l) {
+      const IX at = own[l].blk + (c >> 5);
+      blk[l] = P.bidx ? P.bidx[at] : (int32_t)at;
+      two &= blk[l];
+    }
   }
-  auto at = [&](int l) { return P.pool + (int64_t)(blk[l] & ~kXTwoWeights) * x_block_elems<R>() + slot; };
+  auto at = [&](int l) {
+    if constexpr (SHARED)
+      return P.pool + (int64_t)(blk[l] & ~kXTwoWeights) * x_block_elems<R, true>() + slot;
+    else
+      return P.pool + (int64_t)(own[l].blk + (c >> 5)) * x_block_elems<R, false>() + slot;
+  };
   if constexpr (sizeof(R) == 8) {
     unsigned bad = 0;
     auto exponent = [&](int l) { return reinterpret_cast<const int*>(at(l) - slot + 14 * 32)[slot]; };
-    if (__all_sync(0xffffffffu, two)) {
+    if constexpr (!SHARED) {
+#pragma unroll
+      for (int l = 0; l < PER; ++l) {
+        R t, n[6];
+        x_load(P.T, own[l].base + (IX)c, own[l], dxl, dxh, t, n);
+        const uint2* __restrict__ iw = reinterpret_cast<const uint2*>(at(l));
+        uint2 wi[6];
+#pragma unroll
+        for (int f = 0; f < 6; ++f) wi[f] = iw[f * 32];
+        bool ok;
+        r[l] = x_int_stencil(t, n, wi, x_own_exponent(reinterpret_cast<const int*>(at(l) - slot + 6 * 32)[slot]), false, ok);
+        bad |= ok ? 0u : 1u << l;
+      }
+    } else if (__all_sync(0xffffffffu, two)) {
 #pragma unroll
       for (int l = 0; l < PER; ++l) {
         R t, n[6];
@@ -239,7 +308,11 @@ __device__ __forceinline__ void x_stencil_values(const XProblem<R>& P, const XLi
       for (int l = 0; l < PER; ++l) {
         R t, n[6];
         x_load(P.T, own[l].base + (IX)c, own[l], dxl, dxh, t, n);
-        const R v = x_chain(at(l), t, n);
+        R v;
+        if constexpr (SHARED)
+          v = x_chain(at(l), t, n);
+        else
+          v = x_chain_own(at(l) - slot, slot, t, n);
         r[l] = bad >> l & 1 ? v : r[l];
       }
       asm volatile("mov.u32 %0, 0;" : "=r"(again));
@@ -280,7 +353,7 @@ __device__ __forceinline__ void x_fill_lines(const XProblem<R>& P, int64_t L0, i
 
 // The stencil of the x-lines [L0, L0 + kXStencilLines) up to line_end, columns of chunks ch0, ch0 + dch, ...: right-hand
 // sides into W0.  Called by every thread of a CTA of kXStencilWarps warps; lines: shared memory; sq: the source values.
-template <typename R, bool HAS_Q, typename IX>
+template <typename R, bool HAS_Q, bool SHARED, typename IX>
 __device__ __forceinline__ void x_stencil_lines(const XProblem<R>& P, int64_t L0, int64_t line_end, int ch0, int dch,
                                                 XLine<IX>* lines, const R* sq) {
   constexpr int PER = kXStencilPer;
@@ -293,7 +366,7 @@ __device__ __forceinline__ void x_stencil_lines(const XProblem<R>& P, int64_t L0
   for (int ch = ch0; ch < (int)P.nchunks; ch += dch) {
     const int i = ch * 32 + lane;
     R r[PER];
-    x_stencil_values<R, HAS_Q, PER, IX>(P, own, sq, min(i, (int)P.nx - 1), r);  // lanes past the end repeat the last
+    x_stencil_values<R, HAS_Q, SHARED, PER, IX>(P, own, sq, min(i, (int)P.nx - 1), r);  // lanes past the end repeat the last
 #pragma unroll
     for (int l = 0; l < PER; ++l)
       if (l < mine && i < (int)P.nx) P.W0[own[l].out + i] = r[l];
@@ -593,7 +666,7 @@ __device__ __forceinline__ void x_bar_arrive(int b) {
 
 // The lines [L0, L0 + 16) up to line_end.  Called by every thread of a CTA of kXFusedThreads; the source values are at
 // the start of smem.
-template <bool HAS_Q, typename IX>
+template <bool HAS_Q, bool SHARED, typename IX>
 __device__ __forceinline__ void x_fused_lines(const XProblem<double>& P, int64_t L0, int64_t line_end,
                                               unsigned char* smem) {
   constexpr int PER = 16 / kXStencilWarps, FULL = 1, EMPTY = 3;
@@ -614,7 +687,7 @@ __device__ __forceinline__ void x_fused_lines(const XProblem<double>& P, int64_t
       for (int s = 0; s < 2; ++s) {
         const int i = column(q, s, lane);
         double r[PER];
-        x_stencil_values<double, HAS_Q, PER, IX>(P, own, sq, exists(s, i) ? i : 0, r);
+        x_stencil_values<double, HAS_Q, SHARED, PER, IX>(P, own, sq, exists(s, i) ? i : 0, r);
 #pragma unroll
         for (int l = 0; l < PER; ++l) bufs[q].v[s][warp * PER + l][lane] = r[l];
       }
