@@ -428,10 +428,11 @@ __global__ void adj_seed_kernel(AView v, const double* __restrict__ diff, int64_
 // gradient accumulation of one step; one thread per voxel, each voxel owning its three low faces.
 // FP64 arithmetic bounds it, so what can be had without is: the increments h = y / 2 are halved (the x stage's scale
 // is, exactly, and with it what follows), which takes the factors 1/2 out of the face gradients; a voxel's
-// T + h0 and its difference of mu0 to the left are formed once and shared through shared memory with the
-// neighbour that needs them; the source gradient is skipped where s = 0.  gM accumulates half its value.
-// 29 operations (30 with a source) against 34, five CTAs to an SM (48 registers): 5.86 million voxels 323 us
-// against 375 (the FP64 unit 84% busy; 22 fields of 8 bytes take 154).
+// difference of mu0 to the left is formed once and shared through shared memory with the neighbour that needs it, as
+// are T and h0; the source gradient is skipped where s = 0.  gM accumulates half its value.  (T + h0 is not formed per
+// voxel, which would save one more operation: where T is large against the differences of h0 it loses their digits.)
+// 30 operations (31 with a source) against 34, five CTAs to an SM (48 registers): 5.86 million voxels 342 us
+// against 375 (22 fields of 8 bytes take 154).
 constexpr int kUpdateThreads = 256;
 __global__ void __launch_bounds__(kUpdateThreads, 5) adj_update_kernel(
     AView v, const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
@@ -440,41 +441,35 @@ __global__ void __launch_bounds__(kUpdateThreads, 5) adj_update_kernel(
     const double* __restrict__ mu2, double s, const double* __restrict__ diff, int64_t obs_step,
     double* __restrict__ lam, double* __restrict__ ggx, double* __restrict__ ggy, double* __restrict__ ggz,
     double* __restrict__ gM, double* __restrict__ gq) {
-  __shared__ double sw[kUpdateThreads + 1], sd[kUpdateThreads + 1];
+  __shared__ double sT[kUpdateThreads + 1], sh[kUpdateThreads + 1], sd[kUpdateThreads + 1];
   const int t = threadIdx.x;
   const int64_t p0 = blockIdx.x * (int64_t)kUpdateThreads, p = p0 + t;
   Vox x{};
   if (p < v.nvox) x = vox_at(v, p);
   wait_prior_grid();  // the previous kernel on the stream (programmatic dependent launch)
-  double m0 = 0.0, Tp = 0.0, a0 = 0.0, d0x = 0.0, w = 0.0;
+  double m0 = 0.0, Tp = 0.0, a0 = 0.0, d0x = 0.0;
   if (x.in) {
     m0 = mu0[p];
     Tp = T[p];
     a0 = h0[p];
-    w = Tp + a0;
     if (x.i > 0) d0x = m0 - mu0[p - 1];
   }
-  sw[t + 1] = w;
+  sT[t + 1] = Tp;
+  sh[t + 1] = a0;
   sd[t] = d0x;
-  // the neighbours beyond the block (read by voxels of their row alone): T + h0 on the left, mu0's difference on the right
-  if (t < 2) {
-    const int64_t r = p0 + kUpdateThreads;
-    const double *b0 = t ? mu0 + r : T + p0 - 1, *b1 = t ? mu0 + r - 1 : h0 + p0 - 1;
-    double e0 = 0.0, e1 = 0.0;
-    if (t ? r < v.nvox : p0 > 0) {
-      e0 = *b0;
-      e1 = *b1;
-    }
-    if (t) e1 = -e1;
-    (t ? sd[kUpdateThreads] : sw[0]) = e0 + e1;
+  // the neighbours beyond the block (read by voxels of their row alone): T and h0 on the left, mu0's difference on the right
+  if (t == 0 && p0 > 0) {
+    sT[0] = T[p0 - 1];
+    sh[0] = h0[p0 - 1];
   }
+  if (t == 32 && p0 + kUpdateThreads < v.nvox) sd[kUpdateThreads] = mu0[p0 + kUpdateThreads] - mu0[p0 + kUpdateThreads - 1];
   __syncthreads();
   if (!x.in) return;
   const double m1 = mu1[p], m2 = mu2[p], a1 = h1[p], a2 = h2[p];
   double l = lam[p];
   if (x.i > 0) {
     l = fma(-gx[p], d0x, l);
-    ggx[p] = fma(-d0x, w - sw[t], ggx[p]);
+    ggx[p] = fma(-d0x, (a0 - sh[t]) + (Tp - sT[t]), ggx[p]);
   }
   if (x.j > 0) {
     const int64_t q = p - x.px;
