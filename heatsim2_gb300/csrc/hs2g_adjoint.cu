@@ -218,8 +218,12 @@ __global__ void adj_diag_kernel(AView v, const double* __restrict__ gx, const do
 //     x_m = W_m - a_m z_{m-1} - b_m z_{m+1},   W = rhs scale.
 // Kept: -a = G / (2 p) of the face away from the middle, -b = G / (2 p) of the face towards it, ip = 1 / p (x: half of
 // it, see adj_update_kernel) and mip = M / p, the scale of b = rhs and of b = M rhs.  A pair of lanes takes a line, one
-// end each.  FP64 arithmetic bounds the kernel on many lines: one reciprocal per row and quotients from it by one
-// correction step, 5.86 million voxels 688 us on the three axes against 865 with two divisions.
+// end each.  FP64 arithmetic bounds the kernel on many lines: one reciprocal per row and b from it by one correction step,
+// 5.86 million voxels 688 us on the three axes against 865 with two divisions.  The step is Markstein's (Computation of
+// elementary functions on the IBM RISC System/6000 processor, 1990): y the rounded reciprocal, q = y in to within two
+// units of its last place, q + (in - q p) y with two fused multiply-adds is in / p to within half a unit and 2^-103 of
+// it.  It wants the remainder in - q p exact and y a normal number: with p at most 1e300 (a fixed voxel's row) y is one,
+// and the remainder's last digit stays far above the smallest number for every conductance above 1e-100.
 __global__ void adj_factor_kernel(AView v, int axis, int64_t nlines, const double* __restrict__ M,
                                   const double* __restrict__ g, double* __restrict__ a, double* __restrict__ b,
                                   double* __restrict__ ip, double* __restrict__ mip) {
