@@ -222,8 +222,8 @@ __global__ void adj_diag_kernel(AView v, const double* __restrict__ gx, const do
 // 5.86 million voxels 688 us on the three axes against 865 with two divisions.  The step is Markstein's (Computation of
 // elementary functions on the IBM RISC System/6000 processor, 1990): y the rounded reciprocal, q = y in to within two
 // units of its last place, q + (in - q p) y with two fused multiply-adds is in / p to within half a unit and 2^-103 of
-// it.  It wants the remainder in - q p exact and y a normal number: with p at most 1e300 (a fixed voxel's row) y is one,
-// and the remainder's last digit stays far above the smallest number for every conductance above 1e-100.
+// it.  It wants y and q normal numbers and the remainder in - q p exact: p is at most 1e300 (a fixed voxel's row), whose
+// y is one, and q is for every conductance above 1e-7 there (below, it is off by units of 5e-324, which nothing sees).
 __global__ void adj_factor_kernel(AView v, int axis, int64_t nlines, const double* __restrict__ M,
                                   const double* __restrict__ g, double* __restrict__ a, double* __restrict__ b,
                                   double* __restrict__ ip, double* __restrict__ mip) {
