@@ -58,7 +58,6 @@ struct hs2g_handle {
   double* shape_volumes = nullptr;
   int64_t* shape_tiles = nullptr;
   unsigned long long* err_dev = nullptr;
-  int* status_dev = nullptr;
   bool graph_pdl = true;  // the captured step graphs launch their sweeps with programmatic dependent launch
   bool per_row = false;  // compiled from per-row conductances (hs2g_create_rows): no shared face arrays
   int64_t bytes = 0;
@@ -224,7 +223,6 @@ int alloc_common(hs2g_handle* h, bool faces = true) {
     if ((rc = dalloc(h, &c, 2 * np, "step coefficients"))) return rc;
   h->c.nchunks = (h->d.nx + 31) / 32;
   if ((rc = dalloc(h, &h->err_dev, 1, "error word"))) return rc;
-  if ((rc = dalloc(h, &h->status_dev, 1, "status word"))) return rc;
   h->c.a0 = h->coef[0];
   h->c.b0 = h->coef[0] + np;
   h->c.a1 = h->coef[1];
@@ -232,7 +230,6 @@ int alloc_common(hs2g_handle* h, bool faces = true) {
   h->c.a2 = h->coef[2];
   h->c.b2 = h->coef[2] + np;
   HS2G_CUDA(cudaMemsetAsync(h->err_dev, 0, sizeof(unsigned long long), h->stream), "clear error word");
-  HS2G_CUDA(cudaMemsetAsync(h->status_dev, 0, sizeof(int), h->stream), "clear status word");
   // HS2G_PDL=0: the step graphs' sweeps launched without programmatic dependent launch
   const char* pdl = getenv("HS2G_PDL");
   h->graph_pdl = !(pdl && strcmp(pdl, "0") == 0);
@@ -246,17 +243,7 @@ hs2g::StepArgs make_args(const hs2g_handle* h, const double* T_in, const double*
   a.W0 = h->W0;
   a.W1 = h->W1;
   a.vclass = h->vclass;
-  a.status = h->status_dev;
   return a;
-}
-
-// After a synchronisation: report a bounded device wait that ran out (and clear the word).
-int check_status(hs2g_handle* h) {
-  int v = 0;
-  HS2G_CUDA(cudaMemcpy(&v, h->status_dev, sizeof(int), cudaMemcpyDeviceToHost), "read status word");
-  if (v == 0) return HS2G_OK;
-  cudaMemset(h->status_dev, 0, sizeof(int));
-  return fail(v, "a device wait in a sweep kernel ran out of time (error %d)", v);
 }
 
 int new_handle(int device, const Dims& d, hs2g_handle** out) {
@@ -396,7 +383,7 @@ int step_host_pipelined(hs2g_handle* h, hs2g::StepArgs& a, const hs2g::QTable& q
   }
   HS2G_CUDA(cudaStreamSynchronize(cs), "step");
   HS2G_CUDA(cudaStreamSynchronize(s), "step");
-  return check_status(h);
+  return HS2G_OK;
 }
 
 // Whether host memory at p is page-locked.  Overlapped copies pay only then: the runtime stages pageable memory through
@@ -477,7 +464,6 @@ void hs2g_destroy(hs2g_handle* h) {
   cudaStreamSynchronize(h->stream);
   if (h->own_stream) cudaStreamSynchronize(h->own_stream);
   const int64_t n = h->d.nvox();
-  dfree(h, h->status_dev, 1);
   dfree(h, h->Gz, 0);
   dfree(h, h->Gy, 0);
   dfree(h, h->Gx, 0);
@@ -832,12 +818,8 @@ int hs2g_step(hs2g_handle* h, const double* T_in, double* T_out, const double* q
   if (e != cudaSuccess) return cuda_fail(e, "step kernels");
   if (!dev) {
     HS2G_CUDA(cudaMemcpyAsync(T_out, h->Tout_dev, sizeof(double) * n, cudaMemcpyDeviceToHost, s), "download T");
-    HS2G_CUDA(cudaStreamSynchronize(s), "step");
-    return check_status(h);
-  } else if (flags & HS2G_SYNC) {
-    HS2G_CUDA(cudaStreamSynchronize(s), "step");
-    return check_status(h);
   }
+  if (!dev || (flags & HS2G_SYNC)) HS2G_CUDA(cudaStreamSynchronize(s), "step");
   return HS2G_OK;
 }
 
@@ -1065,12 +1047,8 @@ int run_steps(hs2g_handle* h, int nsteps, const double* T_in, double* T_out, con
     if (history)
       HS2G_CUDA(cudaMemcpyAsync(history, h->hist_dev, sizeof(double) * nsteps * d.nxy(), cudaMemcpyDeviceToHost, s),
                 "download history");
-    HS2G_CUDA(cudaStreamSynchronize(s), "run");
-    return check_status(h);
-  } else if (flags & HS2G_SYNC) {
-    HS2G_CUDA(cudaStreamSynchronize(s), "run");
-    return check_status(h);
   }
+  if (!dev || (flags & HS2G_SYNC)) HS2G_CUDA(cudaStreamSynchronize(s), "run");
   return HS2G_OK;
 }
 }  // namespace
@@ -1177,7 +1155,7 @@ int hs2g_run_timed(hs2g_handle* h, int nsteps, const double* T_in, double* T_out
   }
   if (rc == HS2G_OK) {
     cudaError_t e = cudaStreamSynchronize(s);
-    rc = (e != cudaSuccess) ? cuda_fail(e, "run") : check_status(h);
+    if (e != cudaSuccess) rc = cuda_fail(e, "run");
   }
   kernel_ms[0] = kernel_ms[1] = kernel_ms[2] = kernel_ms[3] = 0.0;
   for (int st = 0; st < nsteps && rc == HS2G_OK; ++st)

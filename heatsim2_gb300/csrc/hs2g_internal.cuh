@@ -246,7 +246,6 @@ struct StepArgs {
   const double* qdense;  // may be null
   const double* qshape;  // per-voxel multiplier of the class sources (null: 1 everywhere)
   bool has_qtab;
-  int* status;           // device word: 0, or HS2G_ERR_TIMEOUT when a bounded wait in a kernel ran out
   bool pdl;              // launch the y and z sweeps with programmatic dependent launch (captured step graphs)
   bool pdl_x;            // the same for the x sweep (not for the first kernel of a graph)
 };

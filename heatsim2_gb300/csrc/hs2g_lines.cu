@@ -1,5 +1,6 @@
 // A bounded device wait and its self-test: a wait on an mbarrier gives up after a limit of %globaltimer time and
-// reports HS2G_ERR_TIMEOUT through a status word, leaving the context usable.
+// reports HS2G_ERR_TIMEOUT through its status word, leaving the context usable.  (The line solves are in hs2g_pair.cuh and
+// hs2g_x.cuh; they have no such wait.)
 #include "hs2g_internal.cuh"
 
 namespace hs2g {

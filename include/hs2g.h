@@ -36,7 +36,7 @@ extern "C" {
 #define HS2G_ERR_FORM (-7)       /* a face flux is not a conservative Crank-Nicolson two-point difference */
 #define HS2G_ERR_CAPACITY (-8)   /* a computed voxel has rho*c/dt <= 0 or not finite */
 #define HS2G_ERR_STATE (-9)      /* handle not in a state that allows this call */
-#define HS2G_ERR_TIMEOUT (-10)   /* a bounded wait inside a kernel ran out; the step's output is invalid */
+#define HS2G_ERR_TIMEOUT (-10)   /* a bounded wait inside a kernel ran out (hs2g_selftest_wait) */
 
 /* flags */
 #define HS2G_DEVICE 1            /* T_in / T_out / qdense / history are device pointers (no copies) */
@@ -375,7 +375,8 @@ int hs2g_adjoint_backward(hs2g_adjoint* a, double* gk, double* gC, double* gq, d
 
 /* Self-test of a bounded wait inside a kernel (failure detection without a fault): one thread waits at most limit_ns
    (<= 10 s) on an mbarrier that receives its one arrival (arrive != 0) or none.  *status receives HS2G_OK, or
-   HS2G_ERR_TIMEOUT -- the status a kernel reports whose wait ran out -- and the device stays usable either way. */
+   HS2G_ERR_TIMEOUT, and the device stays usable either way.  (The sweeps wait on nothing that could fail to come: on the
+   other warps of their CTA, on their own copies, and on the kernel before them.) */
 int hs2g_selftest_wait(int device, int64_t limit_ns, int arrive, int* status);
 
 /* Copy the compiled face conductances and capacities to host buffers (any may be NULL).  A handle made by
