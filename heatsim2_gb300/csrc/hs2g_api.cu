@@ -557,9 +557,9 @@ int hs2g_create_classes(const hs2g_class_problem* p, int device, hs2g_handle** o
     up(h->vclass, p->volumetric, (size_t)n);
   else if (e == cudaSuccess)
     e = cudaMemsetAsync(h->vclass, 0, (size_t)n, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 0, mat, bz, mats, p->nmat, forms, p->nbnd, h->Gz, h->err_dev, table, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 1, mat, by, mats, p->nmat, forms, p->nbnd, h->Gy, h->err_dev, table, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 2, mat, bx, mats, p->nmat, forms, p->nbnd, h->Gx, h->err_dev, table, s);
+  const uint8_t* bclass[3] = {bz, by, bx};
+  double* G[3] = {h->Gz, h->Gy, h->Gx};
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, mat, bclass, mats, p->nmat, forms, p->nbnd, G, h->err_dev, table, s);
   if (e == cudaSuccess)
     e = hs2g::launch_capacity_from_classes(d, mat, mats, p->nmat, h->M, h->compute, h->err_dev, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -560,9 +560,9 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   up(forms, p.forms, sizeof(hs2g_face_form) * p.nbnd * 3);
   if (p.volumetric) up(b.vclass + I.off, p.volumetric, (size_t)n);
   else if (e == cudaSuccess) e = cudaMemsetAsync(b.vclass + I.off, 0, (size_t)n, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 0, mat, bz, mats, p.nmat, forms, p.nbnd, fz, err, table, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 1, mat, by, mats, p.nmat, forms, p.nbnd, fy, err, table, s);
-  if (e == cudaSuccess) e = hs2g::launch_faces(d, 2, mat, bx, mats, p.nmat, forms, p.nbnd, fx, err, table, s);
+  const uint8_t* bclass[3] = {bz, by, bx};
+  double* G[3] = {fz, fy, fx};
+  if (e == cudaSuccess) e = hs2g::launch_faces(d, mat, bclass, mats, p.nmat, forms, p.nbnd, G, err, table, s);
   if (e == cudaSuccess) e = hs2g::launch_capacity_from_classes(d, mat, mats, p.nmat, M, comp, err, s);
   if (e != cudaSuccess) return bcuda(e, "batch compile");
   unsigned long long v = 0;
@@ -591,37 +591,42 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   hs2g::Compressed kept;
   if ((e = hs2g::compress_coeffs(d, faces, comp, s2, c, b.precision, scratch, &kept, s)) != cudaSuccess)
     return bcuda(e, "batch factor");
-  b.coef_mem.push_back(kept.blocks.pool);
+  for (void* m : {kept.mem, kept.own})
+    if (m) b.coef_mem.push_back(m);
   I.pool = kept.blocks.pool;
   I.bidx = kept.blocks.bidx;
   if (!I.bidx) b.dense_blocks = true;
   b.bytes += (int64_t)kept.blocks.bytes;
   const double* coeffs[3][2] = {{c.a0, c.b0}, {c.a1, c.b1}, {c.a2, c.b2}};
+  // in one allocation: float tables beside the classes, and the arrays where the lines have too many classes (whole
+  // 256 bytes each)
+  int64_t count[3] = {}, total = 0;
   for (int ax = 0; ax < 3; ++ax) {
-    hs2g::LineTables& t = kept.lines[ax];
-    if (t.cls) {
-      b.coef_mem.push_back(t.a);
-      b.bytes += (int64_t)t.bytes;
-    } else {
-      b.dense[ax] = true;
-    }
+    const hs2g::LineTables& t = kept.lines[ax];
     I.cls[ax] = t.cls;
-    const void** dst[2] = {&I.a[ax], &I.b[ax]};
+    if (t.cls) b.bytes += (int64_t)t.bytes;
+    else b.dense[ax] = true;
     if (t.cls && f64) {  // the tables as they are
       I.a[ax] = t.a;
       I.b[ax] = t.b;
-      continue;
+    } else {
+      count[ax] = t.cls ? t.nclass * (ax == 0 ? d.nx : ax == 1 ? d.ny : d.nz) : np;
+      total += 2 * ((count[ax] + 63) & ~int64_t(63));
     }
-    // float tables beside the classes, or the arrays where the lines have too many classes
-    const int64_t count = t.cls ? t.nclass * (ax == 0 ? d.nx : ax == 1 ? d.ny : d.nz) : np;
-    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
-      void* m = nullptr;
-      e = cudaMalloc(&m, b.elem() * count);
-      if (e != cudaSuccess) break;
-      b.coef_mem.push_back(m);
-      b.bytes += (int64_t)b.elem() * count;
-      *dst[q] = m;
-      e = hs2g::batch_convert(t.cls ? (q ? t.b : t.a) : coeffs[ax][q], m, count, b.precision, s);
+  }
+  if (total) {
+    unsigned char* m = nullptr;
+    if ((e = cudaMalloc(&m, b.elem() * total)) != cudaSuccess) return bcuda(e, "batch factor");
+    b.coef_mem.push_back(m);
+    b.bytes += (int64_t)b.elem() * total;
+    for (int ax = 0; ax < 3; ++ax) {
+      const hs2g::LineTables& t = kept.lines[ax];
+      const void** dst[2] = {&I.a[ax], &I.b[ax]};
+      for (int q = 0; q < 2 && count[ax] && e == cudaSuccess; ++q) {
+        *dst[q] = m;
+        e = hs2g::batch_convert(t.cls ? (q ? t.b : t.a) : coeffs[ax][q], m, count[ax], b.precision, s);
+        m += b.elem() * ((count[ax] + 63) & ~int64_t(63));
+      }
     }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

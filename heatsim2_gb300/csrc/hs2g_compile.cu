@@ -6,6 +6,7 @@
 // alternatingdirection_c.c:102-199) and its LU factorisation at finalize (tridiag.pyx:9-43,
 // alternatingdirection_c_pyx.pyx:279).  All FP64.  One thread per face (compiler) or per grid line (LU).
 #include <algorithm>
+#include <climits>
 
 #include "hs2g_internal.cuh"
 #include "hs2g_x.cuh"
@@ -51,12 +52,12 @@ __device__ FaceValue face_value(const hs2g_material* __restrict__ mats, int nmat
   if (code == 0 && (mlo >= nmat || mhi >= nmat) && g != 0.0) code = HS2G_ERR_EXTERIOR;
   return {g, code};
 }
-// The values of every (class, low material, high material), nmat standing for outside the grid: one thread each.
-__global__ void face_values_kernel(int axis, const hs2g_material* __restrict__ mats, int nmat,
+// The values of every (axis, class, low material, high material), nmat standing for outside the grid: one thread each.
+__global__ void face_values_kernel(const hs2g_material* __restrict__ mats, int nmat,
                                    const hs2g_face_form* __restrict__ forms, int nbnd, FaceValue* __restrict__ table) {
-  const int m1 = nmat + 1, n = nbnd * m1 * m1;
+  const int m1 = nmat + 1, n = nbnd * m1 * m1, axis = blockIdx.y;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-    table[t] = face_value(mats, nmat, forms[t / (m1 * m1) * 3 + axis], t / m1 % m1, t % m1);
+    table[axis * n + t] = face_value(mats, nmat, forms[t / (m1 * m1) * 3 + axis], t / m1 % m1, t % m1);
 }
 
 // One thread per face of `axis`.  The two voxels that meet at a face are lo (index - 1 along the axis) and hi.
@@ -350,32 +351,50 @@ __global__ void factor_x_kernel(Dims d, F g, const double* __restrict__ M, const
   b0[t * px + m] = -(upper(m, r.hi, piv));
 }
 
-// The eight stage-0 coefficients of column i of x-line t (zeros past the line's end).
+// Column `lane` of stencil block b: its row (k, j), column i (past the line's end: none) and voxel.
+struct BlockColumn {
+  int64_t k, j, i, p;
+};
+__device__ __forceinline__ BlockColumn block_column(const Dims& d, int64_t nchunks, int64_t b, int lane) {
+  int64_t t, k;
+  if (d.nz * d.ny * nchunks < ((int64_t)1 << 31)) {  // (64-bit divisions would take most of a setup kernel's time)
+    t = (unsigned)b / (unsigned)nchunks;
+    k = (unsigned)t / (unsigned)d.ny;
+  } else {
+    t = b / nchunks;
+    k = t / d.ny;
+  }
+  const int64_t i = (b - t * nchunks) * 32 + lane;
+  return {k, t - k * d.ny, i, t * d.nx + i};
+}
+// What its eight stage-0 coefficients are made of (zeros past the line's end): the six conductances and the row scale;
+// blocks are compared by these, without the FP64 unit, whose 12 operations would take the search 200 us of every 262144
+// blocks.  And which of its faces are on the grid's exterior (bit f, in the weights' order; 0 past the line's end).
 template <class F>
-__device__ __forceinline__ void block_values(const Dims& d, const F& g, const uint8_t* __restrict__ compute,
-                                             const double* __restrict__ f0, int64_t t, int64_t i, double (&v)[8]) {
+__device__ __forceinline__ void block_parts(const Dims& d, const F& g, const uint8_t* __restrict__ compute,
+                                            const double* __restrict__ f0, const BlockColumn& c, double (&v)[7]) {
 #pragma unroll
-  for (int c = 0; c < 8; ++c) v[c] = 0.0;
-  const int64_t k = t / d.ny, j = t - k * d.ny, p = t * d.nx + i;
-  if (i >= d.nx || !compute[p]) return;
-  const double gxl = g.xlo(d, p, k, j, i), gxh = g.xhi(d, p, k, j, i);
-  const double gyl = g.ylo(d, p, k, j, i), gyh = g.yhi(d, p, k, j, i);
-  const double gzl = g.zlo(d, p, k, j, i), gzh = g.zhi(d, p, k, j, i);
-  const double f = f0[p];
-  v[0] = f * -(((gxl + gxh) + (gyl + gyh)) + (gzl + gzh));
-  v[1] = f * gxl;
-  v[2] = f * gxh;
-  v[3] = f * gyl;
-  v[4] = f * gyh;
-  v[5] = f * gzl;
-  v[6] = f * gzh;
+  for (int e = 0; e < 7; ++e) v[e] = 0.0;
+  if (c.i >= d.nx || !compute[c.p]) return;
+  v[0] = g.xlo(d, c.p, c.k, c.j, c.i);
+  v[1] = g.xhi(d, c.p, c.k, c.j, c.i);
+  v[2] = g.ylo(d, c.p, c.k, c.j, c.i);
+  v[3] = g.yhi(d, c.p, c.k, c.j, c.i);
+  v[4] = g.zlo(d, c.p, c.k, c.j, c.i);
+  v[5] = g.zhi(d, c.p, c.k, c.j, c.i);
+  v[6] = f0[c.p];
+}
+__device__ __forceinline__ void block_values(const double (&g)[7], double (&v)[8]) {
+  const double f = g[6];
+  v[0] = f * -(((g[0] + g[1]) + (g[2] + g[3])) + (g[4] + g[5]));
+#pragma unroll
+  for (int e = 0; e < 6; ++e) v[1 + e] = f * g[e];
   v[7] = f;
 }
-// which of the voxel's faces are on the grid's exterior (bit f, in the weights' order); 0 past the line's end
-__device__ __forceinline__ int exterior_faces(const Dims& d, int64_t t, int64_t i) {
-  if (i >= d.nx) return 0;
-  const int64_t k = t / d.ny, j = t - k * d.ny;
-  return (i == 0) | (i + 1 == d.nx) << 1 | (j == 0) << 2 | (j + 1 == d.ny) << 3 | (k == 0) << 4 | (k + 1 == d.nz) << 5;
+__device__ __forceinline__ int exterior_faces(const Dims& d, const BlockColumn& c) {
+  if (c.i >= d.nx) return 0;
+  return (c.i == 0) | (c.i + 1 == d.nx) << 1 | (c.j == 0) << 2 | (c.j + 1 == d.ny) << 3 | (c.k == 0) << 4 |
+         (c.k + 1 == d.nz) << 5;
 }
 // writes a block (one warp); true when two products do for each of its voxels (kXTwoWeights)
 template <typename R, bool SHARED>
@@ -420,154 +439,142 @@ __device__ __forceinline__ bool store_block(R* blk, int lane, const double (&v)[
   return two;
 }
 
-// Distinct blocks (one warp per block): hashed into an open-addressing table, numbered, written once each, and every
-// block compared with the one it is replaced by (bit for bit; a clash of hashes clears *same).
+// Distinct blocks (one warp per block): hashed into an open-addressing table, numbered (hs2g_classes.cu), written once
+// each, and every block compared with its owner, bit for bit (a clash of hashes is noted in count[1]).
 template <class F>
 __global__ void hash_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
-                                   int64_t nchunks, unsigned long long* keys, int* owner, int64_t mask, int* slot) {
-  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+                                   int64_t nchunks, ClassTable t) {
+  __shared__ unsigned long long found[8];  // of the CTA's blocks; those alike go to the table as one
+  const int64_t b0 = blockIdx.x * (int64_t)8, b = b0 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (b >= d.nz * d.ny * nchunks) return;
-  double v[8];
-  block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + lane, v);
+  const BlockColumn col = block_column(d, nchunks, min(b, t.n - 1), lane);
+  double v[7];
+  block_parts(d, g, compute, f0, col, v);
   unsigned long long h = (unsigned long long)lane * 0xD6E8FEB86659FD93ull + 1 +
-                         ((unsigned long long)exterior_faces(d, b / nchunks, (b % nchunks) * 32 + lane) << 40);
+                         ((unsigned long long)exterior_faces(d, col) << 40);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < 7; ++c) {
     h = (h ^ (unsigned long long)__double_as_longlong(v[c])) * 0x9E3779B97F4A7C15ull;
     h ^= h >> 29;
   }
   for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-  if (lane) return;
   h = (h ^ (h >> 32)) * 0x9E3779B97F4A7C15ull;
-  if (h == 0) h = 1;
-  int64_t e = (int64_t)(h >> 17) & mask;
-  for (;; e = (e + 1) & mask) {  // the table has twice as many entries as there are blocks
-    const unsigned long long k = atomicCAS(keys + e, 0ull, h);
-    if (k == 0ull || k == h) break;
-  }
-  slot[b] = (int)e;
-  atomicMin(owner + e, (int)b);
-}
-__global__ void number_blocks_kernel(int64_t blocks, const int* owner, const int* slot, int* id, int* count) {
-  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b < blocks && owner[slot[b]] == (int)b) id[slot[b]] = atomicAdd(count, 1);
+  if (lane == 0) found[threadIdx.x >> 5] = b >= t.n ? 0 : h ? h : 1;
+  __syncthreads();
+  if (threadIdx.x >= 8) return;
+  t.insert_all(0xffu, found[lane], (int)b0 + lane);
 }
 // writes the owners' blocks, or (SHARED false) every block at its own place
 template <typename R, bool SHARED, class F>
 __global__ void write_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
-                                    int64_t nchunks, const int* owner, const int* slot, int* id, R* pool) {
-  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (b >= d.nz * d.ny * nchunks) return;
-  if (SHARED && owner[slot[b]] != (int)b) return;
-  double v[8];
-  block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31), v);
-  const int64_t at = SHARED ? (int64_t)id[slot[b]] : b;
-  const bool two = store_block<R, SHARED>(pool + at * x_block_elems<R, SHARED>(), threadIdx.x & 31, v,
-                                          exterior_faces(d, b / nchunks, (b % nchunks) * 32 + (threadIdx.x & 31)));
-  __syncwarp();
-  if (SHARED && two && (threadIdx.x & 31) == 0) id[slot[b]] = (int)at | kXTwoWeights;
-}
-template <class F>
-__global__ void index_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
-                                    int64_t nchunks, const int* owner, const int* slot, const int* id, int32_t* bidx,
-                                    int* same) {
+                                    int64_t nchunks, ClassTable t, R* pool) {
   const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (b >= d.nz * d.ny * nchunks) return;
-  const int64_t o = owner[slot[b]];
-  double v[8], w[8];
-  block_values(d, g, compute, f0, b / nchunks, (b % nchunks) * 32 + lane, v);
-  block_values(d, g, compute, f0, o / nchunks, (o % nchunks) * 32 + lane, w);
-  bool eq = exterior_faces(d, b / nchunks, (b % nchunks) * 32 + lane) == exterior_faces(d, o / nchunks, (o % nchunks) * 32 + lane);
+  if (SHARED && t.owner[t.slot[b]] != (int)b) return;
+  const BlockColumn col = block_column(d, nchunks, b, lane);
+  double parts[7], v[8];
+  block_parts(d, g, compute, f0, col, parts);
+  block_values(parts, v);
+  const int64_t at = SHARED ? (int64_t)t.id[t.slot[b]] : b;
+  const bool two = store_block<R, SHARED>(pool + at * x_block_elems<R, SHARED>(), lane, v, exterior_faces(d, col));
+  __syncwarp();
+  if (SHARED && two && lane == 0) t.id[t.slot[b]] = (int)at | kXTwoWeights;
+}
+template <class F>
+__global__ void index_blocks_kernel(Dims d, F g, const uint8_t* __restrict__ compute, const double* __restrict__ f0,
+                                    int64_t nchunks, ClassTable t, int32_t* bidx) {
+  const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (b >= t.n) return;
+  const BlockColumn col = block_column(d, nchunks, b, lane), own = block_column(d, nchunks, t.owner[t.slot[b]], lane);
+  double v[7], w[7];
+  block_parts(d, g, compute, f0, col, v);
+  block_parts(d, g, compute, f0, own, w);
+  bool eq = exterior_faces(d, col) == exterior_faces(d, own);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) eq &= __double_as_longlong(v[c]) == __double_as_longlong(w[c]);
-  if (!eq) *same = 0;
-  if (lane == 0) bidx[b] = id[slot[b]];
+  for (int c = 0; c < 7; ++c) eq &= __double_as_longlong(v[c]) == __double_as_longlong(w[c]);
+  if (!eq) t.count[1] = 1;
+  if (lane == 0) bidx[b] = t.id[t.slot[b]];
 }
 
 inline int64_t block_count(const Dims& d) { return d.nz * d.ny * ((d.nx + 31) / 32); }
 // things are numbered in 32 bits, and the index keeps a bit for kXTwoWeights
 inline bool blocks_countable(const Dims& d) { return block_count(d) < ((int64_t)1 << 29); }
+inline int64_t searched_lines(const Dims& d, int axis) {
+  const int64_t lines = axis == 0 ? d.nz * d.ny : axis == 1 ? d.nz * d.nx : d.nxy();
+  return lines < ((int64_t)1 << 29) ? lines : 0;
+}
 
 template <typename R, class F>
 cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const double* f0, const Coeffs& c, bool two_ended,
                           unsigned char* scratch, Compressed* out, cudaStream_t s) {
   const int64_t nch = (d.nx + 31) / 32, blocks = block_count(d);
-  const unsigned wgrid = (unsigned)((blocks + 7) / 8), tgrid = (unsigned)((blocks + 255) / 256);
+  const unsigned wgrid = (unsigned)((blocks + 7) / 8);
   const size_t bytes = sizeof(R) * x_block_elems<R, true>(), own_bytes = sizeof(R) * x_block_elems<R, false>();
-  LineJob job[3];
-  job[0].grid = {c.a0, c.b0, d.nz * d.ny, 1, c.px, d.nx, 1};
-  job[0].mid = two_ended ? x_mid(d.nx) : -1;
-  job[1].grid = {c.a1, c.b1, d.nz, d.nx, d.ny * c.px, d.ny, c.px};
-  job[2].grid = {c.a2, c.b2, d.ny, d.nx, c.px, d.nz, d.ny * c.px};
-  // all four searches are queued, then their counts read at once, and the checks' outcomes likewise
-  unsigned char* at = scratch;
-  bool on[4] = {};  // (without scratch none is)
+  LineSearch search{};
+  search.grid[0] = {c.a0, c.b0, d.nz * d.ny, 1, c.px, d.nx, 1};
+  search.grid[1] = {c.a1, c.b1, d.nz, d.nx, d.ny * c.px, d.ny, c.px};
+  search.grid[2] = {c.a2, c.b2, d.ny, d.nx, c.px, d.nz, d.ny * c.px};
+  search.mid[0] = two_ended ? x_mid(d.nx) : -1;
+  search.mid[1] = search.mid[2] = -1;
+  // the lines and the blocks are searched together, their counts read at once, and the checks' outcomes likewise
   int host[4][2] = {};
+  auto counts = [&]() {
+    return cudaMemcpyAsync(host, search.table[0].count, sizeof host, cudaMemcpyDeviceToHost, s);
+  };
+  ClassTable t(scratch && blocks_countable(d) ? blocks : 0);
+  for (int a = 0; a < 3; ++a) search.table[a] = ClassTable(scratch ? searched_lines(d, a) : 0);
   cudaError_t e = cudaSuccess;
-  for (int a = 0; a < 3 && scratch && e == cudaSuccess; ++a) {
-    const int64_t lines = job[a].grid.lines();
-    if (lines >= ((int64_t)1 << 29)) continue;
-    on[a] = true;
-    e = job[a].begin(at, s);
-    at += (LineJob::scratch_bytes(lines) + 255) & ~size_t(255);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(host[a], job[a].table.count, sizeof(int), cudaMemcpyDeviceToHost, s);
-  }
-  ClassTable t(blocks_countable(d) ? blocks : 0);
-  if (e == cudaSuccess && scratch && blocks_countable(d)) {
-    on[3] = true;
-    t.place(at);
-    e = t.clear(s);
-    if (e == cudaSuccess) {
-      hash_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.keys, t.owner, t.cap - 1, t.slot);
-      number_blocks_kernel<<<tgrid, 256, 0, s>>>(blocks, t.owner, t.slot, t.id, t.count);
+  if (scratch) {
+    e = search.begin(scratch, t, s);
+    if (e == cudaSuccess && t.n) {
+      hash_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(host[3], t.count, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = search.number(t, s);
+    if (e == cudaSuccess) e = counts();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  for (int a = 0; a < 3 && e == cudaSuccess; ++a)
-    if (on[a]) {
-      e = job[a].finish(host[a][0], &out->lines[a], s);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(host[a] + 1, job[a].table.count + 1, sizeof(int), cudaMemcpyDeviceToHost, s);
-    }
   // An index is worth it when at most a quarter of the blocks are distinct: the sweep then reads them from L2, and the
   // index costs it a dependent load
   XBlocks& x = out->blocks;
   const size_t index = sizeof(int32_t) * (size_t)blocks;
-  bool shared = on[3] && host[3][0] <= std::max<int64_t>(1, blocks / 4);
-  if (e == cudaSuccess && shared) {
-    x.count = host[3][0];
-    x.bytes = bytes * x.count + index;
-    e = cudaMalloc(&x.pool, x.bytes);
-    if (e == cudaSuccess) {
+  bool shared = t.n && host[3][0] <= std::max<int64_t>(1, blocks / 4);
+  if (e == cudaSuccess && scratch) {
+    x.count = shared ? host[3][0] : 0;
+    x.bytes = shared ? bytes * x.count + index : 0;
+    size_t tables = search.choose({host[0][0], host[1][0], host[2][0]});
+    if (tables + x.bytes) e = cudaMalloc(&out->mem, tables + x.bytes);
+    if (e == cudaErrorMemoryAllocation && tables) {  // no room for the tables: the arrays stay
+      cudaGetLastError();
+      tables = search.choose({INT_MAX, INT_MAX, INT_MAX});
+      e = shared ? cudaMalloc(&out->mem, x.bytes) : cudaSuccess;
+    }
+    if (e == cudaSuccess) e = search.finish((unsigned char*)out->mem, out->lines, s);
+    if (e == cudaSuccess && shared) {
+      x.pool = (unsigned char*)out->mem + tables;
       x.bidx = reinterpret_cast<int32_t*>((unsigned char*)x.pool + bytes * x.count);
-      write_blocks_kernel<R, true><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, (R*)x.pool);
-      index_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t.owner, t.slot, t.id, x.bidx, t.count + 1);
+      write_blocks_kernel<R, true><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t, (R*)x.pool);
+      index_blocks_kernel<<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, t, x.bidx);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(host[3] + 1, t.count + 1, sizeof(int), cudaMemcpyDeviceToHost, s);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  for (int a = 0; a < 3 && e == cudaSuccess; ++a)
-    if (out->lines[a].cls && !host[a][1]) {
-      cudaFree(out->lines[a].a);
-      out->lines[a] = LineTables{};
-    }
-  if (e == cudaSuccess && shared && !host[3][1]) {
-    cudaFree(x.pool);
-    x = XBlocks{};
-    shared = false;
+  if (e == cudaSuccess && scratch) {
+    e = counts();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    for (int a = 0; a < 3 && e == cudaSuccess; ++a)
+      if (out->lines[a].cls && host[a][1]) out->lines[a] = LineTables{};
+    if (e == cudaSuccess && shared && host[3][1]) shared = false;
   }
   if (e == cudaSuccess && !shared) {  // every block for itself
+    x = XBlocks{};
     x.count = blocks;
     x.bytes = own_bytes * blocks;
-    e = cudaMalloc(&x.pool, x.bytes);
+    e = cudaMalloc(&out->own, x.bytes);
     if (e == cudaSuccess) {
-      write_blocks_kernel<R, false><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, nullptr, nullptr, nullptr, (R*)x.pool);
+      x.pool = out->own;
+      write_blocks_kernel<R, false><<<wgrid, 256, 0, s>>>(d, g, compute, f0, nch, ClassTable(), (R*)x.pool);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -608,19 +615,21 @@ inline unsigned grid_for(int64_t n, int threads) {
 
 size_t face_table_bytes(int nmat, int nbnd) {
   const int64_t entries = (int64_t)nbnd * (nmat + 1) * (nmat + 1);
-  return entries <= 65536 ? sizeof(FaceValue) * (size_t)entries : 0;
+  return entries <= 65536 ? 3 * sizeof(FaceValue) * (size_t)entries : 0;
 }
 
-cudaError_t launch_faces(const Dims& d, int axis, const uint8_t* material, const uint8_t* bclass,
-                         const hs2g_material* mats, int nmat, const hs2g_face_form* forms, int nbnd, double* G,
-                         unsigned long long* err, void* table, cudaStream_t s) {
-  const int64_t nfaces = (d.nz + (axis == 0)) * (d.ny + (axis == 1)) * (d.nx + (axis == 2));
+cudaError_t launch_faces(const Dims& d, const uint8_t* material, const uint8_t* const bclass[3], const hs2g_material* mats,
+                         int nmat, const hs2g_face_form* forms, int nbnd, double* const G[3], unsigned long long* err,
+                         void* table, cudaStream_t s) {
   FaceValue* values = face_table_bytes(nmat, nbnd) ? static_cast<FaceValue*>(table) : nullptr;
+  const int64_t entries = (int64_t)nbnd * (nmat + 1) * (nmat + 1);
   if (values)
-    face_values_kernel<<<grid_for((int64_t)nbnd * (nmat + 1) * (nmat + 1), 64), 64, 0, s>>>(axis, mats, nmat, forms, nbnd,
-                                                                                         values);
-  faces_kernel<<<grid_for(nfaces, kThreads), kThreads, 0, s>>>(d, axis, material, bclass, mats, nmat, forms, nbnd,
-                                                               values, G, err);
+    face_values_kernel<<<dim3(grid_for(entries, 64), 3), 64, 0, s>>>(mats, nmat, forms, nbnd, values);
+  for (int axis = 0; axis < 3; ++axis) {
+    const int64_t nfaces = (d.nz + (axis == 0)) * (d.ny + (axis == 1)) * (d.nx + (axis == 2));
+    faces_kernel<<<grid_for(nfaces, kThreads), kThreads, 0, s>>>(d, axis, material, bclass[axis], mats, nmat, forms, nbnd,
+                                                                 values ? values + axis * entries : nullptr, G[axis], err);
+  }
   return cudaGetLastError();
 }
 
@@ -657,16 +666,14 @@ cudaError_t launch_factor(const Dims& d, const Faces& f, const double* M, const 
 }
 
 void Compressed::release() {
-  cudaFree(blocks.pool);
-  for (LineTables& t : lines) cudaFree(t.a);
+  cudaFree(mem);
+  cudaFree(own);
   *this = Compressed{};
 }
 
 size_t compress_scratch(const Dims& d) {
-  size_t n = 256 + (blocks_countable(d) ? ClassTable(block_count(d)).bytes() : 0);
-  for (int64_t lines : {d.nz * d.ny, d.nz * d.nx, d.nxy()})
-    if (lines < ((int64_t)1 << 29)) n += (LineJob::scratch_bytes(lines) + 255) & ~size_t(255);
-  return n;
+  return LineSearch::scratch_bytes({searched_lines(d, 0), searched_lines(d, 1), searched_lines(d, 2)},
+                                   blocks_countable(d) ? block_count(d) : 0);
 }
 
 cudaError_t compress_coeffs(const Dims& d, const Faces& f, const uint8_t* compute, const double* f0, const Coeffs& c,

@@ -47,7 +47,7 @@ struct Coeffs {
 };
 
 // The distinct lines of an axis: a[c*n + r], b[c*n + r] per class and row, cls[line]; cls is null when there are too
-// many.  One device allocation, at a, owned by the caller.
+// many.
 struct LineTables {
   double* a = nullptr;
   double* b = nullptr;
@@ -55,8 +55,7 @@ struct LineTables {
   int64_t nclass = 0;
   size_t bytes = 0;
 };
-// Stencil blocks of a problem: the distinct ones with an index per (line, chunk), or all of them (bidx null).  Device
-// memory owned by the caller.
+// Stencil blocks of a problem: the distinct ones with an index per (line, chunk), or all of them (bidx null).
 struct XBlocks {
   void* pool = nullptr;
   int32_t* bidx = nullptr;
@@ -65,29 +64,37 @@ struct XBlocks {
 };
 
 // An open-addressing table over n things, by 64-bit hash: keys, the smallest thing of each key, the number it gets,
-// each thing's slot, and {count of numbers, 1 while no two different things were found under one key}.
+// each thing's slot, and {count of numbers, 1 once two different things were found under one key}.
 struct ClassTable {
-  int64_t n = 0, cap = 64;
+  int64_t n = 0;
   unsigned long long* keys = nullptr;
   int *owner = nullptr, *id = nullptr, *slot = nullptr, *count = nullptr;
-  explicit ClassTable(int64_t things = 0) : n(things) {
-    while (cap < 2 * n) cap *= 2;
+  __host__ __device__ ClassTable(int64_t things = 0) : n(things) {}
+  __host__ __device__ int64_t cap() const {  // at least twice as many entries as things
+    int64_t c = 64;
+    while (c < 2 * n) c *= 2;
+    return c;
   }
-  size_t bytes() const { return sizeof(*keys) * (size_t)cap + sizeof(int) * (size_t)(2 * cap + n + 2); }
-  unsigned char* place(unsigned char* at) {  // returns what follows it
-    keys = reinterpret_cast<unsigned long long*>(at);
-    owner = reinterpret_cast<int*>(keys + cap);
-    id = owner + cap;
-    slot = id + cap;
-    count = slot + n;
-    return reinterpret_cast<unsigned char*>(count + 2);
+  // the slot of hash h (not 0), thing l among its owners.  (Read before each atomic: of many things alike all but the
+  // first few find what they would write.)
+  __device__ __forceinline__ int insert(unsigned long long h, int l) const {
+    const int64_t mask = cap() - 1;
+    int64_t e = (int64_t)(h >> 17) & mask;
+    for (;; e = (e + 1) & mask) {
+      unsigned long long k = *(volatile unsigned long long*)(keys + e);
+      if (k == 0ull) k = atomicCAS(keys + e, 0ull, h);
+      if (k == 0ull || k == h) break;
+    }
+    if (*(volatile int*)(owner + e) > l) atomicMin(owner + e, l);
+    return (int)e;
   }
-  cudaError_t clear(cudaStream_t s) {
-    static const int start[2] = {0, 1};
-    cudaError_t e = cudaMemsetAsync(keys, 0, sizeof(*keys) * cap, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(owner, 0x7f, sizeof(int) * cap, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(count, start, sizeof start, cudaMemcpyHostToDevice, s);
-    return e;
+  // the slots of the things of a warp's lanes (mask: lanes 0 .. some; things ascending, h 0: none), those alike as one
+  __device__ __forceinline__ void insert_all(unsigned mask, unsigned long long h, int l) const {
+    const int lane = threadIdx.x & 31, leader = __ffs(__match_any_sync(mask, h)) - 1;
+    int e = 0;
+    if (lane == leader && h) e = insert(h, l);
+    e = __shfl_sync(mask, e, leader);
+    if (h) slot[l] = e;
   }
 };
 
@@ -97,22 +104,36 @@ struct LineGrid {
   const double* b;
   int64_t outer, nx, ost, n, rst;
   __host__ __device__ int64_t lines() const { return outer * nx; }
-  __device__ int64_t base(int64_t l) const { return (l / nx) * ost + l % nx; }
+  __device__ int64_t base(int64_t l) const {  // (the search numbers lines in 32 bits)
+    const unsigned o = (unsigned)l / (unsigned)nx;
+    return o * ost + ((unsigned)l - o * (unsigned)nx);
+  }
 };
-// Finding the line classes of an axis (hs2g_classes.cu): begin queues the hashing and numbering, the caller reads
-// table.count[0] (and waits), finish queues the tables and the check that clears table.count[1] on a clash of hashes.
-// mid >= 0: the rows above mid are tabulated last first (row r at position mid + n - r).
-struct LineJob {
-  LineGrid grid{};
-  int64_t mid = -1;
-  ClassTable table;
-  int* rep = nullptr;
+// Finding the line classes of the three axes (hs2g_classes.cu); grid, table[a].n (0: no search on that axis) and mid are
+// the caller's.  begin queues the hashing (and clears the blocks' table beside the lines'), number the numbering of both;
+// the caller reads the counts (2 ints per table from table[0].count on) and waits; choose takes the axes worth tables and
+// returns the bytes of these, finish queues them and the check that sets count[1] on a clash of hashes.  mid >= 0: the rows
+// above mid are tabulated last first (row r at position mid + n - r).
+struct LineSearch {
+  LineGrid grid[3];
+  int64_t mid[3];
+  ClassTable table[3];
+  int* rep[3];  // a line of each class
+  int per[3], first_cta[3];
+  int64_t nclass[3];
+  int32_t* cls[3];
+  double *ta[3], *tb[3];
   // Worth it when the tables are an eighth of the arrays: the classes of a warp's 16 lines then cost it no more than
   // reading the arrays would
-  static int64_t max_class(int64_t lines) { return lines / 8 > 1 ? lines / 8 : 1; }
-  static size_t scratch_bytes(int64_t lines);
-  cudaError_t begin(unsigned char* scratch, cudaStream_t s);
-  cudaError_t finish(int64_t nclass, LineTables* out, cudaStream_t s);
+  __host__ __device__ static int64_t max_class(int64_t lines) { return lines / 8 > 1 ? lines / 8 : 1; }
+  static size_t scratch_bytes(const int64_t (&lines)[3], int64_t nblocks);
+  cudaError_t begin(unsigned char* scratch, ClassTable& blocks, cudaStream_t s);
+  cudaError_t number(const ClassTable& blocks, cudaStream_t s);
+  size_t table_bytes(int a) const {
+    return 2 * sizeof(double) * (size_t)(nclass[a] * grid[a].n) + sizeof(int32_t) * (size_t)table[a].n;
+  }
+  size_t choose(const int (&classes)[3]);
+  cudaError_t finish(unsigned char* m, LineTables (&out)[3], cudaStream_t s);
 };
 
 struct QTable {
@@ -192,9 +213,10 @@ __device__ __forceinline__ void record_error(unsigned long long* err, int code, 
 }
 
 // setup kernels (hs2g_compile.cu)
-cudaError_t launch_faces(const Dims& d, int axis, const uint8_t* material, const uint8_t* bclass,
-                         const hs2g_material* mats, int nmat, const hs2g_face_form* forms, int nbnd, double* G,
-                         unsigned long long* err, void* table, cudaStream_t s);
+// the face conductances of the three axes (z, y, x), from the boundary classes of their faces
+cudaError_t launch_faces(const Dims& d, const uint8_t* material, const uint8_t* const bclass[3], const hs2g_material* mats,
+                         int nmat, const hs2g_face_form* forms, int nbnd, double* const G[3], unsigned long long* err,
+                         void* table, cudaStream_t s);
 size_t face_table_bytes(int nmat, int nbnd);  // of launch_faces's table; 0: it takes none
 cudaError_t launch_capacity_from_classes(const Dims& d, const uint8_t* material, const hs2g_material* mats,
                                          int nmat, double* M, uint8_t* compute, unsigned long long* err,
@@ -217,6 +239,7 @@ cudaError_t launch_factor(const Dims& d, const Faces& f, const double* M, const 
 struct Compressed {
   XBlocks blocks;
   LineTables lines[3];
+  void *mem = nullptr, *own = nullptr;  // device memory of the tables and the distinct blocks, and of all blocks
   void release();
 };
 size_t compress_scratch(const Dims& d);
