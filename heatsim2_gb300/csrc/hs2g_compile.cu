@@ -649,11 +649,11 @@ cudaError_t launch_validate_dense(const Dims& d, const double* Gz, const double*
 template <class F>
 cudaError_t launch_factor_with(const Dims& d, F g, const double* M, const uint8_t* compute, double* s2,
                                double* sigma, const Coeffs& c, cudaStream_t s, bool two_ended) {
-  const int th = 128;
-  factor_z_kernel<F><<<grid_for(d.nxy(), th), th, 0, s>>>(d, g, M, compute, s2, c.a2, c.b2, c.px, two_ended);
-  factor_y_kernel<F><<<grid_for(d.nz * d.nx, th), th, 0, s>>>(d, g, M, compute, s2, sigma, c.a1, c.b1,
-                                                                c.px, two_ended);
-  factor_x_kernel<F><<<grid_for(d.nz * d.ny, th), th, 0, s>>>(d, g, M, compute, sigma, s2, c.a0, c.b0, c.px, two_ended);
+  const int th = 128;  // a thread per line, however many there are
+  auto ctas = [&](int64_t lines) { return (unsigned)((lines + th - 1) / th); };
+  factor_z_kernel<F><<<ctas(d.nxy()), th, 0, s>>>(d, g, M, compute, s2, c.a2, c.b2, c.px, two_ended);
+  factor_y_kernel<F><<<ctas(d.nz * d.nx), th, 0, s>>>(d, g, M, compute, s2, sigma, c.a1, c.b1, c.px, two_ended);
+  factor_x_kernel<F><<<ctas(d.nz * d.ny), th, 0, s>>>(d, g, M, compute, sigma, s2, c.a0, c.b0, c.px, two_ended);
   return cudaGetLastError();
 }
 
