@@ -14,9 +14,9 @@ HBM; ``e2e`` is the same metric through the C ABI with host buffers (host->devic
 device->host copy of T, every step); ``roofline`` is the dominant sweep kernel against the measured HBM copy
 bandwidth, on the algorithmic bytes of a sweep that reads each array it needs once with the face conductances
 and capacities re-read in every sweep (x 56, y 40, z 40 B per voxel: 136 B per step), with this
-implementation's own bytes (x 88 B: T, nine step coefficients, W0) and the ncu-measured DRAM traffic beside
-it; ``kernel_hbm_frac`` gives the same for every sweep; ``step_hbm`` the whole step against the bandwidth
-(both accountings); ``fp64_roofline`` the whole step against the measured FP64 FMA rate;
+implementation's own bytes (x 32 B: T read, the right-hand sides written and read, W0 written; the coefficients
+come from tables in cache) and the ncu-measured DRAM traffic beside it; ``kernel_hbm_frac`` gives the same for
+every sweep; ``step_hbm`` the whole step against the bandwidth (both accountings); ``fp64_roofline`` the whole step against the measured FP64 FMA rate;
 ``cpu_baseline`` the reference (or, where it cannot be built, the oracle) on the host cores.  ``batched`` is
 the 256-instance uneven batch (FP64 and FP32) against a per-instance loop of the plain path; ``adjoint`` the
 gradient evaluations per second of the (32,128,128) steel inverse problem and of the 32-instance batched

@@ -387,8 +387,9 @@ int step_host_pipelined(hs2g_handle* h, hs2g::StepArgs& a, const hs2g::QTable& q
 }
 
 // Whether host memory at p is page-locked.  Overlapped copies pay only then: the runtime stages pageable memory through
-// its own buffers while the caller waits, piece by piece (49x220x200 numpy steps: 1.05 ms with one copy each way, 1.8 ms
-// in four slabs and blocks; page-locked at 65x512x512: 1.80 ms and 1.57 ms).
+// its own buffers while the caller waits, piece by piece.  Steps with one copy each way, and in brackets in four slabs and
+// blocks: pageable 33x200x170 176 us [283], 49x220x200 300 [380], 65x512x512 1860 [1850]; page-locked 33x200x170 165 [170],
+// 49x220x200 277 [264], 65x512x512 1784 [1565].
 bool page_locked(const void* p) {
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {

@@ -1,16 +1,17 @@
 // Batched timestep: many independent problems of uneven size advanced together.
 //
 // All instances live in one concatenated device state (instance b's fields start at voxel offset off[b], each
-// (nz_b, ny_b, nx_b) C-ordered).  The three sweeps are persistent kernels that walk flattened work lists --
-// x: (instance, 32 x-lines), y: (instance, 128 y-lines), z: (instance, 128 z-lines) -- ordered longest lines
-// first so the static round-robin over the persistent grid balances uneven instances.  One timestep (three
-// sweeps + a step-counter increment) is captured once in a CUDA graph and replayed; the per-step source
+// (nz_b, ny_b, nx_b) C-ordered).  A step is four sweep kernels over flattened work lists, a CTA per work item -- the x
+// stencil and the x solve: 64 x-lines of an instance (the stencil a CTA per 16 of them and, split, per part of their
+// columns); y and z: kPairMaxWarps groups of neighbouring lines, a group per warp -- with the instances of the longest
+// lines first, and a step-counter increment.  They are captured once in a CUDA graph and replayed; the per-step source
 // tables are uploaded once and selected on the device by the step counter, so the graph never changes.
 //
 // The arithmetic per line is that of the single-problem kernels (hs2g_sweep.cu, scaled delta-form Douglas
 // ADI), templated on the storage type: double (results equal to the single-problem path bit for bit) or float
 // (coefficients compiled in double, rounded once; its error against double is measured by the caller).
-// Block sizes and persistent grid sizes per axis are chosen by hs2g_batch_autotune (timed on the batch).
+// hs2g_batch_autotune chooses, timed on the batch, how many CTAs share an item's columns in the stencil and whether
+// each axis's forward values stay in shared memory.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -62,11 +63,8 @@ struct BatchView {
   const int* step;         // device step counter
   int nsched, ninst, nclass;
   const XWork* xw;
-  int64_t nx_work;
   const LWork* yw;
-  int64_t ny_work;
   const LWork* zw;
-  int64_t nz_work;
 };
 
 
@@ -238,11 +236,8 @@ BatchView<R> view(const Batch& b) {
   v.ninst = b.ninst;
   v.nclass = b.nclass;
   v.xw = b.xw;
-  v.nx_work = b.nxw;
   v.yw = b.yw;
-  v.ny_work = b.nyw;
   v.zw = b.zw;
-  v.nz_work = b.nzw;
   return v;
 }
 
@@ -423,8 +418,6 @@ cudaError_t batch_time_axis(Batch& b, int axis, const Tuning& t, int reps, float
 
 // Candidate launch shapes per axis, timed on the batch itself.  Returns the report in `report`.
 cudaError_t batch_autotune(Batch& b, std::string& report) {
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b.device);
   Tuning best = b.tune;
   char line[256];
   cudaError_t e = cudaSuccess;
@@ -741,8 +734,6 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   e = cudaMemcpyAsync(b.inst_dev, b.inst.data(), sizeof(hs2g::Inst) * n, cudaMemcpyHostToDevice, b.stream);
   if (e != cudaSuccess) return bail(bcuda(e, "instances"));
   if ((e = hs2g::batch_upload_work(b)) != cudaSuccess) return bail(bcuda(e, "work lists"));
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   for (const hs2g::Inst& I : b.inst) {
     b.max_nx = std::max(b.max_nx, I.d.nx);
     b.max_ny = std::max(b.max_ny, I.d.ny);

@@ -536,8 +536,9 @@ cudaError_t compress_with(const Dims& d, F g, const uint8_t* compute, const doub
     if (e == cudaSuccess) e = counts();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
-  // An index is worth it when at most a quarter of the blocks are distinct: the sweep then reads them from L2, and the
-  // index costs it a dependent load
+  // An index is worth it when at most a quarter of the blocks are distinct: the sweep then reads them from cache, and the
+  // index costs it a dependent load (64x256x512, x sweep with an index and in brackets without: 1/64 of the blocks 162 us
+  // [186], 1/16 190 [212], 1/4 193 [210], 1/2 201 [211], all 220 [214]; 37x192x210 1/4 39 [45], all 51 [48])
   XBlocks& x = out->blocks;
   const size_t index = sizeof(int32_t) * (size_t)blocks;
   bool shared = t.n && host[3][0] <= std::max<int64_t>(1, blocks / 4);

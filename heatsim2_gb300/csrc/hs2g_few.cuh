@@ -90,7 +90,7 @@ __device__ __forceinline__ double few_chain(double* W, const double* A, const do
   return x;
 }
 // the warp that runs the chain: CTAs that share an SM use FP64 units of their own
-__device__ __forceinline__ int few_chain_warp() { return (int)(blockIdx.x / 152) & 3; }
+__device__ __forceinline__ int few_chain_warp() { return (int)(blockIdx.x / (unsigned)kSMs) & 3; }
 
 // y and z lines, coefficients and scale per voxel (pair_solve with SCALE and without TABLE)
 __host__ __device__ constexpr size_t few_smem(int64_t max_len) { return sizeof(double) * 32 * 4 * (size_t)(max_len / 2); }
@@ -226,7 +226,7 @@ __device__ __forceinline__ void few_x_solve(const double* in, const double* sc, 
 // a chain for each of its FP64 units.
 inline bool few_lines(int64_t groups, size_t smem) {
   const int64_t per = (int64_t)(227 * 1024 / (smem + 1024));
-  return groups <= 152 * (per < 4 ? per : 4);
+  return groups <= kSMs * (per < 4 ? per : 4);
 }
 
 }  // namespace hs2g

@@ -14,6 +14,8 @@ struct Dims {
   __host__ __device__ int64_t nxy() const { return ny * nx; }
 };
 
+constexpr int64_t kSMs = 152;  // of a GB300.  Launch shapes fill them; nothing is wrong where there are more or fewer
+
 // middle column of the two-ended x elimination
 __host__ __device__ inline int64_t x_mid(int64_t nx) { return (nx - 1) / 2; }
 
@@ -123,8 +125,10 @@ struct LineSearch {
   int64_t nclass[3];
   int32_t* cls[3];
   double *ta[3], *tb[3];
-  // Worth it when the tables are an eighth of the arrays: the classes of a warp's 16 lines then cost it no more than
-  // reading the arrays would
+  // Worth it when the tables are an eighth of the arrays: they stay in cache, and where neighbouring lines are of one class,
+  // as in a layered specimen, a warp reads one row for its sixteen.  At the worst, all neighbours different, us per sweep
+  // from tables of 1/64, 1/16 and 1/8 of the lines, in brackets from the arrays: 64x256x512 x 186, 212, 212 [190], y 38
+  // [67], z 83 [63]; 37x192x210 x 42, 44, 45 [52], y 20 [19], z 22 [23].
   __host__ __device__ static int64_t max_class(int64_t lines) { return lines / 8 > 1 ? lines / 8 : 1; }
   static size_t scratch_bytes(const int64_t (&lines)[3], int64_t nblocks);
   cudaError_t begin(unsigned char* scratch, ClassTable& blocks, cudaStream_t s);
@@ -154,14 +158,7 @@ struct DevSchedule {
   unsigned int hist_done;  // CTAs of the current history kernel that have finished (the last one advances row)
 };
 
-// L2 eviction policies (createpolicy) and stores that carry one: evict-first for data streamed once, evict-last
-// for a value the same thread block reads back soon (a sweep's forward values), and dropping a 128-byte line
-// without writing it back (its contents are undefined until written again).
-__device__ __forceinline__ uint64_t l2_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
+// Stores with an L2 evict-last policy, for a value the same warp reads back soon (a line's forward values).
 __device__ __forceinline__ uint64_t l2_evict_last() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
@@ -172,9 +169,6 @@ __device__ __forceinline__ void st_hint(double* p, double v, uint64_t policy) {
 }
 __device__ __forceinline__ void st_hint(float* p, float v, uint64_t policy) {
   asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(policy) : "memory");
-}
-__device__ __forceinline__ void l2_discard_line(const void* p) {
-  asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
 }
 
 // Programmatic dependent launch inside the captured step graphs: a sweep launched with the attribute may be set

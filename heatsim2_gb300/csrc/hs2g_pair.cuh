@@ -346,10 +346,10 @@ inline PairShape pair_shape(int64_t max_len, int64_t groups, int force_keep = -1
   const size_t held = pair_smem<R, TWO, ADD_T, true, TABLE, SCALE>(max_len);
   const int64_t per = (int64_t)(kSmem / (held + kReserved));
   PairShape sh;
-  sh.keep = per > 0 && (force_keep >= 0 ? force_keep != 0 : per >= 8 || groups <= 152 * per);
+  sh.keep = per > 0 && (force_keep >= 0 ? force_keep != 0 : per >= 8 || groups <= kSMs * per);
   const size_t each = sh.keep ? held : pair_smem<R, TWO, ADD_T, false, TABLE, SCALE>(max_len);
   sh.warps = 1;
-  while (sh.warps < kPairMaxWarps && groups >= 152 * 8 * sh.warps && 2 * sh.warps * each <= 64 * 1024) sh.warps *= 2;
+  while (sh.warps < kPairMaxWarps && groups >= kSMs * 8 * sh.warps && 2 * sh.warps * each <= 64 * 1024) sh.warps *= 2;
   sh.smem = each * sh.warps;
   return sh;
 }

@@ -1,5 +1,5 @@
-// Slot bookkeeping of the TMA tile rings in hs2g_lines.cu, kept apart from the kernels so that it compiles as
-// plain C++ and is checked on the host (tests/test_ring_bookkeeping.py).
+// Slot bookkeeping of a ring of bulk copies waited for on mbarriers, plain C++ that is checked on the host
+// (tests/test_ring_bookkeeping.py).  No kernel has such a ring any more: the line solves wait on cp.async groups.
 //
 // A ring has up to 32 slots; each slot's copies complete on the slot's mbarrier, whose phase alternates.  The
 // producer marks a slot pending when it issues copies into it.  A wait that saw the phase complete advances

@@ -96,7 +96,7 @@ cudaError_t launch_x(const StepArgs& a, const Coeffs& c, const XTable<SRC>& q, c
   // a CTA walks its lines' chunks, or takes every second, fourth ... of them until there are CTAs enough for the GPU
   const int64_t ctas = (end - begin + kXStencilLines - 1) / kXStencilLines;
   unsigned split = 1;
-  while (split < c.nchunks && split < 32768 && ctas * split < 152 * 8) split *= 2;
+  while (split < c.nchunks && split < 32768 && ctas * split < kSMs * 8) split *= 2;
   const dim3 grid((unsigned)ctas, split), block(32 * kXStencilWarps);
   cudaError_t e = x_index32(a.d, c)
                       ? launch_kernel(x_stencil_kernel<SRC, SHARED, int32_t>, grid, block, 0, s, a.pdl_x, P, q, ds, begin, end)

@@ -23,7 +23,7 @@ namespace hs2g {
 
 constexpr int kXStencilWarps = 4;  // of a CTA of the stencil kernel, each with kXStencilPer lines
 constexpr int kXStencilPer = 4;
-constexpr int kXStencilCtas = 4;   // CTAs per SM the stencil kernel is built for (128 registers)
+constexpr int kXStencilCtas = 4;   // CTAs per SM the stencil kernel is built for (128 registers; 64-bit indices spill a little)
 constexpr int kXStencilLines = kXStencilWarps * kXStencilPer;
 
 // lines of a warp of the line solves
@@ -194,7 +194,7 @@ struct XProblem {
 // for a neighbour of weight 0).
 template <typename IX>
 struct alignas(16) XLine {
-  IX base, blk, out, unused, dyl, dyh, dzl, dzh;
+  IX base, blk, out, pad, dyl, dyh, dzl, dzh;  // (pad: the offsets are one 16-byte load)
 };
 
 // A voxel's seven temperatures, and its stencil as the chain of seven multiply-adds or in integers (FP64).  blk: its
@@ -799,7 +799,7 @@ __device__ __forceinline__ void x_fused_lines(const XProblem<double>& P, int64_t
 template <typename IX>
 inline bool x_fused(int64_t nx, int64_t lines) {
   const size_t need = x_fused_smem<IX>(nx) + 1024;
-  return need <= 227 * 1024 && (lines + 15) / 16 <= 152 * std::min<int64_t>(3, (int64_t)(227 * 1024 / need));
+  return need <= 227 * 1024 && (lines + 15) / 16 <= kSMs * std::min<int64_t>(3, (int64_t)(227 * 1024 / need));
 }
 
 // How a launch of the line solves over `groups` warps runs (as pair_shape)
@@ -809,10 +809,10 @@ inline PairShape x_solve_shape(int64_t max_nx, int64_t groups, int force_keep = 
   const size_t held = x_solve_smem<R, TWO, TABLE, true, SCALE>(max_nx);
   const int64_t per = (int64_t)(kSmem / (held + kReserved));
   PairShape sh;
-  sh.keep = per > 0 && (force_keep >= 0 ? force_keep != 0 : per >= 8 || groups <= 152 * per);
+  sh.keep = per > 0 && (force_keep >= 0 ? force_keep != 0 : per >= 8 || groups <= kSMs * per);
   const size_t each = sh.keep ? held : x_solve_smem<R, TWO, TABLE, false, SCALE>(max_nx);
   sh.warps = 1;
-  while (sh.warps < kPairMaxWarps && groups >= 152 * 8 * sh.warps && 2 * sh.warps * each <= 64 * 1024) sh.warps *= 2;
+  while (sh.warps < kPairMaxWarps && groups >= kSMs * 8 * sh.warps && 2 * sh.warps * each <= 64 * 1024) sh.warps *= 2;
   sh.smem = each * sh.warps;
   return sh;
 }

@@ -301,8 +301,8 @@ int hs2g_step_static(int64_t nz, int64_t ny, int64_t nx, const double* Gz, const
  * whose time loop handles one problem; a loop over run_adi_steps calls is what it replaces).  All instances
  * live in one concatenated state: instance i's (nz_i, ny_i, nx_i) field starts at voxel offsets[i] (see
  * hs2g_batch_layout).  precision 64 stores and computes in double (per instance equal to hs2g_step bit for
- * bit); precision 32 compiles in double and stores / sweeps in float.  A timestep is three persistent sweep
- * kernels over flattened line lists, captured once in a CUDA graph and replayed.
+ * bit); precision 32 compiles in double and stores / sweeps in float.  A timestep is four sweep kernels (the x
+ * stencil, the x, y and z line solves) over flattened work lists, captured once in a CUDA graph and replayed.
  */
 typedef struct hs2g_batch hs2g_batch;
 int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, int device, hs2g_batch** out);
