@@ -99,3 +99,29 @@ def test_few_equal_lines_with_blocks_of_their_own(cuda_ok, nx, negative):
             rhs = lap @ (T[k, j] - 293.0) + q[k, j] / scale[k, j]
             ref = T[k, j] + np.linalg.solve(np.diag(m) - lap / 2, rhs)
             assert rel_err(out[k, j], ref) <= 1e-12
+
+
+@pytest.mark.parametrize("shape", [(1, 2050, 2112), (64, 256, 256)])
+def test_setup_where_the_search_has_no_room(cuda_ok, shape):
+    """200 bytes per voxel left on the device: what a handle keeps (162 and the planes' extra faces) and the factors' two
+    arrays, but not the search for equal lines and blocks beside them.  The same step, bit for bit."""
+    import torch
+    L = _native.load()
+    spec = _random_faces(shape, 50.0 + 37.0 * np.arange(40))
+    args = W.setup_args(hs, spec)
+    T = 293.0 + torch.rand(shape, dtype=torch.float64, device="cuda")
+    out = [torch.empty_like(T), torch.empty_like(T)]
+    hold = None
+    try:
+        for o in out:
+            P, _ = hs.setup(*args)
+            _native.check(L.hs2g_step(P.handle.ptr, T.data_ptr(), o.data_ptr(), None, None, None,
+                                      _native.DEVICE | _native.SYNC))
+            del P
+            if hold is None:
+                torch.cuda.empty_cache()
+                hold = torch.empty(torch.cuda.mem_get_info()[0] - 200 * T.numel(), dtype=torch.uint8, device="cuda")
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert torch.equal(*out)
