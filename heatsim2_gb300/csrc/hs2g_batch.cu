@@ -512,7 +512,7 @@ void batch_free(Batch& b) {
 }
 
 // Compile instance `ib` of problem p into the batch (FP64 workspace ws, then into the batch's storage type).
-int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, unsigned long long* err) {
+int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, bool search, unsigned long long* err) {
   hs2g::Inst& I = b.inst[ib];
   const hs2g::Dims& d = I.d;
   const int64_t n = d.nvox(), np = d.nz * d.ny * I.px;
@@ -540,7 +540,7 @@ int compile_instance(Batch& b, int ib, const hs2g_class_problem& p, double* ws, 
   // then the faces' values per class and material pair, and the scratch of the search for equal lines and blocks
   unsigned char* table = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(forms + 3 * HS2G_MAX_CLASSES) + 255) & ~uintptr_t(255));
-  unsigned char* scratch = table + ((hs2g::face_table_bytes(p.nmat, p.nbnd) + 255) & ~size_t(255));
+  unsigned char* scratch = search ? table + ((hs2g::face_table_bytes(p.nmat, p.nbnd) + 255) & ~size_t(255)) : nullptr;
   cudaError_t e = cudaSuccess;
   auto up = [&](void* dst, const void* src, size_t bytes) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
@@ -677,7 +677,7 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     delete hb;
     return bcuda(e, "cudaStreamCreate");
   }
-  int64_t off = 0, ws = 0;
+  int64_t off = 0, ws = 0, ws_least = 0;  // workspace with and without the scratch of the search
   b.offsets.push_back(0);
   for (int i = 0; i < n; ++i) {
     hs2g::Inst I{};
@@ -697,8 +697,9 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
     const int64_t need = faces + 3 * nn + 6 * d.nz * d.ny * I.px + (faces + 3 * nn) / 8 + 2048 +
                          (int64_t)(sizeof(hs2g_material) * HS2G_MAX_CLASSES + sizeof(hs2g_face_form) * 3 *
                                    HS2G_MAX_CLASSES) / 8 + 512 +
-                         (int64_t)(hs2g::face_table_bytes(problems[i].nmat, problems[i].nbnd) + hs2g::compress_scratch(d)) / 8;
-    ws = std::max(ws, need);
+                         (int64_t)hs2g::face_table_bytes(problems[i].nmat, problems[i].nbnd) / 8;
+    ws_least = std::max(ws_least, need);
+    ws = std::max(ws, need + (int64_t)hs2g::compress_scratch(d) / 8);
   }
   b.nvox = off;
   b.ix32 = true;
@@ -707,11 +708,21 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   const size_t el = b.elem();
   double* wsp = nullptr;
   unsigned long long* err = nullptr;
+  bool search = true;
+  auto workspace = [&]() {
+    cudaError_t w = cudaMalloc(&wsp, sizeof(double) * ws);
+    if (w == cudaErrorMemoryAllocation) {  // no room for the search: everything in voxel order
+      cudaGetLastError();
+      search = false;
+      w = cudaMalloc(&wsp, sizeof(double) * ws_least);
+    }
+    return w;
+  };
   if ((e = balloc(b, &b.inst_dev, n)) != cudaSuccess || (e = balloc(b, (char**)&b.T, b.nvox * el)) != cudaSuccess ||
       (e = balloc(b, (char**)&b.W0, b.nw * el)) != cudaSuccess ||
       (e = balloc(b, (char**)&b.W1, b.nw * el)) != cudaSuccess ||
       (e = balloc(b, &b.vclass, b.nvox)) != cudaSuccess || (e = balloc(b, &b.step, 1)) != cudaSuccess ||
-      (e = cudaMalloc(&wsp, sizeof(double) * ws)) != cudaSuccess ||
+      (e = workspace()) != cudaSuccess ||
       (e = cudaMalloc(&err, sizeof(unsigned long long))) != cudaSuccess) {
     if (wsp) cudaFree(wsp);
     if (err) cudaFree(err);
@@ -723,10 +734,29 @@ int hs2g_batch_create(int n, const hs2g_class_problem* problems, int precision, 
   cudaMemsetAsync(b.W1, 0, b.nw * el, b.stream);
   cudaMemsetAsync(b.vclass, 0, b.nvox, b.stream);
   cudaMemsetAsync(b.step, 0, sizeof(int), b.stream);
-  int rc = HS2G_OK;
-  for (int i = 0; i < n && rc == HS2G_OK; ++i) {
-    cudaMemsetAsync(err, 0, sizeof(unsigned long long), b.stream);
-    rc = compile_instance(b, i, problems[i], wsp, err);
+  const int64_t bytes = b.bytes;
+  auto compile_all = [&]() {
+    int rc = HS2G_OK;
+    for (int i = 0; i < n && rc == HS2G_OK; ++i) {
+      cudaMemsetAsync(err, 0, sizeof(unsigned long long), b.stream);
+      rc = compile_instance(b, i, problems[i], wsp, search, err);
+    }
+    return rc;
+  };
+  int rc = compile_all();
+  if (rc == HS2G_ERR_NOMEM && search) {  // the coefficients did not fit beside the scratch
+    cudaStreamSynchronize(b.stream);
+    for (void* m : b.coef_mem) cudaFree(m);
+    b.coef_mem.clear();
+    b.bytes = bytes;
+    b.dense[0] = b.dense[1] = b.dense[2] = b.dense_blocks = false;
+    cudaFree(wsp);
+    wsp = nullptr;
+    search = false;
+    if (cudaMalloc(&wsp, sizeof(double) * ws_least) == cudaSuccess)
+      rc = compile_all();
+    else
+      cudaGetLastError();
   }
   cudaFree(wsp);
   cudaFree(err);

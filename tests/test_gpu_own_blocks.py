@@ -125,3 +125,28 @@ def test_setup_where_the_search_has_no_room(cuda_ok, shape):
         del hold
         torch.cuda.empty_cache()
     assert torch.equal(*out)
+
+
+def test_batch_where_the_search_has_no_room(cuda_ok):
+    """The same for a batch of one: 260 bytes per voxel left, which state, coefficients and blocks (137) and the
+    compilation's own arrays (99) need without the scratch of the search."""
+    import torch
+    shape = (1, 2050, 2112)
+    spec = _random_faces(shape, 50.0 + 37.0 * np.arange(40))
+    args = W.setup_args(hs, spec)
+    T = 293.0 + np.random.default_rng(1).random(shape)
+    out, hold = [], None
+    try:
+        for _ in range(2):
+            b = Batch([args], precision=64)
+            b.set_temperature([T])
+            b.run(2)
+            out.append(b.get_temperature()[0])
+            del b
+            if hold is None:
+                torch.cuda.empty_cache()
+                hold = torch.empty(torch.cuda.mem_get_info()[0] - 260 * T.size, dtype=torch.uint8, device="cuda")
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    np.testing.assert_array_equal(*out)
